@@ -98,17 +98,19 @@ int tnns_launch_gemm_tc(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const vo
 //                    copy can deliver im2row tiles without any expansion (ternary activations only)
 #define TNNS_IMG_PLANES 1
 #define TNNS_IMG_E2M1 2
+// (quantise_any.cu: any tensor; the copy-engine fed kernel where it applies)
+// PH, PW (4-bit image only): store the image bordered, i.e. every image framed by PH rows / PW columns of
+// the padding value (ternary 0, binary +1), [n][H + 2*PH][W + 2*PW][C/2 bytes]
+// pitch_words (4-bit image only): 64-channel words (32 bytes) from one pixel to the next; 0: as many as the pixel has
 int tnns_launch_quantise(tnns_cuda_ctx* ctx, bool ternary, const float* d_x, const float* d_thr, void* d_image, int N, int C, int H,
-                         int W, int layout, cudaStream_t stream, int format = TNNS_IMG_PLANES);
+                         int W, int layout, cudaStream_t stream, int format = TNNS_IMG_PLANES, int PH = 0, int PW = 0, int pitch_words = 0);
 // the same for NCHW input whose rows the copy engine can fetch (H*W a multiple of four floats,
 // 16-byte aligned base): tensor copies into a shared-memory ring instead of register loads
 bool tnns_quantise_tma_supported(const float* d_x, int H, int W, int layout);
-// PH, PW (4-bit image only): store the image bordered, i.e. every image framed by PH rows / PW columns of
-// the padding value (ternary 0, binary +1), [n][H + 2*PH][W + 2*PW][C/2 bytes]
 // layout TNNS_NHWC: the input is (pixels) x (channels), fetched as 128-byte-swizzled boxes (tnns_quantise_tma_nhwc_supported)
 bool tnns_quantise_tma_nhwc_supported(const float* d_x, int N, int C, int H, int W);
 int tnns_launch_quantise_tma(tnns_cuda_ctx* ctx, bool ternary, const float* d_x, const float* d_thr, void* d_image, int N, int C, int H,
-                             int W, cudaStream_t stream, int format, int PH = 0, int PW = 0, int layout = TNNS_NCHW);
+                             int W, cudaStream_t stream, int format, int PH = 0, int PW = 0, int layout = TNNS_NCHW, int pitch_words = 0);
 // dense form of layers with few input channels (dense.cu): channels of the virtual 1x1 layer, whether a kernel
 // qualifies, the repacked kernel of that layer, and the quantise kernel that writes its 4-bit image
 int tnns_dense_channels(int C, int KH, int KW);

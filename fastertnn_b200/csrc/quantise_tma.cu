@@ -44,7 +44,7 @@ __device__ __forceinline__ uint32_t push_sign_bit(uint32_t acc, float d) { retur
 template <bool TERNARY, int IMG, bool NHWC_IN>
 __global__ void __launch_bounds__(QTHREADS, 1)
 quantise_tma_kernel(const __grid_constant__ CUtensorMap tmap, const float* __restrict__ thr, void* __restrict__ out, int N, int C, int HW,
-                    int Cp, int nbands, unsigned int* status, int W, int Wp, int HpWp, int off0) {
+                    int Cp, int nbands, unsigned int* status, int W, int Wp, int HpWp, int off0, int pitch) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + QSTG * QSTAGE_BYTES);
@@ -84,7 +84,7 @@ quantise_tma_kernel(const __grid_constant__ CUtensorMap tmap, const float* __res
         for (long long t = (long long)blockIdx.x * (QGROUPS * QL) + (tid - 32); t < total; t += (long long)gridDim.x * (QGROUPS * QL)) {
             const int r = (int)(t % HpWp), y = r / Wp, x = r - y * Wp;
             if (y < PH || y >= PH + H || x < PW || x >= PW + W) {
-                uint4* dst = reinterpret_cast<uint4*>(out) + (size_t)t * Cp * 2;
+                uint4* dst = reinterpret_cast<uint4*>(out) + (size_t)t * pitch * 2;
                 for (int u = 0; u < 2 * Cp; u++) dst[u] = pad4;
             }
         }
@@ -192,7 +192,7 @@ quantise_tma_kernel(const __grid_constant__ CUtensorMap tmap, const float* __res
                     tnns_expand32_f4(sg[0], ~nz[0], lo);
                     tnns_expand32_f4(sg[1], ~nz[1], hi);
                     const int y = pix / W, x = pix - y * W;
-                    uint4* dst = reinterpret_cast<uint4*>(out) + (((size_t)n * HpWp + (size_t)y * Wp + x + off0) * Cp + ic) * 2;
+                    uint4* dst = reinterpret_cast<uint4*>(out) + (((size_t)n * HpWp + (size_t)y * Wp + x + off0) * pitch + ic) * 2;
                     dst[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
                     dst[1] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
                 } else {
@@ -227,7 +227,7 @@ bool tnns_quantise_tma_nhwc_supported(const float* d_x, int N, int C, int H, int
 }
 
 int tnns_launch_quantise_tma(tnns_cuda_ctx* ctx, bool ternary, const float* d_x, const float* d_thr, void* d_image, int N, int C, int H,
-                             int W, cudaStream_t stream, int format, int PH, int PW, int layout) {
+                             int W, cudaStream_t stream, int format, int PH, int PW, int layout, int pitch_words) {
     const int HW = H * W;
     if (N == 0) return TNNS_OK;
     if ((PH || PW) && format != TNNS_IMG_E2M1) return tnns_fail(TNNS_ERR_INVALID, "only the 4-bit image has a bordered form");
@@ -256,7 +256,7 @@ int tnns_launch_quantise_tma(tnns_cuda_ctx* ctx, bool ternary, const float* d_x,
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        TNNS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, map, d_thr, d_image, N, C, HW, Cp, nbands, ctx->d_status, W, Wp, HpWp, off0));
+        TNNS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, map, d_thr, d_image, N, C, HW, Cp, nbands, ctx->d_status, W, Wp, HpWp, off0, pitch_words ? pitch_words : Cp));
         tnns_count_launch();
         TNNS_CUDA_TRY(cudaGetLastError());
         return TNNS_OK;

@@ -1,0 +1,63 @@
+"""GPU suite: layers of sizes that are no multiple of anything.  The quantise kernels that read with plain
+loads (unaligned rows, unaligned bases, tiny tensors) against a numpy construction of their images, and whole
+layers with ragged channel counts or binary activations and strides against the checker."""
+import numpy as np
+import pytest
+
+import fastertnn_b200 as ft
+from cases import BNN, BTN, TBN, TNN, act_ternary, make_case, special_value_case, to_nchw, to_nhwc, wgt_ternary
+from fastertnn_b200 import synth
+from fastertnn_b200.workloads import Layer
+from test_gpu_parity import _expand32_f4_numpy
+
+pytestmark = pytest.mark.gpu
+
+
+def numpy_planes(x, thr, tern):
+    """[n][plane][pixel][ic][lo, hi] uint32 of an fp32 NCHW tensor, by the reference's compares."""
+    N, C, H, W = x.shape
+    Cp = (C + 63) // 64
+    t = thr.reshape(N, 1, 1)
+    v = x.reshape(N, C, H * W)
+    bits = np.zeros((2 if tern else 1, N, Cp * 64, H * W), bool)
+    bits[0, :, :C] = v < (-t if tern else t)
+    if tern:
+        bits[1] = True
+        bits[1, :, :C] = ~((v < -t) | (v > t))
+    packed = np.ascontiguousarray(np.packbits(bits.transpose(1, 0, 3, 2), axis=-1, bitorder="little"))   # n, plane, pixel, channel bits
+    return packed.view(np.uint32).reshape(N, 2 if tern else 1, H * W, Cp, 2)
+
+
+@pytest.mark.parametrize("tern", [True, False])
+@pytest.mark.parametrize("N,C,H,W", [(1, 1, 1, 1), (3, 33, 1, 1), (1, 64, 5, 5), (5, 65, 7, 3), (2, 31, 31, 33), (33, 130, 1, 7), (4, 262, 9, 5), (7, 3, 15, 23),
+                                     (2, 64, 8, 8), (3, 192, 6, 6)])
+def test_quantise_with_plain_loads(N, C, H, W, tern, gpu_ctx):
+    """One pixel, one channel, tails on both sides of 32 and 64 channels, pixel counts around 32, warps that straddle
+    images; and sizes the copy engine would take, from a base that is not 16-byte aligned."""
+    ctx = gpu_ctx
+    x = synth.uniform_pm1(300 + C, (N, C, H, W))
+    thr = (synth.uniform_pm1(301, (N,)) * 0.3 + (0.2 if tern else 0.0)).astype(np.float32)
+    flat = x.reshape(-1)
+    flat[:: 5] = np.float32(0.0)
+    flat[1:: 7] = np.repeat(thr, C * H * W)[1:: 7]       # exactly on the threshold: compares are strict
+    want = numpy_planes(x, thr, tern)
+    want4 = _expand32_f4_numpy(want[:, 0], want[:, 1]) if tern else None
+    Cp = (C + 63) // 64
+    nb_p, nb_e = ft.api.packed_image_bytes(tern, N, C, H, W), ft.api.e2m1_image_bytes(N, C, H, W)
+    d_t, d_p, d_e, d_x = ctx.to_device(thr), ctx.malloc(nb_p), ctx.malloc(nb_e), ctx.malloc(x.nbytes + 16)
+    try:
+        for layout in (ft.NCHW, ft.NHWC):
+            for off in (0, 4):
+                ctx.fill(d_x + off, x if layout == ft.NCHW else to_nhwc(x))
+                ctx.fill(d_p, np.full(nb_p // 4, 0x5A5A5A5A, np.uint32))
+                ctx.quantise(tern, d_x + off, d_t, d_p, N, C, H, W, layout)
+                ctx.sync()
+                assert np.array_equal(ctx.to_host(d_p, want.shape, np.uint32), want), ("planes", layout, off)
+                if tern:
+                    ctx.fill(d_e, np.full(nb_e // 4, 0x5A5A5A5A, np.uint32))
+                    ctx.quantise_e2m1(d_x + off, d_t, d_e, N, C, H, W, layout)
+                    ctx.sync()
+                    assert np.array_equal(ctx.to_host(d_e, (N, H * W, Cp, 2, 4), np.uint32), want4), ("4-bit image", layout, off)
+    finally:
+        for p in (d_t, d_p, d_e, d_x):
+            ctx.free(p)
