@@ -273,6 +273,10 @@ static int upload_weights_impl(tnns_cuda_ctx* ctx, int type, const int64_t* pack
         tnns_cuda_free_weights(ctx, w);
         return rc;
     }
+    if ((rc = tnns_build_wide_weights(ctx, w)) != TNNS_OK) {
+        tnns_cuda_free_weights(ctx, w);
+        return rc;
+    }
     if (C > 0 && tnns_dense_eligible(type, C, KH, KW)) {
         // few input channels: also keep the kernel as a 1x1 layer over only the real positions of a window.  The
         // repacked rows are in the reference's packed format, so the same upload builds that layer's operand images.
@@ -313,6 +317,7 @@ void tnns_cuda_free_weights(tnns_cuda_ctx* ctx, tnns_cuda_weights* w) {
     if (w->d_f4) cudaFree(w->d_f4);
     if (w->d_jtab) cudaFree(w->d_jtab);
     if (w->dense) tnns_cuda_free_weights(nullptr, w->dense);
+    if (w->wide) tnns_cuda_free_weights(nullptr, w->wide);
     delete w;
 }
 
@@ -555,6 +560,7 @@ static int conv_slab_impl(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
     TnnsFusedInput f;
     f.d_x = d_x;
     f.d_thr = d_thr;
+    f.C = g.C; f.Cp = g.Cp;
     f.d_sync = reinterpret_cast<unsigned int*>(static_cast<char*>(d_workspace) + slab_image_bytes(g.N, g.C, g.H, g.W, g.PH, g.PW));
     return tnns_launch_gemm_slab(ctx, w, d_workspace, d_y, g, alpha, TNNS_NCHW, (cudaStream_t)stream, pairs, d_image_out, d_thr_next, fmt, bin, next_PH,
                                  next_PW, &f);
@@ -658,10 +664,8 @@ int tnns_cuda_conv_dense_packed_out(tnns_cuda_ctx* ctx, const tnns_cuda_weights*
 int tnns_cuda_conv_auto_algo(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s, const float* d_x, int layout) {
     if (!ctx || !w || !s) return TNNS_GEMM_AUTO;
     if (tnns_cuda_dense_supported(ctx, w, s)) return TNNS_GEMM_F4_DENSE;
-    if (layout == TNNS_NCHW && tnns_cuda_slab_preferred(ctx, w, s) && tnns_cuda_conv_slab_supported(ctx, w, s, d_x, layout))
-        return tnns_cuda_conv_slab_one_launch_preferred(ctx, w, s, d_x, layout) ? TNNS_GEMM_F4_SLAB_FUSED : TNNS_GEMM_F4_SLAB;
-    if (layout == TNNS_NHWC && tnns_cuda_slab_preferred(ctx, w, s) && tnns_quantise_tma_nhwc_supported(d_x, s->N, s->C, s->H, s->W))
-        return TNNS_GEMM_F4_SLAB;  // two launches: the quantiser inside the GEMM kernel reads NCHW only
+    // two launches, whatever the input's layout and alignment (the one-launch form is never preferred)
+    if (tnns_cuda_slab_preferred(ctx, w, s)) return TNNS_GEMM_F4_SLAB;
     if (tnns_cuda_conv_fused_preferred(const_cast<tnns_cuda_ctx*>(ctx), w, s, d_x, layout)) return TNNS_GEMM_F4_FUSED;
     return TNNS_GEMM_F4_TC;
 }
@@ -699,6 +703,7 @@ static int conv_fused_impl(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const
     TnnsFusedInput f;
     f.d_x = d_x;
     f.d_thr = d_thr;
+    f.C = g.C; f.Cp = g.Cp;
     f.d_sync = reinterpret_cast<unsigned int*>(static_cast<char*>(d_workspace) + fused_image_bytes(g.N, g.C, g.H, g.W));
     return tnns_launch_gemm_im2col(ctx, w, d_workspace, d_y, g, alpha, layout, (cudaStream_t)stream, pairs, d_image_out, d_thr_next,
                                    next_format, &f);
@@ -720,14 +725,20 @@ int tnns_cuda_conv_fused_packed_out(tnns_cuda_ctx* ctx, const tnns_cuda_weights*
                            stream);
 }
 
-// The rule tnns_cuda_conv applies with TNNS_GEMM_AUTO: the one-launch route where the layer qualifies
-// and every SM has at least three 128-row tiles (measured, one launch / two launches in us: 32 images of
-// 512x32x32 -> 512, 3.5 tiles per SM: 49 / 54; 256 x 256x14x14 -> 256, 2.6: 43 / 40; 16 images, 1.7: 33 / 31.5).
+// Where the quantise step inside the GEMM launch pays: every SM has at least three 128-row tiles (measured, one launch /
+// two launches in us: 32 images of 512x32x32 -> 512, 3.5 tiles per SM: 49 / 54; 256 x 256x14x14 -> 256, 2.6: 43 / 40;
+// 16 images, 1.7: 33 / 31.5).
+static bool enough_tiles_for_one_launch(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const TnnsGeom& g) {
+    const long long M = (long long)g.N * g.OH * g.OW;
+    const int bn = tnns_i8_tile_n(w->KN);
+    return ((M + 127) / 128) * ((w->KN + bn - 1) / bn) >= 3LL * ctx->sm_count;
+}
+
+// The rule tnns_cuda_conv applies with TNNS_GEMM_AUTO
 int tnns_cuda_conv_fused_preferred(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s, const float* d_x, int layout) {
-    if (!ctx || !tnns_cuda_conv_fused_supported(w, s, d_x, layout)) return 0;
-    const long long tiles = (((long long)s->N * tnns_out_dim(s->H, s->PH, s->KH, s->SH) * tnns_out_dim(s->W, s->PW, s->KW, s->SW) + 127) / 128) *
-                            ((s->KN + 255) / 256);
-    return tiles >= 3LL * ctx->sm_count ? 1 : 0;
+    TnnsGeom g;
+    if (!ctx || !tnns_cuda_conv_fused_supported(w, s, d_x, layout) || tnns_make_geom(s, &g)) return 0;
+    return enough_tiles_for_one_launch(ctx, w, g) ? 1 : 0;
 }
 
 size_t tnns_packed_image_bytes(int ternary, int N, int C, int H, int W) {
@@ -796,6 +807,43 @@ int tnns_cuda_im2row_packed(tnns_cuda_ctx* ctx, int ternary, const void* d_image
                             TNNS_SRC_PACKED_IMAGE, TNNS_PACK_AUTO, (cudaStream_t)stream);
 }
 
+// Layers outside tnns_im2col_supported on the copy-engine fed GEMM all the same: binary activations from an image that
+// stores its padding (any stride), pixels of an odd number of bytes stored at a pitch of whole stage rows (w->wide).
+// gv: the geometry the GEMM sees; PH, PW: the border the quantise step writes.
+struct WidePlan {
+    const tnns_cuda_weights* w;
+    TnnsGeom gv;
+    int PH, PW;
+    size_t image_bytes, bytes;  // the image; with the synchronisation words of the one-launch form behind it
+};
+static bool wide_plan(const tnns_cuda_weights* w, const TnnsGeom& g, WidePlan* pl) {
+    pl->w = w->wide ? w->wide : w;
+    pl->gv = g;
+    pl->gv.C = pl->w->Cp * TNNS_WORD_BITS; pl->gv.Cp = pl->w->Cp; pl->gv.Kw = pl->w->Kw; pl->gv.Kp = pl->w->Kp;
+    pl->PH = pl->PW = 0;
+    if (!type_act_ternary(w->type)) {
+        pl->PH = g.PH; pl->PW = g.PW;
+        pl->gv.H += 2 * g.PH; pl->gv.W += 2 * g.PW;
+        pl->gv.PH = pl->gv.PW = 0;
+    }
+    if (!tnns_im2col_geometry_ok(pl->w, pl->gv)) return false;
+    pl->image_bytes = ((size_t)g.N * pl->gv.H * pl->gv.W * pl->gv.Cp * 32 + 127) & ~(size_t)127;
+    pl->bytes = pl->image_bytes + tnns_fused_sync_bytes(g.N);
+    return true;
+}
+// What any route of a whole layer may want as workspace.
+static size_t conv_workspace_bytes(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s, const TnnsGeom& g) {
+    // room for the im2row matrix (explicit route) and, where the layer qualifies, for the 4-bit
+    // image of the copy-engine routes, which is larger than the matrix for 1x1 kernels
+    size_t need = std::max<size_t>(tnns_packed_bytes(w->type, s), 16);
+    if (tnns_im2col_supported(w, g)) need = std::max(need, tnns_fused_workspace_bytes(g.N, g.C, g.H, g.W));
+    if (tnns_slab_supported(ctx, w, g, false)) need = std::max(need, tnns_slab_workspace_bytes(g.N, g.C, g.H, g.W, g.PH, g.PW));
+    if (tnns_cuda_dense_supported(ctx, w, s)) need = std::max(need, tnns_dense_workspace_bytes(s));
+    WidePlan wide;
+    if (wide_plan(w, g, &wide)) need = std::max(need, wide.bytes);
+    return need;
+}
+
 int tnns_cuda_conv_ws(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const float* d_x, const float* d_thr, float* d_y,
                       void* d_workspace, size_t workspace_bytes, const tnns_shape_t* s, float alpha, int layout, int pack_algo,
                       int gemm_algo, void* stream) {
@@ -814,11 +862,9 @@ int tnns_cuda_conv_ws(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const floa
         const int pick = tnns_cuda_conv_auto_algo(ctx, w, s, d_x, layout);
         if (pick == TNNS_GEMM_F4_DENSE && (reinterpret_cast<uintptr_t>(d_workspace) & 127) == 0 && tnns_dense_workspace_bytes(s) <= workspace_bytes)
             gemm_algo = pick;
-        if (pick == TNNS_GEMM_F4_SLAB || pick == TNNS_GEMM_F4_SLAB_FUSED) {
-            const size_t ws_need = pick == TNNS_GEMM_F4_SLAB_FUSED ? tnns_slab_workspace_bytes(g.N, g.C, g.H, g.W, g.PH, g.PW)
-                                                                   : tnns_bordered_image_bytes(g.N, g.C, g.H, g.W, g.PH, g.PW);
-            if ((reinterpret_cast<uintptr_t>(d_workspace) & 127) == 0 && ws_need <= workspace_bytes) gemm_algo = pick;
-        }
+        if (pick == TNNS_GEMM_F4_SLAB && (reinterpret_cast<uintptr_t>(d_workspace) & 127) == 0 &&
+            tnns_bordered_image_bytes(g.N, g.C, g.H, g.W, g.PH, g.PW) <= workspace_bytes)
+            gemm_algo = pick;
     }
     if (gemm_algo == TNNS_GEMM_F4_DENSE) {
         // few input channels: only the real positions of every window, as a 1x1 layer
@@ -831,11 +877,11 @@ int tnns_cuda_conv_ws(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const floa
         const size_t ws_need = one_launch ? tnns_slab_workspace_bytes(g.N, g.C, g.H, g.W, g.PH, g.PW)
                                           : tnns_bordered_image_bytes(g.N, g.C, g.H, g.W, g.PH, g.PW);
         if (pack_algo != TNNS_PACK_AUTO || (layout != TNNS_NCHW && (one_launch || layout != TNNS_NHWC)) || !tnns_slab_supported(ctx, w, g, one_launch) ||
-            !bordered_quantise_ok(d_x, g.N, g.C, g.H, g.W, layout) || (reinterpret_cast<uintptr_t>(d_workspace) & 127) || ws_need > workspace_bytes)
+            (!auto_both && !bordered_quantise_ok(d_x, g.N, g.C, g.H, g.W, layout)) || (reinterpret_cast<uintptr_t>(d_workspace) & 127) || ws_need > workspace_bytes)
             return tnns_fail(TNNS_ERR_UNSUPPORTED, "layer, layout, workspace size or alignment outside the slab-fed route");
         if (one_launch) return tnns_cuda_conv_slab(ctx, w, d_x, d_thr, d_y, d_workspace, workspace_bytes, s, alpha, 0, stream);
-        rc = tnns_launch_quantise_tma(ctx, type_act_ternary(w->type), d_x, d_thr, d_workspace, g.N, g.C, g.H, g.W, (cudaStream_t)stream, TNNS_IMG_E2M1,
-                                      g.PH, g.PW, quantise_layout(layout, g.H, g.W));
+        rc = tnns_launch_quantise(ctx, type_act_ternary(w->type), d_x, d_thr, d_workspace, g.N, g.C, g.H, g.W, layout, (cudaStream_t)stream, TNNS_IMG_E2M1,
+                                  g.PH, g.PW);
         if (rc) return rc;
         return tnns_launch_gemm_slab(ctx, w, d_workspace, d_y, g, alpha, layout, (cudaStream_t)stream);
     }
@@ -868,6 +914,16 @@ int tnns_cuda_conv_ws(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const floa
         if (rc) return rc;
         return tnns_launch_gemm_im2col(ctx, w, d_workspace, d_y, g, alpha, layout, (cudaStream_t)stream);
     }
+    WidePlan wide;
+    if (auto_route && wide_plan(w, g, &wide) && (reinterpret_cast<uintptr_t>(d_workspace) & 127) == 0 && wide.bytes <= workspace_bytes) {
+        // Measured on B200 against the gathering GEMM that took these layers before (layer call, us): 8 x 320x15x23 -> 320 s2
+        // 18.3 / 12.4, 32 x 192x28x28 -> 192 25.1 / 20.1, NHWC 63 x 262x21x20 -> 512 54 / 41, BTN 8 x 256x14x14 -> 256 s2
+        // 16.2 / 12.7, BNN 32 x 128x28x28 -> 128 s2 13.6 / 11.2, BNN 16 x 320x28x28 -> 320 27.7 / 24.6
+        rc = tnns_launch_quantise(ctx, type_act_ternary(w->type), d_x, d_thr, d_workspace, g.N, g.C, g.H, g.W, layout, (cudaStream_t)stream,
+                                  TNNS_IMG_E2M1, wide.PH, wide.PW, wide.gv.Cp);
+        if (rc) return rc;
+        return tnns_launch_gemm_im2col(ctx, wide.w, d_workspace, d_y, wide.gv, alpha, layout, (cudaStream_t)stream);
+    }
     const size_t image_bytes = tnns_packed_image_bytes(type_act_ternary(w->type), g.N, g.C, g.H, g.W);
     if (pack_algo == TNNS_PACK_AUTO && (gemm_algo == TNNS_GEMM_AUTO || gemm_algo == TNNS_GEMM_F4_TC) && w->d_f4 && w->d_jtab &&
         w->Kp < 65536 && image_bytes <= workspace_bytes) {
@@ -893,12 +949,7 @@ int tnns_cuda_conv(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const float* 
     int rc = tnns_make_geom(s, &g);
     if (rc) return rc;
     TNNS_ENTER(ctx, w);
-    // room for the im2row matrix (explicit route) and, where the layer qualifies, for the 4-bit
-    // image of the copy-engine route, which is larger than the matrix for 1x1 kernels
-    size_t need = std::max<size_t>(tnns_packed_bytes(w->type, s), 16);
-    if (tnns_im2col_supported(w, g)) need = std::max(need, tnns_fused_workspace_bytes(g.N, g.C, g.H, g.W));
-    if (tnns_slab_supported(ctx, w, g, false)) need = std::max(need, tnns_slab_workspace_bytes(g.N, g.C, g.H, g.W, g.PH, g.PW));
-    if (tnns_cuda_dense_supported(ctx, w, s)) need = std::max(need, tnns_dense_workspace_bytes(s));
+    const size_t need = conv_workspace_bytes(ctx, w, s, g);
     if (ctx->workspace_bytes < need) {
         // earlier launches may still read the old workspace
         TNNS_CUDA_TRY(cudaDeviceSynchronize());
@@ -955,8 +1006,9 @@ int tnns_cuda_conv_host(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const fl
     const size_t out_img = (size_t)g.KN * g.OH * g.OW * sizeof(float);
     tnns_shape_t ss = *s;
     ss.N = nb;
-    size_t pack_slice = std::max<size_t>(tnns_packed_bytes(w->type, &ss), 16);
-    if (tnns_im2col_supported(w, g)) pack_slice = std::max(pack_slice, tnns_fused_workspace_bytes(nb, g.C, g.H, g.W));
+    TnnsGeom gs = g;
+    gs.N = nb;
+    const size_t pack_slice = conv_workspace_bytes(ctx, w, &ss, gs);
 
     // staging buffers are shared by both slots' sizes; growing needs the device idle
     bool must_grow = ctx->stage_in_bytes < in_img * nb || ctx->stage_out_bytes < out_img * nb ||

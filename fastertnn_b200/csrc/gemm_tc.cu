@@ -40,6 +40,7 @@
 #include <cuda.h>  // CUtensorMap and the encode prototypes only; the entry point is looked up at run time
 
 #include <algorithm>
+#include <new>
 #include <type_traits>
 #include <vector>
 
@@ -189,6 +190,31 @@ __global__ void expand_weights_kernel(const uint4* __restrict__ packed, unsigned
     }
 }
 
+// The 4-bit image with every tap padded from cp_src to cp_dst (a multiple of four) words: stage c of a row holds the
+// words 4c .. 4c+3 of the padded row; words without a source are zero weights.
+__global__ void expand_weights_wide_kernel(const uint64_t* __restrict__ packed, unsigned char* __restrict__ img, int KN, int Kp, int cp_src,
+                                           int cp_dst, int nch, int BN, int two_planes) {
+    const long long total = (long long)KN * nch;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+        const int kn = (int)(i / nch), c = (int)(i - (long long)kn * nch);
+        const uint64_t* row = packed + (size_t)kn * Kp * (two_planes ? 2 : 1);
+        const int tap = 4 * c / cp_dst, ic0 = 4 * c - tap * cp_dst;  // cp_dst % 4 == 0: a stage never spans two taps
+        uint64_t sw[4], zw[4];
+        for (int q = 0; q < 4; q++) {
+            const int j = tap * cp_src + ic0 + q;
+            const bool real = ic0 + q < cp_src;
+            sw[q] = !real ? 0ull : two_planes ? row[(j >> 2) * 8 + (j & 3)] : row[j];
+            zw[q] = !real ? ~0ull : two_planes ? row[(j >> 2) * 8 + 4 + (j & 3)] : 0ull;
+        }
+        uint4 s[2], z[2];
+        for (int q = 0; q < 2; q++) {
+            s[q] = make_uint4((uint32_t)sw[2 * q], (uint32_t)(sw[2 * q] >> 32), (uint32_t)sw[2 * q + 1], (uint32_t)(sw[2 * q + 1] >> 32));
+            z[q] = make_uint4((uint32_t)zw[2 * q], (uint32_t)(zw[2 * q] >> 32), (uint32_t)zw[2 * q + 1], (uint32_t)(zw[2 * q + 1] >> 32));
+        }
+        store_row_stage_f4(img + ((size_t)(kn / BN) * nch + c) * (size_t)BN * KCH, kn % BN, s, z);
+    }
+}
+
 struct GemmArgs {
     const uint4* A;             // packed activations
     const unsigned char* Bimg;  // expanded weights
@@ -196,7 +222,7 @@ struct GemmArgs {
     long long M;
     int KN, Kp, OHW, layout;
     int a_two_planes;
-    int acc_bias;               // added to the integer dot product (BNN: K_unpack - 64*Kp)
+    int acc_bias;               // added to the integer dot product (BNN: K_unpack minus the positions multiplied)
     float alpha;
     unsigned int* status;
     // optional quantised output for a following layer (instead of y): bit planes [n][plane][pixel][ic]
@@ -223,7 +249,7 @@ struct GemmArgs {
     const float* qthr;
     uint4* qimg;
     unsigned int* q_sync;
-    int qN, qC, q_nbands;
+    int qN, qC, q_nbands, q_cp;  // q_cp: 64-channel words of that input (the image's pixel pitch is Cp)
     int q_nhwc;        // that input is pixel-major (NHWC)
     int q_self_clean;  // the last block to leave zeroes the words again (q_sync[1] counts the blocks that left)
 };
@@ -381,7 +407,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                         // quantiser warps (of any block) have finished them
                         const long long last = min(row0 + BMT, p.M) - 1;
                         const int n_last = (int)(last / p.OHW);
-                        const unsigned int per_image = (unsigned int)(p.q_nbands * p.Cp) * 4u;  // every quantiser warp counts itself
+                        const unsigned int per_image = (unsigned int)(p.q_nbands * p.q_cp) * 4u;  // every quantiser warp counts itself
                         for (int n = a_n; n <= n_last; n++)
                             if (!counter_wait(p.q_sync + Q_FLAG0 + n, per_image, abort_flag, p.status, 6)) goto done;
                         // their plain stores, now visible to this thread, before the copy engine's reads
@@ -600,7 +626,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
     } else if (QF && warp >= Cfg::WARP_Q0) {
         uint64_t* qbars = reinterpret_cast<uint64_t*>(smem + Cfg::Q_OFF + Cfg::QSTG * Cfg::Q_STAGE);
         if (warp < Cfg::WARP_Q0 + 4)
-            quantise_items(plain_quant_args(p.qthr, p.qimg, p.q_sync, p.qN, p.qC, p.q_nbands, p.Cp, p.H, p.W, p.status, p.q_nhwc), &tmap_q, smem + Cfg::Q_OFF, qbars,
+            quantise_items(plain_quant_args(p.qthr, p.qimg, p.q_sync, p.qN, p.qC, p.q_nbands, p.q_cp, p.Cp, p.H, p.W, p.status, p.q_nhwc), &tmap_q, smem + Cfg::Q_OFF, qbars,
                            abort_flag, tid - Cfg::WARP_Q0 * 32);
         else if (lane == 0)
             publish_items(p.q_sync, p.status, qbars, abort_flag);
@@ -978,6 +1004,19 @@ int launch_bn(tnns_cuda_ctx* ctx, const GemmArgs& a, cudaStream_t stream) {
 
 int tnns_i8_tile_n(int KN) { return KN <= 64 ? 64 : (KN <= 128 ? 128 : 256); }
 
+// tap table: plane word j -> kh<<24 | kw<<16 | ic, for kernels whose taps fit those fields
+static int upload_tap_table(tnns_cuda_weights* w) {
+    if (!(w->C > 0 && w->KH < 256 && w->KW < 256 && w->Cp < 65536)) return TNNS_OK;
+    std::vector<uint32_t> tab(w->Kp, 0xFFFFFFFFu);
+    for (int j = 0; j < w->Kw; j++) {
+        const int ic = j % w->Cp, kw = (j / w->Cp) % w->KW, kh = j / (w->Cp * w->KW);
+        tab[j] = ((uint32_t)kh << 24) | ((uint32_t)kw << 16) | (uint32_t)ic;
+    }
+    TNNS_CUDA_TRY(cudaMalloc(&w->d_jtab, tab.size() * sizeof(uint32_t)));
+    TNNS_CUDA_TRY(cudaMemcpy(w->d_jtab, tab.data(), tab.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    return TNNS_OK;
+}
+
 // Builds both operand images of a layer's weights: int8 (128 K elements per 128-byte row and
 // stage) and e2m1 (256 K elements per row and stage).
 int tnns_build_i8_weights(tnns_cuda_ctx* ctx, tnns_cuda_weights* w) {
@@ -994,26 +1033,47 @@ int tnns_build_i8_weights(tnns_cuda_ctx* ctx, tnns_cuda_weights* w) {
         TNNS_CUDA_TRY(cudaMemset(img, 0, bytes));
         const long long total = (long long)w->KN * nch;
         const int blocks = (int)std::min<long long>((total + 127) / 128, 4096);
-        // TBN: ternary activations meet binary weights, whose pad words read +1; the products there are
-        // zero only because the activation pad words are zeros -- writing zero weights instead changes
-        // nothing and lets the tensor-copy form skip those K positions.  (BNN keeps +1: its epilogue
-        // constant counts the padded +1 x +1 products.)
-        const int zero_from = (f4 && w->type == TBN) ? w->Kw : -1;
+        // Binary weights read +1 in the pad-to-four words.  Zeros there instead let the tensor-copy form skip those K
+        // positions: TBN multiplies them with zeros anyway, and BNN's epilogue constant counts real words only.
+        const int zero_from = (f4 && !two) ? w->Kw : -1;
         expand_weights_kernel<<<blocks, 128>>>(reinterpret_cast<const uint4*>(w->d_packed), reinterpret_cast<unsigned char*>(img), w->KN,
                                                 w->Kp, BN, two ? 1 : 0, f4, zero_from);
         tnns_count_launch();
         TNNS_CUDA_TRY(cudaGetLastError());
     }
-    // tap table for the implicit-im2row form: plane word j -> kh<<24 | kw<<16 | ic
-    if (w->C > 0 && w->KH < 256 && w->KW < 256 && w->Cp < 65536) {
-        std::vector<uint32_t> tab(w->Kp, 0xFFFFFFFFu);
-        for (int j = 0; j < w->Kw; j++) {
-            const int ic = j % w->Cp, kw = (j / w->Cp) % w->KW, kh = j / (w->Cp * w->KW);
-            tab[j] = ((uint32_t)kh << 24) | ((uint32_t)kw << 16) | (uint32_t)ic;
-        }
-        TNNS_CUDA_TRY(cudaMalloc(&w->d_jtab, tab.size() * sizeof(uint32_t)));
-        TNNS_CUDA_TRY(cudaMemcpy(w->d_jtab, tab.data(), tab.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    }
+    int rc = upload_tap_table(w);
+    if (rc) return rc;
+    TNNS_CUDA_TRY(cudaDeviceSynchronize());
+    return TNNS_OK;
+}
+
+// The kernel with every tap's words padded to a multiple of four (64 * 4 channels = the 128 bytes of a stage row).
+// A pixel of 96 or 160 bytes cannot fill a stage row from whole copies, and the copy engine's cost is per pixel and
+// copy, not per byte: ceil(Cp / 4) copies of 128 bytes per tap are fewer than Cp copies of 32.  The pad words meet zero
+// weights, so the image may leave them as they are (every 4-bit code is finite).
+int tnns_build_wide_weights(tnns_cuda_ctx* ctx, tnns_cuda_weights* w) {
+    (void)ctx;
+    if (w->C <= 0 || w->Cp <= 2 || w->Cp % 4 == 0 || w->KH >= 256 || w->KW >= 256) return TNNS_OK;
+    const int cp = (w->Cp + 3) & ~3, kw = w->KH * w->KW * cp;
+    if (kw >= 65536) return TNNS_OK;
+    tnns_cuda_weights* v = new (std::nothrow) tnns_cuda_weights();
+    if (!v) return tnns_fail(TNNS_ERR_NOMEM, "host allocation failed");
+    *v = tnns_cuda_weights{};
+    w->wide = v;
+    v->type = w->type; v->KN = w->KN; v->KH = w->KH; v->KW = w->KW; v->device = w->device;
+    v->C = cp * TNNS_WORD_BITS; v->Cp = cp; v->Kw = v->Kp = kw;
+    v->K_unpack = w->K_unpack + 64 * (v->Kw - w->Kw);  // so that K_unpack - 64*Kw stays what it is
+    const int BN = tnns_i8_tile_n(w->KN), ntn = (w->KN + BN - 1) / BN, nch = kw / 4;
+    v->f4_bytes = (size_t)ntn * nch * BN * KCH;
+    TNNS_CUDA_TRY(cudaMalloc(&v->d_f4, v->f4_bytes));
+    TNNS_CUDA_TRY(cudaMemset(v->d_f4, 0, v->f4_bytes));
+    const long long total = (long long)w->KN * nch;
+    const int blocks = (int)std::min<long long>((total + 127) / 128, 4096);
+    expand_weights_wide_kernel<<<blocks, 128>>>(w->d_packed, v->d_f4, w->KN, w->Kp, w->Cp, cp, nch, BN, (w->type == TNN || w->type == BTN) ? 1 : 0);
+    tnns_count_launch();
+    TNNS_CUDA_TRY(cudaGetLastError());
+    int rc = upload_tap_table(v);
+    if (rc) return rc;
     TNNS_CUDA_TRY(cudaDeviceSynchronize());
     return TNNS_OK;
 }
@@ -1037,7 +1097,8 @@ int tnns_launch_gemm_tc(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const vo
     // epilogue writes 16 bytes per lane where the channel-major one would write 4 (rows are KN floats apart either way)
     a.layout = OHW == 1 ? TNNS_NHWC : layout;
     a.a_two_planes = (w->type == TNN || w->type == TBN) ? 1 : 0;
-    a.acc_bias = (w->type == BNN) ? w->K_unpack - 64 * w->Kp : 0;
+    // BNN counts its products; the 4-bit weight image holds zeros in the pad-to-four words, the int8 one +1
+    a.acc_bias = (w->type == BNN) ? w->K_unpack - 64 * (f4 ? w->Kw : w->Kp) : 0;
     a.zero_passes = w->type != TNN;
     a.alpha = alpha;
     a.status = ctx->d_status;
@@ -1050,7 +1111,7 @@ int tnns_launch_gemm_tc(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const vo
     a.img = nullptr;
     a.jtab = nullptr;
     a.H = a.W = a.OW = a.Cp = a.SH = a.SW = a.PH = a.PW = 0;
-    a.qx = a.qthr = nullptr; a.qimg = nullptr; a.q_sync = nullptr; a.qN = a.qC = a.q_nbands = a.q_self_clean = a.q_nhwc = 0;
+    a.qx = a.qthr = nullptr; a.qimg = nullptr; a.q_sync = nullptr; a.qN = a.qC = a.q_nbands = a.q_cp = a.q_self_clean = a.q_nhwc = 0;
     if (implicit_geom) {
         // d_a is the quantised image of the layer input, not an im2row matrix
         if (!f4 || !w->d_jtab) return tnns_fail(TNNS_ERR_UNSUPPORTED, "implicit im2row needs the 4-bit tensor-core GEMM and layer geometry");
@@ -1079,6 +1140,10 @@ int tnns_launch_gemm_tc(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const vo
 // ---------------------------------------------------------------------------------------
 bool tnns_im2col_supported(const tnns_cuda_weights* w, const TnnsGeom& g) {
     if (!(w->type == TNN || w->type == TBN)) return false;   // outside the image the copy engine writes 0, a ternary zero
+    return tnns_im2col_geometry_ok(w, g);
+}
+
+bool tnns_im2col_geometry_ok(const tnns_cuda_weights* w, const TnnsGeom& g) {
     if (!w->d_f4 || !w->d_jtab || w->Kp >= 65536) return false;
     if (tnns_i8_tile_n(w->KN) != 256 && tnns_i8_tile_n(w->KN) != 128 && tnns_i8_tile_n(w->KN) != 64) return false;
     if (g.Cp != 1 && g.Cp != 2 && g.Cp % 4 != 0) return false;  // a 128-byte stage row = 1 tap of 256 channels, 2 of 128 or 4 of 64
@@ -1177,13 +1242,17 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
                             const TnnsFusedInput* fused, int next_PH, int next_PW) {
     const long long M = (long long)g.N * g.OH * g.OW;
     if (M == 0) return TNNS_OK;
-    if (!tnns_im2col_supported(w, g)) return tnns_fail(TNNS_ERR_UNSUPPORTED, "layer shape or type outside the tensor-copy activation path");
+    // binary activations: only from an image that holds the padding itself (their padding is +1, the copy engine's 0)
+    if (!tnns_im2col_geometry_ok(w, g) || ((w->type == BTN || w->type == BNN) && (g.PH || g.PW)))
+        return tnns_fail(TNNS_ERR_UNSUPPORTED, "layer shape or type outside the tensor-copy activation path");
     if (reinterpret_cast<uintptr_t>(d_image) & 15) return tnns_fail(TNNS_ERR_INVALID, "image must be 16-byte aligned");
     unsigned int* fused_words = nullptr;
     int fused_self_clean = 0;
     if (fused) {
         if (!fused->d_x || !fused->d_thr || !fused->d_sync) return tnns_fail(TNNS_ERR_INVALID, "NULL argument");
-        if (!tnns_fused_supported(w, g, fused->d_x, layout))
+        TnnsGeom gx = g;
+        gx.C = fused->C;
+        if (!tnns_fused_supported(w, gx, fused->d_x, layout))
             return tnns_fail(TNNS_ERR_UNSUPPORTED, "fused quantisation needs a 16-byte aligned input: NCHW with H*W a multiple of four, or NHWC with C a multiple of four");
         if (reinterpret_cast<uintptr_t>(fused->d_sync) & 127) return tnns_fail(TNNS_ERR_INVALID, "synchronisation words must be 128-byte aligned");
         int rc0 = tnns_fused_sync_prepare(ctx, g.N, stream, fused->d_sync, &fused_words, &fused_self_clean);
@@ -1202,7 +1271,7 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
     a.OHW = g.OH * g.OW;
     a.layout = a.OHW == 1 ? TNNS_NHWC : layout;  // one pixel per image: same memory, wider stores (see above)
     a.a_two_planes = 1;
-    a.acc_bias = 0;
+    a.acc_bias = (w->type == BNN) ? w->K_unpack - 64 * w->Kw : 0;
     a.zero_passes = w->type != TNN;
     a.alpha = alpha;
     a.status = ctx->d_status;
@@ -1223,7 +1292,7 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
     a.cp_next = (w->KN + TNNS_WORD_BITS - 1) / TNNS_WORD_BITS;
     a.img = nullptr;
     a.jtab = w->d_jtab;
-    a.qx = a.qthr = nullptr; a.qimg = nullptr; a.q_sync = nullptr; a.qN = a.qC = a.q_nbands = a.q_self_clean = a.q_nhwc = 0;
+    a.qx = a.qthr = nullptr; a.qimg = nullptr; a.q_sync = nullptr; a.qN = a.qC = a.q_nbands = a.q_cp = a.q_self_clean = a.q_nhwc = 0;
     a.H = g.H; a.W = g.W; a.OW = g.OW; a.Cp = g.Cp; a.SH = g.SH; a.SW = g.SW; a.PH = g.PH; a.PW = g.PW;
     alignas(64) CUtensorMap map_q;
     if (fused) {
@@ -1231,9 +1300,9 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
         const unsigned long long HW = (unsigned long long)g.H * g.W;
         // (pixel-major input: one row of C floats per pixel of any image; box = 128 pixels x 32 channels, 128-byte swizzle)
         if (layout == TNNS_NHWC)
-            rc = tnns_tensor_map_2d(&map_q, 4, fused->d_x, (unsigned long long)g.C, (unsigned long long)g.N * HW, (unsigned long long)g.C * 4, 32, Q_PIX, 128);
+            rc = tnns_tensor_map_2d(&map_q, 4, fused->d_x, (unsigned long long)fused->C, (unsigned long long)g.N * HW, (unsigned long long)fused->C * 4, 32, Q_PIX, 128);
         else
-            rc = tnns_tensor_map_2d(&map_q, 4, fused->d_x, HW, (unsigned long long)g.N * g.C, HW * 4, Q_PIX, 64);
+            rc = tnns_tensor_map_2d(&map_q, 4, fused->d_x, HW, (unsigned long long)g.N * fused->C, HW * 4, Q_PIX, 64);
         if (rc) return rc;
         a.q_nhwc = layout == TNNS_NHWC;
         a.qx = fused->d_x;
@@ -1242,7 +1311,8 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
         a.q_sync = fused_words;
         a.q_self_clean = fused_self_clean;
         a.qN = g.N;
-        a.qC = g.C;
+        a.qC = fused->C;
+        a.q_cp = fused->Cp;
         a.q_nbands = (g.H * g.W + Q_PIX - 1) / Q_PIX;
     }
     const int taps = g.Cp == 1 ? 4 : (g.Cp == 2 ? 2 : 1);

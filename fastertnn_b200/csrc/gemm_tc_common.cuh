@@ -279,6 +279,7 @@ struct QuantArgs {
     uint4* qimg;
     unsigned int* q_sync;
     int qN, qC, q_nbands, Cp, HW;
+    int pitch;  // 64-channel words from one pixel of the image to the next (>= Cp)
     unsigned int* status;
     // Where pixel (y, x) of image n lands in the 4-bit image: pixel index n*HpWp + y*Wp + x + off0.
     // Plain image: Wp = W, HpWp = H*W, off0 = 0.  Bordered image (the layer's padding stored around
@@ -288,10 +289,10 @@ struct QuantArgs {
     int binary;  // activations in {-1,+1} (x < t), absent channels and the border +1; else ternary, both 0
     int nhwc;    // the fp32 input is pixel-major: an item arrives as two 128-byte-swizzled boxes of 128 pixels x 32 channels
 };
-__device__ __forceinline__ QuantArgs plain_quant_args(const float* qthr, uint4* qimg, unsigned int* q_sync, int qN, int qC, int q_nbands, int Cp,
+__device__ __forceinline__ QuantArgs plain_quant_args(const float* qthr, uint4* qimg, unsigned int* q_sync, int qN, int qC, int q_nbands, int Cp, int pitch,
                                                       int H, int W, unsigned int* status, int nhwc = 0) {
     QuantArgs a;
-    a.qthr = qthr; a.qimg = qimg; a.q_sync = q_sync; a.qN = qN; a.qC = qC; a.q_nbands = q_nbands; a.Cp = Cp; a.HW = H * W; a.status = status;
+    a.qthr = qthr; a.qimg = qimg; a.q_sync = q_sync; a.qN = qN; a.qC = qC; a.q_nbands = q_nbands; a.Cp = Cp; a.pitch = pitch; a.HW = H * W; a.status = status;
     a.W = W; a.Wp = W; a.HpWp = H * W; a.off0 = 0; a.border = 0; a.binary = 0; a.nhwc = nhwc;
     return a;
 }
@@ -442,7 +443,7 @@ __device__ __noinline__ void quantise_items(const QuantArgs p, const CUtensorMap
             for (int tpx = qtid; tpx < p.HpWp; tpx += Q_PIX) {
                 const int y = tpx / p.Wp, x = tpx - y * p.Wp;
                 if (y < PH || y >= PH + H || x < PW || x >= PW + p.W) {
-                    uint4* dst = p.qimg + ((size_t)n * p.HpWp + tpx) * p.Cp * 2;
+                    uint4* dst = p.qimg + ((size_t)n * p.HpWp + tpx) * p.pitch * 2;
                     for (int u = 0; u < 2 * p.Cp; u++) dst[u] = pad4;
                 }
             }
@@ -451,7 +452,7 @@ __device__ __noinline__ void quantise_items(const QuantArgs p, const CUtensorMap
             tnns_expand32_f4(sg[0], ~nz[0], lo);
             tnns_expand32_f4(sg[1], ~nz[1], hi);
             const int y = pix / p.W, x = pix - y * p.W;
-            uint4* dst = p.qimg + (((size_t)n * p.HpWp + (size_t)y * p.Wp + x + p.off0) * p.Cp + ic) * 2;
+            uint4* dst = p.qimg + (((size_t)n * p.HpWp + (size_t)y * p.Wp + x + p.off0) * p.pitch + ic) * 2;
             dst[0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             dst[1] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
         }

@@ -58,6 +58,10 @@ struct tnns_cuda_weights {
     // layers with few input channels: the same kernel as a 1x1 layer over only the real positions of a window
     // (dense.cu), NULL where that form does not apply
     tnns_cuda_weights* dense;
+    // kernels whose pixels are no 32, 64 or multiple of 128 bytes of 4-bit operands: the same kernel with every tap
+    // padded to a multiple of four 64-channel words (zero weights), for an image stored with that pixel pitch; holds
+    // d_f4 and d_jtab only, NULL where the kernel's own form fits
+    tnns_cuda_weights* wide;
 };
 
 // error plumbing (thread local)
@@ -83,6 +87,7 @@ int tnns_launch_gemm_popc(tnns_cuda_ctx* ctx, int type, const void* d_a, const v
 // tensor-core path (gemm_i8_tc.cu)
 int tnns_i8_tile_n(int KN);
 int tnns_build_i8_weights(tnns_cuda_ctx* ctx, tnns_cuda_weights* w);
+int tnns_build_wide_weights(tnns_cuda_ctx* ctx, tnns_cuda_weights* w);
 // d_pimg != NULL: write the next layer's quantised bit planes instead of fp32 (d_y unused)
 int tnns_launch_gemm_tc(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const void* d_a, float* d_y, long long M, int OHW, float alpha,
                         int layout, bool f4, cudaStream_t stream, void* d_pimg = nullptr, const float* d_thr_next = nullptr,
@@ -124,6 +129,8 @@ int tnns_tensor_map_2d(void* map, int elem_bytes, const void* base, unsigned lon
 // 4-bit GEMM + PReLU whose activation tiles the copy engine gathers (im2col tensor copies) from
 // an e2m1 image; needs ternary activations and a channel count that fills 128-byte chunks
 bool tnns_im2col_supported(const tnns_cuda_weights* w, const TnnsGeom& g);
+// the part of that which concerns the geometry alone: any type, where the image holds no padding of another value
+bool tnns_im2col_geometry_ok(const tnns_cuda_weights* w, const TnnsGeom& g);
 // d_pimg != NULL: write the next layer's quantised activations instead of fp32 (next_format 0: binary
 // bit planes, 1: ternary bit planes, 2: ternary 4-bit operand image)
 // fused != NULL: the same launch also quantises the layer's fp32 input into d_image (quantiser
@@ -133,6 +140,7 @@ struct TnnsFusedInput {
     const float* d_x;
     const float* d_thr;
     unsigned int* d_sync;
+    int C, Cp;  // channels of the fp32 input and their 64-channel words (the image's pixel may be padded to more)
 };
 size_t tnns_fused_sync_bytes(int N);
 bool tnns_fused_supported(const tnns_cuda_weights* w, const TnnsGeom& g, const float* d_x, int layout);

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import fastertnn_b200 as ft
-from cases import BNN, BTN, TBN, TNN, act_ternary, make_case, special_value_case, to_nchw, to_nhwc, wgt_ternary
+from cases import BNN, BTN, TBN, TNN, make_case, to_nchw, to_nhwc, wgt_ternary
 from fastertnn_b200 import synth
 from fastertnn_b200.workloads import Layer
 from test_gpu_parity import _expand32_f4_numpy
@@ -61,3 +61,43 @@ def test_quantise_with_plain_loads(N, C, H, W, tern, gpu_ctx):
     finally:
         for p in (d_t, d_p, d_e, d_x):
             ctx.free(p)
+
+
+# ragged channel counts (pixels of 96, 160, 192, 224 bytes of operands), binary activations with strides and paddings,
+# pad-to-four words under binary weights, odd images: layers whose image is stored padded or bordered for the copy engine
+WIDE_LAYERS = [
+    (Layer(130, 9, 7, 40, 3, 3, 1, 1), 3), (Layer(320, 15, 23, 300, 3, 3, 1, 2), 2), (Layer(384, 5, 5, 64, 1, 1, 0, 1), 3),
+    (Layer(420, 6, 6, 129, 5, 3, 2, 2), 2), (Layer(600, 1, 1, 70, 1, 1, 0, 1), 5), (Layer(64, 12, 12, 64, 3, 3, 1, 2), 3),
+    (Layer(128, 9, 9, 33, 3, 3, 1, 3), 3), (Layer(256, 14, 14, 256, 3, 3, 1, 2), 3), (Layer(40, 7, 7, 20, 3, 3, 0, 1), 4),
+    (Layer(96, 8, 8, 200, 2, 2, 3, 1), 2), (Layer(70, 5, 5, 16, 1, 1, 0, 2), 7), (Layer(512, 4, 4, 40, 3, 3, 1, 1), 5),
+]
+
+
+@pytest.mark.parametrize("type_", [TNN, TBN, BTN, BNN])
+@pytest.mark.parametrize("layer,N", WIDE_LAYERS, ids=lambda v: str(v).replace(" ", ""))
+def test_layers_of_any_channel_count_and_alphabet(layer, N, type_, gpu_ctx, checker):
+    """Whole layers through the default call, both layouts, twice over stale workspaces."""
+    case = make_case(type_, layer, N, 8200 + layer.C, "uniform")
+    wp = checker.pack_weights(wgt_ternary(type_), case.w, case.w_thr)
+    want = checker.conv(type_, case.x, case.thr, wp, case.kernel_hw, case.padding, case.stride, case.alpha)
+    ctx = gpu_ctx
+    w = ctx.upload_weights(type_, wp, layer.C, layer.KH, layer.KW)
+    d_t, d_y = ctx.to_device(case.thr), ctx.malloc(want.nbytes)
+    nb = 1 << 22
+    d_ws = ctx.malloc(nb)
+    try:
+        for layout in (ft.NCHW, ft.NHWC):
+            d_x = ctx.to_device(case.x if layout == ft.NCHW else to_nhwc(case.x))
+            for fill in (0x77777777, 0xFFFFFFFF):
+                ctx.fill(d_ws, np.full(nb // 4, fill, np.uint32))
+                ctx.fill(d_y, np.full(want.size, np.nan, np.float32))
+                ctx.conv_ws(w, d_x, d_t, d_y, d_ws, nb, layer.shape(N), case.alpha, layout)
+                ctx.sync()
+                got = ctx.to_host(d_y, want.shape if layout == ft.NCHW else (N, layer.OH, layer.OW, layer.KN), np.float32)
+                got = got if layout == ft.NCHW else to_nchw(got)
+                assert got.tobytes() == want.tobytes(), (layout, fill)
+            ctx.free(d_x)
+    finally:
+        for p in (d_t, d_y, d_ws):
+            ctx.free(p)
+        w.free()
