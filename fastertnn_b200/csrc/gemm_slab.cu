@@ -788,7 +788,7 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
         if (!tnns_quantise_tma_supported(fused->d_x, g.H, g.W, layout))
             return tnns_fail(TNNS_ERR_UNSUPPORTED, "fused quantisation needs NCHW input with H*W a multiple of four and a 16-byte aligned base");
         const unsigned long long HW = (unsigned long long)g.H * g.W;
-        if ((rc = tnns_tensor_map_2d(&map_q, 4, fused->d_x, HW, (unsigned long long)g.N * g.C, HW * 4, Q_PIX, 64))) return rc;
+        if ((rc = tnns_tensor_map_nchw(&map_q, fused->d_x, g.N, g.C, (long long)HW, Q_PIX, 64))) return rc;
         unsigned int* words = nullptr;
         int self_clean = 0;
         if ((rc = tnns_fused_sync_prepare(ctx, g.N, stream, fused->d_sync, &words, &self_clean))) return rc;

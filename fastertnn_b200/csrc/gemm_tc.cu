@@ -1296,13 +1296,13 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
     a.H = g.H; a.W = g.W; a.OW = g.OW; a.Cp = g.Cp; a.SH = g.SH; a.SW = g.SW; a.PH = g.PH; a.PW = g.PW;
     alignas(64) CUtensorMap map_q;
     if (fused) {
-        // the fp32 input as a 2-D tensor: one row of H*W floats per (image, channel); box = 128 pixels x 64 channels
+        // the fp32 input as images x channels x H*W floats; box = 128 pixels x 64 channels of one image
         const unsigned long long HW = (unsigned long long)g.H * g.W;
         // (pixel-major input: one row of C floats per pixel of any image; box = 128 pixels x 32 channels, 128-byte swizzle)
         if (layout == TNNS_NHWC)
             rc = tnns_tensor_map_2d(&map_q, 4, fused->d_x, (unsigned long long)fused->C, (unsigned long long)g.N * HW, (unsigned long long)fused->C * 4, 32, Q_PIX, 128);
         else
-            rc = tnns_tensor_map_2d(&map_q, 4, fused->d_x, HW, (unsigned long long)g.N * fused->C, HW * 4, Q_PIX, 64);
+            rc = tnns_tensor_map_nchw(&map_q, fused->d_x, g.N, fused->C, (long long)HW, Q_PIX, 64);
         if (rc) return rc;
         a.q_nhwc = layout == TNNS_NHWC;
         a.qx = fused->d_x;

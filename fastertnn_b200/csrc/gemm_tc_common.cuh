@@ -265,8 +265,8 @@ __device__ __forceinline__ void store_rows16_at(const float (&f)[32], float* con
 }
 
 // Quantiser role of the fused form, called by the four quantiser warps together (thread = pixel).
-// An item = 128 neighbouring pixels x 64 channels of one image (NCHW, a row of the 2-D tensor
-// (image, channel) x pixels per channel).  The first lane claims items in image order from a
+// An item = 128 neighbouring pixels x 64 channels of one image (NCHW, the tensor images x
+// channels x pixels).  The first lane claims items in image order from a
 // global counter -- so the images the first tiles need are finished first, whichever blocks
 // run -- and requests each as ONE tensor copy into a two-stage ring; every thread then reads its
 // pixel's 64 channels from shared memory (conflict-free), pushes the sign bits of (v + t) and
@@ -327,7 +327,7 @@ __device__ __noinline__ void quantise_items(const QuantArgs p, const CUtensorMap
                 tma_tile2d_g2s(smem_u32(stage0 + s * Q_STAGE), tmap_q, ic * 64, row0, bar_full + 8 * s);
                 tma_tile2d_g2s(smem_u32(stage0 + s * Q_STAGE + Q_STAGE / 2), tmap_q, ic * 64 + 32, row0, bar_full + 8 * s);
             } else {
-                tma_tile2d_g2s(smem_u32(stage0 + s * Q_STAGE), tmap_q, band * Q_PIX, (int)n * p.qC + ic * 64, bar_full + 8 * s);
+                tma_tile3d_g2s(smem_u32(stage0 + s * Q_STAGE), tmap_q, band * Q_PIX, ic * 64, (int)n, bar_full + 8 * s);
             }
         } else {
             mbar_arrive(bar_full + 8 * s);
@@ -378,7 +378,7 @@ __device__ __noinline__ void quantise_items(const QuantArgs p, const CUtensorMap
                 tnns_quantise_row32_swz128<true>(row, nch, t, sg[0], nz[0]);
                 tnns_quantise_row32_swz128<true>(row + Q_STAGE / 2, nch - 32, t, sg[1], nz[1]);
             }
-        } else if (nch == 64 && !p.binary) {
+        } else if (!p.binary) {
 #pragma unroll
             for (int b = 31; b >= 0; b--) {
 #pragma unroll
@@ -388,31 +388,20 @@ __device__ __noinline__ void quantise_items(const QuantArgs p, const CUtensorMap
                     nz[h] = push_sign(nz[h], t - fabsf(v));
                 }
             }
-        } else if (p.binary) {
+        } else {
             // x < t reads -1 (src/tnns/binarize2row_avx2.c:19-21); absent channels are +1: sign 0
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-#pragma unroll 4
-                for (int b = 31; b >= 0; b--) {
-                    if (32 * h + b < nch) sg[h] = push_sign(sg[h], (sp[(32 * h + b) * Q_PIX] + 0.0f) - t);
-                    else sg[h] <<= 1;
-                }
+#pragma unroll 8
+                for (int b = 31; b >= 0; b--) sg[h] = push_sign(sg[h], (sp[(32 * h + b) * Q_PIX] + 0.0f) - t);
                 nz[h] = 0xFFFFFFFFu;  // no zeros in the binary alphabet
             }
-        } else {
+        }
+        if (!p.nhwc && nch < 64) {  // absent channels (zero-filled by the copy): sign 0, ternary non-zero 0
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-#pragma unroll 1
-                for (int b = 31; b >= 0; b--) {
-                    if (32 * h + b < nch) {
-                        const float v = sp[(32 * h + b) * Q_PIX];
-                        sg[h] = push_sign(sg[h], v + t);
-                        nz[h] = push_sign(nz[h], t - fabsf(v));
-                    } else {  // absent channel: sign 0, non-zero 0
-                        sg[h] <<= 1;
-                        nz[h] <<= 1;
-                    }
-                }
+                sg[h] &= tnns_low_bits(nch - 32 * h);
+                if (!p.binary) nz[h] &= tnns_low_bits(nch - 32 * h);
             }
         }
         // every value is in registers: hand the stage back; the issuer refills it at once

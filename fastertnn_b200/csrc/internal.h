@@ -126,6 +126,7 @@ int tnns_launch_dense_quantise(tnns_cuda_ctx* ctx, const float* d_x, const float
 // driver-encoded descriptor of a two-dimensional tensor for the copy engine (128 bytes at `map`)
 int tnns_tensor_map_2d(void* map, int elem_bytes, const void* base, unsigned long long dim0, unsigned long long dim1,
                        unsigned long long stride1_bytes, unsigned box0, unsigned box1, int swizzle_bytes = 0);
+int tnns_tensor_map_nchw(void* map, const void* base, int N, int C, long long HW, unsigned box0, unsigned box1);
 // 4-bit GEMM + PReLU whose activation tiles the copy engine gathers (im2col tensor copies) from
 // an e2m1 image; needs ternary activations and a channel count that fills 128-byte chunks
 bool tnns_im2col_supported(const tnns_cuda_weights* w, const TnnsGeom& g);
@@ -197,31 +198,31 @@ FastDiv tnns_fastdiv(uint32_t d);
 // signbit(v + t); |v| > t <=> signbit(t - |v|); binary v < t <=> signbit(v - t)); channels at or past nch read
 // as absent (sign 0, non-zero 0).  Lanes of a warp = neighbouring pixels: each load instruction spreads over
 // all banks, where a plain [pixel][channel] tile would put every lane on the same one.
+// (Absent channels are masked off at the end: a test per channel would cost every full group as well.)
+__device__ __forceinline__ uint32_t tnns_low_bits(int n) { return n >= 32 ? 0xFFFFFFFFu : n > 0 ? (1u << n) - 1u : 0u; }
 template <bool TERNARY>
 __device__ __forceinline__ void tnns_quantise_row32_swz128(const unsigned char* row, int nch, float t, uint32_t& sg_out, uint32_t& nz_out) {
     const uint32_t x = (static_cast<uint32_t>(__cvta_generic_to_shared(row)) >> 7) & 7u;
     uint32_t sg = 0, nz = 0;
+    if (nch > 0) {
 #pragma unroll
-    for (int c = 7; c >= 0; c--) {
-        const float4 v4 = *reinterpret_cast<const float4*>(row + ((static_cast<uint32_t>(c) ^ x) << 4));
+        for (int c = 7; c >= 0; c--) {
+            const float4 v4 = *reinterpret_cast<const float4*>(row + ((static_cast<uint32_t>(c) ^ x) << 4));
 #pragma unroll
-        for (int e = 3; e >= 0; e--) {
-            const float v = e == 3 ? v4.w : e == 2 ? v4.z : e == 1 ? v4.y : v4.x;
-            if (4 * c + e < nch) {
+            for (int e = 3; e >= 0; e--) {
+                const float v = e == 3 ? v4.w : e == 2 ? v4.z : e == 1 ? v4.y : v4.x;
                 if (TERNARY) {
                     sg = __funnelshift_l(__float_as_uint(v + t), sg, 1);
                     nz = __funnelshift_l(__float_as_uint(t - fabsf(v)), nz, 1);
                 } else {
                     sg = __funnelshift_l(__float_as_uint((v + 0.0f) - t), sg, 1);
                 }
-            } else {
-                sg <<= 1;
-                nz <<= 1;
             }
         }
     }
-    sg_out = sg;
-    nz_out = nz;
+    const uint32_t m = tnns_low_bits(nch);
+    sg_out = sg & m;
+    nz_out = nz & m;
 }
 
 __device__ __forceinline__ void tnns_expand32_f4(uint32_t s, uint32_t z, uint32_t (&w)[4]) {

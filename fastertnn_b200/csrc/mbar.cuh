@@ -78,4 +78,10 @@ __device__ __forceinline__ void tma_tile2d_g2s(uint32_t dst_smem, const void* tm
                  : "memory");
 }
 
+__device__ __forceinline__ void tma_tile3d_g2s(uint32_t dst_smem, const void* tmap, int x, int y, int z, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+                 ::"r"(dst_smem), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(y), "r"(z)
+                 : "memory");
+}
+
 }  // namespace

@@ -2,7 +2,7 @@
 // reference: src/tnns/ternarize2row_avx2.c:438-452, src/tnns/binarize2row_avx2.c:15-22, without
 // the im2row scatter) for NCHW input.
 //
-// The input is read as a two-dimensional tensor: one row per (image, channel) with H*W floats.
+// The input is read as a three-dimensional tensor: images x channels x H*W floats.
 // A persistent block walks work items (image, band of 128 pixels, group of 64 channels); the
 // producer thread requests each item as ONE tensor copy -- a box of 128 pixels x 64 channels,
 // 32 KB -- into a four-deep shared-memory ring, so about 128 KB per SM are in flight towards HBM
@@ -11,6 +11,11 @@
 // consecutive floats), the sign and non-zero bits pushed into the plane words branch-free, the
 // stage handed back, then the pixel's 64 channels stored as one 64-bit word per plane or as
 // 32 bytes of e2m1 operands.  The kernel is bound by HBM traffic: 4 bytes read per input value.
+//
+// A ragged channel group costs no more than a full one: its absent channels are zero-filled by the copy and masked
+// off after the same unrolled 64 reads (a test per channel halved the rate, and as rows of a two-dimensional tensor the
+// box fetched the next image's channels: layer call 62 x 203x72x54 -> 64 1x1 127 -> 61 us, 32 x 96x28x28 -> 96 20.9 ->
+// 12.7, BNN 8 x 3x224x224 -> 64 99 -> 61).
 //
 // NHWC input (NHWC_IN) is the tensor (pixels of all images) x (channels): an item arrives as two
 // copies of 128 pixels x 32 channels, written in the 128-byte swizzle pattern, so that a thread
@@ -104,7 +109,7 @@ quantise_tma_kernel(const __grid_constant__ CUtensorMap tmap, const float* __res
                     tma_tile2d_g2s(smem_u32(smem + s * QSTAGE_BYTES), &tmap, ic * QC, row0, bar_full + 8 * s);
                     tma_tile2d_g2s(smem_u32(smem + s * QSTAGE_BYTES + QSTAGE_BYTES / 2), &tmap, ic * QC + 32, row0, bar_full + 8 * s);
                 } else {
-                    tma_tile2d_g2s(smem_u32(smem + s * QSTAGE_BYTES), &tmap, band * QL, n * C + ic * QC, bar_full + 8 * s);
+                    tma_tile3d_g2s(smem_u32(smem + s * QSTAGE_BYTES), &tmap, band * QL, ic * QC, n, bar_full + 8 * s);
                 }
             }
         }
@@ -150,7 +155,7 @@ quantise_tma_kernel(const __grid_constant__ CUtensorMap tmap, const float* __res
                 const unsigned char* row = smem + s * QSTAGE_BYTES + p * 128;
                 tnns_quantise_row32_swz128<TERNARY>(row, nch, t, sg[0], nz[0]);
                 tnns_quantise_row32_swz128<TERNARY>(row + QSTAGE_BYTES / 2, nch - 32, t, sg[1], nz[1]);
-            } else if (nch == QC) {
+            } else {
 #pragma unroll
                 for (int half = 0; half < 2; half++) {
 #pragma unroll
@@ -163,23 +168,9 @@ quantise_tma_kernel(const __grid_constant__ CUtensorMap tmap, const float* __res
                             sg[half] = push_sign_bit(sg[half], (v + 0.0f) - t);
                         }
                     }
-                }
-            } else {
-#pragma unroll 1
-                for (int c = QC - 1; c >= 0; c--) {
-                    const int half = c >> 5;
-                    if (c < nch) {
-                        const float v = sp[c * QL];
-                        if (TERNARY) {
-                            sg[half] = push_sign_bit(sg[half], v + t);
-                            nz[half] = push_sign_bit(nz[half], t - fabsf(v));
-                        } else {
-                            sg[half] = push_sign_bit(sg[half], (v + 0.0f) - t);
-                        }
-                    } else {  // absent channel: sign 0, non-zero 0
-                        sg[half] <<= 1;
-                        nz[half] <<= 1;
-                    }
+                    // absent channels (zero-filled by the copy): sign 0, non-zero 0
+                    sg[half] &= tnns_low_bits(nch - 32 * half);
+                    nz[half] &= tnns_low_bits(nch - 32 * half);
                 }
             }
             if (!TERNARY) nz[0] = nz[1] = 0xFFFFFFFFu;  // the binary alphabet has no zero; absent channels read +1
@@ -237,7 +228,7 @@ int tnns_launch_quantise_tma(tnns_cuda_ctx* ctx, bool ternary, const float* d_x,
     const int nbands = nhwc ? (int)(((long long)N * HW + QL - 1) / QL) : (HW + QL - 1) / QL;
     alignas(64) CUtensorMap map;
     int rc = nhwc ? tnns_tensor_map_2d(&map, 4, d_x, (unsigned long long)C, (unsigned long long)N * HW, (unsigned long long)C * 4, 32, QL, 128)
-                  : tnns_tensor_map_2d(&map, 4, d_x, (unsigned long long)HW, (unsigned long long)N * C, (unsigned long long)HW * 4, QL, QC);
+                  : tnns_tensor_map_nchw(&map, d_x, N, C, HW, QL, QC);
     if (rc) return rc;
     const long long items = nhwc ? (long long)nbands * Cp : (long long)N * nbands * Cp;
     const int grid = (int)std::min<long long>(items, ctx->sm_count);
