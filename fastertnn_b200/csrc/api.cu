@@ -488,13 +488,14 @@ int tnns_cuda_slab_supported(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* 
 }
 
 // Where the library itself prefers the slab-fed route (tnns_cuda_conv with TNNS_GEMM_AUTO, ConvStack).
-// Measured on B200, quantise + GEMM in us, slab-fed / im2col-fed (or, binary activations, gathering warps):
-//   256 x 64x56x56 -> 64      GEMM alone 55 / 93          256 x 128x28x28 -> 128   55 / 58
-//   1 x 256x56x56 -> 256 BTN  13.1 / 14.0                 64 x 512x32x32 -> 512 BTN  95 / 102
-//   64 x 512x32x32 -> 512     95 / 79 (one launch)        256 x 256x14x14 -> 256   37 / 35
-// The slab removes the per-tap copy requests, which is what bounds 32- and 64-byte pixels, and it is the only
-// copy-engine form of binary activations; on 128-byte pixels the tensor pipe bounds both forms and the padded
-// lattice's extra rows (13 % at 32x32, 31 % at 14x14) decide for the im2col form.
+// The slab removes the per-tap copy requests, which is what bounds 32- and 64-byte pixels on tiles of few kernels; it is
+// paid for with the padded lattice's extra rows (13 % at 32x32, 31 % at 14x14).  Measured on B200, layer call in us,
+// slab-fed / im2col-fed:
+//   251 x 64x32x32 -> 64 3x3    38.6 / 48.5     167 x 128x32x32 -> 64 3x3   38.8 / 46.6
+//   256 x 128x28x28 -> 128 3x3  55 / 58         55 x 512x32x32 -> 64 3x3    48.0 / 44.3
+//   100 x 64x32x32 -> 256 3x3   38.7 / 34.3     83 x 128x32x32 -> 256 3x3   37.8 / 35.0
+//   251 x 64x32x32 -> 64 1x1    34.7 / 35.2     83 x 128x32x32 -> 256 1x1   31.2 / 31.8
+// Binary activations take it at any size (1 x 256x56x56 -> 256 BTN 13.1 against 14.0 gathering).
 int tnns_cuda_slab_preferred(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s) {
     TnnsGeom g;
     if (!ctx || !w || !s || tnns_make_geom(s, &g)) return 0;
@@ -502,7 +503,8 @@ int tnns_cuda_slab_preferred(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* 
     if (!tnns_slab_supported(ctx, w, g, false)) return 0;
     const double useful = (double)g.OH * g.OW / ((double)(g.H + 2 * g.PH) * (g.W + 2 * g.PW));
     if (useful < 0.75) return 0;
-    return (!type_act_ternary(w->type) || g.Cp <= 2) ? 1 : 0;
+    if (!type_act_ternary(w->type)) return 1;
+    return (g.Cp <= 2 && (w->KN <= 128 || g.KH * g.KW == 1)) ? 1 : 0;
 }
 
 // next_format of the public slab entry points -> (format, binary) of the launcher
@@ -665,7 +667,8 @@ int tnns_cuda_conv_auto_algo(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* 
     if (!ctx || !w || !s) return TNNS_GEMM_AUTO;
     if (tnns_cuda_dense_supported(ctx, w, s)) return TNNS_GEMM_F4_DENSE;
     // two launches, whatever the input's layout and alignment (the one-launch form is never preferred)
-    if (tnns_cuda_slab_preferred(ctx, w, s)) return TNNS_GEMM_F4_SLAB;
+    // (pixel-major 1x1 layers: 251 x 64x32x32 -> 64 36.8 us slab-fed, 33.1 im2col-fed)
+    if (tnns_cuda_slab_preferred(ctx, w, s) && !(layout == TNNS_NHWC && type_act_ternary(w->type) && s->KH * s->KW == 1)) return TNNS_GEMM_F4_SLAB;
     if (tnns_cuda_conv_fused_preferred(const_cast<tnns_cuda_ctx*>(ctx), w, s, d_x, layout)) return TNNS_GEMM_F4_FUSED;
     return TNNS_GEMM_F4_TC;
 }
@@ -725,20 +728,26 @@ int tnns_cuda_conv_fused_packed_out(tnns_cuda_ctx* ctx, const tnns_cuda_weights*
                            stream);
 }
 
-// Where the quantise step inside the GEMM launch pays: every SM has at least three 128-row tiles (measured, one launch /
-// two launches in us: 32 images of 512x32x32 -> 512, 3.5 tiles per SM: 49 / 54; 256 x 256x14x14 -> 256, 2.6: 43 / 40;
-// 16 images, 1.7: 33 / 31.5).
-static bool enough_tiles_for_one_launch(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const TnnsGeom& g) {
+// Where the quantise step inside the GEMM launch pays.  Beside the MMAs the quantiser reads the input at about half the
+// rate of the stand-alone kernel, so there must be MMAs to hide it under: multiply time (8.6 POP/s) at least 1.25 x the
+// input's read time (6.5 TB/s), which is KN*KH*KW*OH*OW >= 3300*H*W, and every SM must have at least three 128-row tiles.
+// Measured, one launch / two launches in us: 64 x 512x32x32 -> 512 3x3 (4608 on that scale) 76.8 / 87.5, 32 images (3.5
+// tiles per SM) 48.6 / 51.6; 41 x 512x32x32 -> 256 3x3 (2304) 46.9 / 47.3, NHWC 48.4 / 46.7; 62 x 256x32x32 -> 256 3x3
+// 40.9 / 40.0; 55 x 512x32x32 -> 64 3x3 (576) 50.6 / 44.3; 64 x 512x32x32 -> 512 1x1 (512) 64.0 / 58.7; 100 x 256x32x32
+// -> 64 1x1 43.8 / 32.6; 16 images of the first (1.7 tiles per SM) 33 / 31.5.
+static bool one_launch_pays(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const TnnsGeom& g) {
     const long long M = (long long)g.N * g.OH * g.OW;
     const int bn = tnns_i8_tile_n(w->KN);
-    return ((M + 127) / 128) * ((w->KN + bn - 1) / bn) >= 3LL * ctx->sm_count;
+    const long long tiles = ((M + 127) / 128) * ((w->KN + bn - 1) / bn);
+    const double multiply = (double)w->KN * g.KH * g.KW * g.OH * g.OW, read = (double)g.H * g.W;
+    return tiles >= 3LL * ctx->sm_count && multiply >= 3300.0 * read;
 }
 
 // The rule tnns_cuda_conv applies with TNNS_GEMM_AUTO
 int tnns_cuda_conv_fused_preferred(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s, const float* d_x, int layout) {
     TnnsGeom g;
     if (!ctx || !tnns_cuda_conv_fused_supported(w, s, d_x, layout) || tnns_make_geom(s, &g)) return 0;
-    return enough_tiles_for_one_launch(ctx, w, g) ? 1 : 0;
+    return one_launch_pays(ctx, w, g) ? 1 : 0;
 }
 
 size_t tnns_packed_image_bytes(int ternary, int N, int C, int H, int W) {
@@ -919,6 +928,12 @@ int tnns_cuda_conv_ws(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const floa
         // Measured on B200 against the gathering GEMM that took these layers before (layer call, us): 8 x 320x15x23 -> 320 s2
         // 18.3 / 12.4, 32 x 192x28x28 -> 192 25.1 / 20.1, NHWC 63 x 262x21x20 -> 512 54 / 41, BTN 8 x 256x14x14 -> 256 s2
         // 16.2 / 12.7, BNN 32 x 128x28x28 -> 128 s2 13.6 / 11.2, BNN 16 x 320x28x28 -> 320 27.7 / 24.6
+        if (auto_both && type_act_ternary(w->type) && tnns_fused_supported(wide.w, wide.gv, d_x, layout) && one_launch_pays(ctx, w, g)) {
+            TnnsFusedInput f;
+            f.d_x = d_x; f.d_thr = d_thr; f.C = g.C; f.Cp = g.Cp;
+            f.d_sync = reinterpret_cast<unsigned int*>(static_cast<char*>(d_workspace) + wide.image_bytes);
+            return tnns_launch_gemm_im2col(ctx, wide.w, d_workspace, d_y, wide.gv, alpha, layout, (cudaStream_t)stream, 0, nullptr, nullptr, 1, &f);
+        }
         rc = tnns_launch_quantise(ctx, type_act_ternary(w->type), d_x, d_thr, d_workspace, g.N, g.C, g.H, g.W, layout, (cudaStream_t)stream,
                                   TNNS_IMG_E2M1, wide.PH, wide.PW, wide.gv.Cp);
         if (rc) return rc;

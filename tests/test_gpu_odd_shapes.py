@@ -101,3 +101,25 @@ def test_layers_of_any_channel_count_and_alphabet(layer, N, type_, gpu_ctx, chec
         for p in (d_t, d_y, d_ws):
             ctx.free(p)
         w.free()
+
+
+@pytest.mark.parametrize("layer,N", [(Layer(130, 20, 20, 400, 3, 3, 1, 1), 75), (Layer(192, 24, 24, 368, 3, 3, 1, 1), 52)], ids=lambda v: str(v).replace(" ", ""))
+def test_ragged_channels_in_one_launch(layer, N, gpu_ctx, checker):
+    """Enough tiles for the form that quantises inside the GEMM launch, with pixels padded to whole stage rows."""
+    from cases import threaded_conv
+    case = make_case(TNN, layer, N, 8300, "uniform")
+    wp = checker.pack_weights(True, case.w, case.w_thr)
+    want = threaded_conv(checker, TNN, case.x, case.thr, wp, layer)
+    ctx = gpu_ctx
+    w = ctx.upload_weights(TNN, wp, layer.C, layer.KH, layer.KW)
+    d_t, d_x, d_y = ctx.to_device(case.thr), ctx.to_device(case.x), ctx.malloc(want.nbytes)
+    try:
+        before = ft.api.launch_count()
+        ctx.conv(w, d_x, d_t, d_y, layer.shape(N), case.alpha)
+        assert ft.api.launch_count() - before == 1
+        ctx.sync()
+        assert ctx.to_host(d_y, want.shape, np.float32).tobytes() == want.tobytes()
+    finally:
+        for p in (d_t, d_x, d_y):
+            ctx.free(p)
+        w.free()
