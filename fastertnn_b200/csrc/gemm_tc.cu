@@ -89,7 +89,8 @@ struct TcCfg {
     static constexpr int QSTG = Q_STG, Q_STAGE = 128 * 64 * 4;  // quantiser ring: stages, bytes per stage
     // smem ring depth
     static constexpr int NSTG_QF = (CG == 2) ? 5 : (BN == 256 ? 3 : 4);
-    static constexpr int NSTG = QF ? NSTG_QF : ((CG == 2) ? 6 : ((MT == 1) ? 4 : 3));
+    static constexpr int NSTG_ATMA = CG == 2 ? 6 : (BN == 64 ? 8 : (BN == 128 ? 6 : 4));  // 192 KB whatever the tile
+    static constexpr int NSTG = QF ? NSTG_QF : (ATMA ? NSTG_ATMA : ((MT == 1) ? 4 : 3));
     static constexpr int A_STAGE = MT * A_SUB, B_STAGE = (BN / CG) * KCH;
     static constexpr bool OVL = F4 && MT == 1 && BN == 256;        // overlapping accumulator sets
     static constexpr int NBUF = (OVL || MT * BN <= (F4 ? 128 : 256)) ? 2 : 1;  // accumulator sets in tensor memory
@@ -221,6 +222,7 @@ struct GemmArgs {
     float* y;
     long long M;
     int KN, Kp, OHW, layout;
+    int b_rows;                 // kernels per tile of the weight image: BN, or a multiple of it (tensor-copy form, few tiles)
     int a_two_planes;
     int acc_bias;               // added to the integer dot product (BNN: K_unpack minus the positions multiplied)
     float alpha;
@@ -313,11 +315,11 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int nchunks = F4 ? p.Kp / 4 : p.Kp / 2;  // stages per tile
     const int ntn = (p.KN + BN - 1) / BN;
-    const long long ntm = (p.M + TILE_M - 1) / TILE_M;
-    const long long ntiles = ntm * ntn;
+    const int ntm = (int)((p.M + TILE_M - 1) / TILE_M);
+    const int ntiles = ntm * ntn;  // below 2^31 (checked by the launcher): no 64-bit division per tile
     // a unit = the block (CG = 1) or the block pair (CG = 2) that walks one tile sequence
     const uint32_t rank = (CG == 2) ? cluster_ctarank() : 0u;
-    const long long unit = blockIdx.x / CG, nunits = gridDim.x / CG;
+    const int unit = blockIdx.x / CG, nunits = gridDim.x / CG;
 
     if (p.jtab)
         for (int j = threadIdx.x; j < min(p.Kp, Cfg::TAPMAX); j += blockDim.x) s_taps[j] = __ldg(p.jtab + j);
@@ -379,22 +381,57 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
         tc_fence_after();
     }
 
-    // everything above touched only on-chip state and the layer's constant tables; what follows reads
+    // Stages of the block's first tile whose weight copies are requested before the wait for the launch in front: weights
+    // are constant, so their latency and the descriptors' fetch hide under it; the activation copies of those stages follow
+    // after the wait (from that wait to the first complete stage took 2750 clocks).  32 KB, no more: where the block could
+    // only start when the launch in front left its SM, the first stage's activations queue behind these copies (all
+    // four stages of a 256-kernel tile requested early: 8 x 512x32x32 -> 512 12.9 us against 11.3).
+    constexpr int wpt = 4 / TAPS, SUBA = A_STAGE / TAPS;  // tensor-copy form: plane words and bytes per tap
+    const uint32_t bar_full_lead = (CG == 2) ? mapa_shared(bar_full, 0) : bar_full;  // pair: both blocks' copies report to the first block's barrier
+    constexpr int EARLY = 32768 / B_STAGE < NSTG ? 32768 / B_STAGE : NSTG;
+    const int early = min(EARLY, nchunks);
+    // tile n_tile of BN kernels is rows [n_tile*BN % b_rows, +BN) of an image tile of b_rows kernels: one contiguous piece per stage
+    const size_t b_step = (size_t)p.b_rows * KCH;
+    auto weights_of = [&](int n_tile) {
+        const uint32_t k0 = (uint32_t)n_tile * BN, big = k0 / (uint32_t)p.b_rows;
+        return p.Bimg + (size_t)big * nchunks * b_step + (size_t)(k0 - big * p.b_rows) * KCH;
+    };
+    if (ATMA && warp == WARP_TMA && lane == 0) {
+        prefetch_tensor_map(&tmap_a);
+        if (CG == 2) prefetch_tensor_map(&tmap_b);
+        if (unit < ntiles) {
+            const int n_tile = unit % ntn;
+            const unsigned char* src = weights_of(n_tile);
+            for (int c = 0; c < early; c++) {
+                int a_bytes = 0;
+#pragma unroll
+                for (int q = 0; q < TAPS; q++)
+                    if (tap_at(4 * c + q * wpt) != 0xFFFFFFFFu) a_bytes += SUBA;
+                if (CG == 2) {
+                    if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * c, CG * (B_STAGE + a_bytes));
+                    tma_tile2d_g2s_pair(smem_u32(sB + c * B_STAGE), &tmap_b, 0, (n_tile * nchunks + c) * BN + (int)rank * (BN / CG), bar_full_lead + 8 * c);
+                } else {
+                    mbar_arrive_expect_tx(bar_full + 8 * c, B_STAGE + a_bytes);
+                    bulk_g2s(smem_u32(sB + c * B_STAGE), src + (size_t)c * b_step, B_STAGE, bar_full + 8 * c);
+                }
+            }
+        }
+    }
+
+    // everything above touched only on-chip state and the layer's constant tables and weights; what follows reads
     // and writes tensors that the previous launch on the stream may still be working on
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     if (warp == WARP_TMA) {
         if (lane == 0) {
             uint32_t s = 0, ph = 1;  // ring slot and the parity its "empty" barrier is waited with
-            // pair: both blocks' copies report to the first block's barrier
-            const uint32_t bar_full_lead = (CG == 2) ? mapa_shared(bar_full, 0) : bar_full;
-            for (long long t = unit; t < ntiles; t += nunits) {
-                const int n_tile = (int)(t % ntn);
-                const unsigned char* src = p.Bimg + (size_t)n_tile * nchunks * B_STAGE;
+            for (int t = unit; t < ntiles; t += nunits) {
+                const int n_tile = t % ntn;
+                const unsigned char* src = weights_of(n_tile);
                 // tensor-copy activations: base pixel of the block's first output pixel
                 int a_n = 0, a_h = 0, a_w = 0;
                 if (ATMA) {
-                    long long row0 = (t / ntn) * TILE_M + (long long)rank * BMT;
+                    long long row0 = (long long)(t / ntn) * TILE_M + (int)rank * BMT;
                     if (row0 >= p.M) row0 = 0;  // second block of a pair past the last row: any valid pixels, never stored
                     // 32-bit divisions where the row index allows it (64-bit ones cost this thread hundreds of cycles per tile)
                     a_n = row0 < 0x7FFFFFFFLL ? (int)((uint32_t)row0 / (uint32_t)p.OHW) : (int)(row0 / p.OHW);
@@ -406,7 +443,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                         // the copies of this tile read the images of its rows: wait until the
                         // quantiser warps (of any block) have finished them
                         const long long last = min(row0 + BMT, p.M) - 1;
-                        const int n_last = (int)(last / p.OHW);
+                        const int n_last = last < 0x7FFFFFFFLL ? (int)((uint32_t)last / (uint32_t)p.OHW) : (int)(last / p.OHW);
                         const unsigned int per_image = (unsigned int)(p.q_nbands * p.q_cp) * 4u;  // every quantiser warp counts itself
                         for (int n = a_n; n <= n_last; n++)
                             if (!counter_wait(p.q_sync + Q_FLAG0 + n, per_image, abort_flag, p.status, 6)) goto done;
@@ -414,7 +451,27 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                         asm volatile("fence.proxy.async.global;" ::: "memory");
                     }
                 }
-                for (int c = 0; c < nchunks; c++, s = (s + 1 == NSTG) ? 0 : s + 1, ph ^= (s == 0)) {
+                int c = 0;
+                if (ATMA && t == unit) {
+                    // the stages whose weights were requested before the wait: activations only
+                    for (; c < early; c++) {
+#pragma unroll
+                        for (int q = 0; q < TAPS; q++) {
+                            const uint32_t tap = tap_at(4 * c + q * wpt);
+                            if (tap == 0xFFFFFFFFu) continue;
+                            const uint32_t dst = smem_u32(sA + c * A_STAGE + q * SUBA);
+                            if (CG == 2)
+                                tma_im2col_g2s_pair(dst, &tmap_a, (int)(tap & 0xFFFF) * 32, a_w, a_h, a_n, (unsigned short)((tap >> 16) & 0xFF),
+                                                    (unsigned short)(tap >> 24), bar_full_lead + 8 * c);
+                            else
+                                tma_im2col_g2s(dst, &tmap_a, (int)(tap & 0xFFFF) * 32, a_w, a_h, a_n, (unsigned short)((tap >> 16) & 0xFF),
+                                               (unsigned short)(tap >> 24), bar_full + 8 * c);
+                        }
+                    }
+                    s = early == NSTG ? 0u : (uint32_t)early;
+                    ph = early == NSTG ? 0u : 1u;
+                }
+                for (; c < nchunks; c++, s = (s + 1 == NSTG) ? 0 : s + 1, ph ^= (s == 0)) {
                     if (!mbar_wait(bar_empty + 8 * s, ph, abort_flag, p.status, 1)) goto done;
                     // tensor-copy activations: the stage's four plane words are TAPS filter taps
                     // (TAPS: one tap of 256 channels, two of 128 or four of 64), one copy and one sub-tile
@@ -422,12 +479,11 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                     // it held (any nibble is a finite e2m1 value) and meets zero weights
                     uint32_t tap[4];
                     int a_bytes = 0;
-                    constexpr int wpt = 4 / TAPS, sub = A_STAGE / TAPS;  // plane words and bytes per tap
                     if (ATMA) {
 #pragma unroll
                         for (int q = 0; q < TAPS; q++) {
                             tap[q] = tap_at(4 * c + q * wpt);
-                            if (tap[q] != 0xFFFFFFFFu) a_bytes += sub;
+                            if (tap[q] != 0xFFFFFFFFu) a_bytes += SUBA;
                         }
                     }
                     if (CG == 2) {
@@ -437,17 +493,17 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
 #pragma unroll
                         for (int q = 0; q < TAPS; q++)
                             if (tap[q] != 0xFFFFFFFFu)
-                                tma_im2col_g2s_pair(smem_u32(sA + s * A_STAGE + q * sub), &tmap_a, (int)(tap[q] & 0xFFFF) * 32, a_w, a_h, a_n,
+                                tma_im2col_g2s_pair(smem_u32(sA + s * A_STAGE + q * SUBA), &tmap_a, (int)(tap[q] & 0xFFFF) * 32, a_w, a_h, a_n,
                                                     (unsigned short)((tap[q] >> 16) & 0xFF), (unsigned short)(tap[q] >> 24), bar_full_lead + 8 * s);
                         continue;
                     }
                     mbar_arrive_expect_tx(bar_full + 8 * s, B_STAGE + a_bytes);
-                    bulk_g2s(smem_u32(sB + s * B_STAGE), src + (size_t)c * B_STAGE, B_STAGE, bar_full + 8 * s);
+                    bulk_g2s(smem_u32(sB + s * B_STAGE), src + (size_t)c * b_step, B_STAGE, bar_full + 8 * s);
                     if (ATMA) {
 #pragma unroll
                         for (int q = 0; q < TAPS; q++)
                             if (tap[q] != 0xFFFFFFFFu)
-                                tma_im2col_g2s(smem_u32(sA + s * A_STAGE + q * sub), &tmap_a, (int)(tap[q] & 0xFFFF) * 32, a_w, a_h, a_n,
+                                tma_im2col_g2s(smem_u32(sA + s * A_STAGE + q * SUBA), &tmap_a, (int)(tap[q] & 0xFFFF) * 32, a_w, a_h, a_n,
                                                (unsigned short)((tap[q] >> 16) & 0xFF), (unsigned short)(tap[q] >> 24), bar_full + 8 * s);
                     }
                 }
@@ -469,7 +525,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
             const uint32_t a_lo0 = (uint32_t)da0, a_hi = (uint32_t)(da0 >> 32), b_lo0 = (uint32_t)db0, b_hi = (uint32_t)(db0 >> 32);
             const uint32_t sfa = tmem_base + SF_COL, sfb = tmem_base + SF_COL + 16;
             uint32_t a_lo = a_lo0, b_lo = b_lo0;                // descriptors of ring slot s
-            for (long long t = unit; t < ntiles; t += nunits, lt++) {
+            for (int t = unit; t < ntiles; t += nunits, lt++) {
                 const int buf = lt % NBUF;
                 // overlapping sets: one barrier, completed once per tile when the columns shared
                 // with the previous tile's set have been drained; otherwise one barrier per set
@@ -518,12 +574,12 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
         constexpr int RW = F4 ? 2 : 1;  // uint4 per plane and stage
         uint4 ring_s[PF][RW], ring_z[PF][RW];
         // prefetch cursor: (tile, chunk) of the next load of this group
-        long long pf_t = blockIdx.x;
+        int pf_t = blockIdx.x;  // may run past ntiles by one grid
         int pf_c = grp;
         while (pf_c >= nchunks) { pf_c -= nchunks; pf_t += gridDim.x; }
         // implicit im2row: window origin of this thread's row in the prefetch cursor's tile
         int im_n = 0, im_ih0 = 0, im_iw0 = 0;
-        long long im_tile = -1;
+        int im_tile = -1;
         const size_t img_plane = (size_t)p.H * p.W * p.Cp;  // words per image and plane
         const int img_planes = p.a_two_planes ? 2 : 1;
         auto fetch = [&](uint4 (&ds)[RW], uint4 (&dz)[RW]) {
@@ -531,7 +587,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                 if (F4 && p.img) {
                     if (im_tile != pf_t) {
                         im_tile = pf_t;
-                        const long long row = min((pf_t / ntn) * BMT + r, p.M - 1);
+                        const long long row = min((long long)(pf_t / ntn) * BMT + r, p.M - 1);
                         const long long n_img = row / p.OHW;
                         const int rem = (int)(row - n_img * p.OHW);
                         const int oh = rem / p.OW;
@@ -582,7 +638,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                     while (pf_c >= nchunks) { pf_c -= nchunks; pf_t += gridDim.x; }
                     return;
                 }
-                const uint4* rowp = p.A + (size_t)min((pf_t / ntn) * BMT + r, p.M - 1) * pitch;
+                const uint4* rowp = p.A + (size_t)min((long long)(pf_t / ntn) * BMT + r, p.M - 1) * pitch;
                 if (F4) {
                     const uint4* row = rowp + (size_t)pf_c * gsz;
 #pragma unroll
@@ -652,14 +708,14 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
         const bool rows16 = F4 && p.pimg == nullptr && p.layout == TNNS_NHWC && (p.KN & 1) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
         tnns_thr::Pair qt = {0.f, 0.f};
         long long qt_img = -1;
-        for (long long t = unit; t < ntiles; t += nunits, lt++) {
+        for (int t = unit; t < ntiles; t += nunits, lt++) {
             const int buf = lt % NBUF;
-            const long long m0 = (t / ntn) * TILE_M + (long long)rank * BMT + sub * BM;
-            const int n0 = (int)(t % ntn) * BN;
+            const long long m0 = (long long)(t / ntn) * TILE_M + (int)rank * BMT + sub * BM;
+            const int n0 = (t % ntn) * BN;
             // the row's image (a 64-bit division) and threshold: worked out while the tile's MMAs run
             const long long row = m0 + q * 32 + lane;
             const bool row_ok = row < p.M;
-            const long long n_img = row_ok ? row / p.OHW : 0;
+            const long long n_img = !row_ok ? 0 : row < 0x7FFFFFFFLL ? (long long)((uint32_t)row / (uint32_t)p.OHW) : row / p.OHW;
             const int rem = (int)(row - n_img * p.OHW);
             float* ybase = (p.layout == TNNS_NHWC) ? p.y + (size_t)row * p.KN : p.y + (size_t)n_img * p.KN * p.OHW + rem;
             const float tq = (p.pimg && row_ok) ? __ldg(p.thr_next + n_img) + 0.0f : 0.f;  // + 0.0f: -0 acts as +0
@@ -943,6 +999,7 @@ int launch_cfg(tnns_cuda_ctx* ctx, const GemmArgs& a, cudaStream_t stream, const
         smem_set[ctx->device & 63] = true;
     }
     const long long tiles = ((a.M + CG * MT * BM - 1) / (CG * MT * BM)) * ((a.KN + BN - 1) / BN);
+    if (tiles >= 0x7FFFFFFFLL) return tnns_fail(TNNS_ERR_UNSUPPORTED, "too many output tiles");
     // the launch may be scheduled while its predecessor on the stream drains (the kernel
     // waits for it, griddepcontrol.wait, before it touches global data)
     cudaLaunchAttribute attr[2];
@@ -1092,6 +1149,7 @@ int tnns_launch_gemm_tc(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const vo
     a.M = M;
     a.KN = w->KN;
     a.Kp = w->Kp;
+    a.b_rows = tnns_i8_tile_n(w->KN);
     a.OHW = OHW;
     // one output pixel per image (fully connected layers): both layouts are the same memory, and the pixel-major
     // epilogue writes 16 bytes per lane where the channel-major one would write 4 (rows are KN floats apart either way)
@@ -1197,6 +1255,21 @@ int encode_weight_map(CUtensorMap* map, const tnns_cuda_weights* w, int BN) {
 }
 }  // namespace
 
+namespace {
+// Kernels per tile of the tensor-copy form on single blocks: the weight image's own tile, or the narrowest part of it whose
+// tiles still fit the chip in one wave.  Clocks stamped in the kernel for a tile of 64 / 128 / 256 kernels: a stage 340 /
+// 375 / 567 (its four MMAs, or its bytes at the 86 per clock that reach an SM), the drain of the finished accumulator 1250
+// per 64 kernels (an SM stores about 30 bytes per clock).  Both lie in series when an SM has one tile.  Where there is more
+// than one wave they overlap and a narrower tile only repeats the activation copies (256 x 64x56x56 -> 128 s2: 30 us with
+// tiles of 128, 47 with 64).  GEMM alone, widest / rule: 1 x 256x56x56 -> 256 8.3 / 6.4 us, FC 1024x4096x1024 10.2 / 8.2.
+int tile_n_for(int sm_count, long long M, int KN, int widest) {
+    const long long mt = (M + BM - 1) / BM;
+    int bn = widest;
+    while (bn > 64 && mt * ((KN + bn / 2 - 1) / (bn / 2)) <= sm_count) bn /= 2;
+    return bn;
+}
+}  // namespace
+
 // pairs: 0 = decide by size, 1 = single blocks, 2 = block pairs (kernel tile of 256 only)
 size_t tnns_fused_sync_bytes(int N) { return ((size_t)(Q_FLAG0 + N) * sizeof(unsigned int) + 127) & ~(size_t)127; }
 
@@ -1268,6 +1341,7 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
     a.M = M;
     a.KN = w->KN;
     a.Kp = w->Kp;
+    a.b_rows = tnns_i8_tile_n(w->KN);
     a.OHW = g.OH * g.OW;
     a.layout = a.OHW == 1 ? TNNS_NHWC : layout;  // one pixel per image: same memory, wider stores (see above)
     a.a_two_planes = 1;
@@ -1316,11 +1390,12 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
         a.q_nbands = (g.H * g.W + Q_PIX - 1) / Q_PIX;
     }
     const int taps = g.Cp == 1 ? 4 : (g.Cp == 2 ? 2 : 1);
-    const int bn = tnns_i8_tile_n(w->KN);
+    int bn = tnns_i8_tile_n(w->KN);
     if (pairs == 2 && bn != 256) return tnns_fail(TNNS_ERR_UNSUPPORTED, "block pairs need more than 128 kernels");
     // Block pairs once there are enough 256-row tiles to occupy every SM pair.
     const long long pair_tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((w->KN + bn - 1) / bn);
     const bool use_pairs = bn == 256 && (pairs == 2 || (pairs == 0 && pair_tiles >= ctx->sm_count / 2));
+    if (!use_pairs && !fused) bn = tile_n_for(ctx->sm_count, M, w->KN, bn);
     CUtensorMap map_b;
     if (use_pairs && (rc = encode_weight_map(&map_b, w, bn))) return rc;
     auto go = [&](auto taps_c) -> int {

@@ -20,6 +20,9 @@ constexpr int Q_PIX = 128;    // pixels per quantise item = quantiser threads pe
 constexpr int Q_STG = 2;      // stages of the quantiser warps' ring
 constexpr int Q_PUBN = 8;     // items the quantiser warps may be ahead of the publisher
 
+__device__ __forceinline__ void prefetch_tensor_map(const void* tmap) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
+}
 __device__ __forceinline__ void bulk_g2s(uint32_t dst_smem, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_smem), "l"(src),
                  "r"(bytes), "r"(bar)
