@@ -43,6 +43,7 @@ struct SlabArgs {
     float* y;
     int Mv;                     // virtual rows: N * Hp * Wp
     int KN, nchunks;            // kernels, weight stages per kernel tile
+    int b_rows;                 // kernels per tile of the weight image: BN, or a multiple of it (few tiles)
     int OH, OW, Wp, HpWp;       // output size, padded input lattice
     int KW, T;                  // filter width, taps KH*KW
     int G;                      // 128-byte channel groups per pixel (one slab each); 1 for 64 / 128 channels
@@ -73,13 +74,18 @@ struct SlabCfg {
     static constexpr int B_STAGE = (BN / CG) * KCH;   // bytes of a weight stage in one block
     static constexpr bool OVL = BN == 256;            // overlapping accumulator sets (scales leave 480 columns)
     static constexpr int ACC_OFF = OVL ? BN - 32 : BN;
-    static constexpr int EPW = 2;                     // epilogue warps per lane quadrant
-    static constexpr int WARP_EPI0 = 2, WARP_Q0 = 2 + 4 * EPW;
-    // Two separate accumulator sets and single blocks: a second warp issues the MMAs of every other tile, so that one
-    // issuer's barrier waits and descriptor arithmetic run under the other's MMAs (see the MMA role).
-    static constexpr bool DUAL = !OVL && CG == 1;
-    static constexpr int WARP_MMA2 = 2 + 4 * EPW + (QF ? 5 : 0);
-    static constexpr int NTHREADS = 32 * (2 + 4 * EPW + (QF ? 5 : 0) + (DUAL ? 1 : 0));
+    static constexpr int NBUF = OVL ? 2 : (BN == 64 ? 4 : 3);  // accumulator sets in tensor memory
+    // Epilogue warps: EPW per lane quadrant share a tile's columns, and NSETS such groups take the tiles in turn.  On tiles of
+    // 64 / 128 kernels a tile's drain is a chain of latencies (barrier, row addresses, tensor-memory load, 32 columns of
+    // arithmetic) several times as long as its MMAs, so three tiles are drained at once.  Eight warps on one tile / two sets /
+    // three sets, inside the 11-layer stack: 64 -> 64 @56 48.3 / 39.8 / 33.0 us, 128 -> 128 @28 25.9 / 22.1 / 19.4; four
+    // sets of the 64-kernel form gained nothing more.
+    static constexpr int EPW = OVL ? 2 : 1, NSETS = OVL ? 1 : (QF ? 2 : 3);
+    // (a set's next tile waits for its barrier's phase by parity: the phase before must be complete by then)
+    static_assert(NSETS <= NBUF, "a set may not be a whole turn of the accumulators ahead");
+    static constexpr int NEPI = 4 * EPW * NSETS;      // epilogue warps
+    static constexpr int WARP_EPI0 = 2, WARP_Q0 = 2 + NEPI;
+    static constexpr int NTHREADS = 32 * (2 + NEPI + (QF ? 5 : 0));
     static constexpr int Q_STAGE = Q_PIX * 64 * 4;
     static constexpr int SMEM_MAX = 232448;
 };
@@ -91,6 +97,8 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
     using Cfg = SlabCfg<BN, CG, TAPS, QF>;
     constexpr int RB = Cfg::RB, B_STAGE = Cfg::B_STAGE, WARP_EPI0 = Cfg::WARP_EPI0, EPW = Cfg::EPW, ACC_OFF = Cfg::ACC_OFF;
     constexpr bool OVL = Cfg::OVL;
+    constexpr int NBUF = Cfg::NBUF, NSETS = Cfg::NSETS;
+    static_assert((2 * SL_MAXSLAB + 2 * SL_MAXSTG + 2 * NBUF) * 8 + 8 <= SL_BAR_BYTES, "barriers");
     constexpr int TILE_M = CG * BM;
     // e2m1 A and B (1<<7, 1<<10), ue8m0 scales (1<<23), K-major, N>>3 at bit 17, M>>4 at bit 24
     constexpr uint32_t IDESC = (1u << 23) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)((CG * BM) >> 4) << 24);
@@ -102,8 +110,8 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
     uint64_t* bars = reinterpret_cast<uint64_t*>(sB + p.nstg * B_STAGE);
     const uint32_t bar_sfull = smem_u32(bars), bar_sempty = smem_u32(bars + SL_MAXSLAB), bar_bfull = smem_u32(bars + 2 * SL_MAXSLAB),
                    bar_bempty = smem_u32(bars + 2 * SL_MAXSLAB + SL_MAXSTG), bar_tfull = smem_u32(bars + 2 * SL_MAXSLAB + 2 * SL_MAXSTG),
-                   bar_tempty = smem_u32(bars + 2 * SL_MAXSLAB + 2 * SL_MAXSTG + 2);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * SL_MAXSLAB + 2 * SL_MAXSTG + 4);
+                   bar_tempty = smem_u32(bars + 2 * SL_MAXSLAB + 2 * SL_MAXSTG + NBUF);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * SL_MAXSLAB + 2 * SL_MAXSTG + 2 * NBUF);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     unsigned char* q_ring = reinterpret_cast<unsigned char*>(bars) + SL_BAR_BYTES;
 
@@ -125,7 +133,7 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
             mbar_init(bar_bfull + 8 * s, 1);
             mbar_init(bar_bempty + 8 * s, 1);
         }
-        for (int b = 0; b < 2; b++) {
+        for (int b = 0; b < NBUF; b++) {
             mbar_init(bar_tfull + 8 * b, 1);
             mbar_init(bar_tempty + 8 * b, CG * 4 * EPW);
         }
@@ -171,6 +179,28 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
     if (CG == 2) cluster_sync_all(); else __syncthreads();
     tc_fence_after();
 
+    // weight stage c of kernel tile n_tile -> ring slot; a tile is rows [n_tile*BN % b_rows, +BN) of an image tile of b_rows kernels
+    const uint32_t bfull_lead = (CG == 2) ? mapa_shared(bar_bfull, 0) : bar_bfull;
+    auto request_weights = [&](int n_tile, int c, uint32_t slot) {
+        if (CG == 2) {
+            if (rank == 0) mbar_arrive_expect_tx(bar_bfull + 8 * slot, CG * B_STAGE);
+            tma_tile2d_g2s_pair(smem_u32(sB + slot * B_STAGE), &tmap_b, 0, (n_tile * p.nchunks + c) * BN + (int)rank * (BN / CG), bfull_lead + 8 * slot);
+        } else {
+            const int k0 = n_tile * BN, big = k0 / p.b_rows;
+            mbar_arrive_expect_tx(bar_bfull + 8 * slot, B_STAGE);
+            bulk_g2s(smem_u32(sB + slot * B_STAGE), p.Bimg + ((size_t)(big * p.nchunks + c) * p.b_rows + (k0 - big * p.b_rows)) * KCH, B_STAGE, bar_bfull + 8 * slot);
+        }
+    };
+    // the first stages of the block's first tile, before the wait for the launch in front (32 KB of constant weights; see gemm_tc.cu)
+    const int early = min(min(32768 / B_STAGE, p.nstg), SPG);
+    if (warp == WARP_TMA && lane == 0 && unit < ntiles) {
+        prefetch_tensor_map(&tmap_a);
+        for (int j = 0; j < early; j++) {
+            const int c = (TAPS == 1) ? j * p.G : j;
+            request_weights(unit % ntn, c, p.b_resident ? (uint32_t)c : (uint32_t)j);
+        }
+    }
+
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     if (warp == WARP_TMA) {
@@ -178,7 +208,6 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
             uint32_t sl = 0, slph = 1, s = 0, ph = 1;
             bool first_tile = true;
             const uint32_t sfull_lead = (CG == 2) ? mapa_shared(bar_sfull, 0) : bar_sfull;
-            const uint32_t bfull_lead = (CG == 2) ? mapa_shared(bar_bfull, 0) : bar_bfull;
             const uint32_t copy_bytes = (uint32_t)(p.ncopies * p.copy_rows * RB);
             for (int t = unit; t < ntiles; t += nunits, first_tile = false) {
                 const int n_tile = t % ntn;
@@ -210,27 +239,22 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
                     for (int j = 0; j < SPG; j++) {
                         const int c = (TAPS == 1) ? j * p.G + cg : j;
                         const uint32_t slot = p.b_resident ? (uint32_t)c : s;
-                        if (!p.b_resident && !mbar_wait(bar_bempty + 8 * slot, ph, abort_flag, p.status, 1)) goto done;
-                        if (CG == 2) {
-                            if (rank == 0) mbar_arrive_expect_tx(bar_bfull + 8 * slot, CG * B_STAGE);
-                            tma_tile2d_g2s_pair(smem_u32(sB + slot * B_STAGE), &tmap_b, 0, (n_tile * p.nchunks + c) * BN + (int)rank * (BN / CG),
-                                                bfull_lead + 8 * slot);
-                        } else {
-                            mbar_arrive_expect_tx(bar_bfull + 8 * slot, B_STAGE);
-                            bulk_g2s(smem_u32(sB + slot * B_STAGE), p.Bimg + ((size_t)n_tile * p.nchunks + c) * B_STAGE, B_STAGE, bar_bfull + 8 * slot);
+                        if (!(first_tile && cg == 0 && j < early)) {
+                            if (!p.b_resident && !mbar_wait(bar_bempty + 8 * slot, ph, abort_flag, p.status, 1)) goto done;
+                            request_weights(n_tile, c, slot);
                         }
                         if (!p.b_resident && ++s == (uint32_t)p.nstg) { s = 0; ph ^= 1; }
                     }
                 }
             }
         }
-    } else if (warp == WARP_MMA || (Cfg::DUAL && warp == Cfg::WARP_MMA2)) {
-        if (lane == 0 && rank == 0) {  // pair: the first block issues for both
-            // This one thread's instruction stream paces the tensor pipe.  Two things measured on this loop:
-            // nothing that touches shared memory may stand between two MMAs (a table look-up per tap, queued
-            // behind the MMAs just issued, cost 60 clocks per MMA: tap offsets are running counters), and the
-            // MMAs of a tile must sit in ONE divergent region (issued one by one from `if (leader)` branches of
-            // a warp-wide loop, every reconvergence waited for the MMA before it: three times slower).
+    } else if (warp == WARP_MMA) {
+        if (rank == 0) {  // pair: the first block issues for both
+            // This warp's instruction stream paces the tensor pipe: it runs warp-uniform (see elect_one), nothing that
+            // touches shared memory stands between two MMAs of a slab (a table look-up per tap, queued behind the MMAs just
+            // issued, cost 60 clocks per MMA: tap offsets are registers or running counters), and a slab's MMAs sit in as few
+            // elected regions as the weight waits allow (one by one, every reconvergence waited for the MMA before it).
+            const bool elected = elect_one();
             uint32_t lt = 0, sl = 0, slph = 0, s = 0, ph = 0;
             bool first_tile = true;
             const uint64_t da0 = make_desc_taps(smem_u32(sA), TAPS), db0 = make_desc(smem_u32(sB));
@@ -238,76 +262,67 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
             const uint32_t row16 = (uint32_t)(p.Wp * (RB / 16));  // one image row further down the slab, in descriptor units
             const uint32_t a_lo0 = (uint32_t)da0, a_hi = (uint32_t)(da0 >> 32), b_lo0 = (uint32_t)db0, b_hi = (uint32_t)(db0 >> 32);
             const uint32_t sfa = tmem_base + SF_COL, sfb = tmem_base + SF_COL + 16;
+            auto mma = [&](uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t acc) {
+                if (CG == 2) tc_mma_f4_pair_lh(d_tmem, a_lo, a_hi, b_lo, b_hi, IDESC, sfa, sfb, acc);
+                else tc_mma_f4_lh(d_tmem, a_lo, a_hi, b_lo, b_hi, IDESC, sfa, sfb, acc);
+            };
+            auto commit = [&](uint32_t bar) {
+                if (CG == 2) tc_commit_pair(bar); else tc_commit(bar);
+            };
             const bool fast3x3 = p.T == 9 && p.KW == 3;
-            if (warp != WARP_MMA && !fast3x3) goto done;  // the generic loop has one issuer
             if (fast3x3) {
-                // 3x3 filters: the nine tap offsets live in registers and every MMA of a slab is issued from straight-line
-                // code -- one 32-bit add per operand and MMA.  (The generic loop below spends a dozen dependent
-                // instructions between two MMAs; with the epilogue warps competing for the same scheduler that cost
-                // 250 clocks per MMA on 64-kernel tiles against 85 for the instruction alone.)
-                //
-                // Two issuers (DUAL): this thread takes every other tile of the block's sequence -- its accumulator set is
-                // always the same one -- and steps its ring positions over the other issuer's tiles.  Measured on
-                // 256 x 64x56x56 -> 64 with one issuer: 1560 clocks per tile of which 550 were this thread's two barrier
-                // waits with the tensor pipe idle, and 1010 the issue of nine MMAs that execute in 770.
+                // 3x3 filters: the nine tap offsets live in registers and the MMAs of a slab (or, where weights stream, of a
+                // stage) are straight-line code -- one 32-bit add per operand and MMA
                 uint32_t aoff[9];
 #pragma unroll
                 for (int j = 0; j < 9; j++) aoff[j] = (uint32_t)((j / 3) * p.Wp + (j % 3)) * (RB / 16);
                 constexpr int KPT = 4 / TAPS;               // K steps (32 bytes) per tap: 1, 2 or 4
-                constexpr int NISSUE = Cfg::DUAL ? 2 : 1;
-                const int me = (warp == WARP_MMA) ? 0 : 1;
-                const int stages_per_tile = p.G * ((9 * KPT + 3) / 4);
-                auto skip_tile = [&]() {  // ring positions over a tile the other issuer takes
-                    for (int i = 0; i < p.G; i++)
-                        if (++sl == (uint32_t)p.nslab) { sl = 0; slph ^= 1; }
-                    if (!p.b_resident)
-                        for (int i = 0; i < stages_per_tile; i++)
-                            if (++s == (uint32_t)p.nstg) { s = 0; ph ^= 1; }
-                };
-                if (me == 1) { skip_tile(); lt = 1; }
-                for (int t = unit + me * nunits; t < ntiles; t += NISSUE * nunits, lt += NISSUE, first_tile = false) {
-                    const int buf = lt & 1;
-                    if (!mbar_wait(OVL ? bar_tempty : bar_tempty + 8 * buf, (OVL ? (lt & 1) : ((lt >> 1) & 1)) ^ 1, abort_flag, p.status, 2)) goto done;
+                constexpr int NK = 9 * KPT, NST = (NK + 3) / 4;  // K steps and weight stages of a slab
+                for (int t = unit; t < ntiles; t += nunits, lt++, first_tile = false) {
+                    const int buf = (int)(lt % NBUF);
+                    if (!mbar_wait(OVL ? bar_tempty : bar_tempty + 8 * buf, (OVL ? (lt & 1) : ((lt / NBUF) & 1)) ^ 1, abort_flag, p.status, 2)) goto done;
                     tc_fence_after();
                     const uint32_t d_tmem = tmem_base + buf * ACC_OFF;
-                    uint32_t acc = 0;
                     for (int cg = 0; cg < p.G; cg++) {
                         if (!mbar_wait(bar_sfull + 8 * sl, slph, abort_flag, p.status, 0x13)) goto done;
-                        tc_fence_after();
                         const uint32_t slab_lo = a_lo0 + sl * slab16;
-                        uint32_t b_lo = 0;
+                        if (p.b_resident) {
+                            if (first_tile)
+                                for (int j = 0; j < NST; j++)
+                                    if (!mbar_wait(bar_bfull + 8 * ((TAPS == 1) ? j * p.G + cg : j), 0u, abort_flag, p.status, 3)) goto done;
+                            tc_fence_after();
+                            if (elected) {
 #pragma unroll
-                        for (int q = 0; q < 9 * KPT; q++) {   // K step q: tap q / KPT, stage q / 4
-                            const int k = q & 3;
-                            if (k == 0) {
-                                const int j = q >> 2;
-                                const int c = (TAPS == 1) ? j * p.G + cg : j;
-                                const uint32_t slot = p.b_resident ? (uint32_t)c : s;
-                                if (!p.b_resident || first_tile) {
-                                    if (!mbar_wait(bar_bfull + 8 * slot, p.b_resident ? 0u : ph, abort_flag, p.status, 3)) goto done;
-                                    tc_fence_after();
+                                for (int q = 0; q < NK; q++) {   // K step q: tap q / KPT, stage q / 4
+                                    const uint32_t slot = (TAPS == 1) ? (uint32_t)((q >> 2) * p.G + cg) : (uint32_t)(q >> 2);
+                                    mma(d_tmem, slab_lo + aoff[q / KPT] + 2u * (uint32_t)(q % KPT), b_lo0 + slot * (uint32_t)(B_STAGE >> 4) + 2u * (q & 3), (uint32_t)(cg | q));
                                 }
-                                b_lo = b_lo0 + slot * (uint32_t)(B_STAGE >> 4);
+                                commit(bar_sempty + 8 * sl);
                             }
-                            const uint32_t a_lo = slab_lo + aoff[q / KPT] + 2u * (uint32_t)(q % KPT);
-                            if (CG == 2) tc_mma_f4_pair_lh(d_tmem, a_lo, a_hi, b_lo + 2u * k, b_hi, IDESC, sfa, sfb, acc);
-                            else tc_mma_f4_lh(d_tmem, a_lo, a_hi, b_lo + 2u * k, b_hi, IDESC, sfa, sfb, acc);
-                            acc = 1;
-                            if ((k == 3 || q == 9 * KPT - 1) && !p.b_resident) {
-                                if (CG == 2) tc_commit_pair(bar_bempty + 8 * s); else tc_commit(bar_bempty + 8 * s);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < NST; j++) {
+                                if (!mbar_wait(bar_bfull + 8 * s, ph, abort_flag, p.status, 3)) goto done;
+                                tc_fence_after();
+                                if (elected) {
+                                    const uint32_t b_lo = b_lo0 + s * (uint32_t)(B_STAGE >> 4);
+#pragma unroll
+                                    for (int q = 4 * j; q < 4 * j + 4 && q < NK; q++)
+                                        mma(d_tmem, slab_lo + aoff[q / KPT] + 2u * (uint32_t)(q % KPT), b_lo + 2u * (q & 3), (uint32_t)(cg | q));
+                                    commit(bar_bempty + 8 * s);
+                                    if (j == NST - 1) commit(bar_sempty + 8 * sl);
+                                }
                                 if (++s == (uint32_t)p.nstg) { s = 0; ph ^= 1; }
                             }
                         }
-                        if (CG == 2) tc_commit_pair(bar_sempty + 8 * sl); else tc_commit(bar_sempty + 8 * sl);
                         if (++sl == (uint32_t)p.nslab) { sl = 0; slph ^= 1; }
                     }
-                    if (CG == 2) tc_commit_pair(bar_tfull + 8 * buf); else tc_commit(bar_tfull + 8 * buf);
-                    if (NISSUE == 2) skip_tile();
+                    if (elected) commit(bar_tfull + 8 * buf);
                 }
             } else
             for (int t = unit; t < ntiles; t += nunits, lt++, first_tile = false) {
-                const int buf = lt & 1;
-                if (!mbar_wait(OVL ? bar_tempty : bar_tempty + 8 * buf, (OVL ? (lt & 1) : ((lt >> 1) & 1)) ^ 1, abort_flag, p.status, 2))
+                const int buf = (int)(lt % NBUF);
+                if (!mbar_wait(OVL ? bar_tempty : bar_tempty + 8 * buf, (OVL ? (lt & 1) : ((lt / NBUF) & 1)) ^ 1, abort_flag, p.status, 2))
                     goto done;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * ACC_OFF;
@@ -315,7 +330,7 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
                 for (int cg = 0; cg < p.G; cg++) {
                     if (!mbar_wait(bar_sfull + 8 * sl, slph, abort_flag, p.status, 0x13)) goto done;
                     tc_fence_after();
-                    const uint64_t da = da0 + (uint64_t)(sl * slab16);
+                    const uint32_t slab_lo = a_lo0 + sl * slab16;
                     // tap (kh, kw) starts kh*Wp + kw rows into the slab: kept as running counters -- a table in
                     // shared memory would put a load, queued behind the MMAs just issued, in front of every MMA
                     uint32_t kwc = 0, rowoff = 0, tapoff = 0;
@@ -327,17 +342,15 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
                             if (!mbar_wait(bar_bfull + 8 * slot, p.b_resident ? 0u : ph, abort_flag, p.status, 3)) goto done;
                             tc_fence_after();
                         }
-                        const uint64_t db = db0 + (uint64_t)(slot * (B_STAGE >> 4));
+                        const uint32_t b_lo = b_lo0 + slot * (uint32_t)(B_STAGE >> 4);
+                        // offsets of the stage's four K steps (64 elements = 32 bytes of one tap's pixel row each)
+                        uint32_t ak[4];
+                        int steps = 0;
 #pragma unroll
                         for (int k = 0; k < 4; k++) {
-                            // K step k of the stage = 64 elements = 32 bytes of one tap's pixel row
                             const uint32_t koff = (TAPS == 1) ? 2u * k : (TAPS == 2 ? 2u * (k & 1) : 0u);
-                            if (TAPS == 1 || tap < p.T) {
-                                const uint64_t dak = da + (uint64_t)(tapoff + koff);
-                                if (CG == 2) tc_mma_f4_pair(d_tmem, dak, db + 2 * k, IDESC, tmem_base + SF_COL, tmem_base + SF_COL + 16, acc);
-                                else tc_mma_f4(d_tmem, dak, db + 2 * k, IDESC, tmem_base + SF_COL, tmem_base + SF_COL + 16, acc);
-                                acc = 1;
-                            }
+                            ak[k] = slab_lo + tapoff + koff;
+                            if (TAPS == 1 || tap < p.T) steps = k + 1;
                             // the next K step belongs to the next tap: after every step (32-byte pixels), every second
                             // (64-byte pixels) or the stage's last (128-byte pixels)
                             if (TAPS == 4 || (TAPS == 2 && (k & 1)) || (TAPS == 1 && k == 3)) {
@@ -346,15 +359,19 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
                                 else tapoff += RB / 16;
                             }
                         }
-                        if (!p.b_resident) {
-                            if (CG == 2) tc_commit_pair(bar_bempty + 8 * s); else tc_commit(bar_bempty + 8 * s);
-                            if (++s == (uint32_t)p.nstg) { s = 0; ph ^= 1; }
+                        if (elected) {
+#pragma unroll
+                            for (int k = 0; k < 4; k++)
+                                if (k < steps) mma(d_tmem, ak[k], b_lo + 2u * k, acc | (uint32_t)k);
+                            if (!p.b_resident) commit(bar_bempty + 8 * s);
                         }
+                        acc = 1;
+                        if (!p.b_resident && ++s == (uint32_t)p.nstg) { s = 0; ph ^= 1; }
                     }
-                    if (CG == 2) tc_commit_pair(bar_sempty + 8 * sl); else tc_commit(bar_sempty + 8 * sl);
+                    if (elected) commit(bar_sempty + 8 * sl);
                     if (++sl == (uint32_t)p.nslab) { sl = 0; slph ^= 1; }
                 }
-                if (CG == 2) tc_commit_pair(bar_tfull + 8 * buf); else tc_commit(bar_tfull + 8 * buf);
+                if (elected) commit(bar_tfull + 8 * buf);
             }
         }
     } else if (QF && warp >= Cfg::WARP_Q0) {
@@ -368,16 +385,21 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
         } else if (lane == 0) {
             publish_items(p.q_sync, p.status, qbars, abort_flag);
         }
-    } else if (warp >= WARP_EPI0 && warp < WARP_EPI0 + 4 * EPW) {
+    } else if (warp >= WARP_EPI0 && warp < WARP_EPI0 + Cfg::NEPI) {
         // ---------------- epilogue ----------------
         const int q = warp & 3;                        // tensor-memory lane quadrant this warp may access
-        const int ecol = (warp - WARP_EPI0) >> 2;      // which share of the columns
+        const int ecol = ((warp - WARP_EPI0) >> 2) % EPW;         // which share of the columns
+        const int group = ((warp - WARP_EPI0) >> 2) / EPW;
+        // which tiles: every NSETS-th of the block's sequence; where no block has more than one (the launcher starts
+        // two groups only), the groups share its columns
+        const bool one_tile = NSETS > 1 && ntiles <= nunits;
+        const int set = one_tile ? 0 : group, slice0 = one_tile ? group : 0, slice_step = one_tile ? ONE_TILE_GROUPS : 1;
         constexpr int ECOLS = BN / EPW;
         constexpr int NSL = ECOLS / 32;
         const bool alpha_in_unit = p.alpha > 0.f && p.alpha <= 1.f;
         const float bias_f = (float)p.acc_bias;
         const int OHW = p.OH * p.OW;
-        uint32_t lt = 0;
+        uint32_t lt = (uint32_t)set;
         const uint32_t bar_release = (CG == 2 && rank != 0) ? mapa_shared(bar_tempty, 0) : 0u;
         // quantised output with 0 < alpha <= 1: PReLU and the next layer's rule collapse into thresholds on
         // the accumulator (two instructions per output and plane instead of evaluating the PReLU first).
@@ -390,8 +412,8 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
         int qt_img = -1;
         // pixel-major fp32 output: the accumulator is fetched in the 16x256b shape (four lanes = 32 contiguous bytes of a row)
         const bool rows16 = p.pimg == nullptr && p.layout == TNNS_NHWC && (p.KN & 1) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
-        for (int t = unit; t < ntiles; t += nunits, lt++) {
-            const int buf = lt & 1;
+        for (int t = unit + set * nunits; t < ntiles; t += NSETS * nunits, lt += NSETS) {
+            const int buf = (int)(lt % NBUF);
             const int n0 = (t % ntn) * BN;
             // where this thread's row sits in the lattice, and its image's threshold: worked out while the tile's MMAs run
             const int row = (t / ntn) * TILE_M + (int)rank * BM + q * 32 + lane;  // virtual row
@@ -422,12 +444,12 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
                     }
                 }
             }
-            if (!mbar_wait(bar_tfull + 8 * buf, (lt >> 1) & 1, abort_flag, p.status, 5)) goto done;
+            if (!mbar_wait(bar_tfull + 8 * buf, (lt / NBUF) & 1, abort_flag, p.status, 5)) goto done;
             tc_fence_after();
             int start = 0;
             if (OVL && buf == 0 && ecol == EPW - 1) start = NSL - 1;
 #pragma unroll 1
-            for (int i = 0; i < NSL; i++) {
+            for (int i = slice0; i < NSL; i += slice_step) {
                 const int cb = ecol * ECOLS + ((i + start) % NSL) * 32;
                 uint32_t v[32];
                 const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * ACC_OFF + cb);
@@ -623,7 +645,7 @@ int launch_slab(tnns_cuda_ctx* ctx, const SlabArgs& a, size_t smem, cudaStream_t
     attr[nattr].val.programmaticStreamSerializationAllowed = 1;
     nattr++;
     cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(Cfg::NTHREADS);
+    cfg.blockDim = dim3(!QF && Cfg::NSETS > 1 && tiles <= ctx->sm_count ? 32 * (Cfg::WARP_EPI0 + 4 * ONE_TILE_GROUPS) : Cfg::NTHREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     if (CG == 1) {
@@ -721,6 +743,16 @@ bool choose_form(int sm_count, const tnns_cuda_weights* w, const TnnsGeom& g, in
     ch->b_stage = (pl.bn / (ch->pairs ? 2 : 1)) * KCH;
     ch->fixed = 1024 + SL_BAR_BYTES + (fused ? Q_STG * Q_PIX * 64 * 4 + 128 : 0);
     if (!ring_depths(pl, ch->b_stage, ch->fixed, w->Kp / 4, ch->ntn == 1, &ch->nslab, &ch->nstg, &ch->resident)) return false;
+    if (!ch->pairs && !fused) {
+        // few tiles: narrower ones (what fits with the widest tile fits with these)
+        const int bn = tile_n_for(sm_count, ch->Mv, w->KN, pl.bn);
+        if (bn != pl.bn) {
+            ch->pl.bn = bn;
+            ch->ntn = (w->KN + bn - 1) / bn;
+            ch->b_stage = bn * KCH;
+            if (!ring_depths(pl, ch->b_stage, ch->fixed, w->Kp / 4, ch->ntn == 1, &ch->nslab, &ch->nstg, &ch->resident)) return false;
+        }
+    }
     ch->smem = (size_t)ch->fixed + (size_t)ch->nslab * pl.slab_bytes + (size_t)ch->nstg * ch->b_stage;
     return true;
 }
@@ -756,6 +788,7 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
     a.Mv = Mv;
     a.KN = w->KN;
     a.nchunks = w->Kp / 4;
+    a.b_rows = tnns_i8_tile_n(w->KN);
     a.OH = g.OH; a.OW = g.OW; a.Wp = pl.Wp; a.HpWp = pl.Hp * pl.Wp;
     a.KW = g.KW; a.T = pl.T; a.G = pl.G;
     a.slab_bytes = pl.slab_bytes; a.copy_rows = pl.copy_rows; a.ncopies = pl.ncopies;

@@ -93,16 +93,23 @@ struct TcCfg {
     static constexpr int NSTG = QF ? NSTG_QF : (ATMA ? NSTG_ATMA : ((MT == 1) ? 4 : 3));
     static constexpr int A_STAGE = MT * A_SUB, B_STAGE = (BN / CG) * KCH;
     static constexpr bool OVL = F4 && MT == 1 && BN == 256;        // overlapping accumulator sets
-    static constexpr int NBUF = (OVL || MT * BN <= (F4 ? 128 : 256)) ? 2 : 1;  // accumulator sets in tensor memory
+    // Tensor-copy form on narrow tiles: three groups of four epilogue warps take the tiles in turn (see gemm_slab.cu, where a
+    // narrow tile's drain is the same chain of latencies, longer than its MMAs)
+    static constexpr int NSETS = (ATMA && !QF && CG == 1 && BN <= 128) ? 3 : 1;
+    static constexpr int NBUF = NSETS > 1 ? (BN == 64 ? 4 : 3) : ((OVL || MT * BN <= (F4 ? 128 : 256)) ? 2 : 1);  // accumulator sets in tensor memory
+    static_assert(NSETS <= NBUF || NSETS == 1, "a set may not be a whole turn of the accumulators ahead (parity waits)");
     static constexpr int ACC_OFF = OVL ? BN - 32 : MT * BN;        // column distance between the sets
     // epilogue warps per lane quadrant: two share each quadrant's columns where the drain is
     // not (or only partly) hidden behind the next tile's MMAs
-    static constexpr int EPW = ATMA ? 2 : (((NBUF == 1 || OVL) && MT == 1) ? 2 : 1);
+    static constexpr int EPW = ATMA ? (NSETS > 1 ? 1 : 2) : (((NBUF == 1 || OVL) && MT == 1) ? 2 : 1);
     // expander groups (stages expanded concurrently); 22 warps per block in every MT = 1 form
     static constexpr int NG = ATMA ? 0 : ((MT == 1) ? (EPW == 2 ? 3 : 4) : 2);
     static constexpr int WARP_EPI0 = WARP_EXP0 + 4 * MT * NG;
-    static constexpr int WARP_Q0 = WARP_EPI0 + 4 * MT * EPW;
-    static constexpr int NTHREADS = 32 * (2 + 4 * MT * NG + 4 * MT * EPW + NQ);
+    static constexpr int NEPI = 4 * MT * EPW * NSETS;  // epilogue warps
+    static constexpr int WARP_Q0 = WARP_EPI0 + NEPI;
+    static constexpr int NTHREADS = 32 * (2 + 4 * MT * NG + NEPI + NQ);
+    static constexpr int NBARS = NBUF > 2 ? NBUF : 2;
+    static_assert((2 * NSTG + 2 * NBARS) * 8 + 8 <= 256, "barriers and two words");
     static constexpr int TAPMAX = QF ? 192 : 1024;  // entries of the tap table kept in shared memory (QF: 192 entries + the 256 bytes of barriers = 1 KB, see Q_OFF)
     static constexpr size_t Q_OFF = (size_t)NSTG * (A_STAGE + B_STAGE) + 256 + TAPMAX * sizeof(uint32_t);  // quantiser ring, then its barriers
     static_assert(!QF || Q_OFF % 1024 == 0, "the quantiser ring receives 128-byte-swizzled boxes: its stages start on 1024-byte boundaries");
@@ -297,10 +304,10 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
     unsigned char* sA = smem;
     unsigned char* sB = smem + NSTG * A_STAGE;
     uint64_t* bars = reinterpret_cast<uint64_t*>(sB + NSTG * B_STAGE);
-    // barriers: full[NSTG], empty[NSTG], tmem_full[2], tmem_empty[2]
+    // barriers: full[NSTG], empty[NSTG], tmem_full[NBARS], tmem_empty[NBARS]
     const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + NSTG), bar_tfull = smem_u32(bars + 2 * NSTG),
-                   bar_tempty = smem_u32(bars + 2 * NSTG + 2);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NSTG + 4);
+                   bar_tempty = smem_u32(bars + 2 * NSTG + Cfg::NBARS);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NSTG + 2 * Cfg::NBARS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     // The tap table (plane word -> kh, kw, ic) sits on the producer's critical path once per stage,
     // so its first TAPMAX entries are copied to shared memory; longer tables fall back to global loads.
@@ -328,7 +335,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
             mbar_init(bar_full + 8 * s, ATMA ? 1 : 1 + 4 * MT);  // weight producer + the expander warps
             mbar_init(bar_empty + 8 * s, 1);  // tcgen05.commit
         }
-        for (int b = 0; b < 2; b++) {
+        for (int b = 0; b < Cfg::NBARS; b++) {
             mbar_init(bar_tfull + 8 * b, 1);
             mbar_init(bar_tempty + 8 * b, CG * 4 * MT * EPW);  // the epilogue warps (of both blocks of a pair)
         }
@@ -692,12 +699,17 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
         // ---------------- epilogue ----------------
         const int q = warp & 3;                 // tensor-memory lane quadrant this warp may access
         const int sub = ((warp - WARP_EPI0) >> 2) % MT;   // which 128-row sub-tile (accumulator) it drains
-        const int ecol = ((warp - WARP_EPI0) >> 2) / MT;  // which share of the columns
-        constexpr int ECOLS = BN / EPW;
+        const int ecol = ((warp - WARP_EPI0) >> 2) / MT % EPW;  // which share of the columns
+        constexpr int ECOLS = BN / EPW, NSETS = Cfg::NSETS;
+        // which tiles: every NSETS-th of the block's sequence; where no block has more than one (the launcher starts
+        // two groups only), the groups share its columns
+        const int group = ((warp - WARP_EPI0) >> 2) / (MT * EPW);
+        const bool one_tile = NSETS > 1 && ntiles <= nunits;
+        const int set = one_tile ? 0 : group, slice0 = one_tile ? group : 0, slice_step = one_tile ? ONE_TILE_GROUPS : 1;
         const bool alpha_in_unit = p.alpha > 0.f && p.alpha <= 1.f;
         const int bias_magic = 0x4B400000 + p.acc_bias;
         const float bias_f = (float)p.acc_bias;  // +0.0f when there is none: a + 0.0f also turns a -0 sum into +0
-        uint32_t lt = 0;
+        uint32_t lt = (uint32_t)set;
         const uint32_t bar_release = (CG == 2 && rank != 0) ? mapa_shared(bar_tempty, 0) : 0u;  // pair: the first block's barrier
         // quantised output with 0 < alpha <= 1: PReLU and the next layer's rule collapse into thresholds on
         // the accumulator (two instructions per output and plane instead of evaluating the PReLU first)
@@ -706,11 +718,11 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
         // its mere presence measured one percent of the large layer)
         if (F4 && !QF && p.pimg && p.pimg_e2m1 && p.o_HpWp)
             fill_output_border(reinterpret_cast<uint4*>(p.pimg), p.cp_next, p.OHW / p.OW, p.OW, (int)(p.M / p.OHW), p.o_Wp, p.o_HpWp, p.o_PH, p.o_PW,
-                               (long long)blockIdx.x * (32 * 4 * MT * EPW) + (tid - 32 * WARP_EPI0), (long long)gridDim.x * (32 * 4 * MT * EPW));
+                               (long long)blockIdx.x * (blockDim.x - 32 * WARP_EPI0) + (tid - 32 * WARP_EPI0), (long long)gridDim.x * (blockDim.x - 32 * WARP_EPI0));
         const bool rows16 = F4 && p.pimg == nullptr && p.layout == TNNS_NHWC && (p.KN & 1) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
         tnns_thr::Pair qt = {0.f, 0.f};
         long long qt_img = -1;
-        for (int t = unit; t < ntiles; t += nunits, lt++) {
+        for (int t = unit + set * nunits; t < ntiles; t += NSETS * nunits, lt += NSETS) {
             const int buf = lt % NBUF;
             const long long m0 = (long long)(t / ntn) * TILE_M + (int)rank * BMT + sub * BM;
             const int n0 = (t % ntn) * BN;
@@ -734,7 +746,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
             int start = 0;
             if (OVL && buf == 0 && ecol == EPW - 1) start = NSL - 1;
 #pragma unroll 1
-            for (int i = 0; i < NSL; i++) {
+            for (int i = slice0; i < NSL; i += slice_step) {
                 const int cb = ecol * ECOLS + ((i + start) % NSL) * 32;
                 uint32_t v[32];
                 const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * ACC_OFF + sub * BN + cb);
@@ -1013,7 +1025,7 @@ int launch_cfg(tnns_cuda_ctx* ctx, const GemmArgs& a, cudaStream_t stream, const
         const int grid = (int)std::min<long long>(tiles, ctx->sm_count);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(grid);
-        cfg.blockDim = dim3(Cfg::NTHREADS);
+        cfg.blockDim = dim3(Cfg::NSETS > 1 && tiles <= ctx->sm_count ? 32 * (Cfg::WARP_EPI0 + 4 * ONE_TILE_GROUPS) : Cfg::NTHREADS);
         cfg.dynamicSmemBytes = Cfg::SMEM;
         cfg.stream = stream;
         cfg.attrs = attr;
@@ -1254,21 +1266,6 @@ namespace {
 // of one stage.  The image is stored swizzled already, so the copy itself does not swizzle.
 int encode_weight_map(CUtensorMap* map, const tnns_cuda_weights* w, int BN) {
     return tnns_tensor_map_2d(map, 1, w->d_f4, KCH, w->f4_bytes / KCH, KCH, KCH, BN / 2);
-}
-}  // namespace
-
-namespace {
-// Kernels per tile of the tensor-copy form on single blocks: the weight image's own tile, or the narrowest part of it whose
-// tiles still fit the chip in one wave.  Clocks stamped in the kernel for a tile of 64 / 128 / 256 kernels: a stage 340 /
-// 375 / 567 (its four MMAs, or its bytes at the 86 per clock that reach an SM), the drain of the finished accumulator 1250
-// per 64 kernels (an SM stores about 30 bytes per clock).  Both lie in series when an SM has one tile.  Where there is more
-// than one wave they overlap and a narrower tile only repeats the activation copies (256 x 64x56x56 -> 128 s2: 30 us with
-// tiles of 128, 47 with 64).  GEMM alone, widest / rule: 1 x 256x56x56 -> 256 8.3 / 6.4 us, FC 1024x4096x1024 10.2 / 8.2.
-int tile_n_for(int sm_count, long long M, int KN, int widest) {
-    const long long mt = (M + BM - 1) / BM;
-    int bn = widest;
-    while (bn > 64 && mt * ((KN + bn / 2 - 1) / (bn / 2)) <= sm_count) bn /= 2;
-    return bn;
 }
 }  // namespace
 

@@ -14,12 +14,25 @@ constexpr int BM = 128;        // rows per accumulator (tensor-memory lanes)
 constexpr int KCH = 128;       // K elements = bytes per row and stage (one swizzle atom)
 constexpr int A_SUB = BM * KCH;  // bytes of one 128-row activation sub-tile per stage
 constexpr int WARP_TMA = 0, WARP_MMA = 1, WARP_EXP0 = 2;
+constexpr int ONE_TILE_GROUPS = 2;  // groups of four epilogue warps on narrow tiles where no block has more than one tile
 // fused quantisation (QF)
 constexpr int Q_FLAG0 = 32;   // the per-image words start one 128-byte line after the item counter
 constexpr int Q_PIX = 128;    // pixels per quantise item = quantiser threads per block
 constexpr int Q_STG = 2;      // stages of the quantiser warps' ring
 constexpr int Q_PUBN = 8;     // items the quantiser warps may be ahead of the publisher
 
+// Kernels per tile of the tensor-copy form on single blocks: the weight image's own tile, or the narrowest part of it whose
+// tiles still fit the chip in one wave.  Clocks stamped in the kernel for a tile of 64 / 128 / 256 kernels: a stage 340 /
+// 375 / 567 (its four MMAs, or its bytes at the 86 per clock that reach an SM), the drain of the finished accumulator 1250
+// per 64 kernels (an SM stores about 30 bytes per clock).  Both lie in series when an SM has one tile.  Where there is more
+// than one wave they overlap and a narrower tile only repeats the activation copies (256 x 64x56x56 -> 128 s2: 30 us with
+// tiles of 128, 47 with 64).  GEMM alone, widest / rule: 1 x 256x56x56 -> 256 8.3 / 6.4 us, FC 1024x4096x1024 10.2 / 8.2.
+inline int tile_n_for(int sm_count, long long M, int KN, int widest) {
+    const long long mt = (M + BM - 1) / BM;
+    int bn = widest;
+    while (bn > 64 && mt * ((KN + bn / 2 - 1) / (bn / 2)) <= sm_count) bn /= 2;
+    return bn;
+}
 // One lane of a converged warp.  The MMA issuers run their loops warp-wide, wait for their barriers with all lanes and
 // issue a stage's MMAs and its commit from one `if (elected)` region: loop state then lives in uniform registers, which is
 // where the MMA instruction takes its operands from.  Measured with operands resident in shared memory, a barrier wait

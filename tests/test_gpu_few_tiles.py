@@ -16,6 +16,9 @@ LAYERS = [
     (Layer(128, 14, 14, 191, 3, 3, 1, 2), 5), (Layer(512, 7, 7, 257, 3, 3, 1, 1), 8), (Layer(512, 7, 7, 513, 1, 1, 0, 1), 3),
     (Layer(256, 12, 12, 320, 5, 3, 1, 2), 4), (Layer(1024, 1, 1, 1000, 1, 1, 0, 1), 129), (Layer(256, 16, 16, 256, 1, 1, 0, 1), 18),
     (Layer(256, 16, 16, 256, 1, 1, 0, 1), 19), (Layer(256, 16, 16, 200, 1, 1, 0, 1), 37), (Layer(256, 16, 16, 200, 1, 1, 0, 1), 38),
+    # narrow tiles, some blocks with two and more: drained by groups of warps in turn
+    (Layer(64, 16, 16, 64, 3, 3, 1, 2), 310), (Layer(256, 16, 16, 100, 1, 1, 0, 1), 150), (Layer(64, 16, 16, 60, 3, 3, 1, 1), 150),
+    (Layer(128, 14, 14, 128, 3, 3, 1, 1), 75),
 ]
 
 
