@@ -17,6 +17,7 @@
 // "channels", with every epilogue it has.  Ternary activations only (TNN, TBN): a binary window pads
 // with +1, which the zero positions of this form cannot express.
 #include <algorithm>
+#include <cmath>
 
 #include "internal.h"
 
@@ -53,66 +54,112 @@ __global__ void repack_weights_dense_kernel(const uint64_t* __restrict__ packed,
     }
 }
 
-// One thread = one output pixel's 32 consecutive positions (one 16-byte piece of its row of the virtual image).
-// Neighbouring threads take neighbouring output pixels of the same piece: for every position their loads are SW
-// floats apart (coalesced along the input row), and their 16-byte stores one image row (K'/2 bytes) apart.
-// Pieces that lie entirely past K are written as zeros (binary weights read +1 there, not 0).  The walk over
-// (kh, kw, c) keeps a running pointer and a running "inside the input" flag, so a position costs its load, two
-// additions, two funnel shifts and the flag.
+// A block owns a band of output rows (and a segment of output columns) of one image.
+//   1. The input values its windows cover are quantised once, into two bit rows per input row in shared memory (sign,
+//      non-zero): bit (x - x0)*C + c.  A warp makes a word with one load per lane and two ballots; positions outside the
+//      input are the reference's padding, zero whatever the threshold.
+//   2. In that order the KW*C positions of a window's filter row are CONSECUTIVE bits, starting at ow*SW*C: a thread
+//      collects its output pixel's positions with one funnel shift per filter row (and 32 positions) and plane, and stores
+//      16 bytes of operands for every 32 of them; positions past K are zero.
+// Bound by instructions, so both steps keep their loops free of divisions and every lane on the same path.  (With every
+// position quantised from its own load, 147 per output pixel of a 7x7x3 window, and with one thread per 32 positions of a
+// pixel instead of one per pixel, the first layer of the ResNet-18 table at batch 8, GEMM included, took 29 and 36 us; 23 now.)
+constexpr int DQ_THREADS = 256;
+constexpr int DQ_SMEM = 48 * 1024;
+constexpr int DQ_ROWS = 8;  // loads in flight per lane
+
+struct DenseQ {
+    int N, C, H, W, OH, OW, KH, SH, SW, PH, PW;
+    int R, groups32, pieces;         // positions of one filter row; 32-position pieces of an image row, and how many of them are written
+    int band, seg, rows, words;      // output rows and columns of a unit; input rows and words per bit row it holds
+    int nbands, nsegs;
+    long long units;
+    FastDiv div_c, div_seg;
+};
+
+__device__ __forceinline__ void store_sector(uint4* dst, const uint32_t (&lo)[4], const uint32_t (&hi)[4]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]), "r"(hi[0]),
+                 "r"(hi[1]), "r"(hi[2]), "r"(hi[3])
+                 : "memory");
+}
+
 template <bool NHWC>
-__global__ void __launch_bounds__(256)
-dense_quantise_kernel(const float* __restrict__ x, const float* __restrict__ thr, uint4* __restrict__ img, TnnsGeom g, int K, int groups32,
-                      FastDiv div_rows, FastDiv div_ow, FastDiv div_ohw, FastDiv div_c, FastDiv div_kw, long long total) {
-    const long long cstride = NHWC ? 1 : (long long)g.H * g.W;   // one channel further
-    const long long pstride = NHWC ? g.C : 1;                    // one input pixel to the right
-    const long long rstride = pstride * g.W;                     // one input row down
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int grp = (int)div_rows.div((uint32_t)i);
-        const uint32_t row = (uint32_t)i - (uint32_t)grp * div_rows.d;
-        const uint32_t n = div_ohw.div(row);
-        const uint32_t rem = row - n * (uint32_t)(g.OH * g.OW);
-        const int oh = (int)div_ow.div(rem), ow = (int)(rem - (uint32_t)oh * g.OW);
+__global__ void __launch_bounds__(DQ_THREADS)
+dense_quantise_kernel(const float* __restrict__ x, const float* __restrict__ thr, uint4* __restrict__ img, DenseQ g) {
+    extern __shared__ uint32_t sm_bits[];  // [rows][words] sign, then [rows][words] non-zero; one spare word behind
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the input may be the output of the launch before
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    uint32_t* sm_s = sm_bits;
+    uint32_t* sm_z = sm_bits + g.rows * g.words;
+    const long long cstride = NHWC ? 1 : (long long)g.H * g.W, pstride = NHWC ? g.C : 1, rstride = pstride * g.W;
+    for (long long u = blockIdx.x; u < g.units; u += gridDim.x) {
+        const int sg = (int)(u % g.nsegs);
+        const long long nb = u / g.nsegs;
+        const int n = (int)(nb / g.nbands), oh0 = (int)(nb - (long long)n * g.nbands) * g.band, ow0 = sg * g.seg;
+        const int boh = min(g.band, g.OH - oh0), bow = min(g.seg, g.OW - ow0);
+        const int y0 = oh0 * g.SH - g.PH, x0 = ow0 * g.SW - g.PW;
         const float t = __ldg(thr + n) + 0.0f;  // + 0.0f: a threshold of -0 behaves as +0 in every compare
-        const int ih0 = oh * g.SH - g.PH, iw0 = ow * g.SW - g.PW;
-        const int e0 = grp * 32;
-        if (e0 >= K) {
-            img[(size_t)row * groups32 + grp] = make_uint4(0u, 0u, 0u, 0u);
-            continue;
-        }
-        // position e = (kh*KW + kw)*C + c, walked from the piece's last position down so that position b ends at bit b
-        int e = min(e0 + 31, K - 1);
-        const int tap = (int)div_c.div((uint32_t)e);
-        int c = e - tap * g.C;
-        int kh = (int)div_kw.div((uint32_t)tap), kw = tap - kh * g.KW;
-        const float* px = x + (size_t)n * g.C * g.H * g.W + (long long)c * cstride + (long long)(ih0 + kh) * rstride + (long long)(iw0 + kw) * pstride;
-        bool ok = (unsigned)(ih0 + kh) < (unsigned)g.H && (unsigned)(iw0 + kw) < (unsigned)g.W;
-        uint32_t sg = 0, nz = 0, ins = 0;
-        for (; e >= e0; e--) {
-            const float v = ok ? __ldg(px) : 0.0f;
-            sg = __funnelshift_l(__float_as_uint(v + t), sg, 1);
-            nz = __funnelshift_l(__float_as_uint(t - fabsf(v)), nz, 1);
-            ins = (ins << 1) | (ok ? 1u : 0u);
-            if (--c >= 0) {
-                px -= cstride;
-            } else {
-                c = g.C - 1;
-                if (--kw >= 0) {
-                    px += (long long)(g.C - 1) * cstride - pstride;
-                } else {
-                    kw = g.KW - 1;
-                    kh--;
-                    px += (long long)(g.C - 1) * cstride - rstride + (long long)(g.KW - 1) * pstride;
+        const float* src = x + (size_t)n * g.C * g.H * g.W;
+        const int nrows = (boh - 1) * g.SH + g.KH;
+        const int nchunks = (nrows + DQ_ROWS - 1) / DQ_ROWS;
+        for (int k = warp; k < g.words * nchunks; k += DQ_THREADS / 32) {
+            // one word of up to DQ_ROWS rows: the lane's column and channel are worked out once for all of them
+            const int w = k / nchunks, r0 = (k - w * nchunks) * DQ_ROWS;
+            const uint32_t idx = (uint32_t)w * 32 + lane, xx = g.div_c.div(idx), c = idx - xx * g.C;
+            const int ix = x0 + (int)xx, iy = y0 + r0;
+            const bool col = (unsigned)ix < (unsigned)g.W;
+            const float* p = src + (c * cstride + ix * (long long)pstride + iy * rstride);
+            float v[DQ_ROWS];
+#pragma unroll
+            for (int r = 0; r < DQ_ROWS; r++) v[r] = (col && r0 + r < nrows && (unsigned)(iy + r) < (unsigned)g.H) ? __ldg(p + r * rstride) : NAN;
+#pragma unroll
+            for (int r = 0; r < DQ_ROWS; r++) {
+                // a position outside the input is NaN here: no compare holds, whatever the threshold
+                const uint32_t sgn = __ballot_sync(0xFFFFFFFFu, v[r] < -t), nz = __ballot_sync(0xFFFFFFFFu, fabsf(v[r]) > t);
+                if (lane == 0 && r0 + r < nrows) {
+                    sm_s[(r0 + r) * g.words + w] = sgn;
+                    sm_z[(r0 + r) * g.words + w] = nz;
                 }
-                ok = (unsigned)(ih0 + kh) < (unsigned)g.H && (unsigned)(iw0 + kw) < (unsigned)g.W;
             }
         }
-        // positions outside the input are the reference's padding: zero whatever the threshold (a negative one
-        // would otherwise call the 0 read there "non-zero"); positions past K sit in the high bits, which stay 0
-        sg &= ins;
-        nz &= ins;
-        uint32_t w4[4];
-        tnns_expand32_f4(sg, ~nz, w4);
-        img[(size_t)row * groups32 + grp] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+        __syncthreads();
+        for (int i = tid; i < boh * bow; i += DQ_THREADS) {
+            const int ohl = bow == g.seg ? (int)g.div_seg.div((uint32_t)i) : i / bow, owl = i - ohl * bow;
+            const uint32_t* row_s = sm_s + ohl * g.SH * g.words;
+            const uint32_t* row_z = sm_z + ohl * g.SH * g.words;
+            uint4* dst = img + (((size_t)n * g.OH + oh0 + ohl) * g.OW + ow0 + owl) * g.groups32;
+            const uint32_t bit0 = (uint32_t)(owl * g.SW * g.C);
+            uint64_t as = 0, az = 0;  // collected positions that are not stored yet; always fewer than 32 between two filter rows' pieces
+            int have = 0, grp = 0;
+            uint32_t s0 = 0, z0 = 0;  // an even piece waits for its neighbour: the two are stored as one 32-byte sector
+            auto emit = [&]() {
+                if (grp & 1) {
+                    uint32_t lo[4], hi[4];
+                    tnns_expand32_f4(s0, ~z0, lo);
+                    tnns_expand32_f4((uint32_t)as, ~(uint32_t)az, hi);
+                    store_sector(dst + grp - 1, lo, hi);
+                } else {
+                    s0 = (uint32_t)as;
+                    z0 = (uint32_t)az;
+                }
+                grp++;
+                as >>= 32;
+                az >>= 32;
+                have -= 32;
+            };
+            for (int kh = 0; kh < g.KH; kh++, row_s += g.words, row_z += g.words)
+                for (int off = 0; off < g.R; off += 32) {
+                    const int take = min(g.R - off, 32);
+                    const uint32_t bit = bit0 + off, w = bit >> 5, keep = 0xFFFFFFFFu >> (32 - take);
+                    as |= (uint64_t)(__funnelshift_r(row_s[w], row_s[w + 1], bit & 31) & keep) << have;
+                    az |= (uint64_t)(__funnelshift_r(row_z[w], row_z[w + 1], bit & 31) & keep) << have;
+                    if ((have += take) >= 32) emit();
+                }
+            // what is left of the last piece, then zeros for positions past K
+            while (grp < g.pieces) emit();
+        }
+        __syncthreads();  // the next unit overwrites the bit rows
     }
 }
 
@@ -145,21 +192,51 @@ int tnns_launch_repack_weights_dense(tnns_cuda_ctx* ctx, const tnns_cuda_weights
     return TNNS_OK;
 }
 
-int tnns_launch_dense_quantise(tnns_cuda_ctx* ctx, const float* d_x, const float* d_thr, void* d_img, const TnnsGeom& g, int Kd, int layout,
+int tnns_launch_dense_quantise(tnns_cuda_ctx* ctx, const float* d_x, const float* d_thr, void* d_img, const TnnsGeom& g, int Kd, bool wgt_ternary, int layout,
                                cudaStream_t stream) {
     const long long rows = (long long)g.N * g.OH * g.OW;
     if (rows == 0) return TNNS_OK;
-    const int groups32 = Kd / 32;
-    const int K = g.C * g.KH * g.KW;
-    const long long total = rows * groups32;
-    if (rows >= 0x7FFFFFFFLL || total >= 0xFFFFFFFFLL) return tnns_fail(TNNS_ERR_UNSUPPORTED, "too many output pixels for the dense first-layer form");
-    const int blocks = (int)std::min<long long>((total + 255) / 256, (long long)ctx->sm_count * 16);
-    const FastDiv dg = tnns_fastdiv((uint32_t)rows), dow = tnns_fastdiv((uint32_t)g.OW), dohw = tnns_fastdiv((uint32_t)(g.OH * g.OW)),
-                  dc = tnns_fastdiv((uint32_t)g.C), dkw = tnns_fastdiv((uint32_t)g.KW);
-    if (layout == TNNS_NHWC)
-        dense_quantise_kernel<true><<<blocks, 256, 0, stream>>>(d_x, d_thr, reinterpret_cast<uint4*>(d_img), g, K, groups32, dg, dow, dohw, dc, dkw, total);
-    else
-        dense_quantise_kernel<false><<<blocks, 256, 0, stream>>>(d_x, d_thr, reinterpret_cast<uint4*>(d_img), g, K, groups32, dg, dow, dohw, dc, dkw, total);
+    if (rows >= 0x7FFFFFFFLL || rows * (Kd / 32) >= 0xFFFFFFFFLL) return tnns_fail(TNNS_ERR_UNSUPPORTED, "too many output pixels for the dense first-layer form");
+    DenseQ q;
+    q.N = g.N; q.C = g.C; q.H = g.H; q.W = g.W; q.OH = g.OH; q.OW = g.OW; q.KH = g.KH; q.SH = g.SH; q.SW = g.SW; q.PH = g.PH; q.PW = g.PW;
+    q.R = g.C * g.KW; q.groups32 = Kd / 32;
+    // words past the last real position meet zero weights and stay as they are, unless the weights are binary (+1 there)
+    q.pieces = wgt_ternary ? 2 * ((g.C * g.KH * g.KW + 63) / 64) : q.groups32;
+    // The unit: up to four output rows and 256 output columns, fewer where the chip would not get two units per SM or the
+    // bit rows would not fit shared memory (one output pixel always does: K <= 1024 positions)
+    q.band = std::min(4, g.OH);
+    q.seg = std::min(256, g.OW);
+    auto smem = [&]() -> size_t {
+        q.rows = (q.band - 1) * g.SH + g.KH;
+        q.words = (int)((((long long)(q.seg - 1) * g.SW + g.KW) * g.C + 31) / 32);
+        return ((size_t)q.rows * q.words * 2 + 1) * sizeof(uint32_t);
+    };
+    auto units = [&]() -> long long { return (long long)g.N * ((g.OH + q.band - 1) / q.band) * ((g.OW + q.seg - 1) / q.seg); };
+    const long long want = 2LL * ctx->sm_count;
+    while (q.band > 1 && smem() > DQ_SMEM) q.band = (q.band + 1) / 2;
+    while (q.seg > 1 && smem() > DQ_SMEM) q.seg = (q.seg + 1) / 2;
+    while (q.seg > 64 && units() < want) q.seg = (q.seg + 1) / 2;   // columns first: a row split repeats KH - S rows of every band
+    while (q.band > 1 && units() < want) q.band = (q.band + 1) / 2;
+    while (q.seg > 16 && units() < want) q.seg = (q.seg + 1) / 2;
+    const size_t bytes = smem();
+    q.nbands = (g.OH + q.band - 1) / q.band;
+    q.nsegs = (g.OW + q.seg - 1) / q.seg;
+    q.units = units();
+    q.div_c = tnns_fastdiv((uint32_t)g.C);
+    q.div_seg = tnns_fastdiv((uint32_t)q.seg);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)std::min<long long>(q.units, (long long)ctx->sm_count * 8));
+    cfg.blockDim = dim3(DQ_THREADS);
+    cfg.dynamicSmemBytes = bytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    uint4* img = reinterpret_cast<uint4*>(d_img);
+    if (layout == TNNS_NHWC) TNNS_CUDA_TRY(cudaLaunchKernelEx(&cfg, dense_quantise_kernel<true>, d_x, d_thr, img, q));
+    else TNNS_CUDA_TRY(cudaLaunchKernelEx(&cfg, dense_quantise_kernel<false>, d_x, d_thr, img, q));
     tnns_count_launch();
     TNNS_CUDA_TRY(cudaGetLastError());
     return TNNS_OK;

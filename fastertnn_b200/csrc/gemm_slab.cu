@@ -389,7 +389,7 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
         // ---------------- epilogue ----------------
         const int q = warp & 3;                        // tensor-memory lane quadrant this warp may access
         const int ecol = ((warp - WARP_EPI0) >> 2) % EPW;         // which share of the columns
-        const int group = ((warp - WARP_EPI0) >> 2) / EPW;
+        const int group = NSETS == 1 ? 0 : ((warp - WARP_EPI0) >> 2) / EPW;
         // which tiles: every NSETS-th of the block's sequence; where no block has more than one (the launcher starts
         // two groups only), the groups share its columns
         const bool one_tile = NSETS > 1 && ntiles <= nunits;

@@ -398,8 +398,11 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
     constexpr int EARLY = 32768 / B_STAGE < NSTG ? 32768 / B_STAGE : NSTG;
     const int early = min(EARLY, nchunks);
     // tile n_tile of BN kernels is rows [n_tile*BN % b_rows, +BN) of an image tile of b_rows kernels: one contiguous piece per stage
-    const size_t b_step = (size_t)p.b_rows * KCH;
+    // (only where narrower tiles exist: the expander-fed form is short of registers)
+    constexpr bool PARTS = ATMA && CG == 1 && !QF;
+    const size_t b_step = PARTS ? (size_t)p.b_rows * KCH : (size_t)B_STAGE;
     auto weights_of = [&](int n_tile) {
+        if (!PARTS) return p.Bimg + (size_t)n_tile * nchunks * B_STAGE;
         const uint32_t k0 = (uint32_t)n_tile * BN, big = k0 / (uint32_t)p.b_rows;
         return p.Bimg + (size_t)big * nchunks * b_step + (size_t)(k0 - big * p.b_rows) * KCH;
     };
@@ -703,7 +706,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
         constexpr int ECOLS = BN / EPW, NSETS = Cfg::NSETS;
         // which tiles: every NSETS-th of the block's sequence; where no block has more than one (the launcher starts
         // two groups only), the groups share its columns
-        const int group = ((warp - WARP_EPI0) >> 2) / (MT * EPW);
+        const int group = NSETS == 1 ? 0 : ((warp - WARP_EPI0) >> 2) / (MT * EPW);
         const bool one_tile = NSETS > 1 && ntiles <= nunits;
         const int set = one_tile ? 0 : group, slice0 = one_tile ? group : 0, slice_step = one_tile ? ONE_TILE_GROUPS : 1;
         const bool alpha_in_unit = p.alpha > 0.f && p.alpha <= 1.f;

@@ -19,6 +19,10 @@ DENSE_LAYERS = [
     (TBN, Layer(16, 12, 12, 128, 3, 3, 1, 1), 2),     # 144 positions -> 256, the widest channel count taken
     (TNN, Layer(3, 13, 13, 300, 11, 11, 5, 4), 2),    # 363 positions -> 512 (two 256-position groups), stride 4
     (TNN, Layer(4, 6, 9, 64, 6, 9, 0, 1), 9),         # the filter is the image: one output pixel per image
+    (TBN, Layer(16, 9, 70, 32, 1, 63, 0, 1), 2),      # filter rows of 1008 bits, one input row per output row
+    (TNN, Layer(1, 70, 5, 32, 64, 1, 0, 1), 3),       # filter rows of one bit
+    (TNN, Layer(3, 5, 600, 32, 3, 3, 1, 1), 40),      # several segments of output columns, the last one short
+    (TNN, Layer(2, 40, 40, 32, 3, 5, 3, 9), 90),      # strides past the filter, padding past it, whole bands per unit
 ]
 
 
