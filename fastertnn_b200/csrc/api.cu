@@ -640,7 +640,7 @@ static int conv_dense_impl(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const
     if (workspace_bytes < need) return tnns_fail(TNNS_ERR_INVALID, "workspace of %zu bytes, need %zu", workspace_bytes, need);
     TNNS_ENTER(ctx, w);
     if (g.N == 0) return TNNS_OK;
-    rc = tnns_launch_dense_quantise(ctx, d_x, d_thr, d_workspace, g, gv.C, type_wgt_ternary(w->type), layout, (cudaStream_t)stream);
+    rc = tnns_launch_dense_quantise(ctx, d_x, d_thr, d_workspace, g, gv.C, layout, (cudaStream_t)stream);
     if (rc) return rc;
     return tnns_launch_gemm_im2col(ctx, w->dense, d_workspace, d_y, gv, alpha, layout, (cudaStream_t)stream, 0, d_image_out, d_thr_next, next_format,
                                    nullptr, next_PH, next_PW);

@@ -22,7 +22,7 @@
 // (four plane words), so K steps that only exist because rows are padded to four words are skipped.
 // Weights that fit the ring entirely are fetched once per block and stay (64-kernel layers).
 //
-// Roles per block: producer warp (slabs and weight stages), MMA warp, eight epilogue warps; with QF
+// Roles per block: producer warp (slabs and weight stages), MMA warp, eight or twelve epilogue warps; with QF
 // four quantiser warps and a publisher as in the im2col form (gemm_tc.cu).  Block pairs
 // (tcgen05.mma.cta_group::2) share a 256-row tile, each block with its own slab and half of the
 // weight stage.  Every wait is bounded.
@@ -405,7 +405,7 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
         // the accumulator (two instructions per output and plane instead of evaluating the PReLU first).
         // Taken on 256-kernel tiles only: on narrower tiles, where the epilogue of one tile runs beside the few
         // MMAs of the next, the shorter but denser instruction stream slowed the tensor pipe more than it
-        // saved (256 x 64x56x56 -> 64 with a bordered image out: 60 us against 49).
+        // saved (256 x 64x56x56 -> 64 with a bordered image out: 38.2 us against 33.4; 128 -> 128 @28 21.3 against 19.5).
         const bool next_tern = !p.next_binary && p.next_format != 0;
         const bool by_thr = BN == 256 && p.pimg != nullptr && alpha_in_unit;
         tnns_thr::Pair qt = {0.f, 0.f};

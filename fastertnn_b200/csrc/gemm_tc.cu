@@ -20,7 +20,7 @@
 //                       tile's copies start once the images of its rows are complete)
 //
 // Expander-fed form: one persistent block per SM, 22 warps in four roles (the tensor-copy form
-// keeps warps 0, 1 and eight epilogue warps):
+// keeps warps 0, 1 and eight epilogue warps, twelve on tiles of 64 and 128 kernels):
 //   warp 0      weight producer: one bulk async copy (TMA engine, no multicast, no tensor map)
 //               per stage of a pre-expanded, pre-swizzled weight tile (built once per layer)
 //   warp 1      MMA issuer: one thread issues four tcgen05.mma per stage and commits to the
@@ -268,17 +268,9 @@ struct GemmArgs {
 // Bordered output image (quantising epilogue, next_format 3): the frame around every image holds the next layer's padding
 // value (ternary 0).  Written by the epilogue threads of all blocks after the wait for the launch before, which may still
 // read this buffer.  Kept out of line: inlined, its registers cost the fp32 path of the large layer a percent.
-__device__ __noinline__ void fill_output_border(uint4* img, int cp_next, int H, int W, int nimg, int o_Wp, int o_HpWp, int o_PH, int o_PW,
+__device__ __noinline__ void fill_output_border(uint4* img, int cp_next, int H, int W, int nimg, int o_PH, int o_PW,
                                                 long long first, long long step) {
-    const long long total = (long long)nimg * o_HpWp;
-    const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
-    for (long long i = first; i < total; i += step) {
-        const int r = (int)(i % o_HpWp), y = r / o_Wp, x = r - y * o_Wp;
-        if (y < o_PH || y >= o_PH + H || x < o_PW || x >= o_PW + W) {
-            uint4* dst = img + (size_t)i * cp_next * 2;
-            for (int u = 0; u < 2 * cp_next; u++) dst[u] = z4;
-        }
-    }
+    tnns_fill_frame(img, make_uint4(0u, 0u, 0u, 0u), nimg, H, W, o_PH, o_PW, cp_next * 2, cp_next * 2, first, step);
 }
 
 // TAPS (tensor-copy form): filter taps per 128-byte stage row -- 1: a tap's 256 channels fill the
@@ -586,12 +578,12 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
         constexpr int RW = F4 ? 2 : 1;  // uint4 per plane and stage
         uint4 ring_s[PF][RW], ring_z[PF][RW];
         // prefetch cursor: (tile, chunk) of the next load of this group
-        int pf_t = blockIdx.x;  // may run past ntiles by one grid
+        long long pf_t = blockIdx.x;
         int pf_c = grp;
         while (pf_c >= nchunks) { pf_c -= nchunks; pf_t += gridDim.x; }
         // implicit im2row: window origin of this thread's row in the prefetch cursor's tile
         int im_n = 0, im_ih0 = 0, im_iw0 = 0;
-        int im_tile = -1;
+        long long im_tile = -1;
         const size_t img_plane = (size_t)p.H * p.W * p.Cp;  // words per image and plane
         const int img_planes = p.a_two_planes ? 2 : 1;
         auto fetch = [&](uint4 (&ds)[RW], uint4 (&dz)[RW]) {
@@ -599,7 +591,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                 if (F4 && p.img) {
                     if (im_tile != pf_t) {
                         im_tile = pf_t;
-                        const long long row = min((long long)(pf_t / ntn) * BMT + r, p.M - 1);
+                        const long long row = min((pf_t / ntn) * BMT + r, p.M - 1);
                         const long long n_img = row / p.OHW;
                         const int rem = (int)(row - n_img * p.OHW);
                         const int oh = rem / p.OW;
@@ -650,7 +642,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                     while (pf_c >= nchunks) { pf_c -= nchunks; pf_t += gridDim.x; }
                     return;
                 }
-                const uint4* rowp = p.A + (size_t)min((long long)(pf_t / ntn) * BMT + r, p.M - 1) * pitch;
+                const uint4* rowp = p.A + (size_t)min((pf_t / ntn) * BMT + r, p.M - 1) * pitch;
                 if (F4) {
                     const uint4* row = rowp + (size_t)pf_c * gsz;
 #pragma unroll
@@ -720,8 +712,8 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
         // (not in the one-launch form, whose producers write plain images only: the code is compiled out there, where
         // its mere presence measured one percent of the large layer)
         if (F4 && !QF && p.pimg && p.pimg_e2m1 && p.o_HpWp)
-            fill_output_border(reinterpret_cast<uint4*>(p.pimg), p.cp_next, p.OHW / p.OW, p.OW, (int)(p.M / p.OHW), p.o_Wp, p.o_HpWp, p.o_PH, p.o_PW,
-                               (long long)blockIdx.x * (blockDim.x - 32 * WARP_EPI0) + (tid - 32 * WARP_EPI0), (long long)gridDim.x * (blockDim.x - 32 * WARP_EPI0));
+            fill_output_border(reinterpret_cast<uint4*>(p.pimg), p.cp_next, p.OHW / p.OW, p.OW, (int)(p.M / p.OHW), p.o_PH, p.o_PW,
+                               ((long long)(warp - WARP_EPI0) * gridDim.x + blockIdx.x) * 32 + lane, (long long)gridDim.x * (blockDim.x - 32 * WARP_EPI0));
         const bool rows16 = F4 && p.pimg == nullptr && p.layout == TNNS_NHWC && (p.KN & 1) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
         tnns_thr::Pair qt = {0.f, 0.f};
         long long qt_img = -1;

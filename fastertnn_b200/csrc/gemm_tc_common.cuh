@@ -98,16 +98,7 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
                  "h"((unsigned short)3)
                  : "memory");
 }
-__device__ __forceinline__ void tc_mma_f4_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t sfa, uint32_t sfb,
-                                               uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %6, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%4], [%5], p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
-        : "memory");
-}
-// The same two with the descriptors given as (low word, high word): only a descriptor's low word -- the
+// The MMA on one block and on a pair with the descriptors given as (low word, high word): only a descriptor's low word -- the
 // shared-memory address in 16-byte units -- changes from MMA to MMA, so the issuing thread does 32-bit adds on
 // it and nothing else (its instruction stream paces the tensor pipe).
 __device__ __forceinline__ void tc_mma_f4_lh(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,

@@ -121,7 +121,7 @@ int tnns_launch_quantise_tma(tnns_cuda_ctx* ctx, bool ternary, const float* d_x,
 int tnns_dense_channels(int C, int KH, int KW);
 bool tnns_dense_eligible(int type, int C, int KH, int KW);
 int tnns_launch_repack_weights_dense(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, uint64_t* d_out, int Kp_out);
-int tnns_launch_dense_quantise(tnns_cuda_ctx* ctx, const float* d_x, const float* d_thr, void* d_img, const TnnsGeom& g, int Kd, bool wgt_ternary, int layout,
+int tnns_launch_dense_quantise(tnns_cuda_ctx* ctx, const float* d_x, const float* d_thr, void* d_img, const TnnsGeom& g, int Kd, int layout,
                                cudaStream_t stream);
 // driver-encoded descriptor of a two-dimensional tensor for the copy engine (128 bytes at `map`)
 int tnns_tensor_map_2d(void* map, int elem_bytes, const void* base, unsigned long long dim0, unsigned long long dim1,
@@ -183,6 +183,30 @@ struct FastDiv {
 #endif
 };
 FastDiv tnns_fastdiv(uint32_t d);
+
+#ifdef __CUDACC__
+// Pixel `f` of the frame of PH rows / PW columns around an H x W image, as an index into the (H + 2*PH) x (W + 2*PW) lattice:
+// the two bands of PH rows, then PW columns on either side of every row.  A frame has (H + 2*PH)*(W + 2*PW) - H*W pixels.
+__device__ __forceinline__ int tnns_frame_pixel(int f, int H, int W, int PH, int PW) {
+    const int Wp = W + 2 * PW, band = PH * Wp;
+    if (f < band) return f;
+    if (f < 2 * band) return (H + PH) * Wp + (f - band);
+    const int s = f - 2 * band, row = s / (2 * PW), c = s - row * 2 * PW;
+    return (PH + row) * Wp + (c < PW ? c : W + c);
+}
+// Writes `pad` over the frames of N bordered images of `pitch` uint4 per pixel, the first `pieces` of each.  Consecutive
+// `first` are consecutive pieces, so a warp stores whole lines; only the frame's pixels are visited.
+__device__ __forceinline__ void tnns_fill_frame(uint4* img, uint4 pad, int N, int H, int W, int PH, int PW, int pitch, int pieces, long long first,
+                                                long long step) {
+    const int HpWp = (H + 2 * PH) * (W + 2 * PW), per = HpWp - H * W;
+    const long long total = (long long)N * per * pieces;
+    for (long long i = first; i < total; i += step) {
+        const long long px = i < 0xFFFFFFFFLL ? (long long)((uint32_t)i / (uint32_t)pieces) : i / pieces;
+        const int n = px < 0xFFFFFFFFLL ? (int)((uint32_t)px / (uint32_t)per) : (int)(px / per);
+        img[((size_t)n * HpWp + tnns_frame_pixel((int)(px - (long long)n * per), H, W, PH, PW)) * pitch + (int)(i - px * pieces)] = pad;
+    }
+}
+#endif
 
 #ifdef __CUDACC__
 // 32 elements (one 32-bit lane of the sign plane, one of the zero plane) -> 32 e2m1 nibbles (four

@@ -61,22 +61,11 @@ __device__ __forceinline__ void store_half(const QaGeom& g, void* out, uint32_t 
 // the frame of a bordered image: only its pixels are visited (two bands of PH rows, then PW columns on either side)
 template <bool TERNARY>
 __device__ __forceinline__ void fill_frame(const QaGeom& g, void* out) {
-    const int per = g.HpWp - g.HW, band = g.PH * g.Wp;
-    const long long total = (long long)g.N * per;
     const uint32_t padw = TERNARY ? 0u : 0x22222222u;
     const uint4 pad4 = make_uint4(padw, padw, padw, padw);
-    for (long long i = (long long)blockIdx.x * QA_THREADS + threadIdx.x; i < total; i += (long long)gridDim.x * QA_THREADS) {
-        const int n = (int)(i / per), f = (int)(i - (long long)n * per);
-        int r;
-        if (f < band) r = f;
-        else if (f < 2 * band) r = (g.H + g.PH) * g.Wp + (f - band);
-        else {
-            const int s = f - 2 * band, row = s / (2 * g.PW), c = s - row * 2 * g.PW;
-            r = (g.PH + row) * g.Wp + (c < g.PW ? c : g.W + c);
-        }
-        uint4* dst = reinterpret_cast<uint4*>(out) + ((size_t)n * g.HpWp + r) * g.pitch * 2;
-        for (int u = 0; u < 2 * g.Cp; u++) dst[u] = pad4;
-    }
+    // (whole warps dealt out over the blocks)
+    tnns_fill_frame(reinterpret_cast<uint4*>(out), pad4, g.N, g.H, g.W, g.PH, g.PW, g.pitch * 2, 2 * g.Cp,
+                    ((long long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31), (long long)gridDim.x * QA_THREADS);
 }
 
 template <bool TERNARY, int IMG>

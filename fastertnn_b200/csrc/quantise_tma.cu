@@ -85,14 +85,10 @@ quantise_tma_kernel(const __grid_constant__ CUtensorMap tmap, const float* __res
         const uint32_t padw = TERNARY ? 0u : 0x22222222u;
         const uint4 pad4 = make_uint4(padw, padw, padw, padw);
         const int PH = off0 / Wp, PW = off0 - PH * Wp, H = HW / W;
-        const long long total = (long long)N * HpWp;
-        for (long long t = (long long)blockIdx.x * (QGROUPS * QL) + (tid - 32); t < total; t += (long long)gridDim.x * (QGROUPS * QL)) {
-            const int r = (int)(t % HpWp), y = r / Wp, x = r - y * Wp;
-            if (y < PH || y >= PH + H || x < PW || x >= PW + W) {
-                uint4* dst = reinterpret_cast<uint4*>(out) + (size_t)t * pitch * 2;
-                for (int u = 0; u < 2 * Cp; u++) dst[u] = pad4;
-            }
-        }
+        // (only its own pixels are visited, whole warps dealt out over the blocks: a walk over all pixels kept the consumers
+        // from the first items, 5 us of 256 x 64x56x56, quantise and GEMM 82.0 -> 77.4)
+        tnns_fill_frame(reinterpret_cast<uint4*>(out), pad4, N, H, W, PH, PW, pitch * 2, 2 * Cp, ((long long)(warp - 1) * gridDim.x + blockIdx.x) * 32 + lane,
+                        (long long)gridDim.x * (QGROUPS * QL));
     }
     if (warp == 0) {
         if (lane == 0) {
