@@ -562,7 +562,7 @@ static int conv_slab_impl(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
     TnnsFusedInput f;
     f.d_x = d_x;
     f.d_thr = d_thr;
-    f.C = g.C; f.Cp = g.Cp;
+    f.Cp = g.Cp;
     f.d_sync = reinterpret_cast<unsigned int*>(static_cast<char*>(d_workspace) + slab_image_bytes(g.N, g.C, g.H, g.W, g.PH, g.PW));
     return tnns_launch_gemm_slab(ctx, w, d_workspace, d_y, g, alpha, TNNS_NCHW, (cudaStream_t)stream, pairs, d_image_out, d_thr_next, fmt, bin, next_PH,
                                  next_PW, &f);
@@ -706,7 +706,7 @@ static int conv_fused_impl(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const
     TnnsFusedInput f;
     f.d_x = d_x;
     f.d_thr = d_thr;
-    f.C = g.C; f.Cp = g.Cp;
+    f.Cp = g.Cp;
     f.d_sync = reinterpret_cast<unsigned int*>(static_cast<char*>(d_workspace) + fused_image_bytes(g.N, g.C, g.H, g.W));
     return tnns_launch_gemm_im2col(ctx, w, d_workspace, d_y, g, alpha, layout, (cudaStream_t)stream, pairs, d_image_out, d_thr_next,
                                    next_format, &f);
@@ -818,7 +818,8 @@ int tnns_cuda_im2row_packed(tnns_cuda_ctx* ctx, int ternary, const void* d_image
 
 // Layers outside tnns_im2col_supported on the copy-engine fed GEMM all the same: binary activations from an image that
 // stores its padding (any stride), pixels of an odd number of bytes stored at a pitch of whole stage rows (w->wide).
-// gv: the geometry the GEMM sees; PH, PW: the border the quantise step writes.
+// gv: the geometry the GEMM sees, its pixel (Cp) padded but its C the input's own -- whether the quantise step may run inside
+// the GEMM launch is asked of the tensor that is there; PH, PW: the border the quantise step writes.
 struct WidePlan {
     const tnns_cuda_weights* w;
     TnnsGeom gv;
@@ -828,7 +829,7 @@ struct WidePlan {
 static bool wide_plan(const tnns_cuda_weights* w, const TnnsGeom& g, WidePlan* pl) {
     pl->w = w->wide ? w->wide : w;
     pl->gv = g;
-    pl->gv.C = pl->w->Cp * TNNS_WORD_BITS; pl->gv.Cp = pl->w->Cp; pl->gv.Kw = pl->w->Kw; pl->gv.Kp = pl->w->Kp;
+    pl->gv.Cp = pl->w->Cp; pl->gv.Kw = pl->w->Kw; pl->gv.Kp = pl->w->Kp;
     pl->PH = pl->PW = 0;
     if (!type_act_ternary(w->type)) {
         pl->PH = g.PH; pl->PW = g.PW;
@@ -930,7 +931,7 @@ int tnns_cuda_conv_ws(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const floa
         // 16.2 / 12.7, BNN 32 x 128x28x28 -> 128 s2 13.6 / 11.2, BNN 16 x 320x28x28 -> 320 27.7 / 24.6
         if (auto_both && type_act_ternary(w->type) && tnns_fused_supported(wide.w, wide.gv, d_x, layout) && one_launch_pays(ctx, w, g)) {
             TnnsFusedInput f;
-            f.d_x = d_x; f.d_thr = d_thr; f.C = g.C; f.Cp = g.Cp;
+            f.d_x = d_x; f.d_thr = d_thr; f.Cp = g.Cp;
             f.d_sync = reinterpret_cast<unsigned int*>(static_cast<char*>(d_workspace) + wide.image_bytes);
             return tnns_launch_gemm_im2col(ctx, wide.w, d_workspace, d_y, wide.gv, alpha, layout, (cudaStream_t)stream, 0, nullptr, nullptr, 1, &f);
         }

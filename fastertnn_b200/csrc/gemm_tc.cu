@@ -1317,9 +1317,7 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
     int fused_self_clean = 0;
     if (fused) {
         if (!fused->d_x || !fused->d_thr || !fused->d_sync) return tnns_fail(TNNS_ERR_INVALID, "NULL argument");
-        TnnsGeom gx = g;
-        gx.C = fused->C;
-        if (!tnns_fused_supported(w, gx, fused->d_x, layout))
+        if (!tnns_fused_supported(w, g, fused->d_x, layout))
             return tnns_fail(TNNS_ERR_UNSUPPORTED, "fused quantisation needs a 16-byte aligned input: NCHW with H*W a multiple of four, or NHWC with C a multiple of four");
         if (reinterpret_cast<uintptr_t>(fused->d_sync) & 127) return tnns_fail(TNNS_ERR_INVALID, "synchronisation words must be 128-byte aligned");
         int rc0 = tnns_fused_sync_prepare(ctx, g.N, stream, fused->d_sync, &fused_words, &fused_self_clean);
@@ -1368,9 +1366,9 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
         const unsigned long long HW = (unsigned long long)g.H * g.W;
         // (pixel-major input: one row of C floats per pixel of any image; box = 128 pixels x 32 channels, 128-byte swizzle)
         if (layout == TNNS_NHWC)
-            rc = tnns_tensor_map_2d(&map_q, 4, fused->d_x, (unsigned long long)fused->C, (unsigned long long)g.N * HW, (unsigned long long)fused->C * 4, 32, Q_PIX, 128);
+            rc = tnns_tensor_map_2d(&map_q, 4, fused->d_x, (unsigned long long)g.C, (unsigned long long)g.N * HW, (unsigned long long)g.C * 4, 32, Q_PIX, 128);
         else
-            rc = tnns_tensor_map_nchw(&map_q, fused->d_x, g.N, fused->C, (long long)HW, Q_PIX, 64);
+            rc = tnns_tensor_map_nchw(&map_q, fused->d_x, g.N, g.C, (long long)HW, Q_PIX, 64);
         if (rc) return rc;
         a.q_nhwc = layout == TNNS_NHWC;
         a.qx = fused->d_x;
@@ -1379,7 +1377,7 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
         a.q_sync = fused_words;
         a.q_self_clean = fused_self_clean;
         a.qN = g.N;
-        a.qC = fused->C;
+        a.qC = g.C;
         a.q_cp = fused->Cp;
         a.q_nbands = (g.H * g.W + Q_PIX - 1) / Q_PIX;
     }

@@ -141,7 +141,7 @@ struct TnnsFusedInput {
     const float* d_x;
     const float* d_thr;
     unsigned int* d_sync;
-    int C, Cp;  // channels of the fp32 input and their 64-channel words (the image's pixel may be padded to more)
+    int Cp;  // 64-channel words of the fp32 input's channels (the geometry's Cp is the image's pixel, which may be padded to more)
 };
 size_t tnns_fused_sync_bytes(int N);
 bool tnns_fused_supported(const tnns_cuda_weights* w, const TnnsGeom& g, const float* d_x, int layout);

@@ -123,3 +123,31 @@ def test_ragged_channels_in_one_launch(layer, N, gpu_ctx, checker):
         for p in (d_t, d_x, d_y):
             ctx.free(p)
         w.free()
+
+
+# tiles of 128 rows x 256 kernels on either side of three per SM (148 SMs); the form that quantises inside the GEMM launch fetches
+# pixel-major rows in 16-byte multiples, so C % 4 decides between one launch and two
+@pytest.mark.parametrize("type_,layer,N,launches", [
+    (TNN, Layer(262, 21, 20, 512, 3, 3, 1, 1), 70, 2), (TNN, Layer(262, 21, 20, 512, 3, 3, 1, 1), 63, 2), (TBN, Layer(130, 20, 20, 400, 3, 3, 1, 1), 75, 2),
+    (TNN, Layer(390, 14, 14, 512, 3, 3, 1, 1), 150, 2), (TNN, Layer(262, 1, 1, 4096, 1, 1, 0, 1), 4000, 2), (TNN, Layer(132, 20, 20, 400, 3, 3, 1, 1), 75, 1),
+    (TBN, Layer(192, 24, 24, 368, 3, 3, 1, 1), 52, 1), (TNN, Layer(192, 24, 24, 368, 3, 3, 1, 1), 48, 2)], ids=lambda v: str(v).replace(" ", ""))
+def test_ragged_channels_pixel_major(type_, layer, N, launches, gpu_ctx, checker):
+    from cases import threaded_conv
+    case = make_case(type_, layer, N, 8400 + layer.C, "uniform")
+    wp = checker.pack_weights(wgt_ternary(type_), case.w, case.w_thr)
+    want = threaded_conv(checker, type_, case.x, case.thr, wp, layer)
+    ctx = gpu_ctx
+    w = ctx.upload_weights(type_, wp, layer.C, layer.KH, layer.KW)
+    d_t, d_x, d_y = ctx.to_device(case.thr), ctx.to_device(to_nhwc(case.x)), ctx.malloc(want.nbytes)
+    try:
+        for _ in range(2):
+            ctx.fill(d_y, np.full(want.size, np.nan, np.float32))
+            before = ft.api.launch_count()
+            ctx.conv(w, d_x, d_t, d_y, layer.shape(N), case.alpha, ft.NHWC)
+            assert ft.api.launch_count() - before == launches
+            ctx.sync()
+            assert to_nchw(ctx.to_host(d_y, (N, layer.OH, layer.OW, layer.KN), np.float32)).tobytes() == want.tobytes()
+    finally:
+        for p in (d_t, d_x, d_y):
+            ctx.free(p)
+        w.free()
