@@ -424,6 +424,13 @@ int tnns_cuda_quantise_e2m1(tnns_cuda_ctx* ctx, const float* d_x, const float* d
     return tnns_launch_quantise(ctx, true, d_x, d_thr, d_image, N, C, H, W, layout, (cudaStream_t)stream, TNNS_IMG_E2M1);
 }
 
+// What the public calls on a plain 4-bit image take.  The launcher itself also takes binary activations, from an image that
+// holds +1 for absent channels and padding; the one tnns_cuda_quantise_e2m1 writes is ternary.
+static int im2col_call_ok(const tnns_cuda_weights* w, const TnnsGeom& g) {
+    if (g.N == 0 || tnns_im2col_supported(w, g)) return TNNS_OK;
+    return tnns_fail(TNNS_ERR_UNSUPPORTED, "layer shape or type outside the tensor-copy activation path");
+}
+
 int tnns_cuda_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const void* d_image, float* d_y, const tnns_shape_t* s,
                           float alpha, int layout, int pairs, void* stream) {
     if (pairs < 0 || pairs > 2) return tnns_fail(TNNS_ERR_INVALID, "pairs must be 0, 1 or 2");
@@ -436,6 +443,7 @@ int tnns_cuda_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
     if (layout != TNNS_NCHW && layout != TNNS_NHWC) return tnns_fail(TNNS_ERR_INVALID, "unknown layout %d", layout);
     TNNS_ENTER(ctx, w);
     if (reinterpret_cast<uintptr_t>(d_image) & 31) return tnns_fail(TNNS_ERR_INVALID, "image must be 32-byte aligned");
+    if ((rc = im2col_call_ok(w, g))) return rc;
     return tnns_launch_gemm_im2col(ctx, w, d_image, d_y, g, alpha, layout, (cudaStream_t)stream, pairs);
 }
 
@@ -782,6 +790,7 @@ int tnns_cuda_gemm_im2col_packed_out(tnns_cuda_ctx* ctx, const tnns_cuda_weights
         return tnns_fail(TNNS_ERR_INVALID, "input image must be 32-byte, output image 16-byte aligned");
     if (pairs < 0 || pairs > 2) return tnns_fail(TNNS_ERR_INVALID, "pairs must be 0, 1 or 2");
     if (next_format < 0 || next_format > 2) return tnns_fail(TNNS_ERR_INVALID, "output format must be 0, 1 or 2");
+    if ((rc = im2col_call_ok(w, g))) return rc;
     return tnns_launch_gemm_im2col(ctx, w, d_image, nullptr, g, alpha, TNNS_NCHW, (cudaStream_t)stream, pairs, d_image_out, d_thr_next,
                                    next_format);
 }
@@ -799,6 +808,7 @@ int tnns_cuda_gemm_im2col_bordered_out(tnns_cuda_ctx* ctx, const tnns_cuda_weigh
     if ((reinterpret_cast<uintptr_t>(d_image) & 31) || (reinterpret_cast<uintptr_t>(d_image_out) & 127))
         return tnns_fail(TNNS_ERR_INVALID, "input image must be 32-byte, bordered output image 128-byte aligned");
     if (pairs < 0 || pairs > 2) return tnns_fail(TNNS_ERR_INVALID, "pairs must be 0, 1 or 2");
+    if ((rc = im2col_call_ok(w, g))) return rc;
     return tnns_launch_gemm_im2col(ctx, w, d_image, nullptr, g, alpha, TNNS_NCHW, (cudaStream_t)stream, pairs, d_image_out, d_thr_next, 3, nullptr,
                                    next_PH, next_PW);
 }

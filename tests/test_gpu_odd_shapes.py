@@ -151,3 +151,27 @@ def test_ragged_channels_pixel_major(type_, layer, N, launches, gpu_ctx, checker
         for p in (d_t, d_x, d_y):
             ctx.free(p)
         w.free()
+
+
+@pytest.mark.parametrize("type_", [BTN, BNN])
+def test_im2col_calls_refuse_binary_activations(type_, gpu_ctx, checker):
+    """Unpadded layers too, whose geometry alone would fit: the 4-bit image these calls read is a ternary one."""
+    layer, N = Layer(200, 8, 8, 160, 1, 1, 0, 1), 3
+    case = make_case(type_, layer, N, 8500, "uniform")
+    wp = checker.pack_weights(wgt_ternary(type_), case.w, case.w_thr)
+    ctx, shape = gpu_ctx, layer.shape(N)
+    w = ctx.upload_weights(type_, wp, layer.C, layer.KH, layer.KW)
+    d_t, d_img = ctx.to_device(case.thr), ctx.malloc(ft.api.e2m1_image_bytes(N, layer.C, layer.H, layer.W))
+    d_y = ctx.malloc(4 * N * layer.KN * layer.OH * layer.OW)
+    try:
+        assert not ctx.im2col_supported(w, shape)
+        calls = [lambda: ctx.gemm_im2col(w, d_img, d_y, shape, 0.5), lambda: ctx.gemm_im2col_bordered_out(w, d_img, d_y, d_t, (1, 1), shape, 0.5)]
+        calls += [lambda f=f: ctx.gemm_im2col_packed_out(w, d_img, d_y, d_t, f, shape, 0.5) for f in (0, 1, 2)]
+        for call in calls:
+            with pytest.raises(ft.TnnsError) as e:
+                call()
+            assert e.value.status == 4
+    finally:
+        for p in (d_t, d_img, d_y):
+            ctx.free(p)
+        w.free()
