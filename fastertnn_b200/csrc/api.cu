@@ -851,6 +851,16 @@ static bool wide_plan(const tnns_cuda_weights* w, const TnnsGeom& g, WidePlan* p
     pl->bytes = pl->image_bytes + tnns_fused_sync_bytes(g.N);
     return true;
 }
+// The one-launch form is not recorded for these layers: its synchronisation words may have to be allocated first, which a
+// capture forbids, and a graph may be replayed on any stream while the context's words serve another.
+static bool being_captured(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+        (void)cudaGetLastError();  // the legacy stream while another stream captures: the launches below report it
+        return true;
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
 // What any route of a whole layer may want as workspace.
 static size_t conv_workspace_bytes(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s, const TnnsGeom& g) {
     // room for the im2row matrix (explicit route) and, where the layer qualifies, for the 4-bit
@@ -939,7 +949,8 @@ int tnns_cuda_conv_ws(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const floa
         // Measured on B200 against the gathering GEMM that took these layers before (layer call, us): 8 x 320x15x23 -> 320 s2
         // 18.3 / 12.4, 32 x 192x28x28 -> 192 25.1 / 20.1, NHWC 63 x 262x21x20 -> 512 54 / 41, BTN 8 x 256x14x14 -> 256 s2
         // 16.2 / 12.7, BNN 32 x 128x28x28 -> 128 s2 13.6 / 11.2, BNN 16 x 320x28x28 -> 320 27.7 / 24.6
-        if (auto_both && type_act_ternary(w->type) && tnns_fused_supported(wide.w, wide.gv, d_x, layout) && one_launch_pays(ctx, w, g)) {
+        if (auto_both && type_act_ternary(w->type) && tnns_fused_supported(wide.w, wide.gv, d_x, layout) && one_launch_pays(ctx, w, g) &&
+            !being_captured((cudaStream_t)stream)) {
             TnnsFusedInput f;
             f.d_x = d_x; f.d_thr = d_thr; f.Cp = g.Cp;
             f.d_sync = reinterpret_cast<unsigned int*>(static_cast<char*>(d_workspace) + wide.image_bytes);

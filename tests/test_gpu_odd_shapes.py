@@ -175,3 +175,31 @@ def test_im2col_calls_refuse_binary_activations(type_, gpu_ctx, checker):
         for p in (d_t, d_img, d_y):
             ctx.free(p)
         w.free()
+
+
+def test_ragged_channels_first_call_inside_a_capture(gpu_ctx, checker):
+    """A context whose first call of the layer is recorded into a graph: nothing may be allocated there, and the graph keeps no
+    state of the context's (it is replayed on another stream than it was recorded on)."""
+    import torch
+    from cases import threaded_conv
+    layer, N = Layer(130, 20, 20, 400, 3, 3, 1, 1), 75
+    case = make_case(TNN, layer, N, 8700, "uniform")
+    wp = checker.pack_weights(True, case.w, case.w_thr)
+    want = threaded_conv(checker, TNN, case.x, case.thr, wp, layer)
+    ctx, nb = ft.Context(0), 32 << 20
+    w = ctx.upload_weights(TNN, wp, layer.C, layer.KH, layer.KW)
+    d_t, d_x, d_y, d_ws = ctx.to_device(case.thr), ctx.to_device(case.x), ctx.malloc(want.nbytes), ctx.malloc(nb)
+    try:
+        s, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            ctx.conv_ws(w, d_x, d_t, d_y, d_ws, nb, layer.shape(N), case.alpha, ft.NCHW, ft.PACK_AUTO, ft.GEMM_AUTO, s.cuda_stream)
+        for rep in range(2):
+            ctx.fill(d_y, np.full(want.size, np.nan, np.float32))
+            graph.replay()
+            torch.cuda.synchronize()
+            assert ctx.to_host(d_y, want.shape, np.float32).tobytes() == want.tobytes(), rep
+    finally:
+        for p in (d_t, d_x, d_y, d_ws):
+            ctx.free(p)
+        w.free()
+        ctx.close()
