@@ -907,7 +907,7 @@ int tnns_cuda_conv_ws(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const floa
         const size_t ws_need = one_launch ? tnns_slab_workspace_bytes(g.N, g.C, g.H, g.W, g.PH, g.PW)
                                           : tnns_bordered_image_bytes(g.N, g.C, g.H, g.W, g.PH, g.PW);
         if (pack_algo != TNNS_PACK_AUTO || (layout != TNNS_NCHW && (one_launch || layout != TNNS_NHWC)) || !tnns_slab_supported(ctx, w, g, one_launch) ||
-            (!auto_both && !bordered_quantise_ok(d_x, g.N, g.C, g.H, g.W, layout)) || (reinterpret_cast<uintptr_t>(d_workspace) & 127) || ws_need > workspace_bytes)
+            (one_launch && !bordered_quantise_ok(d_x, g.N, g.C, g.H, g.W, layout)) || (reinterpret_cast<uintptr_t>(d_workspace) & 127) || ws_need > workspace_bytes)
             return tnns_fail(TNNS_ERR_UNSUPPORTED, "layer, layout, workspace size or alignment outside the slab-fed route");
         if (one_launch) return tnns_cuda_conv_slab(ctx, w, d_x, d_thr, d_y, d_workspace, workspace_bytes, s, alpha, 0, stream);
         rc = tnns_launch_quantise(ctx, type_act_ternary(w->type), d_x, d_thr, d_workspace, g.N, g.C, g.H, g.W, layout, (cudaStream_t)stream, TNNS_IMG_E2M1,

@@ -203,3 +203,35 @@ def test_ragged_channels_first_call_inside_a_capture(gpu_ctx, checker):
             ctx.free(p)
         w.free()
         ctx.close()
+
+
+@pytest.mark.parametrize("type_,layer,N,layout,offset", [
+    (TNN, Layer(64, 31, 33, 64, 3, 3, 1, 1), 2, ft.NCHW, 0), (TNN, Layer(64, 32, 32, 64, 3, 3, 1, 1), 2, ft.NCHW, 4), (TBN, Layer(70, 20, 20, 96, 3, 3, 1, 1), 2, ft.NHWC, 0),
+    (BTN, Layer(256, 15, 17, 64, 3, 3, 1, 1), 2, ft.NCHW, 0), (BNN, Layer(128, 1, 1, 64, 1, 1, 0, 1), 5, ft.NHWC, 4)], ids=lambda v: str(v).replace(" ", ""))
+def test_the_reported_algorithm_can_be_asked_for(type_, layer, N, layout, offset, gpu_ctx, checker):
+    """Inputs the copy engine cannot fetch: what conv_auto_algo answers is what the call takes, by itself and on request."""
+    case = make_case(type_, layer, N, 8600 + layer.C, "uniform")
+    wp = checker.pack_weights(wgt_ternary(type_), case.w, case.w_thr)
+    want = checker.conv(type_, case.x, case.thr, wp, case.kernel_hw, case.padding, case.stride, case.alpha)
+    ctx, shape = gpu_ctx, layer.shape(N)
+    w = ctx.upload_weights(type_, wp, layer.C, layer.KH, layer.KW)
+    d_t, d_y, base = ctx.to_device(case.thr), ctx.malloc(want.nbytes), ctx.malloc(case.x.nbytes + 16)
+    d_x = base + offset
+    try:
+        ctx.fill(d_x, case.x if layout == ft.NCHW else to_nhwc(case.x))
+        algo = ctx.conv_auto_algo(w, shape, d_x, layout)
+        assert algo == ft.GEMM_F4_SLAB
+        for how in (ft.GEMM_AUTO, algo):
+            ctx.fill(d_y, np.full(want.size, np.nan, np.float32))
+            ctx.conv(w, d_x, d_t, d_y, shape, case.alpha, layout, ft.PACK_AUTO, how)
+            ctx.sync()
+            got = ctx.to_host(d_y, want.shape if layout == ft.NCHW else (N, layer.OH, layer.OW, layer.KN), np.float32)
+            assert (got if layout == ft.NCHW else to_nchw(got)).tobytes() == want.tobytes(), how
+        # the one launch reads through the copy engine: still refused
+        with pytest.raises(ft.TnnsError) as e:
+            ctx.conv(w, d_x, d_t, d_y, shape, case.alpha, layout, ft.PACK_AUTO, ft.GEMM_F4_SLAB_FUSED)
+        assert e.value.status == 4
+    finally:
+        for p in (d_t, d_y, base):
+            ctx.free(p)
+        w.free()
