@@ -97,6 +97,7 @@ SIGNATURES = {
     "tnns_cuda_multi_free_weights": (None, [_vp, _vp]),
     "tnns_cuda_multi_conv_host": (_i, [_vp, _vp, _vp, _vp, _vp, _pshape, _f, _i, C.POINTER(_i)]),
     "tnns_cuda_noalloc_scratch_bytes": (_sz, []),
+    "tnns_cuda_conv_workspace_bytes": (_sz, [_vp, _vp, _pshape]),
     "tnns_cuda_conv_noalloc": (_i, [_i, _vp, _vp, _vp, _vp, _pshape, _f, _i, _vp]),
     "tnns_cuda_pipe_rate": (_i, [_vp, _i, C.POINTER(C.c_double)]),
     "tnns_cuda_selftest_wait_expiry": (_i, [_vp]),

@@ -278,6 +278,10 @@ class Context:
         _check(self.lib.tnns_cuda_conv(self.handle, w.handle, d_x, d_thr, d_y, C.byref(shape), alpha, layout, pack_algo,
                                        gemm_algo, stream))
 
+    def conv_workspace_bytes(self, w: Weights, shape: Shape) -> int:
+        """Workspace with which conv_ws (AUTO algorithms) has every route of this layer to choose from; 128-byte aligned."""
+        return int(self.lib.tnns_cuda_conv_workspace_bytes(self.handle, w.handle, C.byref(shape)))
+
     def conv_ws(self, w: Weights, d_x: int, d_thr: int, d_y: int, d_ws: int, ws_bytes: int, shape: Shape, alpha: float,
                 layout=NCHW, pack_algo=PACK_AUTO, gemm_algo=GEMM_AUTO, stream=0):
         _check(self.lib.tnns_cuda_conv_ws(self.handle, w.handle, d_x, d_thr, d_y, d_ws, ws_bytes, C.byref(shape), alpha, layout,

@@ -861,17 +861,28 @@ static bool being_captured(cudaStream_t stream) {
     }
     return status != cudaStreamCaptureStatusNone;
 }
-// What any route of a whole layer may want as workspace.
-static size_t conv_workspace_bytes(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s, const TnnsGeom& g) {
-    // room for the im2row matrix (explicit route) and, where the layer qualifies, for the 4-bit
-    // image of the copy-engine routes, which is larger than the matrix for 1x1 kernels
-    size_t need = std::max<size_t>(tnns_packed_bytes(w->type, s), 16);
+// What the default algorithms may want as workspace: the image of every copy-engine route the layer qualifies for, and what is
+// left without one -- the gathering GEMM's bit planes, or the packed matrix where no kernel gathers.
+static size_t auto_workspace_bytes(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s, const TnnsGeom& g) {
+    const bool gathers = w->d_f4 && w->d_jtab && w->Kp < 65536;
+    size_t need = gathers ? tnns_packed_image_bytes(type_act_ternary(w->type), g.N, g.C, g.H, g.W) : tnns_packed_bytes(w->type, s);
     if (tnns_im2col_supported(w, g)) need = std::max(need, tnns_fused_workspace_bytes(g.N, g.C, g.H, g.W));
     if (tnns_slab_supported(ctx, w, g, false)) need = std::max(need, tnns_slab_workspace_bytes(g.N, g.C, g.H, g.W, g.PH, g.PW));
     if (tnns_cuda_dense_supported(ctx, w, s)) need = std::max(need, tnns_dense_workspace_bytes(s));
     WidePlan wide;
     if (wide_plan(w, g, &wide)) need = std::max(need, wide.bytes);
     return need;
+}
+// ... and what any route may want, the explicit one with its packed matrix included
+static size_t conv_workspace_bytes(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s, const TnnsGeom& g) {
+    return std::max(std::max<size_t>(tnns_packed_bytes(w->type, s), 16), auto_workspace_bytes(ctx, w, s, g));
+}
+
+size_t tnns_cuda_conv_workspace_bytes(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s) {
+    TnnsGeom g;
+    if (!ctx || !w || !s || tnns_make_geom(s, &g)) return 0;
+    if (s->KN != w->KN || s->C != w->C || s->KH != w->KH || s->KW != w->KW) return 0;
+    return std::max<size_t>(auto_workspace_bytes(ctx, w, s, g), 16);
 }
 
 int tnns_cuda_conv_ws(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const float* d_x, const float* d_thr, float* d_y,

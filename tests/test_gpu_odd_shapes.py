@@ -83,7 +83,7 @@ def test_layers_of_any_channel_count_and_alphabet(layer, N, type_, gpu_ctx, chec
     ctx = gpu_ctx
     w = ctx.upload_weights(type_, wp, layer.C, layer.KH, layer.KW)
     d_t, d_y = ctx.to_device(case.thr), ctx.malloc(want.nbytes)
-    nb = 1 << 22
+    nb = -(-ctx.conv_workspace_bytes(w, layer.shape(N)) // 4) * 4
     d_ws = ctx.malloc(nb)
     try:
         for layout in (ft.NCHW, ft.NHWC):
@@ -235,3 +235,88 @@ def test_the_reported_algorithm_can_be_asked_for(type_, layer, N, layout, offset
         for p in (d_t, d_y, base):
             ctx.free(p)
         w.free()
+
+
+@pytest.mark.parametrize("type_", [TNN, TBN, BTN, BNN])
+@pytest.mark.parametrize("layer,N", WIDE_LAYERS + [(Layer(320, 12, 12, 64, 1, 1, 0, 1), 2), (Layer(3, 12, 12, 64, 3, 3, 1, 1), 2), (Layer(64, 30, 30, 64, 3, 3, 1, 1), 1)],
+                         ids=lambda v: str(v).replace(" ", ""))
+def test_workspace_of_the_queried_size_holds_every_route(layer, N, type_, gpu_ctx, checker):
+    """conv_ws in exactly conv_workspace_bytes() bytes writes the image of the route conv() takes, not that of one with a smaller
+    workspace, and nothing past them."""
+    case = make_case(type_, layer, N, 8900 + layer.C, "uniform")
+    wp = checker.pack_weights(wgt_ternary(type_), case.w, case.w_thr)
+    want = checker.conv(type_, case.x, case.thr, wp, case.kernel_hw, case.padding, case.stride, case.alpha)
+    ctx, shape = gpu_ctx, layer.shape(N)
+    w = ctx.upload_weights(type_, wp, layer.C, layer.KH, layer.KW)
+    nb = ctx.conv_workspace_bytes(w, shape)
+    tern, cp = type_ in (TNN, TBN), (layer.C + 63) // 64
+    assert nb >= ft.api.packed_image_bytes(tern, N, layer.C, layer.H, layer.W)
+    if ctx.im2col_supported(w, shape):
+        assert nb >= ft.api.fused_workspace_bytes(N, layer.C, layer.H, layer.W)
+    if ctx.slab_supported(w, shape):
+        assert nb >= ft.api.slab_workspace_bytes(N, layer.C, layer.H, layer.W, layer.P, layer.P)
+    if ctx.dense_supported(w, shape):
+        assert nb >= ft.api.dense_workspace_bytes(shape)
+    assert ctx.conv_workspace_bytes(w, Layer(layer.C + 1, layer.H, layer.W, layer.KN, layer.KH, layer.KW, layer.P, layer.S).shape(N)) == 0
+    guard = 4096
+    d_t, d_x, d_y, d_ws = ctx.to_device(case.thr), ctx.to_device(case.x), ctx.malloc(want.nbytes), ctx.malloc((nb + 3) // 4 * 4 + guard)
+    try:
+        ctx.fill(d_ws, np.full((nb + 3) // 4 + guard // 4, 0x55555555, np.uint32))   # no 4-bit operand is a 5
+        ctx.fill(d_y, np.full(want.size, np.nan, np.float32))
+        ctx.conv_ws(w, d_x, d_t, d_y, d_ws, nb, shape, case.alpha)
+        ctx.sync()
+        assert ctx.to_host(d_y, want.shape, np.float32).tobytes() == want.tobytes()
+        ws = ctx.to_host(d_ws, ((nb + 3) // 4 * 4 + guard,), np.uint8)
+        assert (ws[nb:] == 0x55).all(), "past the workspace"
+        if ctx.conv_auto_algo(w, shape, d_x) != ft.GEMM_F4_DENSE:
+            border = layer.P if not tern or ctx.conv_auto_algo(w, shape, d_x) == ft.GEMM_F4_SLAB else 0
+            pitch = 32 * (cp if cp <= 2 else -(-cp // 4) * 4)
+            last = N * (layer.H + 2 * border) * (layer.W + 2 * border) * pitch - pitch   # the last pixel of the 4-bit image
+            px = ws[last:last + 32 * cp]
+            assert np.isin(px & 15, (0, 2, 10)).all() and np.isin(px >> 4, (0, 2, 10)).all()
+    finally:
+        for p in (d_t, d_x, d_y, d_ws):
+            ctx.free(p)
+        w.free()
+
+
+@pytest.mark.parametrize("type_", [TNN, TBN])
+def test_ragged_channels_in_one_launch_on_two_streams(type_, checker):
+    """The context's own synchronisation words serve the stream that came first, the words behind the image any other one."""
+    import torch
+    from cases import threaded_conv
+    layer, N = Layer(130, 20, 20, 400, 3, 3, 1, 1), 75
+    case = make_case(type_, layer, N, 8350, "uniform")
+    wp = checker.pack_weights(wgt_ternary(type_), case.w, case.w_thr)
+    want = threaded_conv(checker, type_, case.x, case.thr, wp, layer)
+    ctx = ft.Context(0)
+    w = ctx.upload_weights(type_, wp, layer.C, layer.KH, layer.KW)
+    shape = layer.shape(N)
+    nb = ctx.conv_workspace_bytes(w, shape)
+    d_t, d_x = ctx.to_device(case.thr), ctx.to_device(case.x)
+    d_y, d_ws = [ctx.malloc(want.nbytes) for _ in range(2)], [ctx.malloc(nb) for _ in range(2)]
+    side = torch.cuda.Stream()
+    streams = [0, side.cuda_stream]
+    try:
+        for k in range(2):
+            ctx.fill(d_y[k], np.full(want.size, np.nan, np.float32))
+            ctx.fill(d_ws[k], np.full(nb // 4, 0xFFFFFFFF, np.uint32))
+        before = ft.api.launch_count()
+        for rep in range(3):
+            for k in range(2):
+                ctx.conv_ws(w, d_x, d_t, d_y[k], d_ws[k], nb, shape, case.alpha, ft.NCHW, ft.PACK_AUTO, ft.GEMM_AUTO, streams[k])
+        assert ft.api.launch_count() - before == 6, "one launch each"
+        torch.cuda.synchronize()
+        ctx.sync()
+        for k in range(2):
+            assert ctx.to_host(d_y[k], want.shape, np.float32).tobytes() == want.tobytes(), k
+        # a workspace too small for the words behind the image: two launches
+        ctx.conv_ws(w, d_x, d_t, d_y[0], d_ws[0], nb - 128, shape, case.alpha)
+        ctx.sync()
+        assert ctx.to_host(d_y[0], want.shape, np.float32).tobytes() == want.tobytes()
+        assert ft.api.launch_count() - before == 8
+    finally:
+        for p in [d_t, d_x] + d_y + d_ws:
+            ctx.free(p)
+        w.free()
+        ctx.close()
