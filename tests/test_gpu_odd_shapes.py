@@ -30,7 +30,7 @@ def numpy_planes(x, thr, tern):
 
 @pytest.mark.parametrize("tern", [True, False])
 @pytest.mark.parametrize("N,C,H,W", [(1, 1, 1, 1), (3, 33, 1, 1), (1, 64, 5, 5), (5, 65, 7, 3), (2, 31, 31, 33), (33, 130, 1, 7), (4, 262, 9, 5), (7, 3, 15, 23),
-                                     (2, 64, 8, 8), (3, 192, 6, 6)])
+                                     (2, 64, 8, 8), (3, 192, 6, 6), (2, 8, 7, 5), (2, 9, 7, 5), (2, 16, 7, 5), (2, 17, 7, 5), (2, 24, 7, 5), (2, 25, 7, 5), (2, 126, 7, 5)])
 def test_quantise_with_plain_loads(N, C, H, W, tern, gpu_ctx):
     """One pixel, one channel, tails on both sides of 32 and 64 channels, pixel counts around 32, warps that straddle
     images; and sizes the copy engine would take, from a base that is not 16-byte aligned."""
