@@ -427,7 +427,9 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
         tnns_thr::Pair qt = {0.f, 0.f};
         int qt_img = -1;
         // pixel-major fp32 output: the accumulator is fetched in the 16x256b shape (four lanes = 32 contiguous bytes of a row)
-        const bool rows16 = p.pimg == nullptr && p.layout == TNNS_NHWC && (p.KN & 1) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
+        // (float pairs; on narrow tiles single floats as well)
+        const bool row_pairs = (p.KN & 1) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
+        const bool rows16 = p.pimg == nullptr && p.layout == TNNS_NHWC && (NSETS > 1 || row_pairs);
         for (int t = unit + set * nunits; t < ntiles; t += NSETS * nunits, lt += NSETS) {
             const int buf = (int)(lt % NBUF);
             const int n0 = (t % ntn) * BN;
@@ -486,7 +488,8 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
                     const int c0 = n0 + cb;
                     float* const yrow[4] = {yrow0[0] ? yrow0[0] + c0 : nullptr, yrow0[1] ? yrow0[1] + c0 : nullptr,
                                             yrow0[2] ? yrow0[2] + c0 : nullptr, yrow0[3] ? yrow0[3] + c0 : nullptr};
-                    store_rows16_at(f, yrow, p.KN - c0, lane);
+                    if (NSETS == 1 || row_pairs) store_rows16_at(f, yrow, p.KN - c0, lane);
+                    else store_rows16_at<false>(f, yrow, p.KN - c0, lane);
                     continue;
                 }
                 asm volatile(

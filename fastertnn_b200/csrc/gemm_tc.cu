@@ -714,7 +714,10 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
         if (F4 && !QF && p.pimg && p.pimg_e2m1 && p.o_HpWp)
             fill_output_border(reinterpret_cast<uint4*>(p.pimg), p.cp_next, p.OHW / p.OW, p.OW, (int)(p.M / p.OHW), p.o_PH, p.o_PW,
                                ((long long)(warp - WARP_EPI0) * gridDim.x + blockIdx.x) * 32 + lane, (long long)gridDim.x * (blockDim.x - 32 * WARP_EPI0));
-        const bool rows16 = F4 && p.pimg == nullptr && p.layout == TNNS_NHWC && (p.KN & 1) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
+        // pixel-major fp32 output in the 16x256b shape: float pairs, on narrow tiles single floats as well (64 x 64x56x56 -> 25
+        // 41.9 us per layer call with a row per lane, 24.4 so; -> 63 84.8 and 43.5)
+        const bool row_pairs = (p.KN & 1) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
+        const bool rows16 = F4 && p.pimg == nullptr && p.layout == TNNS_NHWC && (NSETS > 1 || row_pairs);
         tnns_thr::Pair qt = {0.f, 0.f};
         long long qt_img = -1;
         for (int t = unit + set * nunits; t < ntiles; t += NSETS * nunits, lt += NSETS) {
@@ -762,7 +765,9 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                     if (row0 < p.M) {
                         float f[32];
                         prelu32_f4(v, f, alpha_in_unit, p.acc_bias, bias_f, p.alpha, p.zero_passes);
-                        store_rows16(f, p.y + (size_t)row0 * p.KN + (n0 + cb), p.KN, p.M - row0, p.KN - (n0 + cb), lane);
+                        float* y0 = p.y + (size_t)row0 * p.KN + (n0 + cb);
+                        if (NSETS == 1 || row_pairs) store_rows16(f, y0, p.KN, p.M - row0, p.KN - (n0 + cb), lane);
+                        else store_rows16<false>(f, y0, p.KN, p.M - row0, p.KN - (n0 + cb), lane);
                     }
                     continue;
                 }
