@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(NTHREADS) gemm_popc_tiled_kernel(const uint32_
         const int c0 = n0 + warp * 8 + ln * 4;
         if (layout == TNNS_NHWC) {
             float* dst = y + (size_t)r * KN + c0;
-            if (c0 + 3 < KN && (KN & 3) == 0) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+            if (c0 + 3 < KN && (KN & 3) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0) *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
             else {
 #pragma unroll
                 for (int j = 0; j < RN; j++) if (c0 + j < KN) dst[j] = v[j];

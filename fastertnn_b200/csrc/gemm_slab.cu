@@ -44,6 +44,7 @@ struct SlabArgs {
     int Mv;                     // virtual rows: N * Hp * Wp
     int KN, nchunks;            // kernels, weight stages per kernel tile
     int b_rows;                 // kernels per tile of the weight image: BN, or a multiple of it (few tiles)
+    int y_vec;                  // floats of a pixel-major output row that may be stored at once: 4, 2 or 1
     int OH, OW, Wp, HpWp;       // output size, padded input lattice
     int KW, T;                  // filter width, taps KH*KW
     int G;                      // 128-byte channel groups per pixel (one slab each); 1 for 64 / 128 channels
@@ -286,9 +287,10 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
                     for (int cg = 0; cg < p.G; cg++) {
                         if (!mbar_wait(bar_sfull + 8 * sl, slph, abort_flag, p.status, 0x13)) goto done;
                         const uint32_t slab_lo = a_lo0 + sl * slab16;
-                        if (p.b_resident && first_tile) {
+                        if (BN == 256 && p.b_resident && first_tile) {
                             // stage by stage as the weights land (waiting for all of them first: 40 x 128x14x14 -> 256 BNN, one
-                            // tile per SM, 11.3 us per layer call against 10.3); rolled up, it runs once per block and group
+                            // tile per SM, 11.3 us per layer call against 10.3; on narrower tiles most of them were requested before the
+                            // wait for the launch in front); rolled up, it runs once per block and group
 #pragma unroll 1
                             for (int j = 0; j < NST; j++) {
                                 const uint32_t slot = (TAPS == 1) ? (uint32_t)(j * p.G + cg) : (uint32_t)j;
@@ -306,6 +308,9 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
                                 }
                             }
                         } else if (p.b_resident) {
+                            if (BN != 256 && first_tile)
+                                for (int j = 0; j < NST; j++)
+                                    if (!mbar_wait(bar_bfull + 8 * ((TAPS == 1) ? j * p.G + cg : j), 0u, abort_flag, p.status, 3)) goto done;
                             tc_fence_after();
                             if (elected) {
 #pragma unroll
@@ -428,8 +433,7 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
         int qt_img = -1;
         // pixel-major fp32 output: the accumulator is fetched in the 16x256b shape (four lanes = 32 contiguous bytes of a row)
         // (float pairs; on narrow tiles single floats as well)
-        const bool row_pairs = (p.KN & 1) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
-        const bool rows16 = p.pimg == nullptr && p.layout == TNNS_NHWC && (NSETS > 1 || row_pairs);
+        const bool rows16 = p.pimg == nullptr && p.layout == TNNS_NHWC && (NSETS > 1 || p.y_vec > 1);
         for (int t = unit + set * nunits; t < ntiles; t += NSETS * nunits, lt += NSETS) {
             const int buf = (int)(lt % NBUF);
             const int n0 = (t % ntn) * BN;
@@ -488,8 +492,8 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
                     const int c0 = n0 + cb;
                     float* const yrow[4] = {yrow0[0] ? yrow0[0] + c0 : nullptr, yrow0[1] ? yrow0[1] + c0 : nullptr,
                                             yrow0[2] ? yrow0[2] + c0 : nullptr, yrow0[3] ? yrow0[3] + c0 : nullptr};
-                    if (NSETS == 1 || row_pairs) store_rows16_at(f, yrow, p.KN - c0, lane);
-                    else store_rows16_at<false>(f, yrow, p.KN - c0, lane);
+                    if (NSETS == 1 || p.y_vec > 1) store_rows16_at(f, yrow, p.KN - c0, lane);
+                    else store_rows16_single(f, yrow, p.KN - c0, lane);
                     continue;
                 }
                 asm volatile(
@@ -581,7 +585,7 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
                             }
                         }
                     } else if (p.layout == TNNS_NHWC) {
-                        if (full && (p.KN & 3) == 0) {
+                        if (full && p.y_vec == 4) {
 #pragma unroll
                             for (int j = 0; j < 32; j += 4)
                                 __stcs(reinterpret_cast<float4*>(ybase + c0 + j), make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]));
@@ -808,6 +812,7 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
     a.KN = w->KN;
     a.nchunks = w->Kp / 4;
     a.b_rows = tnns_i8_tile_n(w->KN);
+    a.y_vec = tnns_row_vec(d_y, w->KN);
     a.OH = g.OH; a.OW = g.OW; a.Wp = pl.Wp; a.HpWp = pl.Hp * pl.Wp;
     a.KW = g.KW; a.T = pl.T; a.G = pl.G;
     a.slab_bytes = pl.slab_bytes; a.copy_rows = pl.copy_rows; a.ncopies = pl.ncopies;

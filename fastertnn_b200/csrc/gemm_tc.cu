@@ -230,6 +230,7 @@ struct GemmArgs {
     long long M;
     int KN, Kp, OHW, layout;
     int b_rows;                 // kernels per tile of the weight image: BN, or a multiple of it (tensor-copy form, few tiles)
+    int y_vec;                  // floats of a pixel-major output row that may be stored at once: 4, 2 or 1
     int a_two_planes;
     int acc_bias;               // added to the integer dot product (BNN: K_unpack minus the positions multiplied)
     float alpha;
@@ -716,8 +717,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                                ((long long)(warp - WARP_EPI0) * gridDim.x + blockIdx.x) * 32 + lane, (long long)gridDim.x * (blockDim.x - 32 * WARP_EPI0));
         // pixel-major fp32 output in the 16x256b shape: float pairs, on narrow tiles single floats as well (64 x 64x56x56 -> 25
         // 41.9 us per layer call with a row per lane, 24.4 so; -> 63 84.8 and 43.5)
-        const bool row_pairs = (p.KN & 1) == 0 && (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
-        const bool rows16 = F4 && p.pimg == nullptr && p.layout == TNNS_NHWC && (NSETS > 1 || row_pairs);
+        const bool rows16 = F4 && p.pimg == nullptr && p.layout == TNNS_NHWC && (NSETS > 1 || p.y_vec > 1);
         tnns_thr::Pair qt = {0.f, 0.f};
         long long qt_img = -1;
         for (int t = unit + set * nunits; t < ntiles; t += NSETS * nunits, lt += NSETS) {
@@ -765,9 +765,17 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                     if (row0 < p.M) {
                         float f[32];
                         prelu32_f4(v, f, alpha_in_unit, p.acc_bias, bias_f, p.alpha, p.zero_passes);
-                        float* y0 = p.y + (size_t)row0 * p.KN + (n0 + cb);
-                        if (NSETS == 1 || row_pairs) store_rows16(f, y0, p.KN, p.M - row0, p.KN - (n0 + cb), lane);
-                        else store_rows16<false>(f, y0, p.KN, p.M - row0, p.KN - (n0 + cb), lane);
+                        if (NSETS == 1 || p.y_vec > 1) {
+                            store_rows16(f, p.y + (size_t)row0 * p.KN + (n0 + cb), p.KN, p.M - row0, p.KN - (n0 + cb), lane);
+                        } else {
+                            float* yrow[4];
+#pragma unroll
+                            for (int h = 0; h < 4; h++) {
+                                const long long r = row0 + 8 * h + (lane >> 2);
+                                yrow[h] = r < p.M ? p.y + (size_t)r * p.KN + (n0 + cb) : nullptr;
+                            }
+                            store_rows16_single(f, yrow, p.KN - (n0 + cb), lane);
+                        }
                     }
                     continue;
                 }
@@ -855,7 +863,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                             }
                         }
                     } else if (p.layout == TNNS_NHWC) {
-                        if (full && (p.KN & 3) == 0) {
+                        if (full && p.y_vec == 4) {
 #pragma unroll
                             for (int j = 0; j < 32; j += 4)
                                 __stcs(reinterpret_cast<float4*>(ybase + c0 + j), make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]));
@@ -1164,6 +1172,7 @@ int tnns_launch_gemm_tc(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const vo
     a.KN = w->KN;
     a.Kp = w->Kp;
     a.b_rows = tnns_i8_tile_n(w->KN);
+    a.y_vec = tnns_row_vec(d_y, w->KN);
     a.OHW = OHW;
     // one output pixel per image (fully connected layers): both layouts are the same memory, and the pixel-major
     // epilogue writes 16 bytes per lane where the channel-major one would write 4 (rows are KN floats apart either way)
@@ -1339,6 +1348,7 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
     a.KN = w->KN;
     a.Kp = w->Kp;
     a.b_rows = tnns_i8_tile_n(w->KN);
+    a.y_vec = tnns_row_vec(d_y, w->KN);
     a.OHW = g.OH * g.OW;
     a.layout = a.OHW == 1 ? TNNS_NHWC : layout;  // one pixel per image: same memory, wider stores (see above)
     a.a_two_planes = 1;

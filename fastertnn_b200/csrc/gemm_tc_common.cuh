@@ -249,19 +249,7 @@ __device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t* w) 
 
 // Stores what two such loads (lanes 0..15 and 16..31 of the warp's quadrant) delivered: f[16*hh + 4k + 2*b + {0,1}] is
 // row 16*hh + 8*b + lane/4 of the quadrant, columns 8k + 2(lane%4) and + 1 of the slice.  y_quad = the quadrant's first
-// row at the slice's first column; rows_left / cols_left = rows and columns that exist from there on.  PAIRS: KN is even and y
-// 8-byte aligned; else the two floats are stored one by one (narrow tiles only), two pieces of a sector back to back where a
-// row per lane would write it in eight.
-template <bool PAIRS>
-__device__ __forceinline__ void store_pair(float* y, float a, float b, int cols_left) {
-    if (PAIRS) {
-        if (cols_left > 0) __stcs(reinterpret_cast<float2*>(y), make_float2(a, b));
-    } else {
-        if (cols_left > 0) __stcs(y, a);
-        if (cols_left > 1) __stcs(y + 1, b);
-    }
-}
-template <bool PAIRS = true>
+// row at the slice's first column; rows_left / cols_left = rows and columns that exist from there on; KN is even.
 __device__ __forceinline__ void store_rows16(const float (&f)[32], float* y_quad, int KN, long long rows_left, int cols_left, int lane) {
     const int cc = 2 * (lane & 3);
 #pragma unroll
@@ -271,14 +259,14 @@ __device__ __forceinline__ void store_rows16(const float (&f)[32], float* y_quad
             float* yr = y_quad + (size_t)r * KN + cc;
 #pragma unroll
             for (int k = 0; k < 4; k++)
-                store_pair<PAIRS>(yr + 8 * k, f[16 * (h >> 1) + 4 * k + 2 * (h & 1)], f[16 * (h >> 1) + 4 * k + 2 * (h & 1) + 1], cols_left - 8 * k - cc);
+                if (8 * k + cc < cols_left)
+                    __stcs(reinterpret_cast<float2*>(yr + 8 * k), make_float2(f[16 * (h >> 1) + 4 * k + 2 * (h & 1)], f[16 * (h >> 1) + 4 * k + 2 * (h & 1) + 1]));
         }
     }
 }
 
 // The same for rows that are not neighbours in memory (the slab-fed GEMM's rows are positions of the padded lattice):
 // yrow[h] = where row 8*h + lane/4 of the quadrant starts at the slice's first column, or nullptr if that row is not stored.
-template <bool PAIRS = true>
 __device__ __forceinline__ void store_rows16_at(const float (&f)[32], float* const (&yrow)[4], int cols_left, int lane) {
     const int cc = 2 * (lane & 3);
 #pragma unroll
@@ -287,7 +275,25 @@ __device__ __forceinline__ void store_rows16_at(const float (&f)[32], float* con
             float* yr = yrow[h] + cc;
 #pragma unroll
             for (int k = 0; k < 4; k++)
-                store_pair<PAIRS>(yr + 8 * k, f[16 * (h >> 1) + 4 * k + 2 * (h & 1)], f[16 * (h >> 1) + 4 * k + 2 * (h & 1) + 1], cols_left - 8 * k - cc);
+                if (8 * k + cc < cols_left)
+                    __stcs(reinterpret_cast<float2*>(yr + 8 * k), make_float2(f[16 * (h >> 1) + 4 * k + 2 * (h & 1)], f[16 * (h >> 1) + 4 * k + 2 * (h & 1) + 1]));
+        }
+    }
+}
+
+// Either for rows whose floats cannot be stored in pairs (an odd KN, a base of 4 bytes): the two floats one by one, two pieces of a
+// sector back to back where a row per lane would write it in eight.
+__device__ __forceinline__ void store_rows16_single(const float (&f)[32], float* const (&yrow)[4], int cols_left, int lane) {
+    const int cc = 2 * (lane & 3);
+#pragma unroll
+    for (int h = 0; h < 4; h++) {
+        if (yrow[h]) {
+            float* yr = yrow[h] + cc;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (8 * k + cc < cols_left) __stcs(yr + 8 * k, f[16 * (h >> 1) + 4 * k + 2 * (h & 1)]);
+                if (8 * k + cc + 1 < cols_left) __stcs(yr + 8 * k + 1, f[16 * (h >> 1) + 4 * k + 2 * (h & 1) + 1]);
+            }
         }
     }
 }

@@ -171,6 +171,12 @@ int tnns_launch_pack_weights(tnns_cuda_ctx* ctx, bool ternary, const float* d_w,
 int tnns_launch_mma_rate(tnns_cuda_ctx* ctx, bool f4, int iters, double* ops, cudaStream_t stream);
 int tnns_launch_wait_selftest(tnns_cuda_ctx* ctx, cudaStream_t stream);
 
+// Floats that may be stored at once everywhere in a matrix of KN floats per row: rows and base allow 16, 8 or 4 bytes.
+static inline int tnns_row_vec(const float* y, int KN) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(y) | ((uintptr_t)KN * sizeof(float));
+    return (at & 15) == 0 ? 4 : (at & 7) == 0 ? 2 : 1;
+}
+
 // Division by a runtime-constant divisor without the hardware divide sequence.
 // Exact for every 32-bit unsigned numerator (Granlund-Montgomery round-up method).
 struct FastDiv {

@@ -320,3 +320,29 @@ def test_ragged_channels_in_one_launch_on_two_streams(type_, checker):
             ctx.free(p)
         w.free()
         ctx.close()
+
+
+# narrow and wide tiles of every GEMM: odd and even kernel counts (ragged last pairs), row bases that hold no pair or quad of floats
+@pytest.mark.parametrize("type_,layer,N", [
+    (TNN, Layer(64, 20, 20, 25, 3, 3, 1, 1), 30), (TNN, Layer(256, 14, 14, 101, 3, 3, 1, 1), 60), (BNN, Layer(128, 20, 20, 1, 3, 3, 1, 1), 5), (BTN, Layer(64, 20, 20, 64, 3, 3, 1, 1), 9),
+    (TBN, Layer(64, 15, 15, 127, 3, 3, 1, 2), 7), (TNN, Layer(3, 30, 30, 33, 3, 3, 1, 1), 40), (TNN, Layer(256, 14, 14, 300, 1, 1, 0, 1), 60)], ids=lambda v: str(v).replace(" ", ""))
+def test_pixel_major_rows_of_any_width_and_alignment(type_, layer, N, gpu_ctx, checker):
+    case = make_case(type_, layer, N, 9000 + layer.C, "uniform")
+    wp = checker.pack_weights(wgt_ternary(type_), case.w, case.w_thr)
+    want = to_nhwc(checker.conv(type_, case.x, case.thr, wp, case.kernel_hw, case.padding, case.stride, case.alpha))
+    ctx = gpu_ctx
+    w = ctx.upload_weights(type_, wp, layer.C, layer.KH, layer.KW)
+    d_t, d_x, d_y = ctx.to_device(case.thr), ctx.to_device(to_nhwc(case.x)), ctx.malloc(want.nbytes + 64)
+    try:
+        for off in (0, 4, 8):
+            for algo in (ft.GEMM_AUTO, ft.GEMM_F4_TC, ft.GEMM_I8_TC, ft.GEMM_POPC_TILED, ft.GEMM_POPC_SIMPLE):
+                ctx.fill(d_y, np.full(want.size + 16, np.nan, np.float32))
+                ctx.conv(w, d_x, d_t, d_y + off, layer.shape(N), case.alpha, ft.NHWC, ft.PACK_AUTO, algo)
+                ctx.sync()
+                got = ctx.to_host(d_y, (want.size + 16,), np.float32)
+                assert got[off // 4:off // 4 + want.size].tobytes() == want.tobytes(), (off, algo)
+                assert np.isnan(got[:off // 4]).all() and np.isnan(got[off // 4 + want.size:]).all(), (off, algo)
+    finally:
+        for p in (d_t, d_x, d_y):
+            ctx.free(p)
+        w.free()
