@@ -23,6 +23,13 @@ DENSE_LAYERS = [
     (TNN, Layer(1, 70, 5, 32, 64, 1, 0, 1), 3),       # filter rows of one bit
     (TNN, Layer(3, 5, 600, 32, 3, 3, 1, 1), 40),      # several segments of output columns, the last one short
     (TNN, Layer(2, 40, 40, 32, 3, 5, 3, 9), 90),      # strides past the filter, padding past it, whole bands per unit
+    (TNN, Layer(12, 11, 45, 40, 3, 3, 1, 2), 5),      # from twelve channels a lane reads a column: words of bits of three and four columns,
+    (TBN, Layer(13, 10, 70, 33, 5, 5, 2, 1), 2),      # rows of several 32-column pieces,
+    (TNN, Layer(15, 9, 33, 25, 3, 3, 1, 1), 3),       # units of few pixels, several threads to a pixel,
+    (TNN, Layer(16, 8, 8, 40, 7, 7, 3, 2), 2),        # 1024 positions,
+    (TBN, Layer(12, 9, 9, 33, 7, 7, 3, 2), 3),        # 768 (no power of two of sectors),
+    (TNN, Layer(15, 31, 40, 25, 7, 7, 3, 2), 2),      # the same over several units
+    (TNN, Layer(14, 6, 40, 32, 3, 3, 1, 1), 300),     # and whole bands per unit
 ]
 
 
