@@ -322,6 +322,76 @@ def test_ragged_channels_in_one_launch_on_two_streams(type_, checker):
         ctx.close()
 
 
+def with_special_values(x, thr, nan=False):
+    """Every third value one where a quantiser can go wrong: +-0, +-threshold and the floats beside it, denormals, infinities."""
+    f = np.float32
+    specials = []
+    for t in np.unique(np.abs(thr)):
+        for s in (f(t), f(-t)):
+            specials += [s, np.nextafter(s, f(np.inf)), np.nextafter(s, f(-np.inf))]
+    specials += [f(0.0), f(-0.0), f(1e-45), f(-1e-45), f(1e-39), f(-1e-39), f(np.inf), f(-np.inf), f(3e38), f(-3e38)] + ([f(np.nan), -f(np.nan)] if nan else [])
+    flat = x.reshape(-1)
+    flat[::3] = np.resize(np.array(specials, f), flat[::3].size)
+    return x
+
+
+SPECIAL_THR = np.array([0.25, 0.0, -0.0, 0.75], np.float32)
+
+
+@pytest.mark.parametrize("tern", [True, False])
+@pytest.mark.parametrize("C,H,W", [(40, 7, 7), (96, 8, 8), (65, 5, 9), (192, 6, 6)])
+def test_quantise_special_values(C, H, W, tern, gpu_ctx):
+    """Plain-load and copy-engine fed kernels, full and ragged channel groups, both layouts; NaN is a ternary zero, a binary +1."""
+    ctx, N = gpu_ctx, 4
+    x = with_special_values(synth.uniform_pm1(400 + C, (N, C, H, W)), SPECIAL_THR, nan=True)
+    want = numpy_planes(x, SPECIAL_THR, tern)
+    nb_p, nb_e = ft.api.packed_image_bytes(tern, N, C, H, W), ft.api.e2m1_image_bytes(N, C, H, W)
+    d_t, d_p, d_e = ctx.to_device(SPECIAL_THR), ctx.malloc(nb_p), ctx.malloc(nb_e)
+    try:
+        for layout in (ft.NCHW, ft.NHWC):
+            d_x = ctx.to_device(x if layout == ft.NCHW else to_nhwc(x))
+            ctx.quantise(tern, d_x, d_t, d_p, N, C, H, W, layout)
+            ctx.sync()
+            assert np.array_equal(ctx.to_host(d_p, want.shape, np.uint32), want), layout
+            if tern:
+                ctx.quantise_e2m1(d_x, d_t, d_e, N, C, H, W, layout)
+                ctx.sync()
+                want4 = _expand32_f4_numpy(want[:, 0], want[:, 1])
+                assert np.array_equal(ctx.to_host(d_e, want4.shape, np.uint32), want4), ("4-bit image", layout)
+            ctx.free(d_x)
+    finally:
+        for p in (d_t, d_p, d_e):
+            ctx.free(p)
+
+
+# the dense form, pixels stored padded, images stored bordered, and the plain image from plain loads
+@pytest.mark.parametrize("type_,layer", [
+    (TNN, Layer(3, 18, 21, 40, 7, 7, 3, 2)), (TBN, Layer(4, 9, 9, 33, 3, 3, 1, 1)), (TNN, Layer(130, 7, 7, 40, 3, 3, 1, 1)), (TBN, Layer(192, 8, 8, 64, 3, 3, 1, 2)),
+    (BTN, Layer(130, 7, 7, 40, 3, 3, 1, 2)), (BNN, Layer(96, 9, 9, 70, 3, 3, 1, 2)), (TNN, Layer(256, 7, 7, 64, 3, 3, 1, 2))], ids=lambda v: str(v).replace(" ", ""))
+def test_layers_with_special_values(type_, layer, gpu_ctx, checker):
+    case = make_case(type_, layer, 4, 8800 + layer.C, "uniform")
+    case.thr[:] = SPECIAL_THR
+    with_special_values(case.x, SPECIAL_THR)
+    wp = checker.pack_weights(wgt_ternary(type_), case.w, case.w_thr)
+    want = checker.conv(type_, case.x, case.thr, wp, case.kernel_hw, case.padding, case.stride, case.alpha)
+    ctx = gpu_ctx
+    w = ctx.upload_weights(type_, wp, layer.C, layer.KH, layer.KW)
+    d_t, d_y = ctx.to_device(case.thr), ctx.malloc(want.nbytes)
+    try:
+        for layout in (ft.NCHW, ft.NHWC):
+            d_x = ctx.to_device(case.x if layout == ft.NCHW else to_nhwc(case.x))
+            ctx.conv(w, d_x, d_t, d_y, layer.shape(4), case.alpha, layout)
+            ctx.sync()
+            got = ctx.to_host(d_y, want.shape if layout == ft.NCHW else (4, layer.OH, layer.OW, layer.KN), np.float32)
+            assert (got if layout == ft.NCHW else to_nchw(got)).tobytes() == want.tobytes(), layout
+            ctx.free(d_x)
+    finally:
+        for p in (d_t, d_y):
+            ctx.free(p)
+        w.free()
+
+
+
 # narrow and wide tiles of every GEMM: odd and even kernel counts (ragged last pairs), row bases that hold no pair or quad of floats
 @pytest.mark.parametrize("type_,layer,N", [
     (TNN, Layer(64, 20, 20, 25, 3, 3, 1, 1), 30), (TNN, Layer(256, 14, 14, 101, 3, 3, 1, 1), 60), (BNN, Layer(128, 20, 20, 1, 3, 3, 1, 1), 5), (BTN, Layer(64, 20, 20, 64, 3, 3, 1, 1), 9),
