@@ -930,16 +930,11 @@ int tnns_cuda_conv_ws(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const floa
     // the 4-bit tensor-core GEMM gather its im2row rows from it, so the KH*KW-times larger im2row
     // matrix is never written.  Forcing a pack or GEMM algorithm selects the explicit two-kernel
     // route (pack to the im2row matrix, then GEMM).
-    // Where the layer qualifies (ternary activations, C a multiple of 256) the image is written as
-    // 4-bit operands and the copy engine delivers the GEMM's activation tiles (im2col tensor copies).
+    // Where the layer qualifies the image is written as 4-bit operands and the copy engine delivers the GEMM's
+    // activation tiles (im2col tensor copies); bit planes and gathering warps are what is left.
     if (gemm_algo == TNNS_GEMM_F4_FUSED || auto_both) {
-        // one launch: the quantise step runs inside the GEMM kernel.  Taken on request, and by
-        // default where every SM has several tiles, so that the quantisation of later images hides
-        // under the MMAs of earlier ones (with one or two tiles per SM the two steps mostly run one
-        // after the other anyway, and the stand-alone quantise kernel is the faster of the two).
-        // Measured on B200, fused / two launches in us: 64 x 512x32x32 -> 512 (6.9 tiles per SM)
-        // 81 / 95, 256 x 128x28x28 -> 128 (10.6) 58 / 66, 256 x 64x56x56 -> 64 (42) 130 / 142;
-        // 256 x 256x14x14 -> 256 (2.6) 43 / 40, 16 x 512x32x32 -> 512 (1.7) 37 / 37.
+        // one launch: the quantise step runs inside the GEMM kernel.  Taken on request, and by default where the
+        // quantisation of later images hides under the MMAs of earlier ones (one_launch_pays, measurements there)
         const bool can = pack_algo == TNNS_PACK_AUTO && tnns_fused_supported(w, g, d_x, layout) &&
                          (reinterpret_cast<uintptr_t>(d_workspace) & 127) == 0 &&
                          tnns_fused_workspace_bytes(g.N, g.C, g.H, g.W) <= workspace_bytes;

@@ -60,7 +60,7 @@ __global__ void repack_weights_dense_kernel(const uint64_t* __restrict__ packed,
 //      A warp makes a word with one load per lane and two ballots (COLUMNS false), or, NCHW from twelve channels on, a lane
 //      reads all channels of one column and the lanes put their bits together by shuffles (true): with a lane per bit a load
 //      touches C rows of the input, 12 or more sectors, and each sector again for the next words -- from L2 where the GEMM
-//      in front or behind leaves little L1 (layer call, us, per bit / per column: 32 x 16x75x111 -> 64 7x7 s2 78 / 38,
+//      in front or behind leaves little L1 (layer call, us, per bit / per column: 32 x 16x75x111 -> 64 7x7 s2 78 / 43,
 //      32 x 12x75x111 -> 25 3x3 s2 42 / 22; below twelve channels most of its eight or sixteen loads would be repeats:
 //      4 x 4x224x224 7x7 s2 25 / 47).
 //   2. In that order the KW*C positions of a window's filter row are CONSECUTIVE bits, starting at ow*SW*C: a thread
@@ -71,7 +71,7 @@ __global__ void repack_weights_dense_kernel(const uint64_t* __restrict__ packed,
 // on the same path, and units are single blocks, scheduled as SMs come free (a resident grid that walks them ran a
 // nearly empty second round wherever their number was a little above it: 24 x 3x224x224 -> 64 7x7 s2 51 us per layer call,
 // 43 so).  Six of them fit an SM, five with a column's sixteen values in registers (40 and 48 registers, no spills).  Layer
-// call, one load per position of every window / now: 8 x 3x224x224 -> 64 7x7 s2 31 / 24, 32 x 15x75x111 -> 96 7x7 s2 62 / 39.
+// call, one load per position of every window / now: 8 x 3x224x224 -> 64 7x7 s2 31 / 24, 32 x 15x75x111 -> 96 7x7 s2 62 / 45.
 constexpr int DQ_THREADS = 256;
 constexpr int DQ_SMEM = 48 * 1024;
 constexpr int DQ_ROWS = 8;      // loads in flight per lane (one bit per lane)

@@ -23,8 +23,8 @@
 // keeps warps 0, 1 and eight epilogue warps, twelve on tiles of 64 and 128 kernels):
 //   warp 0      weight producer: one bulk async copy (TMA engine, no multicast, no tensor map)
 //               per stage of a pre-expanded, pre-swizzled weight tile (built once per layer)
-//   warp 1      MMA issuer: one thread issues four tcgen05.mma per stage and commits to the
-//               stage's "empty" barrier; owns the tensor-memory allocation
+//   warp 1      MMA issuer: a warp-uniform loop whose elected lane issues four tcgen05.mma per stage
+//               and commits to the stage's "empty" barrier; owns the tensor-memory allocation
 //   12-16 warps activation expanders in NG groups: thread = row; group k fills stages k, k+NG, ...
 //               so NG stages are expanded at once; packed planes come from global memory through
 //               a register prefetch ring and are stored in the 128-byte-swizzled K-major layout

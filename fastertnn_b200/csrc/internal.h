@@ -84,7 +84,7 @@ int tnns_launch_gemm_popc(tnns_cuda_ctx* ctx, int type, const void* d_a, const v
                           int KN, int Kp, int OHW, int K_unpack, float alpha, int layout, bool tiled,
                           cudaStream_t stream);
 
-// tensor-core path (gemm_i8_tc.cu)
+// tensor-core path (gemm_tc.cu)
 int tnns_i8_tile_n(int KN);
 int tnns_build_i8_weights(tnns_cuda_ctx* ctx, tnns_cuda_weights* w);
 int tnns_build_wide_weights(tnns_cuda_ctx* ctx, tnns_cuda_weights* w);

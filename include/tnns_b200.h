@@ -198,7 +198,9 @@ size_t tnns_packed_bytes(int type, const tnns_shape_t* s);
 
 /* Copies packed weights (host or device memory; reference layout for `type`: packing-2 for TNN/BTN,
  * one-plane for TBN/BNN) to the device and prepares the per-kernel constants and the
- * operand images the GEMM kernels need.  Done once per layer. */
+ * operand images the GEMM kernels need: int8 and 4-bit, a second 4-bit one with padded taps where ceil(C/64)
+ * is above 2 and no multiple of four (at most 1.6 times the first), and that of the dense form for few input
+ * channels.  Synchronises the device.  Done once per layer. */
 int tnns_cuda_upload_weights(tnns_cuda_ctx* ctx, int type, const int64_t* packed_host, int KN, int C, int KH,
                              int KW, tnns_cuda_weights** out);
 /* Weight packing on the device: fp32 [KN][C][KH][KW] and one threshold per kernel, both in device
@@ -269,7 +271,8 @@ int tnns_cuda_quantise(tnns_cuda_ctx* ctx, int ternary, const float* d_x, const 
                        int W, int layout, void* stream);
 /* GEMM + PReLU that gathers the im2row rows of layer `s` itself from the packed image of the
  * layer's input (implicit im2row: the KH*KW-times larger im2row matrix is never materialised).
- * Same result as tnns_cuda_pack + tnns_cuda_gemm.  tnns_cuda_conv takes this route by default. */
+ * Same result as tnns_cuda_pack + tnns_cuda_gemm.  tnns_cuda_conv takes this route where no copy-engine
+ * route applies or the workspace holds none of their images. */
 int tnns_cuda_gemm_implicit(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const void* d_image, float* d_y, const tnns_shape_t* s,
                             float alpha, int layout, void* stream);
 /* The same route with the copy engine doing the gather (ternary activations; 64-channel groups per
@@ -303,13 +306,15 @@ int tnns_cuda_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
  * other stream use the words in the workspace, which the call clears on `stream` first.  The first
  * call may allocate those words (and synchronise the device); keep it out of stream capture.  Same
  * result as every other route.  tnns_cuda_conv / _conv_ws take it with gemm_algo
- * TNNS_GEMM_F4_FUSED, and with TNNS_GEMM_AUTO where the layer has at least three tiles per SM. */
+ * TNNS_GEMM_F4_FUSED, and with TNNS_GEMM_AUTO where tnns_cuda_conv_fused_preferred says so; those two also
+ * from NHWC input with C a multiple of four. */
 size_t tnns_fused_workspace_bytes(int N, int C, int H, int W);
 int tnns_cuda_conv_fused_supported(const tnns_cuda_weights* w, const tnns_shape_t* s, const float* d_x, int layout);
 int tnns_cuda_conv_fused(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const float* d_x, const float* d_thr, float* d_y,
                          void* d_workspace, size_t workspace_bytes, const tnns_shape_t* s, float alpha, int pairs, void* stream);
-/* 1 where tnns_cuda_conv with TNNS_GEMM_AUTO takes that route by itself (the layer qualifies and
- * every SM has at least three 128-row tiles), else 0. */
+/* 1 where tnns_cuda_conv with TNNS_GEMM_AUTO takes that route by itself, unless a dense or slab-fed one comes
+ * first (the layer qualifies, every SM has at least three 128-row tiles, and the multiply hides the input's
+ * read: KN*KH*KW*OH*OW >= 3300*H*W), else 0. */
 int tnns_cuda_conv_fused_preferred(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s, const float* d_x, int layout);
 /* The same launch as the first layer of a chain (src/timing_layers.c:188-201 chains layers through fp32
  * buffers): fp32 input in, and instead of the fp32 output the next layer's quantised activations
@@ -341,14 +346,17 @@ int tnns_cuda_conv_fused_packed_out(tnns_cuda_ctx* ctx, const tnns_cuda_weights*
  *   tnns_cuda_conv_slab(_packed_out)  ONE launch: quantiser warps write the bordered image inside the GEMM
  *                                     kernel (workspace: tnns_slab_workspace_bytes, 128-byte aligned; the
  *                                     synchronisation words follow the rules of tnns_cuda_conv_fused).
- * tnns_cuda_conv / _conv_ws take these routes with gemm_algo TNNS_GEMM_F4_SLAB / _SLAB_FUSED. */
+ * tnns_cuda_conv / _conv_ws take these routes with gemm_algo TNNS_GEMM_F4_SLAB (any input, plain loads
+ * where the copy engine cannot fetch it) / _SLAB_FUSED. */
 size_t tnns_e2m1_bordered_image_bytes(int N, int C, int H, int W, int PH, int PW);
 size_t tnns_slab_workspace_bytes(int N, int C, int H, int W, int PH, int PW);
 int tnns_cuda_slab_supported(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s);
 /* 1 where the library's own rule (tnns_cuda_conv with TNNS_GEMM_AUTO) takes the slab-fed route for this layer. */
 int tnns_cuda_slab_preferred(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s);
 /* The tnns_gemm_algo that tnns_cuda_conv / _conv_ws resolve TNNS_GEMM_AUTO to for this layer and input
- * (workspace permitting): _F4_SLAB_FUSED, _F4_SLAB, _F4_FUSED, or _F4_TC for the two-launch forms. */
+ * (workspace permitting): _F4_DENSE, _F4_SLAB, _F4_FUSED, or _F4_TC for the rest (a 4-bit image stored
+ * plain, padded or bordered and the im2col-fed GEMM -- in one launch where that pays and pixels are stored
+ * padded -- else the gathering GEMM).  The answer may be passed back as gemm_algo. */
 int tnns_cuda_conv_auto_algo(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s, const float* d_x, int layout);
 int tnns_cuda_conv_slab_one_launch_preferred(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s, const float* d_x, int layout);
 int tnns_cuda_conv_slab_supported(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const tnns_shape_t* s, const float* d_x, int layout);
