@@ -91,7 +91,7 @@ struct SlabCfg {
     static constexpr int SMEM_MAX = 232448;
 };
 
-template <int BN, int CG, int TAPS, bool QF>
+template <int BN, int CG, int TAPS, bool QF, bool SINGLE>
 __global__ void __launch_bounds__(SlabCfg<BN, CG, TAPS, QF>::NTHREADS, 1)
 gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const __grid_constant__ CUtensorMap tmap_q) {
@@ -432,8 +432,8 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
         tnns_thr::Pair qt = {0.f, 0.f};
         int qt_img = -1;
         // pixel-major fp32 output: the accumulator is fetched in the 16x256b shape (four lanes = 32 contiguous bytes of a row)
-        // (float pairs; on narrow tiles single floats as well)
-        const bool rows16 = p.pimg == nullptr && p.layout == TNNS_NHWC && (NSETS > 1 || p.y_vec > 1);
+        // -- float pairs (y_vec), or, in kernels of their own, single floats (SINGLE)
+        const bool rows16 = p.pimg == nullptr && p.layout == TNNS_NHWC && (SINGLE || p.y_vec > 1);
         for (int t = unit + set * nunits; t < ntiles; t += NSETS * nunits, lt += NSETS) {
             const int buf = (int)(lt % NBUF);
             const int n0 = (t % ntn) * BN;
@@ -492,8 +492,8 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
                     const int c0 = n0 + cb;
                     float* const yrow[4] = {yrow0[0] ? yrow0[0] + c0 : nullptr, yrow0[1] ? yrow0[1] + c0 : nullptr,
                                             yrow0[2] ? yrow0[2] + c0 : nullptr, yrow0[3] ? yrow0[3] + c0 : nullptr};
-                    if (NSETS == 1 || p.y_vec > 1) store_rows16_at(f, yrow, p.KN - c0, lane);
-                    else store_rows16_single(f, yrow, p.KN - c0, lane);
+                    if (SINGLE) store_rows16_single(f, yrow, p.KN - c0, lane);
+                    else store_rows16_at(f, yrow, p.KN - c0, lane);
                     continue;
                 }
                 asm volatile(
@@ -650,11 +650,11 @@ done:
     }
 }
 
-template <int BN, int CG, int TAPS, bool QF>
+template <int BN, int CG, int TAPS, bool QF, bool SINGLE = false>
 int launch_slab(tnns_cuda_ctx* ctx, const SlabArgs& a, size_t smem, cudaStream_t stream, const CUtensorMap* tmap_a, const CUtensorMap* tmap_b,
                 const CUtensorMap* tmap_q) {
     using Cfg = SlabCfg<BN, CG, TAPS, QF>;
-    auto kern = gemm_slab_kernel<BN, CG, TAPS, QF>;
+    auto kern = gemm_slab_kernel<BN, CG, TAPS, QF, SINGLE>;
     static const CUtensorMap no_map = {};
     static bool smem_set[64] = {false};  // once per kernel and device
     if (!smem_set[ctx->device & 63]) {
@@ -868,6 +868,10 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
             }
         }
         if (use_pairs) return launch_slab<256, 2, T, false>(ctx, a, smem, stream, &map_a, &map_b, nullptr);
+        if (pl.bn < 256 && single_floats(a.layout, a.y_vec, d_pimg)) {
+            if (pl.bn == 64) return launch_slab<64, 1, T, false, true>(ctx, a, smem, stream, &map_a, nullptr, nullptr);
+            return launch_slab<128, 1, T, false, true>(ctx, a, smem, stream, &map_a, nullptr, nullptr);
+        }
         switch (pl.bn) {
             case 64: return launch_slab<64, 1, T, false>(ctx, a, smem, stream, &map_a, nullptr, nullptr);
             case 128: return launch_slab<128, 1, T, false>(ctx, a, smem, stream, &map_a, nullptr, nullptr);

@@ -277,7 +277,7 @@ __device__ __noinline__ void fill_output_border(uint4* img, int cp_next, int H, 
 // TAPS (tensor-copy form): filter taps per 128-byte stage row -- 1: a tap's 256 channels fill the
 // row (C_pack % 4 == 0); 2: C_pack = 2, two taps of 128 channels in two 64-byte-swizzled sub-tiles;
 // 4: C_pack = 1, four taps of 64 channels in four 32-byte-swizzled sub-tiles.
-template <int BN, int MT, bool F4, bool ATMA, int CG, int TAPS, bool QF>
+template <int BN, int MT, bool F4, bool ATMA, int CG, int TAPS, bool QF, bool SINGLE>
 __global__ void __launch_bounds__(TcCfg<BN, MT, F4, ATMA, CG, TAPS, QF>::NTHREADS, 1)
 gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                const __grid_constant__ CUtensorMap tmap_q) {
@@ -715,9 +715,8 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
         if (F4 && !QF && p.pimg && p.pimg_e2m1 && p.o_HpWp)
             fill_output_border(reinterpret_cast<uint4*>(p.pimg), p.cp_next, p.OHW / p.OW, p.OW, (int)(p.M / p.OHW), p.o_PH, p.o_PW,
                                ((long long)(warp - WARP_EPI0) * gridDim.x + blockIdx.x) * 32 + lane, (long long)gridDim.x * (blockDim.x - 32 * WARP_EPI0));
-        // pixel-major fp32 output in the 16x256b shape: float pairs, on narrow tiles single floats as well (64 x 64x56x56 -> 25
-        // 41.9 us per layer call with a row per lane, 24.4 so; -> 63 84.8 and 43.5)
-        const bool rows16 = F4 && p.pimg == nullptr && p.layout == TNNS_NHWC && (NSETS > 1 || p.y_vec > 1);
+        // pixel-major fp32 output in the 16x256b shape: float pairs (y_vec), or, in kernels of their own, single floats (SINGLE)
+        const bool rows16 = F4 && p.pimg == nullptr && p.layout == TNNS_NHWC && (SINGLE || p.y_vec > 1);
         tnns_thr::Pair qt = {0.f, 0.f};
         long long qt_img = -1;
         for (int t = unit + set * nunits; t < ntiles; t += NSETS * nunits, lt += NSETS) {
@@ -765,7 +764,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                     if (row0 < p.M) {
                         float f[32];
                         prelu32_f4(v, f, alpha_in_unit, p.acc_bias, bias_f, p.alpha, p.zero_passes);
-                        if (NSETS == 1 || p.y_vec > 1) {
+                        if (!SINGLE) {
                             store_rows16(f, p.y + (size_t)row0 * p.KN + (n0 + cb), p.KN, p.M - row0, p.KN - (n0 + cb), lane);
                         } else {
                             float* yrow[4];
@@ -1008,11 +1007,11 @@ __global__ void __launch_bounds__(128, 1) mma_rate_kernel(int iters, unsigned in
     }
 }
 
-template <int BN, int MT, bool F4, bool ATMA = false, int CG = 1, int TAPS = 1, bool QF = false>
+template <int BN, int MT, bool F4, bool ATMA = false, int CG = 1, int TAPS = 1, bool QF = false, bool SINGLE = false>
 int launch_cfg(tnns_cuda_ctx* ctx, const GemmArgs& a, cudaStream_t stream, const CUtensorMap* tmap_a = nullptr,
                const CUtensorMap* tmap_b = nullptr, const CUtensorMap* tmap_q = nullptr) {
     using Cfg = TcCfg<BN, MT, F4, ATMA, CG, TAPS, QF>;
-    auto kern = gemm_tc_kernel<BN, MT, F4, ATMA, CG, TAPS, QF>;
+    auto kern = gemm_tc_kernel<BN, MT, F4, ATMA, CG, TAPS, QF, SINGLE>;
     static const CUtensorMap no_map = {};
     // once per kernel and device: the attribute belongs to (function, device), and the call costs a microsecond per launch
     static bool smem_set[64] = {false};
@@ -1416,6 +1415,10 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
             }
         }
         if (use_pairs) return launch_cfg<256, 1, true, true, 2, T>(ctx, a, stream, &map, &map_b);
+        if (bn < 256 && single_floats(a.layout, a.y_vec, d_pimg)) {
+            if (bn == 64) return launch_cfg<64, 1, true, true, 1, T, false, true>(ctx, a, stream, &map);
+            return launch_cfg<128, 1, true, true, 1, T, false, true>(ctx, a, stream, &map);
+        }
         switch (bn) {
             case 64: return launch_cfg<64, 1, true, true, 1, T>(ctx, a, stream, &map);
             case 128: return launch_cfg<128, 1, true, true, 1, T>(ctx, a, stream, &map);
