@@ -69,7 +69,7 @@ __global__ void repack_weights_dense_kernel(const uint64_t* __restrict__ packed,
 //      share them, each with its own sectors of the rows.
 // Bound by instructions and by the latencies of one unit, so both steps keep their loops free of divisions and every lane
 // on the same path, and units are single blocks, scheduled as SMs come free (a resident grid that walks them ran a
-// nearly empty second round wherever their number was a little above it: 24 x 3x224x224 -> 64 7x7 s2 51 us per layer call,
+// nearly empty second wave wherever their number was a little above it: 24 x 3x224x224 -> 64 7x7 s2 51 us per layer call,
 // 43 so).  Six of them fit an SM, five with a column's sixteen values in registers (40 and 48 registers, no spills).  Layer
 // call, one load per position of every window / now: 8 x 3x224x224 -> 64 7x7 s2 31 / 24, 32 x 15x75x111 -> 96 7x7 s2 62 / 45.
 constexpr int DQ_THREADS = 256;
