@@ -43,13 +43,13 @@ struct SlabArgs {
     float* y;
     int Mv;                     // virtual rows: N * Hp * Wp
     int KN, nchunks;            // kernels, weight stages per kernel tile
-    int b_rows;                 // kernels per tile of the weight image: BN, or a multiple of it (few tiles)
+    int b_rows, b_shift;        // kernels per tile of the weight image (a power of two) and its logarithm: BN, or a multiple of it (few tiles)
     int y_vec;                  // floats of a pixel-major output row that may be stored at once: 4, 2 or 1
     int OH, OW, Wp, HpWp;       // output size, padded input lattice
     int KW, T;                  // filter width, taps KH*KW
     int G;                      // 128-byte channel groups per pixel (one slab each); 1 for 64 / 128 channels
     int slab_bytes, copy_rows, ncopies;  // slab buffer size; rows per tensor copy and copies per slab
-    int nslab, nstg;            // ring depths
+    int nslab, nstg;            // ring depths: slabs, weight stages
     int b_resident;             // the kernel tile's weight stages all fit the ring: fetched once per block
     int layout, zero_passes, acc_bias;
     float alpha;
@@ -66,7 +66,7 @@ struct SlabArgs {
     uint4* qimg;
     unsigned int* q_sync;
     int qN, qC, q_nbands, q_H, q_W, q_PH, q_PW, q_binary, q_self_clean, Cp;
-    FastDiv div_hpwp, div_wp;
+    FastDiv div_hpwp, div_wp, div_ntn;
 };
 
 template <int BN, int CG, int TAPS, bool QF>
@@ -91,11 +91,16 @@ struct SlabCfg {
     static constexpr int SMEM_MAX = 232448;
 };
 
-template <int BN, int CG, int TAPS, bool QF, bool SINGLE>
+// GRP = weight stages per slot of their ring (one pair of barriers per slot).  3: a filter row of a 3x3 layer of 128-byte pixels on
+// tiles of 64 or 128 kernels whose weights stream.  There the producer's wait, announcement and copy take some 300 clocks a
+// slot and the MMA warp's wait and commit another 80, the four MMAs of a stage of 64 kernels 192.  GEMM alone, one stage a slot and a
+// division per stage / so: 8 x 512x14x14 -> 512 8.8 / 6.4 us, 8 x 1024x14x14 -> 1024 16.0 / 11.3, 8 x 256x28x28 -> 256 7.2 / 6.1.
+template <int BN, int CG, int TAPS, bool QF, bool SINGLE, int GRP>
 __global__ void __launch_bounds__(SlabCfg<BN, CG, TAPS, QF>::NTHREADS, 1)
-gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                 const __grid_constant__ CUtensorMap tmap_q) {
+gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> maps) {
+    const CUtensorMap &tmap_a = maps.m[0], &tmap_b = maps.m[CG == 2 ? 1 : 0], &tmap_q = maps.m[QF ? 2 : 0];
     using Cfg = SlabCfg<BN, CG, TAPS, QF>;
+    static_assert(GRP == 1 || (GRP == 3 && TAPS == 1 && CG == 1 && !QF), "slots of three stages: streamed 3x3 weights of 128-byte pixels");
     constexpr int RB = Cfg::RB, B_STAGE = Cfg::B_STAGE, WARP_EPI0 = Cfg::WARP_EPI0, EPW = Cfg::EPW, ACC_OFF = Cfg::ACC_OFF;
     constexpr bool OVL = Cfg::OVL;
     constexpr int NBUF = Cfg::NBUF, NSETS = Cfg::NSETS;
@@ -117,7 +122,6 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
     unsigned char* q_ring = reinterpret_cast<unsigned char*>(bars) + SL_BAR_BYTES;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int ntn = (p.KN + BN - 1) / BN;
     const int ntm = (p.Mv + TILE_M - 1) / TILE_M;
     const int ntiles = ntm * ntn;
@@ -161,11 +165,21 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
+        // dependents may be placed once this block holds its tensor memory, and the producer of a single block goes ahead of the rest
+        // of the set-up (gemm_tc.cu has the reasons for both)
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
-    tc_fence_before();
-    if (CG == 2) cluster_sync_all(); else __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
+    constexpr bool LONE = CG == 1;
+    const bool ahead = LONE && warp == WARP_TMA;
+    uint32_t tmem_base = 0;
+    if (ahead) {
+        named_arrive(1, blockDim.x);
+    } else {
+        tc_fence_before();
+        if (CG == 2) cluster_sync_all(); else named_sync(1, blockDim.x);
+        tc_fence_after();
+        tmem_base = *tmem_slot;
+    }
     // unit block scales (ue8m0 0x7F) in columns 480..511, as in the im2col form
     if (warp >= WARP_EPI0 && warp < WARP_EPI0 + 4) {
         const uint32_t one = 0x7F7F7F7Fu;
@@ -176,29 +190,44 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     }
-    tc_fence_before();
-    if (CG == 2) cluster_sync_all(); else __syncthreads();
-    tc_fence_after();
+    if (!ahead) {
+        tc_fence_before();
+        if (CG == 2) cluster_sync_all(); else named_sync(2, blockDim.x - 32);
+        tc_fence_after();
+    }
 
     // weight stage c of kernel tile n_tile -> ring slot; a tile is rows [n_tile*BN % b_rows, +BN) of an image tile of b_rows kernels
     const uint32_t bfull_lead = (CG == 2) ? mapa_shared(bar_bfull, 0) : bar_bfull;
-    auto request_weights = [&](int n_tile, int c, uint32_t slot) {
+    // (no division and little arithmetic per stage: with one of each the producer took 500 clocks a stage)
+    const size_t b_step = (size_t)p.b_rows * KCH;
+    auto weights_of = [&](int n_tile) -> const unsigned char* {
+        const uint32_t k0 = (uint32_t)(n_tile * BN), big = k0 >> p.b_shift;
+        return p.Bimg + (size_t)big * p.nchunks * b_step + (size_t)(k0 & (uint32_t)(p.b_rows - 1)) * KCH;
+    };
+    const size_t j_step = (TAPS == 1) ? (size_t)p.G * b_step : b_step;  // from a stage of a slab to the next
+    // the GRP stages from w (stage c of the tile) on -> the slot whose first ring stage is `at`
+    auto request_weights = [&](const unsigned char* w, int n_tile, int c, uint32_t at, uint32_t slot) {
         if (CG == 2) {
             if (rank == 0) mbar_arrive_expect_tx(bar_bfull + 8 * slot, CG * B_STAGE);
-            tma_tile2d_g2s_pair(smem_u32(sB + slot * B_STAGE), &tmap_b, 0, (n_tile * p.nchunks + c) * BN + (int)rank * (BN / CG), bfull_lead + 8 * slot);
+            tma_tile2d_g2s_pair(smem_u32(sB + at * B_STAGE), &tmap_b, 0, (n_tile * p.nchunks + c) * BN + (int)rank * (BN / CG), bfull_lead + 8 * slot);
         } else {
-            const int k0 = n_tile * BN, big = k0 / p.b_rows;
-            mbar_arrive_expect_tx(bar_bfull + 8 * slot, B_STAGE);
-            bulk_g2s(smem_u32(sB + slot * B_STAGE), p.Bimg + ((size_t)(big * p.nchunks + c) * p.b_rows + (k0 - big * p.b_rows)) * KCH, B_STAGE, bar_bfull + 8 * slot);
+            mbar_arrive_expect_tx(bar_bfull + 8 * slot, (uint32_t)(GRP * B_STAGE));
+#pragma unroll
+            for (int g = 0; g < GRP; g++) bulk_g2s(smem_u32(sB + (at + g) * B_STAGE), w + g * j_step, B_STAGE, bar_bfull + 8 * slot);
         }
     };
     // the first stages of the block's first tile, before the wait for the launch in front (32 KB of constant weights; see gemm_tc.cu)
-    const int early = min(min(32768 / B_STAGE, p.nstg), SPG);
+    // -- whole slots of the first slab's stages
+    constexpr int EARLY = 32768 / (GRP * B_STAGE) > 0 ? 32768 / (GRP * B_STAGE) * GRP : GRP;
+    const int early = min(min(EARLY, p.nstg), SPG);
     if (warp == WARP_TMA && lane == 0 && unit < ntiles) {
         prefetch_tensor_map(&tmap_a);
-        for (int j = 0; j < early; j++) {
+        const int n_tile = unit - (int)p.div_ntn.div((uint32_t)unit) * ntn;
+        const unsigned char* src = weights_of(n_tile);
+        for (int j = 0; j < early; j += GRP) {
             const int c = (TAPS == 1) ? j * p.G : j;
-            request_weights(unit % ntn, c, p.b_resident ? (uint32_t)c : (uint32_t)j);
+            const uint32_t at = p.b_resident ? (uint32_t)c : (uint32_t)j;
+            request_weights(src + (size_t)j * j_step, n_tile, c, at, at / GRP);
         }
     }
 
@@ -207,12 +236,15 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
     if (warp == WARP_TMA) {
         if (lane == 0) {
             uint32_t sl = 0, slph = 1, s = 0, ph = 1;
+            const uint32_t nslots = (uint32_t)p.nstg / GRP;
+            bool free_slot = false;  // slot s has been seen free
             bool first_tile = true;
             const uint32_t sfull_lead = (CG == 2) ? mapa_shared(bar_sfull, 0) : bar_sfull;
             const uint32_t copy_bytes = (uint32_t)(p.ncopies * p.copy_rows * RB);
             for (int t = unit; t < ntiles; t += nunits, first_tile = false) {
-                const int n_tile = t % ntn;
-                const int q0 = (t / ntn) * TILE_M + (int)rank * BM;  // first virtual row = first pixel of the block's slab
+                const int m_tile = (int)p.div_ntn.div((uint32_t)t), n_tile = t - m_tile * ntn;
+                const unsigned char* src = weights_of(n_tile);
+                const int q0 = m_tile * TILE_M + (int)rank * BM;  // first virtual row = first pixel of the block's slab
                 if (QF && q0 < p.Mv) {
                     // the slab reads the images its pixels belong to: wait until the quantiser warps (of any
                     // block) have finished them, border item included
@@ -236,15 +268,30 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
                             tma_tile2d_g2s(dst + i * p.copy_rows * RB, &tmap_a, cg * KCH, q0 + i * p.copy_rows, bar_sfull + 8 * sl);
                     }
                     if (++sl == (uint32_t)p.nslab) { sl = 0; slph ^= 1; }
-                    if (p.b_resident && !first_tile) continue;
-                    for (int j = 0; j < SPG; j++) {
-                        const int c = (TAPS == 1) ? j * p.G + cg : j;
-                        const uint32_t slot = p.b_resident ? (uint32_t)c : s;
-                        if (!(first_tile && cg == 0 && j < early)) {
-                            if (!p.b_resident && !mbar_wait(bar_bempty + 8 * slot, ph, abort_flag, p.status, 1)) goto done;
-                            request_weights(n_tile, c, slot);
-                        }
-                        if (!p.b_resident && ++s == (uint32_t)p.nstg) { s = 0; ph ^= 1; }
+                    if (p.b_resident) {
+                        if (first_tile)
+                            for (int j = cg == 0 ? early : 0; j < SPG; j++) {
+                                const int c = (TAPS == 1) ? j * p.G + cg : j;
+                                request_weights(src + (size_t)c * b_step, n_tile, c, (uint32_t)c, (uint32_t)c);
+                            }
+                        continue;
+                    }
+                    const unsigned char* w = src + ((TAPS == 1) ? (size_t)cg * b_step : 0);
+                    int j = 0;
+                    if (first_tile && cg == 0) {
+                        j = early;
+                        s = (uint32_t)early / GRP;
+                        if (s == nslots) { s = 0; ph ^= 1; }
+                        w += (size_t)early * j_step;
+                    }
+                    for (; j < SPG; j += GRP) {
+                        if (!free_slot && !mbar_wait(bar_bempty + 8 * s, ph, abort_flag, p.status, 1)) goto done;
+                        const uint32_t s1 = s + 1 == nslots ? 0u : s + 1;
+                        free_slot = mbar_test(bar_bempty + 8 * s1, ph ^ (s1 == 0 ? 1u : 0u));  // the next slot
+                        request_weights(w, n_tile, (TAPS == 1) ? j * p.G + cg : j, s * GRP, s);
+                        w += GRP * j_step;
+                        s = s1;
+                        if (s1 == 0) ph ^= 1;
                     }
                 }
             }
@@ -270,24 +317,53 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
             auto commit = [&](uint32_t bar) {
                 if (CG == 2) tc_commit_pair(bar); else tc_commit(bar);
             };
-            const bool fast3x3 = p.T == 9 && p.KW == 3;
+            const bool fast3x3 = GRP == 3 || (p.T == 9 && p.KW == 3);
             if (fast3x3) {
-                // 3x3 filters: the nine tap offsets live in registers and the MMAs of a slab (or, where weights stream, of a
-                // stage) are straight-line code -- one 32-bit add per operand and MMA
-                uint32_t aoff[9];
-#pragma unroll
-                for (int j = 0; j < 9; j++) aoff[j] = (uint32_t)((j / 3) * p.Wp + (j % 3)) * (RB / 16);
+                // 3x3 filters: the MMAs of a slab (or, where weights stream, of a stage) are straight-line code, every operand one
+                // of four uniform values (the slab's first three image rows, the weights) plus a constant.
+                const uint32_t nslots = (uint32_t)p.nstg / GRP;
+                bool there = false;  // slot s has been seen complete
                 constexpr int KPT = 4 / TAPS;               // K steps (32 bytes) per tap: 1, 2 or 4
                 constexpr int NK = 9 * KPT, NST = (NK + 3) / 4;  // K steps and weight stages of a slab
+                bool acc_free = false, slab_there = false;  // the tile's accumulator / the slab sl has been seen free / complete
                 for (int t = unit; t < ntiles; t += nunits, lt++, first_tile = false) {
                     const int buf = (int)(lt % NBUF);
-                    if (!mbar_wait(OVL ? bar_tempty : bar_tempty + 8 * buf, (OVL ? (lt & 1) : ((lt / NBUF) & 1)) ^ 1, abort_flag, p.status, 2)) goto done;
+                    if (!acc_free && !mbar_wait(OVL ? bar_tempty : bar_tempty + 8 * buf, (OVL ? (lt & 1) : ((lt / NBUF) & 1)) ^ 1, abort_flag, p.status, 2)) goto done;
                     tc_fence_after();
                     const uint32_t d_tmem = tmem_base + buf * ACC_OFF;
                     for (int cg = 0; cg < p.G; cg++) {
-                        if (!mbar_wait(bar_sfull + 8 * sl, slph, abort_flag, p.status, 0x13)) goto done;
-                        const uint32_t slab_lo = a_lo0 + sl * slab16;
-                        if (BN == 256 && p.b_resident && first_tile) {
+                        if (!slab_there && !mbar_wait(bar_sfull + 8 * sl, slph, abort_flag, p.status, 0x13)) goto done;
+                        // look at what comes next now: the answers arrive while this slab's MMAs are issued
+                        const uint32_t sl1 = sl + 1 == (uint32_t)p.nslab ? 0u : sl + 1;
+                        slab_there = mbar_test(bar_sfull + 8 * sl1, slph ^ (sl1 == 0 ? 1u : 0u));
+                        if (!OVL) acc_free = mbar_test(bar_tempty + 8 * ((lt + 1) % NBUF), (((lt + 1) / NBUF) & 1) ^ 1);
+                        const uint32_t slab_lo = a_lo0 + sl * slab16, slab_lo1 = slab_lo + row16, slab_lo2 = slab_lo1 + row16;
+                        // K step q of the slab: 32 bytes x (q % KPT) into the pixels of tap q / KPT
+                        auto a_of = [&](int q) {
+                            const int tap = q / KPT;
+                            return (tap < 3 ? slab_lo : tap < 6 ? slab_lo1 : slab_lo2) + (uint32_t)((tap % 3) * (RB / 16) + 2 * (q % KPT));
+                        };
+                        if (GRP == 3) {
+                            // a slot = the three taps of one filter row
+                            uint32_t row_lo = slab_lo;
+#pragma unroll 1
+                            for (int kh = 0; kh < 3; kh++, row_lo += row16) {
+                                if (!there && !mbar_wait(bar_bfull + 8 * s, ph, abort_flag, p.status, 3)) goto done;
+                                tc_fence_after();
+                                const uint32_t s1 = s + 1 == nslots ? 0u : s + 1;
+                                there = mbar_test(bar_bfull + 8 * s1, ph ^ (s1 == 0 ? 1u : 0u));  // the next slot
+                                const uint32_t b_lo = b_lo0 + s * (uint32_t)(GRP * (B_STAGE >> 4));
+                                if (elected) {
+#pragma unroll
+                                    for (int q = 0; q < 12; q++)
+                                        mma(d_tmem, row_lo + (uint32_t)((q / 4) * (RB / 16) + 2 * (q % 4)), b_lo + (uint32_t)((q / 4) * (B_STAGE >> 4) + 2 * (q % 4)), (uint32_t)(cg | kh | q));
+                                    commit(bar_bempty + 8 * s);
+                                    if (kh == 2) commit(bar_sempty + 8 * sl);
+                                }
+                                s = s1;
+                                if (s1 == 0) ph ^= 1;
+                            }
+                        } else if (BN == 256 && p.b_resident && first_tile) {
                             // stage by stage as the weights land (waiting for all of them first: 40 x 128x14x14 -> 256 BNN, one
                             // tile per SM, 11.3 us per layer call against 10.3; on narrower tiles most of them were requested before the
                             // wait for the launch in front); rolled up, it runs once per block and group
@@ -314,26 +390,27 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
                             tc_fence_after();
                             if (elected) {
 #pragma unroll
-                                for (int q = 0; q < NK; q++) {   // K step q: tap q / KPT, stage q / 4
-                                    const uint32_t slot = (TAPS == 1) ? (uint32_t)((q >> 2) * p.G + cg) : (uint32_t)(q >> 2);
-                                    mma(d_tmem, slab_lo + aoff[q / KPT] + 2u * (uint32_t)(q % KPT), b_lo0 + slot * (uint32_t)(B_STAGE >> 4) + 2u * (q & 3), (uint32_t)(cg | q));
-                                }
+                                for (int q = 0; q < NK; q++)  // stage q / 4 is slot q / 4: nine taps of one channel group fill the ring (G = 1)
+                                    mma(d_tmem, a_of(q), b_lo0 + (uint32_t)((q >> 2) * (B_STAGE >> 4) + 2 * (q & 3)), (uint32_t)q);
                                 commit(bar_sempty + 8 * sl);
                             }
                         } else {
 #pragma unroll
                             for (int j = 0; j < NST; j++) {
-                                if (!mbar_wait(bar_bfull + 8 * s, ph, abort_flag, p.status, 3)) goto done;
+                                if (!there && !mbar_wait(bar_bfull + 8 * s, ph, abort_flag, p.status, 3)) goto done;
                                 tc_fence_after();
+                                const uint32_t s1 = s + 1 == nslots ? 0u : s + 1;
+                                there = mbar_test(bar_bfull + 8 * s1, ph ^ (s1 == 0 ? 1u : 0u));  // the next slot
+                                const uint32_t b_lo = b_lo0 + s * (uint32_t)(B_STAGE >> 4);
                                 if (elected) {
-                                    const uint32_t b_lo = b_lo0 + s * (uint32_t)(B_STAGE >> 4);
 #pragma unroll
                                     for (int q = 4 * j; q < 4 * j + 4 && q < NK; q++)
-                                        mma(d_tmem, slab_lo + aoff[q / KPT] + 2u * (uint32_t)(q % KPT), b_lo + 2u * (q & 3), (uint32_t)(cg | q));
+                                        mma(d_tmem, a_of(q), b_lo + 2u * (q & 3), (uint32_t)(cg | q));
                                     commit(bar_bempty + 8 * s);
                                     if (j == NST - 1) commit(bar_sempty + 8 * sl);
                                 }
-                                if (++s == (uint32_t)p.nstg) { s = 0; ph ^= 1; }
+                                s = s1;
+                                if (s1 == 0) ph ^= 1;
                             }
                         }
                         if (++sl == (uint32_t)p.nslab) { sl = 0; slph ^= 1; }
@@ -436,9 +513,9 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
         const bool rows16 = p.pimg == nullptr && p.layout == TNNS_NHWC && (SINGLE || p.y_vec > 1);
         for (int t = unit + set * nunits; t < ntiles; t += NSETS * nunits, lt += NSETS) {
             const int buf = (int)(lt % NBUF);
-            const int n0 = (t % ntn) * BN;
+            const int m_tile = (int)p.div_ntn.div((uint32_t)t), n0 = (t - m_tile * ntn) * BN;
             // where this thread's row sits in the lattice, and its image's threshold: worked out while the tile's MMAs run
-            const int row = (t / ntn) * TILE_M + (int)rank * BM + q * 32 + lane;  // virtual row
+            const int row = m_tile * TILE_M + (int)rank * BM + q * 32 + lane;  // virtual row
             const bool row_ok = row < p.Mv;
             const int n_img = row_ok ? (int)p.div_hpwp.div((uint32_t)row) : 0;
             const int rem = row - n_img * p.HpWp;
@@ -457,7 +534,7 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ CUtensorMap tmap_a, const _
             if (rows16) {
 #pragma unroll
                 for (int h = 0; h < 4; h++) {
-                    const int r = (t / ntn) * TILE_M + (int)rank * BM + q * 32 + 8 * h + (lane >> 2);
+                    const int r = m_tile * TILE_M + (int)rank * BM + q * 32 + 8 * h + (lane >> 2);
                     if (r < p.Mv) {
                         const int ni = (int)p.div_hpwp.div((uint32_t)r);
                         const int rm = r - ni * p.HpWp;
@@ -650,12 +727,12 @@ done:
     }
 }
 
-template <int BN, int CG, int TAPS, bool QF, bool SINGLE = false>
+template <int BN, int CG, int TAPS, bool QF, bool SINGLE = false, int GRP = 1>
 int launch_slab(tnns_cuda_ctx* ctx, const SlabArgs& a, size_t smem, cudaStream_t stream, const CUtensorMap* tmap_a, const CUtensorMap* tmap_b,
                 const CUtensorMap* tmap_q) {
     using Cfg = SlabCfg<BN, CG, TAPS, QF>;
-    auto kern = gemm_slab_kernel<BN, CG, TAPS, QF, SINGLE>;
-    static const CUtensorMap no_map = {};
+    auto kern = gemm_slab_kernel<BN, CG, TAPS, QF, SINGLE, GRP>;
+    const auto maps = tensor_maps<maps_of(CG, QF)>(tmap_a, tmap_b, tmap_q);
     static bool smem_set[64] = {false};  // once per kernel and device
     if (!smem_set[ctx->device & 63]) {
         TNNS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_MAX));
@@ -696,7 +773,7 @@ int launch_slab(tnns_cuda_ctx* ctx, const SlabArgs& a, size_t smem, cudaStream_t
     }
     cfg.attrs = attr;
     cfg.numAttrs = nattr;
-    TNNS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a, tmap_a ? *tmap_a : no_map, tmap_b ? *tmap_b : no_map, tmap_q ? *tmap_q : no_map));
+    TNNS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a, maps));
     tnns_count_launch();
     TNNS_CUDA_TRY(cudaGetLastError());
     return TNNS_OK;
@@ -751,7 +828,7 @@ namespace {
 struct SlabChoice {
     SlabPlan pl;
     bool pairs;
-    int b_stage, fixed, nslab, nstg, resident, Mv, ntn;
+    int b_stage, fixed, nslab, nstg, resident, grp, Mv, ntn;
     size_t smem;
 };
 // The form a launch takes: single blocks or block pairs (pairs_req 0 = by size, 1, 2), ring depths.
@@ -776,6 +853,9 @@ bool choose_form(int sm_count, const tnns_cuda_weights* w, const TnnsGeom& g, in
             if (!ring_depths(pl, ch->b_stage, ch->fixed, w->Kp / 4, ch->ntn == 1, &ch->nslab, &ch->nstg, &ch->resident)) return false;
         }
     }
+    // three weight stages a slot (see the kernel's GRP) where two slots fit
+    ch->grp = (pl.taps == 1 && g.KH == 3 && g.KW == 3 && !ch->resident && !ch->pairs && !fused && ch->pl.bn <= 128 && ch->nstg >= 6) ? 3 : 1;
+    ch->nstg -= ch->nstg % ch->grp;
     ch->smem = (size_t)ch->fixed + (size_t)ch->nslab * pl.slab_bytes + (size_t)ch->nstg * ch->b_stage;
     return true;
 }
@@ -812,6 +892,8 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
     a.KN = w->KN;
     a.nchunks = w->Kp / 4;
     a.b_rows = tnns_i8_tile_n(w->KN);
+    a.b_shift = a.b_rows == 64 ? 6 : a.b_rows == 128 ? 7 : 8;
+    a.div_ntn = tnns_fastdiv((uint32_t)ch.ntn);
     a.y_vec = tnns_row_vec(d_y, w->KN);
     a.OH = g.OH; a.OW = g.OW; a.Wp = pl.Wp; a.HpWp = pl.Hp * pl.Wp;
     a.KW = g.KW; a.T = pl.T; a.G = pl.G;
@@ -868,7 +950,15 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
             }
         }
         if (use_pairs) return launch_slab<256, 2, T, false>(ctx, a, smem, stream, &map_a, &map_b, nullptr);
-        if (pl.bn < 256 && single_floats(a.layout, a.y_vec, d_pimg)) {
+        const bool single = pl.bn < 256 && single_floats(a.layout, a.y_vec, d_pimg);
+        if constexpr (T == 1)
+            if (ch.grp == 3) {
+                if (pl.bn == 64) return single ? launch_slab<64, 1, T, false, true, 3>(ctx, a, smem, stream, &map_a, nullptr, nullptr)
+                                               : launch_slab<64, 1, T, false, false, 3>(ctx, a, smem, stream, &map_a, nullptr, nullptr);
+                return single ? launch_slab<128, 1, T, false, true, 3>(ctx, a, smem, stream, &map_a, nullptr, nullptr)
+                              : launch_slab<128, 1, T, false, false, 3>(ctx, a, smem, stream, &map_a, nullptr, nullptr);
+            }
+        if (single) {
             if (pl.bn == 64) return launch_slab<64, 1, T, false, true>(ctx, a, smem, stream, &map_a, nullptr, nullptr);
             return launch_slab<128, 1, T, false, true>(ctx, a, smem, stream, &map_a, nullptr, nullptr);
         }

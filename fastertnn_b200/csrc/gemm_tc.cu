@@ -91,6 +91,11 @@ struct TcCfg {
     static constexpr int NSTG_QF = (CG == 2) ? 5 : (BN == 256 ? 3 : 4);
     static constexpr int NSTG_ATMA = CG == 2 ? 6 : (BN == 64 ? 8 : (BN == 128 ? 6 : 4));  // 192 KB whatever the tile
     static constexpr int NSTG = QF ? NSTG_QF : (ATMA ? NSTG_ATMA : ((MT == 1) ? 4 : 3));
+    // Stages per slot of the ring (one pair of barriers per slot).  On narrow tiles of single blocks two: a wait that finds its barrier
+    // complete takes 110-140 clocks, a copy request 70, the four MMAs of a stage 192 (64 kernels) or 256 (128).  GEMM alone, one
+    // stage a slot / two: 8 x 512x14x14 -> 512 7.8 / 7.2 us, 8 x 1024x14x14 -> 1024 13.9 / 12.2, 8 x 256x28x28 -> 256 6.6 / 6.3.
+    static constexpr int GRP = (ATMA && !QF && CG == 1 && BN <= 128) ? 2 : 1, NSLOT = NSTG / GRP;
+    static_assert(NSTG % GRP == 0, "whole slots");
     static constexpr int A_STAGE = MT * A_SUB, B_STAGE = (BN / CG) * KCH;
     static constexpr bool OVL = F4 && MT == 1 && BN == 256;        // overlapping accumulator sets
     // Tensor-copy form on narrow tiles: three groups of four epilogue warps take the tiles in turn (see gemm_slab.cu, where a
@@ -110,8 +115,8 @@ struct TcCfg {
     static constexpr int NTHREADS = 32 * (2 + 4 * MT * NG + NEPI + NQ);
     static constexpr int NBARS = NBUF > 2 ? NBUF : 2;
     static_assert((2 * NSTG + 2 * NBARS) * 8 + 8 <= 256, "barriers and two words");
-    static constexpr int TAPMAX = QF ? 192 : 1024;  // entries of the tap table kept in shared memory (QF: 192 entries + the 256 bytes of barriers = 1 KB, see Q_OFF)
-    static constexpr size_t Q_OFF = (size_t)NSTG * (A_STAGE + B_STAGE) + 256 + TAPMAX * sizeof(uint32_t);  // quantiser ring, then its barriers
+    static constexpr int TAPMAX = ATMA ? 0 : 1024;  // entries of the tap table kept in shared memory (gathering form)
+    static constexpr size_t Q_OFF = (size_t)NSTG * (A_STAGE + B_STAGE) + (QF ? 1024 : 256) + TAPMAX * sizeof(uint32_t);  // quantiser ring, then its barriers
     static_assert(!QF || Q_OFF % 1024 == 0, "the quantiser ring receives 128-byte-swizzled boxes: its stages start on 1024-byte boundaries");
     static constexpr size_t SMEM = 1024 + Q_OFF + (QF ? QSTG * Q_STAGE + 128 : 0);
     static_assert(SMEM <= 232448, "shared memory per block");
@@ -229,7 +234,7 @@ struct GemmArgs {
     float* y;
     long long M;
     int KN, Kp, OHW, layout;
-    int b_rows;                 // kernels per tile of the weight image: BN, or a multiple of it (tensor-copy form, few tiles)
+    int b_rows, b_shift;        // kernels per tile of the weight image (a power of two) and its logarithm: BN, or a multiple of it (tensor-copy form, few tiles)
     int y_vec;                  // floats of a pixel-major output row that may be stored at once: 4, 2 or 1
     int a_two_planes;
     int acc_bias;               // added to the integer dot product (BNN: K_unpack minus the positions multiplied)
@@ -251,6 +256,8 @@ struct GemmArgs {
     const uint64_t* img;
     const uint32_t* jtab;       // per plane word j: kh<<24 | kw<<16 | ic, 0xFFFFFFFF for pad words
     int H, W, OW, Cp, SH, SW, PH, PW;
+    int KH, KW;                 // filter size (tensor-copy form)
+    FastDiv div_ntn, div_ohw, div_ow;  // kernel tiles, output pixels per image, output width: a division costs a thread some 100 clocks
     // fused quantisation (QF): the layer's fp32 NCHW input and per-image thresholds, the 4-bit image
     // the quantiser warps write (the tensor the activation copies read), and the launch's
     // synchronisation words, zero when the launch starts: q_sync[0] = next item to claim,
@@ -279,10 +286,10 @@ __device__ __noinline__ void fill_output_border(uint4* img, int cp_next, int H, 
 // 4: C_pack = 1, four taps of 64 channels in four 32-byte-swizzled sub-tiles.
 template <int BN, int MT, bool F4, bool ATMA, int CG, int TAPS, bool QF, bool SINGLE>
 __global__ void __launch_bounds__(TcCfg<BN, MT, F4, ATMA, CG, TAPS, QF>::NTHREADS, 1)
-gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-               const __grid_constant__ CUtensorMap tmap_q) {
+gemm_tc_kernel(GemmArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> maps) {
+    const CUtensorMap &tmap_a = maps.m[0], &tmap_b = maps.m[CG == 2 ? 1 : 0], &tmap_q = maps.m[QF ? 2 : 0];
     using Cfg = TcCfg<BN, MT, F4, ATMA, CG, TAPS, QF>;
-    constexpr int NSTG = Cfg::NSTG, A_STAGE = Cfg::A_STAGE, B_STAGE = Cfg::B_STAGE, NBUF = Cfg::NBUF, WARP_EPI0 = Cfg::WARP_EPI0, NG = Cfg::NG, EPW = Cfg::EPW;
+    constexpr int NSTG = Cfg::NSTG, GRP = Cfg::GRP, NSLOT = Cfg::NSLOT, A_STAGE = Cfg::A_STAGE, B_STAGE = Cfg::B_STAGE, NBUF = Cfg::NBUF, WARP_EPI0 = Cfg::WARP_EPI0, NG = Cfg::NG, EPW = Cfg::EPW;
     constexpr int BMT = MT * BM;      // rows per block
     constexpr int TILE_M = CG * BMT;  // rows per tile (a block pair shares one 256-row tile)
     // instruction descriptor: i8 -- s32 accumulate (2<<4), signed 8-bit A and B (1<<7, 1<<10);
@@ -302,8 +309,8 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                    bar_tempty = smem_u32(bars + 2 * NSTG + Cfg::NBARS);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NSTG + 2 * Cfg::NBARS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    // The tap table (plane word -> kh, kw, ic) sits on the producer's critical path once per stage,
-    // so its first TAPMAX entries are copied to shared memory; longer tables fall back to global loads.
+    // Gathering form: the first TAPMAX entries of the tap table (plane word -> kh, kw, ic) are copied to shared memory;
+    // longer tables fall back to global loads.
     uint32_t* s_taps = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(bars) + 256);
     auto tap_at = [&](int j) -> uint32_t { return j < Cfg::TAPMAX ? s_taps[j] : __ldg(p.jtab + j); };
 
@@ -311,8 +318,8 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
     // Programmatic dependent launch: a following launch of this kind may place its
     // blocks on SMs as the blocks of this one leave, run its set-up there, and wait (below, before
     // it touches any global data) until this launch has completed.  All blocks of a launch are
-    // resident at once, so letting the dependents in early cannot starve this launch of SMs.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // resident at once, so letting the dependents in early cannot starve this launch of SMs.  The block says so once it holds its
+    // tensor memory (below): a dependent's block on the same SM must not take columns this block still waits for.
     const int nchunks = F4 ? p.Kp / 4 : p.Kp / 2;  // stages per tile
     const int ntn = (p.KN + BN - 1) / BN;
     const int ntm = (int)((p.M + TILE_M - 1) / TILE_M);
@@ -321,7 +328,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
     const uint32_t rank = (CG == 2) ? cluster_ctarank() : 0u;
     const int unit = blockIdx.x / CG, nunits = gridDim.x / CG;
 
-    if (p.jtab)
+    if (!ATMA && p.jtab)
         for (int j = threadIdx.x; j < min(p.Kp, Cfg::TAPMAX); j += blockDim.x) s_taps[j] = __ldg(p.jtab + j);
     if (tid == 0) {
         for (int s = 0; s < NSTG; s++) {
@@ -356,13 +363,23 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
             asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
         }
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
-    tc_fence_before();
-    // pair: no remote arrive, copy completion or multicast commit may reach a barrier before its block initialised it
-    if (CG == 2) cluster_sync_all(); else __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = *tmem_slot;
-    if (F4) {
+    // The producer of a single block (LONE) needs none of the tensor-memory set-up: it initialised the barriers itself, says so, and
+    // goes on to its first copies while the others finish (1.35 us from block start to the end of the set-up, which used to
+    // stand between the end of the launch in front and the first activation copy of every block that was placed late).
+    constexpr bool LONE = ATMA && CG == 1;
+    uint32_t tmem_base = 0;
+    if (LONE && warp == WARP_TMA) {
+        named_arrive(1, blockDim.x);
+    } else {
+        tc_fence_before();
+        // pair: no remote arrive, copy completion or multicast commit may reach a barrier before its block initialised it
+        if (CG == 2) cluster_sync_all(); else if (LONE) named_sync(1, blockDim.x); else __syncthreads();
+        tc_fence_after();
+        tmem_base = *tmem_slot;
+    }
+    if (F4 && !(LONE && warp == WARP_TMA)) {
         // block scales: ue8m0 0x7F = 2^0 in every byte of columns 480..511 (16 columns for the
         // row scales, 16 for the column scales; one MMA reads at most four of each), so whatever
         // bytes the MMA picks as scale of a row block or column block, it reads 1.0
@@ -377,7 +394,8 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         }
         tc_fence_before();
-        if (CG == 2) cluster_sync_all(); else __syncthreads();  // pair: the first block's MMAs read both blocks' scales
+        // pair: the first block's MMAs read both blocks' scales
+        if (CG == 2) cluster_sync_all(); else if (LONE) named_sync(2, blockDim.x - 32); else __syncthreads();
         tc_fence_after();
     }
 
@@ -386,36 +404,55 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
     // after the wait (from that wait to the first complete stage took 2750 clocks).  32 KB, no more: where the block could
     // only start when the launch in front left its SM, the first stage's activations queue behind these copies (all
     // four stages of a 256-kernel tile requested early: 8 x 512x32x32 -> 512 12.9 us against 11.3).
-    constexpr int wpt = 4 / TAPS, SUBA = A_STAGE / TAPS;  // tensor-copy form: plane words and bytes per tap
+    constexpr int SUBA = A_STAGE / TAPS;  // tensor-copy form: bytes per tap
+    // Tensor-copy form: a stage's four plane words are TAPS filter taps (one of 256 channels, two of 128 or four of 64), one
+    // copy and one sub-tile each.  Words added by the pad-to-four have no tap: their sub-tile keeps what it held (any nibble is
+    // a finite e2m1 value) and meets zero weights.
+    const int T = p.KH * p.KW;
+    auto slot_bytes = [&](int c) {  // of the slot that begins with stage c
+        const int n = min(GRP, nchunks - c);
+        return (uint32_t)(n * B_STAGE + (TAPS == 1 ? n : min(n * TAPS, T - c * TAPS)) * SUBA);
+    };
+    auto copy_taps = [&](uint32_t s, int& ic, int& kw, int& kh, int a_w, int a_h, int a_n, uint32_t bar) {
+#pragma unroll
+        for (int q = 0; q < TAPS; q++) {
+            if (TAPS == 1 || kh < p.KH) {
+                const uint32_t dst = smem_u32(sA + s * A_STAGE + q * SUBA);
+                if (CG == 2) tma_im2col_g2s_pair(dst, &tmap_a, ic * 32, a_w, a_h, a_n, (unsigned short)kw, (unsigned short)kh, bar);
+                else tma_im2col_g2s(dst, &tmap_a, ic * 32, a_w, a_h, a_n, (unsigned short)kw, (unsigned short)kh, bar);
+            }
+            if (TAPS == 1 && (ic += 4) != p.Cp) continue;
+            ic = 0;
+            if (++kw == p.KW) { kw = 0; kh++; }
+        }
+    };
     const uint32_t bar_full_lead = (CG == 2) ? mapa_shared(bar_full, 0) : bar_full;  // pair: both blocks' copies report to the first block's barrier
-    constexpr int EARLY = 32768 / B_STAGE < NSTG ? 32768 / B_STAGE : NSTG;
-    const int early = min(EARLY, nchunks);
+    constexpr int EARLY = 32768 / (GRP * B_STAGE) < NSLOT ? 32768 / (GRP * B_STAGE) : NSLOT;
+    const int early = min(EARLY, (nchunks + GRP - 1) / GRP);  // slots
     // tile n_tile of BN kernels is rows [n_tile*BN % b_rows, +BN) of an image tile of b_rows kernels: one contiguous piece per stage
     // (only where narrower tiles exist: the expander-fed form is short of registers)
     constexpr bool PARTS = ATMA && CG == 1 && !QF;
     const size_t b_step = PARTS ? (size_t)p.b_rows * KCH : (size_t)B_STAGE;
     auto weights_of = [&](int n_tile) {
         if (!PARTS) return p.Bimg + (size_t)n_tile * nchunks * B_STAGE;
-        const uint32_t k0 = (uint32_t)n_tile * BN, big = k0 / (uint32_t)p.b_rows;
-        return p.Bimg + (size_t)big * nchunks * b_step + (size_t)(k0 - big * p.b_rows) * KCH;
+        const uint32_t k0 = (uint32_t)n_tile * BN, big = k0 >> p.b_shift;
+        return p.Bimg + (size_t)big * nchunks * b_step + (size_t)(k0 & (uint32_t)(p.b_rows - 1)) * KCH;
     };
     if (ATMA && warp == WARP_TMA && lane == 0) {
         prefetch_tensor_map(&tmap_a);
         if (CG == 2) prefetch_tensor_map(&tmap_b);
         if (unit < ntiles) {
-            const int n_tile = unit % ntn;
+            const int n_tile = unit - (int)p.div_ntn.div((uint32_t)unit) * ntn;
             const unsigned char* src = weights_of(n_tile);
-            for (int c = 0; c < early; c++) {
-                int a_bytes = 0;
-#pragma unroll
-                for (int q = 0; q < TAPS; q++)
-                    if (tap_at(4 * c + q * wpt) != 0xFFFFFFFFu) a_bytes += SUBA;
+            for (int e = 0; e < early; e++) {
                 if (CG == 2) {
-                    if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * c, CG * (B_STAGE + a_bytes));
-                    tma_tile2d_g2s_pair(smem_u32(sB + c * B_STAGE), &tmap_b, 0, (n_tile * nchunks + c) * BN + (int)rank * (BN / CG), bar_full_lead + 8 * c);
+                    if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * e, CG * slot_bytes(e));
+                    tma_tile2d_g2s_pair(smem_u32(sB + e * B_STAGE), &tmap_b, 0, (n_tile * nchunks + e) * BN + (int)rank * (BN / CG), bar_full_lead + 8 * e);
                 } else {
-                    mbar_arrive_expect_tx(bar_full + 8 * c, B_STAGE + a_bytes);
-                    bulk_g2s(smem_u32(sB + c * B_STAGE), src + (size_t)c * b_step, B_STAGE, bar_full + 8 * c);
+                    mbar_arrive_expect_tx(bar_full + 8 * e, slot_bytes(e * GRP));
+#pragma unroll
+                    for (int c = e * GRP; c < (e + 1) * GRP; c++)
+                        if (c < nchunks) bulk_g2s(smem_u32(sB + c * B_STAGE), src + (size_t)c * b_step, B_STAGE, bar_full + 8 * e);
                 }
             }
         }
@@ -429,24 +466,24 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
         if (lane == 0) {
             uint32_t s = 0, ph = 1;  // ring slot and the parity its "empty" barrier is waited with
             for (int t = unit; t < ntiles; t += nunits) {
-                const int n_tile = t % ntn;
+                const int m_tile = (int)p.div_ntn.div((uint32_t)t), n_tile = t - m_tile * ntn;
                 const unsigned char* src = weights_of(n_tile);
                 // tensor-copy activations: base pixel of the block's first output pixel
                 int a_n = 0, a_h = 0, a_w = 0;
                 if (ATMA) {
-                    long long row0 = (long long)(t / ntn) * TILE_M + (int)rank * BMT;
+                    long long row0 = (long long)m_tile * TILE_M + (int)rank * BMT;
                     if (row0 >= p.M) row0 = 0;  // second block of a pair past the last row: any valid pixels, never stored
-                    // 32-bit divisions where the row index allows it (64-bit ones cost this thread hundreds of cycles per tile)
-                    a_n = row0 < 0x7FFFFFFFLL ? (int)((uint32_t)row0 / (uint32_t)p.OHW) : (int)(row0 / p.OHW);
+                    // (64-bit divisions cost this thread hundreds of cycles per tile)
+                    a_n = row0 < 0x7FFFFFFFLL ? (int)p.div_ohw.div((uint32_t)row0) : (int)(row0 / p.OHW);
                     const int rem = (int)(row0 - (long long)a_n * p.OHW);
-                    const int oh = rem / p.OW;
+                    const int oh = (int)p.div_ow.div((uint32_t)rem);
                     a_h = oh * p.SH - p.PH;
                     a_w = (rem - oh * p.OW) * p.SW - p.PW;
                     if (QF) {
                         // the copies of this tile read the images of its rows: wait until the
                         // quantiser warps (of any block) have finished them
                         const long long last = min(row0 + BMT, p.M) - 1;
-                        const int n_last = last < 0x7FFFFFFFLL ? (int)((uint32_t)last / (uint32_t)p.OHW) : (int)(last / p.OHW);
+                        const int n_last = last < 0x7FFFFFFFLL ? (int)p.div_ohw.div((uint32_t)last) : (int)(last / p.OHW);
                         const unsigned int per_image = (unsigned int)(p.q_nbands * p.q_cp) * 4u;  // every quantiser warp counts itself
                         for (int n = a_n; n <= n_last; n++)
                             if (!counter_wait(p.q_sync + Q_FLAG0 + n, per_image, abort_flag, p.status, 6)) goto done;
@@ -454,60 +491,28 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                         asm volatile("fence.proxy.async.global;" ::: "memory");
                     }
                 }
-                int c = 0;
+                int c = 0, ic = 0, kw = 0, kh = 0;  // stage; channel word and tap its first copy takes
                 if (ATMA && t == unit) {
-                    // the stages whose weights were requested before the wait: activations only
-                    for (; c < early; c++) {
-#pragma unroll
-                        for (int q = 0; q < TAPS; q++) {
-                            const uint32_t tap = tap_at(4 * c + q * wpt);
-                            if (tap == 0xFFFFFFFFu) continue;
-                            const uint32_t dst = smem_u32(sA + c * A_STAGE + q * SUBA);
-                            if (CG == 2)
-                                tma_im2col_g2s_pair(dst, &tmap_a, (int)(tap & 0xFFFF) * 32, a_w, a_h, a_n, (unsigned short)((tap >> 16) & 0xFF),
-                                                    (unsigned short)(tap >> 24), bar_full_lead + 8 * c);
-                            else
-                                tma_im2col_g2s(dst, &tmap_a, (int)(tap & 0xFFFF) * 32, a_w, a_h, a_n, (unsigned short)((tap >> 16) & 0xFF),
-                                               (unsigned short)(tap >> 24), bar_full + 8 * c);
-                        }
-                    }
-                    s = early == NSTG ? 0u : (uint32_t)early;
-                    ph = early == NSTG ? 0u : 1u;
+                    // the slots whose weights were requested before the wait: activations only
+                    for (; c < early * GRP && c < nchunks; c++) copy_taps((uint32_t)c, ic, kw, kh, a_w, a_h, a_n, bar_full_lead + 8 * (c / GRP));
+                    s = early == NSLOT ? 0u : (uint32_t)early;
+                    ph = early == NSLOT ? 0u : 1u;
                 }
-                for (; c < nchunks; c++, s = (s + 1 == NSTG) ? 0 : s + 1, ph ^= (s == 0)) {
+                for (; c < nchunks; c += GRP, s = (s + 1 == NSLOT) ? 0 : s + 1, ph ^= (s == 0)) {
                     if (!mbar_wait(bar_empty + 8 * s, ph, abort_flag, p.status, 1)) goto done;
-                    // tensor-copy activations: the stage's four plane words are TAPS filter taps
-                    // (TAPS: one tap of 256 channels, two of 128 or four of 64), one copy and one sub-tile
-                    // each; words added by the pad-to-four have no tap: their sub-tile keeps what
-                    // it held (any nibble is a finite e2m1 value) and meets zero weights
-                    uint32_t tap[4];
-                    int a_bytes = 0;
-                    if (ATMA) {
-#pragma unroll
-                        for (int q = 0; q < TAPS; q++) {
-                            tap[q] = tap_at(4 * c + q * wpt);
-                            if (tap[q] != 0xFFFFFFFFu) a_bytes += SUBA;
-                        }
-                    }
                     if (CG == 2) {
-                        if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * s, CG * (B_STAGE + a_bytes));
+                        if (rank == 0) mbar_arrive_expect_tx(bar_full + 8 * s, CG * slot_bytes(c));
                         tma_tile2d_g2s_pair(smem_u32(sB + s * B_STAGE), &tmap_b, 0, (n_tile * nchunks + c) * BN + (int)rank * (BN / CG),
                                             bar_full_lead + 8 * s);
-#pragma unroll
-                        for (int q = 0; q < TAPS; q++)
-                            if (tap[q] != 0xFFFFFFFFu)
-                                tma_im2col_g2s_pair(smem_u32(sA + s * A_STAGE + q * SUBA), &tmap_a, (int)(tap[q] & 0xFFFF) * 32, a_w, a_h, a_n,
-                                                    (unsigned short)((tap[q] >> 16) & 0xFF), (unsigned short)(tap[q] >> 24), bar_full_lead + 8 * s);
+                        copy_taps(s, ic, kw, kh, a_w, a_h, a_n, bar_full_lead + 8 * s);
                         continue;
                     }
-                    mbar_arrive_expect_tx(bar_full + 8 * s, B_STAGE + a_bytes);
-                    bulk_g2s(smem_u32(sB + s * B_STAGE), src + (size_t)c * b_step, B_STAGE, bar_full + 8 * s);
-                    if (ATMA) {
+                    mbar_arrive_expect_tx(bar_full + 8 * s, ATMA ? slot_bytes(c) : (uint32_t)B_STAGE);
 #pragma unroll
-                        for (int q = 0; q < TAPS; q++)
-                            if (tap[q] != 0xFFFFFFFFu)
-                                tma_im2col_g2s(smem_u32(sA + s * A_STAGE + q * SUBA), &tmap_a, (int)(tap[q] & 0xFFFF) * 32, a_w, a_h, a_n,
-                                               (unsigned short)((tap[q] >> 16) & 0xFF), (unsigned short)(tap[q] >> 24), bar_full + 8 * s);
+                    for (int g = 0; g < GRP; g++) {
+                        if (g && c + g >= nchunks) break;
+                        bulk_g2s(smem_u32(sB + (s * GRP + g) * B_STAGE), src + (size_t)(c + g) * b_step, B_STAGE, bar_full + 8 * s);
+                        if (ATMA) copy_taps(s * GRP + g, ic, kw, kh, a_w, a_h, a_n, bar_full + 8 * s);
                     }
                 }
             }
@@ -534,28 +539,33 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * ACC_OFF;
                 uint32_t acc = 0;
-                for (int c = 0; c < nchunks; c++) {
+                for (int c = 0; c < nchunks; c += GRP) {
                     if (!mbar_wait(bar_full + 8 * s, ph, abort_flag, p.status, 3)) goto done;
                     tc_fence_after();
                     if (elected) {
 #pragma unroll
-                        for (int mt = 0; mt < MT; mt++) {
+                        for (int g = 0; g < GRP; g++) {
+                            if (g && c + g >= nchunks) break;
 #pragma unroll
-                            for (int k = 0; k < KCH / 32; k++) {
-                                // K step k: sub-tile k / KPS, 32 bytes x (k % KPS) into its rows
-                                constexpr int SUB16 = (A_STAGE / TAPS) >> 4;
-                                const uint32_t ak = a_lo + (uint32_t)(mt * (A_SUB >> 4) + (k / KPS) * SUB16 + 2 * (k % KPS));
-                                if (CG == 2) tc_mma_f4_pair_lh(d_tmem, ak, a_hi, b_lo + 2 * k, b_hi, IDESC, sfa, sfb, acc | (uint32_t)k);
-                                else if (F4) tc_mma_f4_lh(d_tmem + mt * BN, ak, a_hi, b_lo + 2 * k, b_hi, IDESC, sfa, sfb, acc | (uint32_t)k);
-                                else tc_mma_i8(d_tmem + mt * BN, ((uint64_t)a_hi << 32) | ak, ((uint64_t)b_hi << 32) | (b_lo + 2 * k), IDESC, (c | k) ? 1u : 0u);
+                            for (int mt = 0; mt < MT; mt++) {
+#pragma unroll
+                                for (int k = 0; k < KCH / 32; k++) {
+                                    // K step k: sub-tile k / KPS, 32 bytes x (k % KPS) into its rows
+                                    constexpr int SUB16 = (A_STAGE / TAPS) >> 4;
+                                    const uint32_t ak = a_lo + (uint32_t)(g * (A_STAGE >> 4) + mt * (A_SUB >> 4) + (k / KPS) * SUB16 + 2 * (k % KPS));
+                                    const uint32_t bk = b_lo + (uint32_t)(g * (B_STAGE >> 4) + 2 * k);
+                                    if (CG == 2) tc_mma_f4_pair_lh(d_tmem, ak, a_hi, bk, b_hi, IDESC, sfa, sfb, acc | (uint32_t)(g | k));
+                                    else if (F4) tc_mma_f4_lh(d_tmem + mt * BN, ak, a_hi, bk, b_hi, IDESC, sfa, sfb, acc | (uint32_t)(g | k));
+                                    else tc_mma_i8(d_tmem + mt * BN, ((uint64_t)a_hi << 32) | ak, ((uint64_t)b_hi << 32) | bk, IDESC, (c | k) ? 1u : 0u);
+                                }
                             }
                         }
-                        // stage reusable once these MMAs have read it (pair: in both blocks)
+                        // slot reusable once these MMAs have read it (pair: in both blocks)
                         if (CG == 2) tc_commit_pair(bar_empty + 8 * s); else tc_commit(bar_empty + 8 * s);
                     }
                     acc = 1;
-                    if (++s == NSTG) { s = 0; ph ^= 1; a_lo = a_lo0; b_lo = b_lo0; }
-                    else { a_lo += A_STAGE >> 4; b_lo += B_STAGE >> 4; }
+                    if (++s == NSLOT) { s = 0; ph ^= 1; a_lo = a_lo0; b_lo = b_lo0; }
+                    else { a_lo += GRP * (A_STAGE >> 4); b_lo += GRP * (B_STAGE >> 4); }
                 }
                 // accumulator complete (pair: each block's epilogue drains its own 128 rows)
                 if (elected) {
@@ -721,12 +731,13 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
         long long qt_img = -1;
         for (int t = unit + set * nunits; t < ntiles; t += NSETS * nunits, lt += NSETS) {
             const int buf = lt % NBUF;
-            const long long m0 = (long long)(t / ntn) * TILE_M + (int)rank * BMT + sub * BM;
-            const int n0 = (t % ntn) * BN;
+            const int m_tile = (int)p.div_ntn.div((uint32_t)t);
+            const long long m0 = (long long)m_tile * TILE_M + (int)rank * BMT + sub * BM;
+            const int n0 = (t - m_tile * ntn) * BN;
             // the row's image (a 64-bit division) and threshold: worked out while the tile's MMAs run
             const long long row = m0 + q * 32 + lane;
             const bool row_ok = row < p.M;
-            const long long n_img = !row_ok ? 0 : row < 0x7FFFFFFFLL ? (long long)((uint32_t)row / (uint32_t)p.OHW) : row / p.OHW;
+            const long long n_img = !row_ok ? 0 : row < 0x7FFFFFFFLL ? (long long)p.div_ohw.div((uint32_t)row) : row / p.OHW;
             const int rem = (int)(row - n_img * p.OHW);
             float* ybase = (p.layout == TNNS_NHWC) ? p.y + (size_t)row * p.KN : p.y + (size_t)n_img * p.KN * p.OHW + rem;
             const float tq = (p.pimg && row_ok) ? __ldg(p.thr_next + n_img) + 0.0f : 0.f;  // + 0.0f: -0 acts as +0
@@ -848,7 +859,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ CUtensorMap tmap_a, const __g
                                 // branch that stores it: as a value kept across the slices it cost the fp32 path 3 % on the large layer)
                                 long long opix = n_img * p.OHW + rem;
                                 if (!QF && p.o_HpWp) {
-                                    const int oh = rem / p.OW;
+                                    const int oh = (int)p.div_ow.div((uint32_t)rem);
                                     opix = n_img * p.o_HpWp + (long long)(oh + p.o_PH) * p.o_Wp + (rem - oh * p.OW) + p.o_PW;
                                 }
                                 uint4* px = reinterpret_cast<uint4*>(p.pimg) + (size_t)opix * ((size_t)p.cp_next * 2) + (c0 >> 5);
@@ -1008,17 +1019,18 @@ __global__ void __launch_bounds__(128, 1) mma_rate_kernel(int iters, unsigned in
 }
 
 template <int BN, int MT, bool F4, bool ATMA = false, int CG = 1, int TAPS = 1, bool QF = false, bool SINGLE = false>
-int launch_cfg(tnns_cuda_ctx* ctx, const GemmArgs& a, cudaStream_t stream, const CUtensorMap* tmap_a = nullptr,
+int launch_cfg(tnns_cuda_ctx* ctx, GemmArgs a, cudaStream_t stream, const CUtensorMap* tmap_a = nullptr,
                const CUtensorMap* tmap_b = nullptr, const CUtensorMap* tmap_q = nullptr) {
     using Cfg = TcCfg<BN, MT, F4, ATMA, CG, TAPS, QF>;
     auto kern = gemm_tc_kernel<BN, MT, F4, ATMA, CG, TAPS, QF, SINGLE>;
-    static const CUtensorMap no_map = {};
+    const auto maps = tensor_maps<maps_of(CG, QF)>(tmap_a, tmap_b, tmap_q);
     // once per kernel and device: the attribute belongs to (function, device), and the call costs a microsecond per launch
     static bool smem_set[64] = {false};
     if (!smem_set[ctx->device & 63]) {
         TNNS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM));
         smem_set[ctx->device & 63] = true;
     }
+    a.div_ntn = tnns_fastdiv((uint32_t)((a.KN + BN - 1) / BN));
     const long long tiles = ((a.M + CG * MT * BM - 1) / (CG * MT * BM)) * ((a.KN + BN - 1) / BN);
     if (tiles >= 0x7FFFFFFFLL) return tnns_fail(TNNS_ERR_UNSUPPORTED, "too many output tiles");
     // the launch may be scheduled while its predecessor on the stream drains (the kernel
@@ -1037,7 +1049,7 @@ int launch_cfg(tnns_cuda_ctx* ctx, const GemmArgs& a, cudaStream_t stream, const
         cfg.stream = stream;
         cfg.attrs = attr;
         cfg.numAttrs = nattr;
-        TNNS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a, tmap_a ? *tmap_a : no_map, no_map, tmap_q ? *tmap_q : no_map));
+        TNNS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a, maps));
     } else {
         // block pairs: clusters of two consecutive blocks, as many as can be resident at once (the
         // kernel is persistent; a pair that had to wait for a free TPC would start its whole tile
@@ -1063,7 +1075,7 @@ int launch_cfg(tnns_cuda_ctx* ctx, const GemmArgs& a, cudaStream_t stream, const
             mp = std::min(n, ctx->sm_count / CG);
         }
         cfg.gridDim = dim3(CG * (int)std::min<long long>(tiles, mp));
-        TNNS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a, tmap_a ? *tmap_a : no_map, tmap_b ? *tmap_b : no_map, tmap_q ? *tmap_q : no_map));
+        TNNS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, a, maps));
     }
     tnns_count_launch();
     TNNS_CUDA_TRY(cudaGetLastError());
@@ -1171,8 +1183,10 @@ int tnns_launch_gemm_tc(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const vo
     a.KN = w->KN;
     a.Kp = w->Kp;
     a.b_rows = tnns_i8_tile_n(w->KN);
+    a.b_shift = a.b_rows == 64 ? 6 : a.b_rows == 128 ? 7 : 8;
     a.y_vec = tnns_row_vec(d_y, w->KN);
     a.OHW = OHW;
+    a.div_ohw = a.div_ow = tnns_fastdiv((uint32_t)std::max(OHW, 1));
     // one output pixel per image (fully connected layers): both layouts are the same memory, and the pixel-major
     // epilogue writes 16 bytes per lane where the channel-major one would write 4 (rows are KN floats apart either way)
     a.layout = OHW == 1 ? TNNS_NHWC : layout;
@@ -1190,7 +1204,7 @@ int tnns_launch_gemm_tc(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const vo
     a.cp_next = (w->KN + TNNS_WORD_BITS - 1) / TNNS_WORD_BITS;
     a.img = nullptr;
     a.jtab = nullptr;
-    a.H = a.W = a.OW = a.Cp = a.SH = a.SW = a.PH = a.PW = 0;
+    a.H = a.W = a.OW = a.Cp = a.SH = a.SW = a.PH = a.PW = a.KH = a.KW = 0;
     a.qx = a.qthr = nullptr; a.qimg = nullptr; a.q_sync = nullptr; a.qN = a.qC = a.q_nbands = a.q_cp = a.q_self_clean = a.q_nhwc = 0;
     if (implicit_geom) {
         // d_a is the quantised image of the layer input, not an im2row matrix
@@ -1262,8 +1276,8 @@ int encode_im2col_map(CUtensorMap* map, const void* d_image, const TnnsGeom& g) 
     if (r != CUDA_SUCCESS) return tnns_fail(TNNS_ERR_CUDA, "cuTensorMapEncodeIm2col failed with driver error %d", (int)r);
     // Drivers up to 13.1 set a flag in im2col maps of tensors below 128 KiB that must be clear
     // (the correction CUTLASS applies to its im2col descriptors, cute/atom/copy_traits_sm90_im2col.hpp).
-    int driver = 0;
-    TNNS_CUDA_TRY(cudaDriverGetVersion(&driver));
+    static int driver = 0;
+    if (!driver) TNNS_CUDA_TRY(cudaDriverGetVersion(&driver));
     if (driver <= 13010 && cbytes * g.W * g.H * g.N < 131072) reinterpret_cast<uint64_t*>(map)[1] &= ~(1ull << 21);
     return TNNS_OK;
 }
@@ -1347,6 +1361,7 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
     a.KN = w->KN;
     a.Kp = w->Kp;
     a.b_rows = tnns_i8_tile_n(w->KN);
+    a.b_shift = a.b_rows == 64 ? 6 : a.b_rows == 128 ? 7 : 8;
     a.y_vec = tnns_row_vec(d_y, w->KN);
     a.OHW = g.OH * g.OW;
     a.layout = a.OHW == 1 ? TNNS_NHWC : layout;  // one pixel per image: same memory, wider stores (see above)
@@ -1371,9 +1386,12 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
     }
     a.cp_next = (w->KN + TNNS_WORD_BITS - 1) / TNNS_WORD_BITS;
     a.img = nullptr;
-    a.jtab = w->d_jtab;
+    a.jtab = nullptr;
     a.qx = a.qthr = nullptr; a.qimg = nullptr; a.q_sync = nullptr; a.qN = a.qC = a.q_nbands = a.q_cp = a.q_self_clean = a.q_nhwc = 0;
     a.H = g.H; a.W = g.W; a.OW = g.OW; a.Cp = g.Cp; a.SH = g.SH; a.SW = g.SW; a.PH = g.PH; a.PW = g.PW;
+    a.KH = g.KH; a.KW = g.KW;
+    a.div_ohw = tnns_fastdiv((uint32_t)a.OHW);
+    a.div_ow = tnns_fastdiv((uint32_t)g.OW);
     alignas(64) CUtensorMap map_q;
     if (fused) {
         // the fp32 input as images x channels x H*W floats; box = 128 pixels x 64 channels of one image

@@ -43,6 +43,24 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}" : "=r"(p));
     return p != 0;
 }
+// Named barrier `id` of `threads` threads: warps that only announce what they did, and those that wait for it.
+__device__ __forceinline__ void named_arrive(int id, int threads) { asm volatile("barrier.cta.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+// The tensor maps a kernel reads, as one parameter: activations; with block pairs weights; with quantiser warps the fp32 input
+// (a launch pays for every byte of its parameters).
+constexpr int maps_of(int CG, bool QF) { return QF ? 3 : CG == 2 ? 2 : 1; }
+template <int N>
+struct alignas(64) TensorMaps {
+    CUtensorMap m[N];
+};
+template <int N>
+inline TensorMaps<N> tensor_maps(const CUtensorMap* a, const CUtensorMap* b, const CUtensorMap* q) {
+    TensorMaps<N> t = {};
+    if (a) t.m[0] = *a;
+    if constexpr (N > 1) { if (b) t.m[1] = *b; }
+    if constexpr (N > 2) { if (q) t.m[2] = *q; }
+    return t;
+}
 __device__ __forceinline__ void prefetch_tensor_map(const void* tmap) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
 }

@@ -347,8 +347,7 @@ FastDiv tnns_fastdiv(uint32_t d) {
     FastDiv f;
     f.d = d;
     if (d <= 1) { f.mul = 0; f.sh1 = 0; f.sh2 = 0; return f; }  // t=0 -> (0 + (n>>0)) >> 0 = n
-    uint32_t l = 0;
-    while ((1ull << l) < d) l++;
+    const uint32_t l = 32 - (uint32_t)__builtin_clz(d - 1);  // the least l with 2^l >= d
     const uint64_t m = ((1ull << 32) * ((1ull << l) - d)) / d + 1;
     f.mul = (uint32_t)m;
     f.sh1 = 1;
