@@ -33,12 +33,13 @@
 
 namespace {
 
-constexpr int SL_MAXSLAB = 4;    // slab buffers at most
+constexpr int SL_MAXSLAB = 8;    // slab buffers at most
 constexpr int SL_MAXSTG = 12;    // weight ring depth at most
 constexpr int SL_TAPMAX = 4096;  // filter taps at most
 constexpr int SL_BAR_BYTES = 512;
 
 struct SlabArgs {
+    const unsigned char* Aimg;  // the bordered image
     const unsigned char* Bimg;  // expanded weights [n_tile][stage][BN rows][128 B]
     float* y;
     int Mv;                     // virtual rows: N * Hp * Wp
@@ -48,7 +49,7 @@ struct SlabArgs {
     int OH, OW, Wp, HpWp;       // output size, padded input lattice
     int KW, T;                  // filter width, taps KH*KW
     int G;                      // 128-byte channel groups per pixel (one slab each); 1 for 64 / 128 channels
-    int slab_bytes, copy_rows, ncopies;  // slab buffer size; rows per tensor copy and copies per slab
+    int slab_bytes, slab_rows, copy_rows, ncopies;  // slab buffer size, rows; rows per tensor copy and copies per slab
     int nslab, nstg;            // ring depths: slabs, weight stages
     int b_resident;             // the kernel tile's weight stages all fit the ring: fetched once per block
     int layout, zero_passes, acc_bias;
@@ -69,7 +70,15 @@ struct SlabArgs {
     FastDiv div_hpwp, div_wp, div_ntn;
 };
 
-template <int BN, int CG, int TAPS, bool QF>
+// 16 bytes, global -> shared memory by this thread's own copy; the last `16 - bytes` of them zeros
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// IMG: quantised output for a following layer, in kernels of its own: either epilogue's registers and code cost the other (the
+// one-launch forms, which the library never picks by itself, keep both).  On single blocks with 32- or 64-byte pixels it comes with
+// slab loaders and, on tiles of 64 kernels, two MMA issuers and a set of epilogue warps per accumulator.
+template <int BN, int CG, int TAPS, bool QF, bool IMG>
 struct SlabCfg {
     static constexpr int RB = 128 / TAPS;             // bytes of a pixel in a slab row
     static constexpr int B_STAGE = (BN / CG) * KCH;   // bytes of a weight stage in one block
@@ -81,12 +90,22 @@ struct SlabCfg {
     // arithmetic) several times as long as its MMAs, so three tiles are drained at once.  Eight warps on one tile / two sets /
     // three sets, inside the 11-layer stack: 64 -> 64 @56 48.3 / 39.8 / 33.0 us, 128 -> 128 @28 25.9 / 22.1 / 19.4; four
     // sets of the 64-kernel form gained nothing more.
-    static constexpr int EPW = OVL ? 2 : 1, NSETS = OVL ? 1 : (QF ? 2 : 3);
+    static constexpr bool LOADER = IMG && CG == 1 && TAPS > 1 && !QF;
+    static constexpr bool TWO = LOADER && BN == 64;   // two MMA issuers (see the kernel)
+    static constexpr int EPW = OVL ? 2 : 1, NSETS = OVL ? 1 : TWO ? 4 : (QF ? 2 : 3);
     // (a set's next tile waits for its barrier's phase by parity: the phase before must be complete by then)
     static_assert(NSETS <= NBUF, "a set may not be a whole turn of the accumulators ahead");
     static constexpr int NEPI = 4 * EPW * NSETS;      // epilogue warps
-    static constexpr int WARP_EPI0 = 2, WARP_Q0 = 2 + NEPI;
-    static constexpr int NTHREADS = 32 * (2 + NEPI + (QF ? 5 : 0));
+    // issuers may finish their tiles out of turn: every accumulator then belongs to one issuer and one set
+    static_assert(!TWO || (NBUF % 2 == 0 && NSETS == NBUF), "waits by parity: everyone meets a barrier in successive phases");
+    // Slab loaders.  A tiled tensor copy moves one box row in about 2.6 clocks whatever its length, so slabs of 32-byte pixels came
+    // at 640 clocks a tile of 64 kernels (246 rows at 56x56), whose MMAs take 432.  The slab is contiguous in the image: two warps
+    // fetch it in 16-byte pieces and place them in the swizzle pattern.  Image out, one GEMM, before loaders, second issuer and the
+    // epilogue of quantise32_e2m1 / after: 256 x 64x56x56 -> 64 34.3 / 26.0 us, 256 x 128x28x28 -> 128 20.6 / 17.5, 8 x 64x112x112 ->
+    // 64 7.4 / 6.8 (the drain alone takes some 900 clocks a tile of 64 kernels, the MMAs alone 475).
+    static constexpr int NLOAD = LOADER ? 2 : 0, WARP_LOAD0 = 2;
+    static constexpr int WARP_EPI0 = 2 + NLOAD, WARP_Q0 = WARP_EPI0 + NEPI;
+    static constexpr int NTHREADS = 32 * (WARP_EPI0 + NEPI + (QF ? 5 : 0));
     static constexpr int Q_STAGE = Q_PIX * 64 * 4;
     static constexpr int SMEM_MAX = 232448;
 };
@@ -95,11 +114,11 @@ struct SlabCfg {
 // tiles of 64 or 128 kernels whose weights stream.  There the producer's wait, announcement and copy take some 300 clocks a
 // slot and the MMA warp's wait and commit another 80, the four MMAs of a stage of 64 kernels 192.  GEMM alone, one stage a slot and a
 // division per stage / so: 8 x 512x14x14 -> 512 8.8 / 6.4 us, 8 x 1024x14x14 -> 1024 16.0 / 11.3, 8 x 256x28x28 -> 256 7.2 / 6.1.
-template <int BN, int CG, int TAPS, bool QF, bool SINGLE, int GRP>
-__global__ void __launch_bounds__(SlabCfg<BN, CG, TAPS, QF>::NTHREADS, 1)
+template <int BN, int CG, int TAPS, bool QF, bool SINGLE, int GRP, bool IMG>
+__global__ void __launch_bounds__(SlabCfg<BN, CG, TAPS, QF, IMG>::NTHREADS, 1)
 gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> maps) {
     const CUtensorMap &tmap_a = maps.m[0], &tmap_b = maps.m[CG == 2 ? 1 : 0], &tmap_q = maps.m[QF ? 2 : 0];
-    using Cfg = SlabCfg<BN, CG, TAPS, QF>;
+    using Cfg = SlabCfg<BN, CG, TAPS, QF, IMG>;
     static_assert(GRP == 1 || (GRP == 3 && TAPS == 1 && CG == 1 && !QF), "slots of three stages: streamed 3x3 weights of 128-byte pixels");
     constexpr int RB = Cfg::RB, B_STAGE = Cfg::B_STAGE, WARP_EPI0 = Cfg::WARP_EPI0, EPW = Cfg::EPW, ACC_OFF = Cfg::ACC_OFF;
     constexpr bool OVL = Cfg::OVL;
@@ -171,6 +190,10 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
     }
     constexpr bool LONE = CG == 1;
     const bool ahead = LONE && warp == WARP_TMA;
+    // Two warps issue the MMAs of every other tile each where a tile has few of them and the weights stay: the producer's warp has
+    // nothing left to do, and a tile's two waits (110-140 clocks each even when complete) pass beside the other's MMAs.  Both take an
+    // even number of slabs and accumulators in turn, so each meets the same ones in successive phases.
+    const bool two = Cfg::TWO && p.b_resident && p.T == 9 && p.KW == 3;
     uint32_t tmem_base = 0;
     if (ahead) {
         named_arrive(1, blockDim.x);
@@ -192,7 +215,7 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
     }
     if (!ahead) {
         tc_fence_before();
-        if (CG == 2) cluster_sync_all(); else named_sync(2, blockDim.x - 32);
+        if (CG == 2) cluster_sync_all(); else named_sync(2, two ? blockDim.x : blockDim.x - 32);
         tc_fence_after();
     }
 
@@ -221,7 +244,7 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
     constexpr int EARLY = 32768 / (GRP * B_STAGE) > 0 ? 32768 / (GRP * B_STAGE) * GRP : GRP;
     const int early = min(min(EARLY, p.nstg), SPG);
     if (warp == WARP_TMA && lane == 0 && unit < ntiles) {
-        prefetch_tensor_map(&tmap_a);
+        if (!Cfg::LOADER) prefetch_tensor_map(&tmap_a);
         const int n_tile = unit - (int)p.div_ntn.div((uint32_t)unit) * ntn;
         const unsigned char* src = weights_of(n_tile);
         for (int j = 0; j < early; j += GRP) {
@@ -231,17 +254,24 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
         }
     }
 
+    if (two && warp == WARP_TMA) {
+        __syncwarp();
+        named_sync(2, blockDim.x);
+        tc_fence_after();
+        tmem_base = *tmem_slot;
+    }
+
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     if (warp == WARP_TMA) {
         if (lane == 0) {
             uint32_t sl = 0, slph = 1, s = 0, ph = 1;
             const uint32_t nslots = (uint32_t)p.nstg / GRP;
-            bool free_slot = false;  // slot s has been seen free
             bool first_tile = true;
             const uint32_t sfull_lead = (CG == 2) ? mapa_shared(bar_sfull, 0) : bar_sfull;
             const uint32_t copy_bytes = (uint32_t)(p.ncopies * p.copy_rows * RB);
-            for (int t = unit; t < ntiles; t += nunits, first_tile = false) {
+            // (with loaders and weights that stay only the first tile's weights are left to request)
+            for (int t = unit; t < ntiles && !(Cfg::LOADER && p.b_resident && !first_tile); t += nunits, first_tile = false) {
                 const int m_tile = (int)p.div_ntn.div((uint32_t)t), n_tile = t - m_tile * ntn;
                 const unsigned char* src = weights_of(n_tile);
                 const int q0 = m_tile * TILE_M + (int)rank * BM;  // first virtual row = first pixel of the block's slab
@@ -256,9 +286,10 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
                     asm volatile("fence.proxy.async.global;" ::: "memory");
                 }
                 for (int cg = 0; cg < p.G; cg++) {
-                    if (!mbar_wait(bar_sempty + 8 * sl, slph, abort_flag, p.status, 0x11)) goto done;
+                    if (!Cfg::LOADER && !mbar_wait(bar_sempty + 8 * sl, slph, abort_flag, p.status, 0x11)) goto done;
                     const uint32_t dst = smem_u32(sA + sl * p.slab_bytes);
-                    if (CG == 2) {
+                    if (Cfg::LOADER) {
+                    } else if (CG == 2) {
                         if (rank == 0) mbar_arrive_expect_tx(bar_sfull + 8 * sl, CG * copy_bytes);
                         for (int i = 0; i < p.ncopies; i++)
                             tma_tile2d_g2s_pair(dst + i * p.copy_rows * RB, &tmap_a, cg * KCH, q0 + i * p.copy_rows, sfull_lead + 8 * sl);
@@ -285,9 +316,8 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
                         w += (size_t)early * j_step;
                     }
                     for (; j < SPG; j += GRP) {
-                        if (!free_slot && !mbar_wait(bar_bempty + 8 * s, ph, abort_flag, p.status, 1)) goto done;
+                        if (!mbar_wait(bar_bempty + 8 * s, ph, abort_flag, p.status, 1)) goto done;
                         const uint32_t s1 = s + 1 == nslots ? 0u : s + 1;
-                        free_slot = mbar_test(bar_bempty + 8 * s1, ph ^ (s1 == 0 ? 1u : 0u));  // the next slot
                         request_weights(w, n_tile, (TAPS == 1) ? j * p.G + cg : j, s * GRP, s);
                         w += GRP * j_step;
                         s = s1;
@@ -296,14 +326,17 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
                 }
             }
         }
-    } else if (warp == WARP_MMA) {
+        __syncwarp();
+    }
+    if (warp == WARP_MMA || (two && warp == WARP_TMA)) {
         if (rank == 0) {  // pair: the first block issues for both
             // This warp's instruction stream paces the tensor pipe: it runs warp-uniform (see elect_one), nothing that
             // touches shared memory stands between two MMAs of a slab (a table look-up per tap, queued behind the MMAs just
             // issued, cost 60 clocks per MMA: tap offsets are registers or running counters), and a slab's MMAs sit in as few
             // elected regions as the weight waits allow (one by one, every reconvergence waited for the MMA before it).
             const bool elected = elect_one();
-            uint32_t lt = 0, sl = 0, slph = 0, s = 0, ph = 0;
+            const uint32_t step = two ? 2u : 1u;  // issuers that take the tiles in turn
+            uint32_t lt = warp == WARP_MMA ? 0u : 1u, sl = lt, slph = 0, s = 0, ph = 0;
             bool first_tile = true;
             const uint64_t da0 = make_desc_taps(smem_u32(sA), TAPS), db0 = make_desc(smem_u32(sB));
             const uint32_t slab16 = (uint32_t)(p.slab_bytes >> 4);
@@ -322,21 +355,15 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
                 // 3x3 filters: the MMAs of a slab (or, where weights stream, of a stage) are straight-line code, every operand one
                 // of four uniform values (the slab's first three image rows, the weights) plus a constant.
                 const uint32_t nslots = (uint32_t)p.nstg / GRP;
-                bool there = false;  // slot s has been seen complete
                 constexpr int KPT = 4 / TAPS;               // K steps (32 bytes) per tap: 1, 2 or 4
                 constexpr int NK = 9 * KPT, NST = (NK + 3) / 4;  // K steps and weight stages of a slab
-                bool acc_free = false, slab_there = false;  // the tile's accumulator / the slab sl has been seen free / complete
-                for (int t = unit; t < ntiles; t += nunits, lt++, first_tile = false) {
+                for (int t = unit + (int)lt * nunits; t < ntiles; t += (int)step * nunits, lt += step, first_tile = false) {
                     const int buf = (int)(lt % NBUF);
-                    if (!acc_free && !mbar_wait(OVL ? bar_tempty : bar_tempty + 8 * buf, (OVL ? (lt & 1) : ((lt / NBUF) & 1)) ^ 1, abort_flag, p.status, 2)) goto done;
+                    if (!mbar_wait(OVL ? bar_tempty : bar_tempty + 8 * buf, (OVL ? (lt & 1) : ((lt / NBUF) & 1)) ^ 1, abort_flag, p.status, 2)) goto done;
                     tc_fence_after();
                     const uint32_t d_tmem = tmem_base + buf * ACC_OFF;
                     for (int cg = 0; cg < p.G; cg++) {
-                        if (!slab_there && !mbar_wait(bar_sfull + 8 * sl, slph, abort_flag, p.status, 0x13)) goto done;
-                        // look at what comes next now: the answers arrive while this slab's MMAs are issued
-                        const uint32_t sl1 = sl + 1 == (uint32_t)p.nslab ? 0u : sl + 1;
-                        slab_there = mbar_test(bar_sfull + 8 * sl1, slph ^ (sl1 == 0 ? 1u : 0u));
-                        if (!OVL) acc_free = mbar_test(bar_tempty + 8 * ((lt + 1) % NBUF), (((lt + 1) / NBUF) & 1) ^ 1);
+                        if (!mbar_wait(bar_sfull + 8 * sl, slph, abort_flag, p.status, 0x13)) goto done;
                         const uint32_t slab_lo = a_lo0 + sl * slab16, slab_lo1 = slab_lo + row16, slab_lo2 = slab_lo1 + row16;
                         // K step q of the slab: 32 bytes x (q % KPT) into the pixels of tap q / KPT
                         auto a_of = [&](int q) {
@@ -348,10 +375,9 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
                             uint32_t row_lo = slab_lo;
 #pragma unroll 1
                             for (int kh = 0; kh < 3; kh++, row_lo += row16) {
-                                if (!there && !mbar_wait(bar_bfull + 8 * s, ph, abort_flag, p.status, 3)) goto done;
+                                if (!mbar_wait(bar_bfull + 8 * s, ph, abort_flag, p.status, 3)) goto done;
                                 tc_fence_after();
                                 const uint32_t s1 = s + 1 == nslots ? 0u : s + 1;
-                                there = mbar_test(bar_bfull + 8 * s1, ph ^ (s1 == 0 ? 1u : 0u));  // the next slot
                                 const uint32_t b_lo = b_lo0 + s * (uint32_t)(GRP * (B_STAGE >> 4));
                                 if (elected) {
 #pragma unroll
@@ -397,10 +423,9 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
                         } else {
 #pragma unroll
                             for (int j = 0; j < NST; j++) {
-                                if (!there && !mbar_wait(bar_bfull + 8 * s, ph, abort_flag, p.status, 3)) goto done;
+                                if (!mbar_wait(bar_bfull + 8 * s, ph, abort_flag, p.status, 3)) goto done;
                                 tc_fence_after();
                                 const uint32_t s1 = s + 1 == nslots ? 0u : s + 1;
-                                there = mbar_test(bar_bfull + 8 * s1, ph ^ (s1 == 0 ? 1u : 0u));  // the next slot
                                 const uint32_t b_lo = b_lo0 + s * (uint32_t)(B_STAGE >> 4);
                                 if (elected) {
 #pragma unroll
@@ -413,7 +438,7 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
                                 if (s1 == 0) ph ^= 1;
                             }
                         }
-                        if (++sl == (uint32_t)p.nslab) { sl = 0; slph ^= 1; }
+                        if ((sl += step) >= (uint32_t)p.nslab) { sl -= (uint32_t)p.nslab; slph ^= 1; }
                     }
                     if (elected) commit(bar_tfull + 8 * buf);
                 }
@@ -472,6 +497,67 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
                 if (elected) commit(bar_tfull + 8 * buf);
             }
         }
+    } else if (warp == WARP_TMA) {
+        // (done above)
+    } else if (Cfg::LOADER && warp < WARP_EPI0) {
+        // ---------------- slab loaders: every NLOAD-th tile of the block's sequence ----------------
+        constexpr int NLOAD = Cfg::LOADER ? Cfg::NLOAD : 1;
+        const int me = warp - Cfg::WARP_LOAD0;
+        // piece i of a slab goes to byte 16*i with the swizzle pattern applied: address bits 4.. are XORed with bits 7.. (one bit for
+        // 32-byte rows, two for 64-byte rows), and since a warp's 32 pieces are 512 bytes only the lane decides those
+        const uint32_t lane_dst = (uint32_t)(lane * 16) ^ ((uint32_t)((lane >> 3) & (RB / 16 - 1)) << 4);
+        const int pieces = p.slab_rows * (RB / 16);
+        const long long total = (long long)p.Mv * (RB / 16);  // pieces of the image; past its end a slab is filled with zeros
+        // Slabs requested and not yet announced, oldest first.  A fill may have to wait for the slab nslab fills before it to be
+        // multiplied, so those this warp holds back must be younger than that.
+        const int hold = min(2, (p.nslab - 1) / NLOAD);
+        int held = 0;
+        uint32_t sl = (uint32_t)me, slph = 1, oldest = (uint32_t)me;
+        auto announce = [&]() {
+            fence_proxy_async();  // these lanes' pieces -> visible to the tensor core's async proxy
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_sfull + 8 * oldest);
+            oldest += NLOAD;
+            if (oldest >= (uint32_t)p.nslab) oldest -= (uint32_t)p.nslab;
+            held--;
+        };
+        for (int t = unit + me * nunits; t < ntiles; t += NLOAD * nunits) {
+            const long long piece0 = (long long)p.div_ntn.div((uint32_t)t) * (TILE_M * (RB / 16));
+            if (!mbar_wait(bar_sempty + 8 * sl, slph, abort_flag, p.status, 0x11)) goto done;
+            const uint32_t dst = smem_u32(sA + sl * p.slab_bytes) + lane_dst;
+            const unsigned char* src = p.Aimg + (size_t)piece0 * 16 + lane * 16;
+            if (piece0 + pieces <= total) {
+                int i = lane;
+#pragma unroll 1
+                for (; i + 7 * 32 < pieces; i += 8 * 32, src += 8 * 512) {
+#pragma unroll
+                    for (int u = 0; u < 8; u++) cp_async16(dst + (uint32_t)(i - lane + u * 32) * 16, src + u * 512, 16);
+                }
+                for (; i < pieces; i += 32, src += 512) cp_async16(dst + (uint32_t)(i - lane) * 16, src, 16);
+            } else {
+                for (int i = lane; i < pieces; i += 32, src += 512) {
+                    const bool there = piece0 + i < total;
+                    cp_async16(dst + (uint32_t)(i - lane) * 16, there ? src : p.Aimg, there ? 16 : 0);
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (++held > hold) {
+                if (hold == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
+                else if (hold == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+                else asm volatile("cp.async.wait_group 0;" ::: "memory");
+                announce();
+            }
+            sl += NLOAD;
+            if (sl >= (uint32_t)p.nslab) { sl -= (uint32_t)p.nslab; slph ^= 1; }
+        }
+        if (held == 2) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            announce();
+        }
+        if (held == 1) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            announce();
+        }
     } else if (QF && warp >= Cfg::WARP_Q0) {
         uint64_t* qbars = reinterpret_cast<uint64_t*>(q_ring + Q_STG * Cfg::Q_STAGE);
         if (warp < Cfg::WARP_Q0 + 4) {
@@ -499,18 +585,17 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
         const int OHW = p.OH * p.OW;
         uint32_t lt = (uint32_t)set;
         const uint32_t bar_release = (CG == 2 && rank != 0) ? mapa_shared(bar_tempty, 0) : 0u;
-        // quantised output with 0 < alpha <= 1: PReLU and the next layer's rule collapse into thresholds on
-        // the accumulator (two instructions per output and plane instead of evaluating the PReLU first).
-        // Taken on 256-kernel tiles only: on narrower tiles, where the epilogue of one tile runs beside the few
-        // MMAs of the next, the shorter but denser instruction stream slowed the tensor pipe more than it
-        // saved (256 x 64x56x56 -> 64 with a bordered image out: 38.2 us against 33.4; 128 -> 128 @28 21.3 against 19.5).
+        // quantised output with 0 < alpha <= 1: PReLU and the next layer's rule collapse into thresholds on the accumulator
         const bool next_tern = !p.next_binary && p.next_format != 0;
-        const bool by_thr = BN == 256 && p.pimg != nullptr && alpha_in_unit;
+        const bool img_out = IMG || (QF && p.pimg != nullptr);
+        const bool by_thr = img_out && alpha_in_unit && (BN == 256 || p.next_format >= 2);
         tnns_thr::Pair qt = {0.f, 0.f};
-        int qt_img = -1;
+        E2m1Rule qe = {0.f, 0.f};
+        float qt_t = 0.f;
+        bool qt_set = false;
         // pixel-major fp32 output: the accumulator is fetched in the 16x256b shape (four lanes = 32 contiguous bytes of a row)
         // -- float pairs (y_vec), or, in kernels of their own, single floats (SINGLE)
-        const bool rows16 = p.pimg == nullptr && p.layout == TNNS_NHWC && (SINGLE || p.y_vec > 1);
+        const bool rows16 = !img_out && p.layout == TNNS_NHWC && (SINGLE || p.y_vec > 1);
         for (int t = unit + set * nunits; t < ntiles; t += NSETS * nunits, lt += NSETS) {
             const int buf = (int)(lt % NBUF);
             const int m_tile = (int)p.div_ntn.div((uint32_t)t), n0 = (t - m_tile * ntn) * BN;
@@ -522,12 +607,30 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
             const int yy = (int)p.div_wp.div((uint32_t)max(rem, 0)), xx = rem - yy * p.Wp;
             const bool valid = row_ok && yy < p.OH && xx < p.OW;   // a real output pixel (oh, ow) = (yy, xx)
             const int opix = yy * p.OW + xx;
-            float* ybase = (p.layout == TNNS_NHWC) ? p.y + ((size_t)n_img * OHW + opix) * p.KN : p.y + (size_t)n_img * p.KN * OHW + opix;
-            const float tq = (p.pimg && valid) ? __ldg(p.thr_next + n_img) + 0.0f : 0.f;
-            if (by_thr && valid && n_img != qt_img) {
-                // the next layer's rule as thresholds on the raw accumulator, once per image this thread meets
+            // (worked out here, while the tile's MMAs run: in the loop below it cost the fp32 layers up to a tenth)
+            float* ybase = IMG ? nullptr : (p.layout == TNNS_NHWC) ? p.y + ((size_t)n_img * OHW + opix) * p.KN : p.y + (size_t)n_img * p.KN * OHW + opix;
+            // 4-bit image out: where the row's pixel goes, nullptr if it has none.  In a bordered image a row that is no output pixel
+            // (yy >= OH or xx >= OW) stands for one border pixel -- the next layer's padded lattice is this layer's: shifted by the
+            // border and wrapped, the rows that are output pixels cover the interior and these rows exactly the frame.  They
+            // write the padding value, so every launch rewrites the whole image and nothing has to be cleared beforehand.
+            uint4* e_out = nullptr;
+            if (img_out && p.next_format >= 2 && (valid || (row_ok && p.next_format == 3))) {
+                uint32_t px = (uint32_t)(n_img * OHW + opix);
+                if (p.next_format == 3) {
+                    int y2 = yy + p.o_PH, x2 = xx + p.o_PW;
+                    if (y2 >= p.o_Hp) y2 -= p.o_Hp;
+                    if (x2 >= p.o_Wp) x2 -= p.o_Wp;
+                    px = (uint32_t)(n_img * p.HpWp + y2 * p.o_Wp + x2);  // o_Hp * o_Wp = HpWp (checked by the launcher)
+                }
+                e_out = reinterpret_cast<uint4*>(p.pimg) + (size_t)px * (uint32_t)(p.cp_next * 2);
+            }
+            const float tq = (img_out && valid) ? __ldg(p.thr_next + n_img) + 0.0f : 0.f;
+            if (by_thr && valid && !(qt_set && tq == qt_t)) {
+                // the next layer's rule as thresholds on the raw accumulator, once per threshold this thread meets (images often share one)
                 qt = tnns_thr::make(tq, p.alpha, bias_f, next_tern);
-                qt_img = n_img;
+                qe = e2m1_rule(qt);
+                qt_t = tq;
+                qt_set = true;
             }
             // rows16: the four rows of the quadrant this thread stores (8*h + lane/4), each mapped to its output pixel
             float* yrow0[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -593,7 +696,15 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
                     }
                 }
                 const int c0 = n0 + cb;
-                if (valid) {
+                if (by_thr && p.next_format >= 2 && c0 + 32 <= p.KN) {
+                    if (e_out) {
+                        uint32_t w4[4];
+                        if (next_tern) quantise32_e2m1<true>(v, qe, w4);
+                        else quantise32_e2m1<false>(v, qe, w4);
+                        const uint32_t padw = next_tern ? 0u : 0x22222222u;
+                        e_out[c0 >> 5] = valid ? make_uint4(w4[0], w4[1], w4[2], w4[3]) : make_uint4(padw, padw, padw, padw);
+                    }
+                } else if (valid) {
                     float f[32];
                     uint32_t sg = 0, nz = 0;
                     if (by_thr) {
@@ -632,7 +743,7 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
                         }
                     }
                     const bool full = c0 + 32 <= p.KN;
-                    if (p.pimg) {
+                    if (img_out) {
                         if (c0 < p.cp_next * 64) {
                             const bool tern = next_tern;
                             if (!by_thr) {
@@ -645,14 +756,7 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
                                 // the 32 channels as 16 bytes of e2m1 operands; channels past KN: ternary 0, binary +1
                                 uint32_t w4[4];
                                 tnns_expand32_f4(sg & vmask, tern ? ~(nz & vmask) : 0u, w4);
-                                size_t px;
-                                if (p.next_format == 3) {
-                                    int y2 = yy + p.o_PH, x2 = xx + p.o_PW;
-                                    px = (size_t)n_img * ((size_t)p.o_Hp * p.o_Wp) + (size_t)y2 * p.o_Wp + x2;
-                                } else {
-                                    px = (size_t)n_img * OHW + opix;
-                                }
-                                *(reinterpret_cast<uint4*>(p.pimg) + px * ((size_t)p.cp_next * 2) + (c0 >> 5)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+                                e_out[c0 >> 5] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
                             } else {
                                 const int planes = tern ? 2 : 1;
                                 const size_t lanes = (size_t)p.cp_next * 2;
@@ -682,18 +786,9 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
                                 if (c0 + j < p.KN) __stcs(yc, f[j]);
                         }
                     }
-                } else if (row_ok && p.pimg && p.next_format == 3 && c0 < p.cp_next * 64) {
-                    // A virtual row that is no output pixel (yy >= OH or xx >= OW) stands for one border
-                    // pixel of the next layer's image, whose padded lattice is this layer's: shifted by the
-                    // border and wrapped, the rows that are output pixels cover the interior and these
-                    // rows exactly the frame.  They write the padding value, so every launch rewrites the
-                    // whole image and nothing has to be cleared beforehand.
-                    int y2 = yy + p.o_PH, x2 = xx + p.o_PW;
-                    if (y2 >= p.o_Hp) y2 -= p.o_Hp;
-                    if (x2 >= p.o_Wp) x2 -= p.o_Wp;
+                } else if (e_out && c0 < p.cp_next * 64) {
                     const uint32_t padw = p.next_binary ? 0x22222222u : 0u;
-                    const size_t px = (size_t)n_img * ((size_t)p.o_Hp * p.o_Wp) + (size_t)y2 * p.o_Wp + x2;
-                    *(reinterpret_cast<uint4*>(p.pimg) + px * ((size_t)p.cp_next * 2) + (c0 >> 5)) = make_uint4(padw, padw, padw, padw);
+                    e_out[c0 >> 5] = make_uint4(padw, padw, padw, padw);
                 }
             }
         }
@@ -727,11 +822,11 @@ done:
     }
 }
 
-template <int BN, int CG, int TAPS, bool QF, bool SINGLE = false, int GRP = 1>
+template <int BN, int CG, int TAPS, bool QF, bool SINGLE = false, int GRP = 1, bool IMG = false>
 int launch_slab(tnns_cuda_ctx* ctx, const SlabArgs& a, size_t smem, cudaStream_t stream, const CUtensorMap* tmap_a, const CUtensorMap* tmap_b,
                 const CUtensorMap* tmap_q) {
-    using Cfg = SlabCfg<BN, CG, TAPS, QF>;
-    auto kern = gemm_slab_kernel<BN, CG, TAPS, QF, SINGLE, GRP>;
+    using Cfg = SlabCfg<BN, CG, TAPS, QF, IMG>;
+    auto kern = gemm_slab_kernel<BN, CG, TAPS, QF, SINGLE, GRP, IMG>;
     const auto maps = tensor_maps<maps_of(CG, QF)>(tmap_a, tmap_b, tmap_q);
     static bool smem_set[64] = {false};  // once per kernel and device
     if (!smem_set[ctx->device & 63]) {
@@ -806,15 +901,16 @@ bool make_plan(const tnns_cuda_weights* w, const TnnsGeom& g, SlabPlan* pl) {
 }
 
 // ring depths for a configuration; false when not even two slabs and three weight stages fit
-bool ring_depths(const SlabPlan& pl, int b_stage, int fixed, int nchunks, bool one_kernel_tile, int* nslab, int* nstg, int* resident) {
+bool ring_depths(const SlabPlan& pl, int b_stage, int fixed, int nchunks, bool one_kernel_tile, bool loaders, int* nslab, int* nstg, int* resident) {
     const int avail = 232448 - fixed;
-    int ns = pl.slab_bytes <= 16384 ? 4 : (pl.slab_bytes <= 32768 ? 3 : 2);
+    int ns = pl.slab_bytes <= 16384 ? (loaders ? SL_MAXSLAB : 4) : (pl.slab_bytes <= 32768 ? 3 : 2);
     for (; ns >= 2; ns--) {
         const int rest = avail - ns * pl.slab_bytes;
         if (rest < 3 * b_stage) continue;
         int nb = std::min(SL_MAXSTG, rest / b_stage);
         *resident = (one_kernel_tile && nchunks <= nb) ? 1 : 0;
         if (*resident) nb = nchunks;
+        if (loaders) ns &= ~1;  // two MMA issuers take them in turn
         *nslab = ns;
         *nstg = nb;
         return true;
@@ -828,11 +924,12 @@ namespace {
 struct SlabChoice {
     SlabPlan pl;
     bool pairs;
+    bool loaders;
     int b_stage, fixed, nslab, nstg, resident, grp, Mv, ntn;
     size_t smem;
 };
 // The form a launch takes: single blocks or block pairs (pairs_req 0 = by size, 1, 2), ring depths.
-bool choose_form(int sm_count, const tnns_cuda_weights* w, const TnnsGeom& g, int pairs_req, bool fused, SlabChoice* ch) {
+bool choose_form(int sm_count, const tnns_cuda_weights* w, const TnnsGeom& g, int pairs_req, bool fused, bool image_out, SlabChoice* ch) {
     if (!make_plan(w, g, &ch->pl)) return false;
     const SlabPlan& pl = ch->pl;
     ch->Mv = g.N * pl.Hp * pl.Wp;
@@ -840,9 +937,12 @@ bool choose_form(int sm_count, const tnns_cuda_weights* w, const TnnsGeom& g, in
     const long long pair_tiles = (long long)((ch->Mv + 2 * BM - 1) / (2 * BM)) * ch->ntn;
     if (pairs_req == 2 && pl.bn != 256) return false;
     ch->pairs = pl.bn == 256 && (pairs_req == 2 || (pairs_req == 0 && pair_tiles >= sm_count / 2));
+    // Slab loaders (SlabCfg::LOADER) where 32- or 64-byte pixels become an image.  fp32 outputs keep the tensor copies: the loaders'
+    // pieces would queue behind the output's stores in the same unit (256 x 64x56x56 -> 64 fp32 out, copies / loaders: 52 / 60 us).
+    ch->loaders = image_out && pl.taps > 1 && !ch->pairs && !fused;
     ch->b_stage = (pl.bn / (ch->pairs ? 2 : 1)) * KCH;
     ch->fixed = 1024 + SL_BAR_BYTES + (fused ? Q_STG * Q_PIX * 64 * 4 + 128 : 0);
-    if (!ring_depths(pl, ch->b_stage, ch->fixed, w->Kp / 4, ch->ntn == 1, &ch->nslab, &ch->nstg, &ch->resident)) return false;
+    if (!ring_depths(pl, ch->b_stage, ch->fixed, w->Kp / 4, ch->ntn == 1, ch->loaders, &ch->nslab, &ch->nstg, &ch->resident)) return false;
     if (!ch->pairs && !fused) {
         // few tiles: narrower ones (what fits with the widest tile fits with these)
         const int bn = tile_n_for(sm_count, ch->Mv, w->KN, pl.bn);
@@ -850,7 +950,7 @@ bool choose_form(int sm_count, const tnns_cuda_weights* w, const TnnsGeom& g, in
             ch->pl.bn = bn;
             ch->ntn = (w->KN + bn - 1) / bn;
             ch->b_stage = bn * KCH;
-            if (!ring_depths(pl, ch->b_stage, ch->fixed, w->Kp / 4, ch->ntn == 1, &ch->nslab, &ch->nstg, &ch->resident)) return false;
+            if (!ring_depths(pl, ch->b_stage, ch->fixed, w->Kp / 4, ch->ntn == 1, ch->loaders, &ch->nslab, &ch->nstg, &ch->resident)) return false;
         }
     }
     // three weight stages a slot (see the kernel's GRP) where two slots fit
@@ -863,7 +963,7 @@ bool choose_form(int sm_count, const tnns_cuda_weights* w, const TnnsGeom& g, in
 
 bool tnns_slab_supported(const tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const TnnsGeom& g, bool fused) {
     SlabChoice ch;
-    return choose_form(ctx->sm_count, w, g, 0, fused, &ch);
+    return choose_form(ctx->sm_count, w, g, 0, fused, false, &ch);
 }
 
 size_t tnns_bordered_image_bytes(int N, int C, int H, int W, int PH, int PW) {
@@ -876,7 +976,7 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
                           int next_PW, const TnnsFusedInput* fused) {
     if (g.N == 0) return TNNS_OK;
     SlabChoice ch;
-    if (!choose_form(ctx->sm_count, w, g, pairs, fused != nullptr, &ch))
+    if (!choose_form(ctx->sm_count, w, g, pairs, fused != nullptr, d_pimg != nullptr, &ch))
         return tnns_fail(TNNS_ERR_UNSUPPORTED, "layer outside the slab-fed GEMM (stride 1; 64, 128 or 256*k channels; slab and weight ring within shared memory)");
     const SlabPlan& pl = ch.pl;
     if (reinterpret_cast<uintptr_t>(d_image) & 127) return tnns_fail(TNNS_ERR_INVALID, "bordered image must be 128-byte aligned");
@@ -897,6 +997,8 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
     a.y_vec = tnns_row_vec(d_y, w->KN);
     a.OH = g.OH; a.OW = g.OW; a.Wp = pl.Wp; a.HpWp = pl.Hp * pl.Wp;
     a.KW = g.KW; a.T = pl.T; a.G = pl.G;
+    a.Aimg = reinterpret_cast<const unsigned char*>(d_image);
+    a.slab_rows = pl.slab_rows;
     a.slab_bytes = pl.slab_bytes; a.copy_rows = pl.copy_rows; a.ncopies = pl.ncopies;
     a.layout = (g.OH * g.OW == 1) ? TNNS_NHWC : layout;  // one pixel per image: both layouts are the same memory, the pixel-major epilogue stores 16 bytes per lane
     a.zero_passes = w->type != TNN;
@@ -918,7 +1020,7 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
     a.div_wp = tnns_fastdiv((uint32_t)pl.Wp);
     // the bordered image as rows of pixels: (bytes of a pixel) x (all padded pixels of the batch)
     alignas(64) CUtensorMap map_a, map_b, map_q;
-    int rc = tnns_tensor_map_2d(&map_a, 1, d_image, (unsigned long long)g.Cp * 32, (unsigned long long)Mv, (unsigned long long)g.Cp * 32, pl.rb,
+    int rc = ch.loaders ? TNNS_OK : tnns_tensor_map_2d(&map_a, 1, d_image, (unsigned long long)g.Cp * 32, (unsigned long long)Mv, (unsigned long long)g.Cp * 32, pl.rb,
                                 pl.copy_rows, pl.rb);
     if (rc) return rc;
     if (use_pairs && (rc = tnns_tensor_map_2d(&map_b, 1, w->d_f4, KCH, w->f4_bytes / KCH, KCH, KCH, pl.bn / 2))) return rc;
@@ -947,6 +1049,18 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
                 case 64: return launch_slab<64, 1, T, true>(ctx, a, smem, stream, &map_a, nullptr, &map_q);
                 case 128: return launch_slab<128, 1, T, true>(ctx, a, smem, stream, &map_a, nullptr, &map_q);
                 default: return launch_slab<256, 1, T, true>(ctx, a, smem, stream, &map_a, nullptr, &map_q);
+            }
+        }
+        const CUtensorMap* ma = ch.loaders ? nullptr : &map_a;
+        if (d_pimg) {
+            if (use_pairs) return launch_slab<256, 2, T, false, false, 1, true>(ctx, a, smem, stream, ma, &map_b, nullptr);
+            if constexpr (T == 1)
+                if (ch.grp == 3) return pl.bn == 64 ? launch_slab<64, 1, T, false, false, 3, true>(ctx, a, smem, stream, ma, nullptr, nullptr)
+                                                    : launch_slab<128, 1, T, false, false, 3, true>(ctx, a, smem, stream, ma, nullptr, nullptr);
+            switch (pl.bn) {
+                case 64: return launch_slab<64, 1, T, false, false, 1, true>(ctx, a, smem, stream, ma, nullptr, nullptr);
+                case 128: return launch_slab<128, 1, T, false, false, 1, true>(ctx, a, smem, stream, ma, nullptr, nullptr);
+                default: return launch_slab<256, 1, T, false, false, 1, true>(ctx, a, smem, stream, ma, nullptr, nullptr);
             }
         }
         if (use_pairs) return launch_slab<256, 2, T, false>(ctx, a, smem, stream, &map_a, &map_b, nullptr);

@@ -284,7 +284,9 @@ __device__ __noinline__ void fill_output_border(uint4* img, int cp_next, int H, 
 // TAPS (tensor-copy form): filter taps per 128-byte stage row -- 1: a tap's 256 channels fill the
 // row (C_pack % 4 == 0); 2: C_pack = 2, two taps of 128 channels in two 64-byte-swizzled sub-tiles;
 // 4: C_pack = 1, four taps of 64 channels in four 32-byte-swizzled sub-tiles.
-template <int BN, int MT, bool F4, bool ATMA, int CG, int TAPS, bool QF, bool SINGLE>
+// IMG: quantised output for a following layer (tensor-copy form without quantiser warps: in kernels of its own, since either epilogue's
+// registers and code cost the other; the other forms decide at run time).
+template <int BN, int MT, bool F4, bool ATMA, int CG, int TAPS, bool QF, bool SINGLE, bool IMG>
 __global__ void __launch_bounds__(TcCfg<BN, MT, F4, ATMA, CG, TAPS, QF>::NTHREADS, 1)
 gemm_tc_kernel(GemmArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> maps) {
     const CUtensorMap &tmap_a = maps.m[0], &tmap_b = maps.m[CG == 2 ? 1 : 0], &tmap_q = maps.m[QF ? 2 : 0];
@@ -719,16 +721,19 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> m
         const uint32_t bar_release = (CG == 2 && rank != 0) ? mapa_shared(bar_tempty, 0) : 0u;  // pair: the first block's barrier
         // quantised output with 0 < alpha <= 1: PReLU and the next layer's rule collapse into thresholds on
         // the accumulator (two instructions per output and plane instead of evaluating the PReLU first)
-        const bool by_thr = F4 && p.pimg != nullptr && alpha_in_unit;
+        const bool img_out = IMG || ((QF || !ATMA) && p.pimg != nullptr);
+        const bool by_thr = F4 && img_out && alpha_in_unit;
         // (not in the one-launch form, whose producers write plain images only: the code is compiled out there, where
         // its mere presence measured one percent of the large layer)
-        if (F4 && !QF && p.pimg && p.pimg_e2m1 && p.o_HpWp)
+        if (F4 && !QF && img_out && p.pimg_e2m1 && p.o_HpWp)
             fill_output_border(reinterpret_cast<uint4*>(p.pimg), p.cp_next, p.OHW / p.OW, p.OW, (int)(p.M / p.OHW), p.o_PH, p.o_PW,
                                ((long long)(warp - WARP_EPI0) * gridDim.x + blockIdx.x) * 32 + lane, (long long)gridDim.x * (blockDim.x - 32 * WARP_EPI0));
         // pixel-major fp32 output in the 16x256b shape: float pairs (y_vec), or, in kernels of their own, single floats (SINGLE)
-        const bool rows16 = F4 && p.pimg == nullptr && p.layout == TNNS_NHWC && (SINGLE || p.y_vec > 1);
+        const bool rows16 = F4 && !img_out && p.layout == TNNS_NHWC && (SINGLE || p.y_vec > 1);
         tnns_thr::Pair qt = {0.f, 0.f};
-        long long qt_img = -1;
+        E2m1Rule qe = {0.f, 0.f};
+        float qt_t = 0.f;
+        bool qt_set = false;
         for (int t = unit + set * nunits; t < ntiles; t += NSETS * nunits, lt += NSETS) {
             const int buf = lt % NBUF;
             const int m_tile = (int)p.div_ntn.div((uint32_t)t);
@@ -740,11 +745,23 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> m
             const long long n_img = !row_ok ? 0 : row < 0x7FFFFFFFLL ? (long long)p.div_ohw.div((uint32_t)row) : row / p.OHW;
             const int rem = (int)(row - n_img * p.OHW);
             float* ybase = (p.layout == TNNS_NHWC) ? p.y + (size_t)row * p.KN : p.y + (size_t)n_img * p.KN * p.OHW + rem;
-            const float tq = (p.pimg && row_ok) ? __ldg(p.thr_next + n_img) + 0.0f : 0.f;  // + 0.0f: -0 acts as +0
-            if (by_thr && row_ok && n_img != qt_img) {
-                // the next layer's rule as thresholds on the raw accumulator, once per image this thread meets
+            // 4-bit image out: where the row's pixel goes in the next layer's image, plain or inside its border
+            uint4* e_out = nullptr;
+            if (F4 && img_out && p.pimg_e2m1 && row_ok) {
+                long long opix = n_img * p.OHW + rem;
+                if (!QF && p.o_HpWp) {
+                    const int oh = (int)p.div_ow.div((uint32_t)rem);
+                    opix = n_img * p.o_HpWp + (long long)(oh + p.o_PH) * p.o_Wp + (rem - oh * p.OW) + p.o_PW;
+                }
+                e_out = reinterpret_cast<uint4*>(p.pimg) + (size_t)opix * ((size_t)p.cp_next * 2);
+            }
+            const float tq = (img_out && row_ok) ? __ldg(p.thr_next + n_img) + 0.0f : 0.f;  // + 0.0f: -0 acts as +0
+            if (by_thr && row_ok && !(qt_set && tq == qt_t)) {
+                // the next layer's rule as thresholds on the raw accumulator, once per threshold this thread meets (images often share one)
                 qt = tnns_thr::make(tq, p.alpha, bias_f, p.next_ternary != 0);
-                qt_img = n_img;
+                qe = e2m1_rule(qt);
+                qt_t = tq;
+                qt_set = true;
             }
             if (!mbar_wait(bar_tfull + 8 * buf, (lt / NBUF) & 1, abort_flag, p.status, 5)) goto done;
             tc_fence_after();
@@ -810,7 +827,14 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> m
                         else mbar_arrive(OVL ? bar_tempty : bar_tempty + 8 * buf);
                     }
                 }
-                if (row_ok) {
+                if (F4 && by_thr && p.pimg_e2m1 && n0 + cb + 32 <= p.KN) {
+                    // (the 4-bit image is written for ternary layers only)
+                    if (row_ok) {
+                        uint32_t w4[4];
+                        quantise32_e2m1<true>(v, qe, w4);
+                        e_out[(n0 + cb) >> 5] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+                    }
+                } else if (row_ok) {
                     float f[32];
                     uint32_t sg = 0, nz = 0;
                     if (by_thr) {
@@ -839,7 +863,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> m
                     }
                     const int c0 = n0 + cb;
                     const bool full = c0 + 32 <= p.KN;
-                    if (p.pimg) {
+                    if (img_out) {
                         // Quantise the 32 channels this thread holds for its pixel straight into one
                         // 32-bit lane of the next layer's bit planes (same rules as the pack kernel:
                         // sign = f < -t, non-zero = |f| > t; binary: f < t), channels past KN absent.
@@ -855,15 +879,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> m
                                 // of the next layer expects them (same expansion routine as everywhere)
                                 uint32_t w4[4];
                                 tnns_expand32_f4(sg & valid, ~(nz & valid), w4);
-                                // the row's pixel in the next layer's image: plain, or inside its border (worked out here, in the
-                                // branch that stores it: as a value kept across the slices it cost the fp32 path 3 % on the large layer)
-                                long long opix = n_img * p.OHW + rem;
-                                if (!QF && p.o_HpWp) {
-                                    const int oh = (int)p.div_ow.div((uint32_t)rem);
-                                    opix = n_img * p.o_HpWp + (long long)(oh + p.o_PH) * p.o_Wp + (rem - oh * p.OW) + p.o_PW;
-                                }
-                                uint4* px = reinterpret_cast<uint4*>(p.pimg) + (size_t)opix * ((size_t)p.cp_next * 2) + (c0 >> 5);
-                                *px = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+                                e_out[c0 >> 5] = make_uint4(w4[0], w4[1], w4[2], w4[3]);
                             } else {
                                 const int planes = p.next_ternary ? 2 : 1;
                                 const size_t lanes = (size_t)p.cp_next * 2;  // 32-bit lanes per pixel and plane
@@ -1018,11 +1034,11 @@ __global__ void __launch_bounds__(128, 1) mma_rate_kernel(int iters, unsigned in
     }
 }
 
-template <int BN, int MT, bool F4, bool ATMA = false, int CG = 1, int TAPS = 1, bool QF = false, bool SINGLE = false>
+template <int BN, int MT, bool F4, bool ATMA = false, int CG = 1, int TAPS = 1, bool QF = false, bool SINGLE = false, bool IMG = false>
 int launch_cfg(tnns_cuda_ctx* ctx, GemmArgs a, cudaStream_t stream, const CUtensorMap* tmap_a = nullptr,
                const CUtensorMap* tmap_b = nullptr, const CUtensorMap* tmap_q = nullptr) {
     using Cfg = TcCfg<BN, MT, F4, ATMA, CG, TAPS, QF>;
-    auto kern = gemm_tc_kernel<BN, MT, F4, ATMA, CG, TAPS, QF, SINGLE>;
+    auto kern = gemm_tc_kernel<BN, MT, F4, ATMA, CG, TAPS, QF, SINGLE, IMG>;
     const auto maps = tensor_maps<maps_of(CG, QF)>(tmap_a, tmap_b, tmap_q);
     // once per kernel and device: the attribute belongs to (function, device), and the call costs a microsecond per launch
     static bool smem_set[64] = {false};
@@ -1430,6 +1446,14 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
                 case 64: return launch_cfg<64, 1, true, true, 1, T, true>(ctx, a, stream, &map, nullptr, &map_q);
                 case 128: return launch_cfg<128, 1, true, true, 1, T, true>(ctx, a, stream, &map, nullptr, &map_q);
                 default: return launch_cfg<256, 1, true, true, 1, T, true>(ctx, a, stream, &map, nullptr, &map_q);
+            }
+        }
+        if (d_pimg) {
+            if (use_pairs) return launch_cfg<256, 1, true, true, 2, T, false, false, true>(ctx, a, stream, &map, &map_b);
+            switch (bn) {
+                case 64: return launch_cfg<64, 1, true, true, 1, T, false, false, true>(ctx, a, stream, &map);
+                case 128: return launch_cfg<128, 1, true, true, 1, T, false, false, true>(ctx, a, stream, &map);
+                default: return launch_cfg<256, 1, true, true, 1, T, false, false, true>(ctx, a, stream, &map);
             }
         }
         if (use_pairs) return launch_cfg<256, 1, true, true, 2, T>(ctx, a, stream, &map, &map_b);

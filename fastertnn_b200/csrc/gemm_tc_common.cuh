@@ -221,6 +221,48 @@ __device__ __forceinline__ uint32_t quantise32_binary(const float (&f)[32], floa
     return sg;
 }
 
+// 32 accumulators of one pixel -> the 16 bytes of e2m1 operands tnns_expand32_f4 would make of its plane words, by thresholds on
+// the accumulator v (prelu_thresholds.cuh; an integer, so that a saturating multiply-add between two integers is a step):
+//     n = sat(-2v + cn)   1 where v < L        p = sat(2v + cp)   1 where v > U and not v < L
+// nibble = 0xA where n, 0x2 where p (binary: where not n), else 0: u = 5n + p (4n + 1) doubled, collected four nibbles to a float by
+// multiply-adds, 128*16^4 = 2^23 in front so that the float's low mantissa bits are those 16 bits.  Four full-rate
+// instructions per value; through the PReLU and two planes of sign bits it was nine issue slots (the maximum and the
+// funnel shifts run at half rate) and the expansion (GEMM with an image out: 64 x 256x14x14 -> 256 7.2 / 6.4 us).
+struct E2m1Rule {
+    float cn, cp;
+};
+__device__ __forceinline__ E2m1Rule e2m1_rule(const tnns_thr::Pair& t) {
+    E2m1Rule r;
+    r.cn = fmaf(-2.0f, t.n1, -1.0f);                       // L = -n1
+    r.cp = fmaf(-2.0f, fmaxf(t.t2, -t.n1 - 1.0f), -1.0f);  // a negative threshold lets v be both below L and above U: -1 then
+    return r;
+}
+__device__ __forceinline__ float fma_sat(float a, float b, float c) {
+    float r;
+    asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+template <bool TERNARY>
+__device__ __forceinline__ void quantise32_e2m1(const uint32_t (&v)[32], const E2m1Rule& t, uint32_t (&w)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        uint32_t half[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            float acc = 128.0f;
+#pragma unroll
+            for (int k = 4 * h + 3; k >= 4 * h; k--) {  // nibble k of word i is channel 4k + 3 - i
+                const float a = __uint_as_float(v[4 * k + 3 - i]);
+                const float n = fma_sat(a, -2.0f, t.cn);
+                const float u = TERNARY ? fmaf(n, 5.0f, fma_sat(a, 2.0f, t.cp)) : fmaf(n, 4.0f, 1.0f);
+                acc = fmaf(acc, 16.0f, u);
+            }
+            half[h] = __float_as_uint(acc);
+        }
+        w[i] = __byte_perm(half[0], half[1], 0x5410) << 1;
+    }
+}
+
 // PReLU of 32 fp32 accumulators (4-bit form), as the reference evaluates it on an integer sum
 // (src/tnns/mm_p2_final_tnn_avx2.c:90-93; zero_passes: the tbn / btn / bnn forms pass a zero sum through).
 // The run-time choices sit outside the unrolled loops: inside, every element pays for both sides of each.
