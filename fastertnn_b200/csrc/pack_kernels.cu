@@ -16,10 +16,10 @@
 
 namespace {
 
-constexpr int kPackThreads = 256;
-#ifndef TNNS_PACK_MINCTA
-#define TNNS_PACK_MINCTA 4
-#endif
+// Threads per block of the staged kernel: 256, and 512 where the grid leaves every SM at most two blocks.  A thread loads its 32
+// channels in four batches of eight, each a round trip to memory, so what a small layer takes is the number of batches in
+// series: 8 x 512x32x32 3x3 (256 blocks of three input rows), pack and GEMM 36.9 / 34.4 us, words of 64 channels per thread of 256 / so.
+constexpr int kPackThreads = 256, kPackThreadsMax = 512;
 
 // ---------------------------------------------------------------------------------------
 // Reference-shaped kernel: one thread per plane word, channels fetched straight from
@@ -132,7 +132,7 @@ __device__ __forceinline__ void quantise_batch(const float* __restrict__ q, size
 }
 
 template <bool TERNARY, int LAYOUT, int VEC, bool PAIR>
-__global__ void __launch_bounds__(kPackThreads, TNNS_PACK_MINCTA)
+__global__ void __launch_bounds__(kPackThreadsMax, 2)
 pack_staged_kernel(const float* __restrict__ x, const float* __restrict__ thr, uint4* __restrict__ out, TnnsGeom g,
                    int BOH, int nbands, int Lmax, FastDiv divU, FastDiv divOW, FastDiv divL) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -142,7 +142,9 @@ pack_staged_kernel(const float* __restrict__ x, const float* __restrict__ thr, u
     int* joff = reinterpret_cast<int*>(sm_sign + (size_t)PLANES * Lmax * g.Cp);
     uint32_t* jtap = reinterpret_cast<uint32_t*>(joff + g.Kp);
 
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, nthreads = blockDim.x;
+    // launched as a programmatic dependent, and its own dependents' blocks may take SMs as its blocks leave
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int n = blockIdx.x / nbands;
     const int band = blockIdx.x - n * nbands;
     const int oh0 = band * BOH;
@@ -151,9 +153,8 @@ pack_staged_kernel(const float* __restrict__ x, const float* __restrict__ thr, u
     const int ih_hi = min((oh0 + boh - 1) * g.SH - g.PH + g.KH, g.H);  // exclusive
     const int nrow = max(ih_hi - ih_lo, 0);                              // input rows held in smem
     const int L = nrow * g.W;                                            // pixels held in smem
-    const float t = (LAYOUT == 2) ? 0.f : thr[n] + 0.0f, nt = -t;  // + 0.0f: a threshold of -0 behaves as +0 in every compare
 
-    for (int j = tid; j < g.Kp; j += kPackThreads) {
+    for (int j = tid; j < g.Kp; j += nthreads) {
         int off = kPadWord;
         uint32_t tap = 0;
         if (j < g.Kw) {
@@ -164,6 +165,9 @@ pack_staged_kernel(const float* __restrict__ x, const float* __restrict__ thr, u
         joff[j] = off;
         jtap[j] = tap;
     }
+    // the input may be the output of the launch before, the matrix an operand of it
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const float t = (LAYOUT == 2) ? 0.f : thr[n] + 0.0f, nt = -t;  // + 0.0f: a threshold of -0 behaves as +0 in every compare
 
     // ---------------- phase 1: quantise + pack the band's input pixels ----------------
     if (LAYOUT == 2) {
@@ -171,62 +175,60 @@ pack_staged_kernel(const float* __restrict__ x, const float* __restrict__ thr, u
         const size_t HWC = (size_t)g.H * g.W * g.Cp;
         const uint64_t* src_s = planes + (size_t)n * PLANES * HWC + (size_t)ih_lo * g.W * g.Cp;
         const int words = L * g.Cp;
-        for (int i = tid; i < words; i += kPackThreads) {
+        for (int i = tid; i < words; i += nthreads) {
             sm_sign[i] = __ldg(src_s + i);
             if (TERNARY) sm_zero[i] = __ldg(src_s + HWC + i);
         }
     } else if (LAYOUT == 0) {
         const size_t HW = (size_t)g.H * g.W;
         const int LV = L / VEC;  // VEC divides L by construction (host checks W % VEC == 0)
-        const int items = g.Cp * LV;
-        for (int id = tid; id < items; id += kPackThreads) {
-            const int ic = (LV == (int)divL.d) ? (int)divL.div((uint32_t)id) : id / LV;
-            const int p = (id - ic * LV) * VEC;
-            const int nch = min(TNNS_WORD_BITS, g.C - ic * TNNS_WORD_BITS);
-            const float* src = x + ((size_t)n * g.C + (size_t)ic * TNNS_WORD_BITS) * HW + (size_t)ih_lo * g.W + p;
-            uint32_t sg[2][VEC], nzb[2][VEC];
+        uint32_t* sm_sign32 = reinterpret_cast<uint32_t*>(sm_sign);
+        uint32_t* sm_zero32 = reinterpret_cast<uint32_t*>(sm_zero);
+        const int items = 2 * g.Cp * LV;  // VEC pixels x 32 channels
+        for (int id = tid; id < items; id += nthreads) {
+            const int h = (LV == (int)divL.d) ? (int)divL.div((uint32_t)id) : id / LV;  // half-word: channels 32*h ..
+            const int p = (id - h * LV) * VEC;
+            const int lim = g.C - 32 * h;  // channels present from there on; may be <= 0
+            const float* src = x + ((size_t)n * g.C + (size_t)32 * h) * HW + (size_t)ih_lo * g.W + p;
+            uint32_t sg[VEC], nzb[VEC];
 #pragma unroll
-            for (int v = 0; v < VEC; v++) { sg[0][v] = sg[1][v] = 0; nzb[0][v] = nzb[1][v] = 0; }
-#pragma unroll
-            for (int half = 0; half < 2; half++) {
-                if (nch >= 32 * half + 32) {
+            for (int v = 0; v < VEC; v++) sg[v] = nzb[v] = 0;
+            if (lim >= 32) {
 #pragma unroll 1
-                    for (int b0 = 24; b0 >= 0; b0 -= 8)  // one batch of eight loads in flight per thread
-                        quantise_batch<TERNARY, VEC>(src + (size_t)(32 * half + b0) * HW, HW, t, sg[half], nzb[half]);
-                } else {
-                    const int lim = nch - 32 * half;  // channels present in this half-word; may be <= 0
-                    for (int b = 31; b >= 0; b--) {
-                        const float* q = src + (size_t)(32 * half + b) * HW;
+                for (int b0 = 24; b0 >= 0; b0 -= 8)  // one batch of eight loads in flight per thread
+                    quantise_batch<TERNARY, VEC>(src + (size_t)b0 * HW, HW, t, sg, nzb);
+            } else {
+                for (int b = 31; b >= 0; b--) {
+                    const float* q = src + (size_t)b * HW;
 #pragma unroll
-                        for (int v = 0; v < VEC; v++) {
-                            if (b < lim) {
-                                const float val = __ldg(q + v);
-                                if (TERNARY) {
-                                    sg[half][v] = push_sign(sg[half][v], val + t);
-                                    nzb[half][v] = push_sign(nzb[half][v], t - fabsf(val));
-                                } else {
-                                    sg[half][v] = push_sign(sg[half][v], (val + 0.0f) - t);
-                                }
-                            } else {  // absent channel: sign 0, non-zero 0
-                                sg[half][v] <<= 1;
-                                if (TERNARY) nzb[half][v] <<= 1;
+                    for (int v = 0; v < VEC; v++) {
+                        if (b < lim) {
+                            const float val = __ldg(q + v);
+                            if (TERNARY) {
+                                sg[v] = push_sign(sg[v], val + t);
+                                nzb[v] = push_sign(nzb[v], t - fabsf(val));
+                            } else {
+                                sg[v] = push_sign(sg[v], (val + 0.0f) - t);
                             }
+                        } else {  // absent channel: sign 0, non-zero 0
+                            sg[v] <<= 1;
+                            if (TERNARY) nzb[v] <<= 1;
                         }
                     }
                 }
             }
 #pragma unroll
             for (int v = 0; v < VEC; v++) {
-                const int at = (p + v) * g.Cp + ic;
-                sm_sign[at] = ((uint64_t)sg[1][v] << 32) | sg[0][v];
-                if (TERNARY) sm_zero[at] = ~(((uint64_t)nzb[1][v] << 32) | nzb[0][v]);
+                const int at = (p + v) * g.Cp * 2 + h;
+                sm_sign32[at] = sg[v];
+                if (TERNARY) sm_zero32[at] = ~nzb[v];
             }
         }
     } else {
         // NHWC: the band's pixels are one contiguous run of L*C floats.
         const float* base = x + ((size_t)n * g.H + ih_lo) * g.W * g.C;
         const int lane = tid & 31, warp = tid >> 5;
-        constexpr int NWARP = kPackThreads / 32;
+        const int NWARP = nthreads / 32;
         uint32_t* sm_sign32 = reinterpret_cast<uint32_t*>(sm_sign);
         uint32_t* sm_zero32 = reinterpret_cast<uint32_t*>(sm_zero);
         if ((g.C & 63) == 0) {
@@ -279,7 +281,7 @@ pack_staged_kernel(const float* __restrict__ x, const float* __restrict__ thr, u
     const uint32_t U = TERNARY ? (uint32_t)g.Kp : (uint32_t)g.Kp / 2;   // 16-byte chunks per row
     const uint32_t units = (uint32_t)(boh * g.OW) * UP;
     uint4* dst = out + ((size_t)n * g.OH + oh0) * g.OW * U;
-    for (uint32_t q = tid; q < units; q += kPackThreads) {
+    for (uint32_t q = tid; q < units; q += nthreads) {
         const uint32_t row = divU.div(q);
         const uint32_t k = q - row * UP;
         const uint32_t ohl = divOW.div(row);
@@ -332,8 +334,18 @@ int launch_staged(tnns_cuda_ctx* ctx, const float* d_x, const float* d_thr, void
         // sizes cannot lower each other's limit between this call and the launch
         if (smem > 48 * 1024)
             TNNS_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(smem, ctx->smem_optin)));
-        kern<<<g.N * nbands, kPackThreads, smem, stream>>>(d_x, d_thr, reinterpret_cast<uint4*>(d_packed), g, BOH, nbands, Lmax,
-                                                           tnns_fastdiv(UP), tnns_fastdiv(g.OW), tnns_fastdiv(LV));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(g.N * nbands));
+        cfg.blockDim = dim3(g.N * (long long)nbands <= 2LL * ctx->sm_count ? kPackThreadsMax : kPackThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        TNNS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, d_x, d_thr, reinterpret_cast<uint4*>(d_packed), g, BOH, nbands, Lmax, tnns_fastdiv(UP),
+                                         tnns_fastdiv(g.OW), tnns_fastdiv(LV)));
         tnns_count_launch();
         TNNS_CUDA_TRY(cudaGetLastError());
         return TNNS_OK;
