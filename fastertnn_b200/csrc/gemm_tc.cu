@@ -79,8 +79,13 @@ namespace {
 // word in global memory; the producer thread starts a tile's tensor copies once the images its
 // rows belong to are complete.  The quantisation (HBM-bound) then runs underneath the MMAs
 // (tensor-bound) of earlier tiles.
-template <int BN, int MT, bool F4, bool ATMA = false, int CG = 1, int TAPS = 1, bool QF = false>
+// PK (expander-fed 4-bit form over an explicit packed matrix): the packed rows of a stage -- 64 bytes each, 32 of binary rows -- come
+// as one swizzled tensor copy into a ring of their own, requested by one more warp, and the expanders read shared memory.
+// Loaded from global memory by the expanders a warp's 16-byte load touched 32 rows, 32 passes through the load unit, which took
+// longer than the stage's MMAs: 8 x 512x32x32 -> 512 3x3 (M 8192, K 4608), GEMM alone 21 -> 13.0 us (14.4 with three expander groups).
+template <int BN, int MT, bool F4, bool ATMA = false, int CG = 1, int TAPS = 1, bool QF = false, bool PK = false>
 struct TcCfg {
+    static_assert(!PK || (F4 && !ATMA && MT == 1), "packed rows by tensor copy: expander-fed 4-bit form");
     static_assert(!QF || ATMA, "fused quantisation: tensor-copy form only");
     static constexpr int NQ = QF ? 5 : 0;  // four quantiser warps (thread = pixel of a 128-pixel item) and the publisher's warp
     static_assert(TAPS == 1 || (ATMA && (TAPS == 2 || TAPS == 4)), "taps per stage row: tensor-copy form only");
@@ -108,17 +113,22 @@ struct TcCfg {
     // not (or only partly) hidden behind the next tile's MMAs
     static constexpr int EPW = ATMA ? (NSETS > 1 ? 1 : 2) : (((NBUF == 1 || OVL) && MT == 1) ? 2 : 1);
     // expander groups (stages expanded concurrently); 22 warps per block in every MT = 1 form
-    static constexpr int NG = ATMA ? 0 : ((MT == 1) ? (EPW == 2 ? 3 : 4) : 2);
+    // (two suffice for 256 kernels where the rows come by tensor copy, and leave the epilogue 96 registers instead of 80)
+    static constexpr int NG = ATMA ? 0 : ((MT == 1) ? (EPW == 2 ? (PK ? 2 : 3) : 4) : 2);
     static constexpr int WARP_EPI0 = WARP_EXP0 + 4 * MT * NG;
     static constexpr int NEPI = 4 * MT * EPW * NSETS;  // epilogue warps
     static constexpr int WARP_Q0 = WARP_EPI0 + NEPI;
-    static constexpr int NTHREADS = 32 * (2 + 4 * MT * NG + NEPI + NQ);
+    static constexpr int WARP_PK = WARP_EPI0 + NEPI;
+    static constexpr int NTHREADS = 32 * (2 + 4 * MT * NG + NEPI + NQ + (PK ? 1 : 0));
+    // Packed-row ring: every slot belongs to one expander group, which then meets it in successive phases.
+    static constexpr int NPK = PK ? 2 * NG : 0, PK_STAGE = BM * 64;
     static constexpr int NBARS = NBUF > 2 ? NBUF : 2;
-    static_assert((2 * NSTG + 2 * NBARS) * 8 + 8 <= 256, "barriers and two words");
-    static constexpr int TAPMAX = ATMA ? 0 : 1024;  // entries of the tap table kept in shared memory (gathering form)
+    static_assert((2 * NSTG + 2 * NBARS + 2 * NPK) * 8 + 8 <= 256, "barriers and two words");
+    static constexpr int TAPMAX = ATMA || PK ? 0 : 1024;  // entries of the tap table kept in shared memory (gathering form)
     static constexpr size_t Q_OFF = (size_t)NSTG * (A_STAGE + B_STAGE) + (QF ? 1024 : 256) + TAPMAX * sizeof(uint32_t);  // quantiser ring, then its barriers
     static_assert(!QF || Q_OFF % 1024 == 0, "the quantiser ring receives 128-byte-swizzled boxes: its stages start on 1024-byte boundaries");
-    static constexpr size_t SMEM = 1024 + Q_OFF + (QF ? QSTG * Q_STAGE + 128 : 0);
+    static constexpr size_t PK_OFF = (size_t)NSTG * (A_STAGE + B_STAGE) + 1024;  // packed-row ring (1024-byte aligned), behind the barriers
+    static constexpr size_t SMEM = 1024 + (PK ? PK_OFF + NPK * PK_STAGE : Q_OFF + (QF ? QSTG * Q_STAGE + 128 : 0));
     static_assert(SMEM <= 232448, "shared memory per block");
 };
 
@@ -286,11 +296,11 @@ __device__ __noinline__ void fill_output_border(uint4* img, int cp_next, int H, 
 // 4: C_pack = 1, four taps of 64 channels in four 32-byte-swizzled sub-tiles.
 // IMG: quantised output for a following layer (tensor-copy form without quantiser warps: in kernels of its own, since either epilogue's
 // registers and code cost the other; the other forms decide at run time).
-template <int BN, int MT, bool F4, bool ATMA, int CG, int TAPS, bool QF, bool SINGLE, bool IMG>
-__global__ void __launch_bounds__(TcCfg<BN, MT, F4, ATMA, CG, TAPS, QF>::NTHREADS, 1)
+template <int BN, int MT, bool F4, bool ATMA, int CG, int TAPS, bool QF, bool SINGLE, bool IMG, bool PK>
+__global__ void __launch_bounds__(TcCfg<BN, MT, F4, ATMA, CG, TAPS, QF, PK>::NTHREADS, 1)
 gemm_tc_kernel(GemmArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> maps) {
     const CUtensorMap &tmap_a = maps.m[0], &tmap_b = maps.m[CG == 2 ? 1 : 0], &tmap_q = maps.m[QF ? 2 : 0];
-    using Cfg = TcCfg<BN, MT, F4, ATMA, CG, TAPS, QF>;
+    using Cfg = TcCfg<BN, MT, F4, ATMA, CG, TAPS, QF, PK>;
     constexpr int NSTG = Cfg::NSTG, GRP = Cfg::GRP, NSLOT = Cfg::NSLOT, A_STAGE = Cfg::A_STAGE, B_STAGE = Cfg::B_STAGE, NBUF = Cfg::NBUF, WARP_EPI0 = Cfg::WARP_EPI0, NG = Cfg::NG, EPW = Cfg::EPW;
     constexpr int BMT = MT * BM;      // rows per block
     constexpr int TILE_M = CG * BMT;  // rows per tile (a block pair shares one 256-row tile)
@@ -309,7 +319,8 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> m
     // barriers: full[NSTG], empty[NSTG], tmem_full[NBARS], tmem_empty[NBARS]
     const uint32_t bar_full = smem_u32(bars), bar_empty = smem_u32(bars + NSTG), bar_tfull = smem_u32(bars + 2 * NSTG),
                    bar_tempty = smem_u32(bars + 2 * NSTG + Cfg::NBARS);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NSTG + 2 * Cfg::NBARS);
+    const uint32_t bar_pfull = smem_u32(bars + 2 * NSTG + 2 * Cfg::NBARS), bar_pempty = bar_pfull + 8 * Cfg::NPK;  // PK
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * NSTG + 2 * Cfg::NBARS + 2 * Cfg::NPK);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     // Gathering form: the first TAPMAX entries of the tap table (plane word -> kh, kw, ic) are copied to shared memory;
     // longer tables fall back to global loads.
@@ -330,7 +341,7 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> m
     const uint32_t rank = (CG == 2) ? cluster_ctarank() : 0u;
     const int unit = blockIdx.x / CG, nunits = gridDim.x / CG;
 
-    if (!ATMA && p.jtab)
+    if (!ATMA && !PK && p.jtab)
         for (int j = threadIdx.x; j < min(p.Kp, Cfg::TAPMAX); j += blockDim.x) s_taps[j] = __ldg(p.jtab + j);
     if (tid == 0) {
         for (int s = 0; s < NSTG; s++) {
@@ -340,6 +351,10 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> m
         for (int b = 0; b < Cfg::NBARS; b++) {
             mbar_init(bar_tfull + 8 * b, 1);
             mbar_init(bar_tempty + 8 * b, CG * 4 * MT * EPW);  // the epilogue warps (of both blocks of a pair)
+        }
+        for (int s = 0; s < Cfg::NPK; s++) {
+            mbar_init(bar_pfull + 8 * s, 1);   // the copy's bytes
+            mbar_init(bar_pempty + 8 * s, 4);  // the warps of the group that reads it
         }
         if (QF) {
             uint64_t* qbars = reinterpret_cast<uint64_t*>(smem + Cfg::Q_OFF + Cfg::QSTG * Cfg::Q_STAGE);
@@ -574,6 +589,54 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> m
                     if (CG == 2) tc_commit_pair(bar_tfull + 8 * buf); else tc_commit(bar_tfull + 8 * buf);
                 }
             }
+        }
+    } else if (PK && warp == Cfg::WARP_PK) {
+        // ---------------- packed rows: one tensor copy per stage, ahead of the expanders across tiles ----------------
+        if (lane == 0) {
+            prefetch_tensor_map(&tmap_a);
+            const int row_bytes = p.a_two_planes ? 64 : 32;  // of a stage
+            uint32_t s = 0, ph = 1;
+            for (int t = unit; t < ntiles; t += nunits) {
+                const int row0 = (int)p.div_ntn.div((uint32_t)t) * BMT;  // M below 2^31 (checked by the launcher)
+                for (int c = 0; c < nchunks; c++) {
+                    if (!mbar_wait(bar_pempty + 8 * s, ph, abort_flag, p.status, 11)) goto done;
+                    mbar_arrive_expect_tx(bar_pfull + 8 * s, (uint32_t)(BM * row_bytes));
+                    tma_tile2d_g2s(smem_u32(smem + Cfg::PK_OFF + s * Cfg::PK_STAGE), &tmap_a, c * row_bytes, row0, bar_pfull + 8 * s);
+                    if (++s == Cfg::NPK) { s = 0; ph ^= 1; }
+                }
+            }
+        }
+    } else if (PK && warp < WARP_EPI0) {
+        // ---------------- expanders from the packed-row ring: thread = row, group k takes the stages k, k+NG, ... ----------------
+        constexpr int NG1 = NG > 0 ? NG : 1, NPK1 = Cfg::NPK > 0 ? Cfg::NPK : 1;
+        const int e = tid - WARP_EXP0 * 32, grp = e / BM, r = e - grp * BM;
+        const int my_tiles = (int)blockIdx.x < ntiles ? (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+        const long long total_it = (long long)my_tiles * nchunks;
+        uint32_t s = (uint32_t)grp % NSTG, ph = (((uint32_t)grp / NSTG) & 1) ^ 1;  // slot of the operand ring, parity of its "empty"
+        uint32_t ps = (uint32_t)grp, pph = 0;                                       // slot of the packed-row ring
+        for (long long it = grp; it < total_it; it += NG1) {
+            uint4 ds[2], dz[2];
+            if (!mbar_wait(bar_pfull + 8 * ps, pph, abort_flag, p.status, 12)) goto done;
+            const unsigned char* slot = smem + Cfg::PK_OFF + ps * Cfg::PK_STAGE;
+            if (p.a_two_planes) {
+                const uint4* row = reinterpret_cast<const uint4*>(slot + r * 64);  // 64-byte swizzle: piece index ^ (row / 2) % 4
+                const int x = (r >> 1) & 3;
+                ds[0] = row[x]; ds[1] = row[1 ^ x]; dz[0] = row[2 ^ x]; dz[1] = row[3 ^ x];
+            } else {
+                const uint4* row = reinterpret_cast<const uint4*>(slot + r * 32);  // 32-byte swizzle: piece index ^ (row / 4) % 2
+                const int x = (r >> 2) & 1;
+                ds[0] = row[x]; ds[1] = row[1 ^ x];
+                dz[0] = dz[1] = make_uint4(0, 0, 0, 0);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_pempty + 8 * ps);
+            if ((ps += NG1) >= (uint32_t)NPK1) { ps = (uint32_t)grp; pph ^= 1; }
+            if (!mbar_wait(bar_empty + 8 * s, ph, abort_flag, p.status, 4)) goto done;
+            store_row_stage_f4(sA + s * A_STAGE, r, ds, dz);
+            fence_proxy_async();  // generic-proxy smem writes -> visible to the tensor core's async proxy
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_full + 8 * s);
+            if ((s += NG1) >= (uint32_t)NSTG) { s -= NSTG; ph ^= 1; }
         }
     } else if (!ATMA && warp < WARP_EPI0) {
         // ---------------- activation expanders ----------------
@@ -1034,11 +1097,11 @@ __global__ void __launch_bounds__(128, 1) mma_rate_kernel(int iters, unsigned in
     }
 }
 
-template <int BN, int MT, bool F4, bool ATMA = false, int CG = 1, int TAPS = 1, bool QF = false, bool SINGLE = false, bool IMG = false>
+template <int BN, int MT, bool F4, bool ATMA = false, int CG = 1, int TAPS = 1, bool QF = false, bool SINGLE = false, bool IMG = false, bool PK = false>
 int launch_cfg(tnns_cuda_ctx* ctx, GemmArgs a, cudaStream_t stream, const CUtensorMap* tmap_a = nullptr,
                const CUtensorMap* tmap_b = nullptr, const CUtensorMap* tmap_q = nullptr) {
-    using Cfg = TcCfg<BN, MT, F4, ATMA, CG, TAPS, QF>;
-    auto kern = gemm_tc_kernel<BN, MT, F4, ATMA, CG, TAPS, QF, SINGLE, IMG>;
+    using Cfg = TcCfg<BN, MT, F4, ATMA, CG, TAPS, QF, PK>;
+    auto kern = gemm_tc_kernel<BN, MT, F4, ATMA, CG, TAPS, QF, SINGLE, IMG, PK>;
     const auto maps = tensor_maps<maps_of(CG, QF)>(tmap_a, tmap_b, tmap_q);
     // once per kernel and device: the attribute belongs to (function, device), and the call costs a microsecond per launch
     static bool smem_set[64] = {false};
@@ -1231,6 +1294,19 @@ int tnns_launch_gemm_tc(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const vo
         a.H = g.H; a.W = g.W; a.OW = g.OW; a.Cp = g.Cp; a.SH = g.SH; a.SW = g.SW; a.PH = g.PH; a.PW = g.PW;
     }
     const int bn = tnns_i8_tile_n(w->KN);
+    if (f4 && !implicit_geom && M < 0x7FFFFFFFLL) {
+        // the packed matrix, its rows fetched by tensor copies: box = one stage of 128 rows
+        const unsigned row_bytes = a.a_two_planes ? 64 : 32;
+        const unsigned long long pitch = (unsigned long long)w->Kp * (a.a_two_planes ? 16 : 8);
+        alignas(64) CUtensorMap map;
+        int rc = tnns_tensor_map_2d(&map, 1, d_a, pitch, (unsigned long long)M, pitch, row_bytes, BM, (int)row_bytes);
+        if (rc) return rc;
+        switch (bn) {
+            case 64: return launch_cfg<64, 1, true, false, 1, 1, false, false, false, true>(ctx, a, stream, &map);
+            case 128: return launch_cfg<128, 1, true, false, 1, 1, false, false, false, true>(ctx, a, stream, &map);
+            default: return launch_cfg<256, 1, true, false, 1, 1, false, false, false, true>(ctx, a, stream, &map);
+        }
+    }
     if (f4) {
         switch (bn) {
             case 64: return launch_bn<64, true>(ctx, a, stream);
