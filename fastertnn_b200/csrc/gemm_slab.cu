@@ -22,7 +22,8 @@
 // (four plane words), so K steps that only exist because rows are padded to four words are skipped.
 // Weights that fit the ring entirely are fetched once per block and stay (64-kernel layers).
 //
-// Roles per block: producer warp (slabs and weight stages), MMA warp, eight or twelve epilogue warps; with QF
+// Roles per block: producer warp (slabs and weight stages), MMA warp, eight or twelve epilogue warps; image outputs of 32- and
+// 64-byte pixels: two more warps that fetch the slabs, sixteen epilogue warps on tiles of 64 kernels; with QF
 // four quantiser warps and a publisher as in the im2col form (gemm_tc.cu).  Block pairs
 // (tcgen05.mma.cta_group::2) share a 256-row tile, each block with its own slab and half of the
 // weight stage.  Every wait is bounded.

@@ -19,16 +19,17 @@
 //                       four quantiser warps and a publisher thread beside the GEMM's roles; a
 //                       tile's copies start once the images of its rows are complete)
 //
-// Expander-fed form: one persistent block per SM, 22 warps in four roles (the tensor-copy form
+// Expander-fed form: one persistent block per SM, 19 to 23 warps in four or five roles (the tensor-copy form
 // keeps warps 0, 1 and eight epilogue warps, twelve on tiles of 64 and 128 kernels):
 //   warp 0      weight producer: one bulk async copy (TMA engine, no multicast, no tensor map)
 //               per stage of a pre-expanded, pre-swizzled weight tile (built once per layer)
 //   warp 1      MMA issuer: a warp-uniform loop whose elected lane issues four tcgen05.mma per stage
 //               and commits to the stage's "empty" barrier; owns the tensor-memory allocation
-//   12-16 warps activation expanders in NG groups: thread = row; group k fills stages k, k+NG, ...
-//               so NG stages are expanded at once; packed planes come from global memory through
-//               a register prefetch ring and are stored in the 128-byte-swizzled K-major layout
-//               the MMA descriptor expects
+//   8-16 warps  activation expanders in NG groups: thread = row; group k fills stages k, k+NG, ...
+//               so NG stages are expanded at once; packed planes come from a ring that one more warp
+//               keeps filled with tensor copies of the packed matrix (4-bit form), or from global memory
+//               through a register prefetch ring, and are stored in the 128-byte-swizzled K-major
+//               layout the MMA descriptor expects
 //   4-8 warps   epilogue: tcgen05.ld the finished accumulator, apply the BNN constant and PReLU,
 //               store fp32 (NCHW: 32 consecutive pixels per warp and kernel -> 128-byte stores)
 // Every mbarrier wait is bounded; on expiry the kernel raises a status word, all roles leave
@@ -112,7 +113,7 @@ struct TcCfg {
     // epilogue warps per lane quadrant: two share each quadrant's columns where the drain is
     // not (or only partly) hidden behind the next tile's MMAs
     static constexpr int EPW = ATMA ? (NSETS > 1 ? 1 : 2) : (((NBUF == 1 || OVL) && MT == 1) ? 2 : 1);
-    // expander groups (stages expanded concurrently); 22 warps per block in every MT = 1 form
+    // expander groups (stages expanded concurrently)
     // (two suffice for 256 kernels where the rows come by tensor copy, and leave the epilogue 96 registers instead of 80)
     static constexpr int NG = ATMA ? 0 : ((MT == 1) ? (EPW == 2 ? (PK ? 2 : 3) : 4) : 2);
     static constexpr int WARP_EPI0 = WARP_EXP0 + 4 * MT * NG;
