@@ -1064,8 +1064,9 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
                 default: return launch_slab<256, 1, T, false, false, 1, true>(ctx, a, smem, stream, ma, nullptr, nullptr);
             }
         }
-        if (use_pairs) return launch_slab<256, 2, T, false>(ctx, a, smem, stream, &map_a, &map_b, nullptr);
-        const bool single = pl.bn < 256 && single_floats(a.layout, a.y_vec, d_pimg);
+        const bool single = single_floats(a.layout, a.y_vec, d_pimg);
+        if (use_pairs) return single ? launch_slab<256, 2, T, false, true>(ctx, a, smem, stream, &map_a, &map_b, nullptr)
+                                     : launch_slab<256, 2, T, false>(ctx, a, smem, stream, &map_a, &map_b, nullptr);
         if constexpr (T == 1)
             if (ch.grp == 3) {
                 if (pl.bn == 64) return single ? launch_slab<64, 1, T, false, true, 3>(ctx, a, smem, stream, &map_a, nullptr, nullptr)
@@ -1074,8 +1075,11 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
                               : launch_slab<128, 1, T, false, false, 3>(ctx, a, smem, stream, &map_a, nullptr, nullptr);
             }
         if (single) {
-            if (pl.bn == 64) return launch_slab<64, 1, T, false, true>(ctx, a, smem, stream, &map_a, nullptr, nullptr);
-            return launch_slab<128, 1, T, false, true>(ctx, a, smem, stream, &map_a, nullptr, nullptr);
+            switch (pl.bn) {
+                case 64: return launch_slab<64, 1, T, false, true>(ctx, a, smem, stream, &map_a, nullptr, nullptr);
+                case 128: return launch_slab<128, 1, T, false, true>(ctx, a, smem, stream, &map_a, nullptr, nullptr);
+                default: return launch_slab<256, 1, T, false, true>(ctx, a, smem, stream, &map_a, nullptr, nullptr);
+            }
         }
         switch (pl.bn) {
             case 64: return launch_slab<64, 1, T, false>(ctx, a, smem, stream, &map_a, nullptr, nullptr);

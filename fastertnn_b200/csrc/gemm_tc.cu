@@ -1533,11 +1533,15 @@ int tnns_launch_gemm_im2col(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, cons
                 default: return launch_cfg<256, 1, true, true, 1, T, false, false, true>(ctx, a, stream, &map);
             }
         }
-        if (use_pairs) return launch_cfg<256, 1, true, true, 2, T>(ctx, a, stream, &map, &map_b);
-        if (bn < 256 && single_floats(a.layout, a.y_vec, d_pimg)) {
-            if (bn == 64) return launch_cfg<64, 1, true, true, 1, T, false, true>(ctx, a, stream, &map);
-            return launch_cfg<128, 1, true, true, 1, T, false, true>(ctx, a, stream, &map);
+        if (single_floats(a.layout, a.y_vec, d_pimg)) {
+            if (use_pairs) return launch_cfg<256, 1, true, true, 2, T, false, true>(ctx, a, stream, &map, &map_b);
+            switch (bn) {
+                case 64: return launch_cfg<64, 1, true, true, 1, T, false, true>(ctx, a, stream, &map);
+                case 128: return launch_cfg<128, 1, true, true, 1, T, false, true>(ctx, a, stream, &map);
+                default: return launch_cfg<256, 1, true, true, 1, T, false, true>(ctx, a, stream, &map);
+            }
         }
+        if (use_pairs) return launch_cfg<256, 1, true, true, 2, T>(ctx, a, stream, &map, &map_b);
         switch (bn) {
             case 64: return launch_cfg<64, 1, true, true, 1, T>(ctx, a, stream, &map);
             case 128: return launch_cfg<128, 1, true, true, 1, T>(ctx, a, stream, &map);
