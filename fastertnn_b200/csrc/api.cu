@@ -1043,13 +1043,12 @@ int tnns_cuda_conv_host(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const fl
     // (Letting the one-launch kernel work on page-locked host buffers directly -- tensor copies and
     // epilogue stores over PCIe, no staging -- measured slower than the copy engines: 4.2 ms against
     // 3.2 ms on the large layer; the SMs' reads of host memory reach about 32 GB/s.)
-    // Slice the batch so that copies and kernels overlap; nb = images of a full slice.  About eight slices, but one below 4 MB of
-    // input and output: a slice costs two copies, two launches and six event calls, which a small batch does not earn back
-    // (the drop-in call on 8 x 256x14x14 -> 256 s2, 2 MB of pageable memory: 508 us in eight slices, 250 in one; two to four slices
-    // of 4 MB for batches of 13 to 16 MB looked slower than eight on a box with a noisy host, so those keep eight).
+    // Slice the batch so that copies and kernels overlap; nb = images of a full slice.  About eight slices, but none below 4 MB of
+    // input and output: a slice costs two copies, two launches and six event calls, which a small one does not earn back
+    // (the drop-in call on 8 x 256x14x14 -> 256 s2, 2 MB of pageable memory: 508 us in eight slices, 250 in one).
     const size_t in_img = (size_t)g.C * g.H * g.W * sizeof(float);
     const size_t out_img = (size_t)g.KN * g.OH * g.OW * sizeof(float);
-    const int nslices = (in_img + out_img) * (size_t)g.N < (4u << 20) ? 1 : 8;
+    const int nslices = (int)std::min<size_t>(8, std::max<size_t>(1, (in_img + out_img) * (size_t)g.N / (4u << 20)));
     const int nb = std::max(1, (g.N + nslices - 1) / nslices);
     tnns_shape_t ss = *s;
     ss.N = nb;
