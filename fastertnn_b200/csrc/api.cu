@@ -556,7 +556,7 @@ int tnns_cuda_gemm_slab_packed_out(tnns_cuda_ctx* ctx, const tnns_cuda_weights* 
 
 static int conv_slab_impl(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const float* d_x, const float* d_thr, float* d_y, void* d_image_out,
                           const float* d_thr_next, int fmt, int bin, int next_PH, int next_PW, void* d_workspace, size_t workspace_bytes,
-                          const tnns_shape_t* s, float alpha, int pairs, void* stream) {
+                          const tnns_shape_t* s, float alpha, int pairs, void* stream, bool starve = false) {
     if (!ctx || !w || !d_x || !d_thr || !d_workspace) return tnns_fail(TNNS_ERR_INVALID, "NULL argument");
     if (pairs < 0 || pairs > 2) return tnns_fail(TNNS_ERR_INVALID, "pairs must be 0, 1 or 2");
     TnnsGeom g;
@@ -571,6 +571,7 @@ static int conv_slab_impl(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
     f.d_x = d_x;
     f.d_thr = d_thr;
     f.Cp = g.Cp;
+    f.starve = starve;
     f.d_sync = reinterpret_cast<unsigned int*>(static_cast<char*>(d_workspace) + slab_image_bytes(g.N, g.C, g.H, g.W, g.PH, g.PW));
     return tnns_launch_gemm_slab(ctx, w, d_workspace, d_y, g, alpha, TNNS_NCHW, (cudaStream_t)stream, pairs, d_image_out, d_thr_next, fmt, bin, next_PH,
                                  next_PW, &f);
@@ -580,6 +581,14 @@ int tnns_cuda_conv_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const fl
                         size_t workspace_bytes, const tnns_shape_t* s, float alpha, int pairs, void* stream) {
     if (!d_y) return tnns_fail(TNNS_ERR_INVALID, "NULL argument");
     return conv_slab_impl(ctx, w, d_x, d_thr, d_y, nullptr, nullptr, 2, 0, 0, 0, d_workspace, workspace_bytes, s, alpha, pairs, stream);
+}
+
+// Failure-detection self-test of a whole layer kernel: its quantiser warps are told that there is no image, so the producers wait for
+// images that never come.  The waits give up after about a second, all roles of every block leave, and the context stays usable.
+int tnns_cuda_selftest_slab_wait_expiry(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const float* d_x, const float* d_thr, float* d_y,
+                                        void* d_workspace, size_t workspace_bytes, const tnns_shape_t* s, int pairs, void* stream) {
+    if (!d_y) return tnns_fail(TNNS_ERR_INVALID, "NULL argument");
+    return conv_slab_impl(ctx, w, d_x, d_thr, d_y, nullptr, nullptr, 2, 0, 0, 0, d_workspace, workspace_bytes, s, 0.5f, pairs, stream, true);
 }
 
 int tnns_cuda_conv_slab_packed_out(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const float* d_x, const float* d_thr, void* d_image_out,

@@ -327,7 +327,9 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
                 }
             }
         }
-        __syncwarp();
+        // On to issuing: lane 0 left no wait behind that could have sent it to `done` (loaders, weights that stay).  In every other form
+        // its failed wait goes to `done` directly, and a barrier here would leave it one warp barrier behind the other lanes.
+        if (two) __syncwarp();
     }
     if (warp == WARP_MMA || (two && warp == WARP_TMA)) {
         if (rank == 0) {  // pair: the first block issues for both
@@ -1038,7 +1040,7 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
         a.qimg = reinterpret_cast<uint4*>(const_cast<void*>(d_image));
         a.q_sync = words;
         a.q_self_clean = self_clean;
-        a.qN = g.N; a.qC = g.C; a.q_H = g.H; a.q_W = g.W; a.q_PH = g.PH; a.q_PW = g.PW;
+        a.qN = fused->starve ? 0 : g.N; a.qC = g.C; a.q_H = g.H; a.q_W = g.W; a.q_PH = g.PH; a.q_PW = g.PW;
         a.q_nbands = (g.H * g.W + Q_PIX - 1) / Q_PIX;
         a.q_binary = act_binary ? 1 : 0;
     }

@@ -142,6 +142,7 @@ struct TnnsFusedInput {
     const float* d_thr;
     unsigned int* d_sync;
     int Cp;  // 64-channel words of the fp32 input's channels (the geometry's Cp is the image's pixel, which may be padded to more)
+    bool starve = false;  // self-test (slab form): the quantiser warps are told of no image, so that every producer's wait runs out
 };
 size_t tnns_fused_sync_bytes(int N);
 bool tnns_fused_supported(const tnns_cuda_weights* w, const TnnsGeom& g, const float* d_x, int layout);

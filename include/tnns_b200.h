@@ -493,6 +493,10 @@ int tnns_cuda_sync(tnns_cuda_ctx* ctx);
  * the following tnns_cuda_sync returns TNNS_ERR_DEVICE_WAIT.  The kernel returns normally and the
  * context remains usable. */
 int tnns_cuda_selftest_wait_expiry(tnns_cuda_ctx* ctx);
+/* The same of a whole layer kernel, the one-launch slab form (arguments as tnns_cuda_conv_slab): its producers wait
+ * for images that no warp writes, every role of every block leaves within seconds, d_y keeps what it held. */
+int tnns_cuda_selftest_slab_wait_expiry(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const float* d_x, const float* d_thr, float* d_y,
+                                        void* d_workspace, size_t workspace_bytes, const tnns_shape_t* s, int pairs, void* stream);
 
 /* The rule of the quantising epilogues, on the host (no GPU needed; no reference counterpart).  A layer
  * that writes the next layer's quantised activations applies, for 0 < alpha <= 1, thresholds to its raw
