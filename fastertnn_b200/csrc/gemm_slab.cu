@@ -31,11 +31,10 @@
 #include <type_traits>
 
 #include "gemm_tc_common.cuh"
+#include "slab_rings.h"
 
 namespace {
 
-constexpr int SL_MAXSLAB = 8;    // slab buffers at most
-constexpr int SL_MAXSTG = 12;    // weight ring depth at most
 constexpr int SL_TAPMAX = 4096;  // filter taps at most
 constexpr int SL_BAR_BYTES = 512;
 
@@ -903,24 +902,6 @@ bool make_plan(const tnns_cuda_weights* w, const TnnsGeom& g, SlabPlan* pl) {
     return true;
 }
 
-// ring depths for a configuration; false when not even two slabs and three weight stages fit
-bool ring_depths(const SlabPlan& pl, int b_stage, int fixed, int nchunks, bool one_kernel_tile, bool loaders, int* nslab, int* nstg, int* resident) {
-    const int avail = 232448 - fixed;
-    int ns = pl.slab_bytes <= 16384 ? (loaders ? SL_MAXSLAB : 4) : (pl.slab_bytes <= 32768 ? 3 : 2);
-    for (; ns >= 2; ns--) {
-        const int rest = avail - ns * pl.slab_bytes;
-        if (rest < 3 * b_stage) continue;
-        int nb = std::min(SL_MAXSTG, rest / b_stage);
-        *resident = (one_kernel_tile && nchunks <= nb) ? 1 : 0;
-        if (*resident) nb = nchunks;
-        if (loaders) ns &= ~1;  // two MMA issuers take them in turn
-        *nslab = ns;
-        *nstg = nb;
-        return true;
-    }
-    return false;
-}
-
 }  // namespace
 
 namespace {
@@ -928,7 +909,8 @@ struct SlabChoice {
     SlabPlan pl;
     bool pairs;
     bool loaders;
-    int b_stage, fixed, nslab, nstg, resident, grp, Mv, ntn;
+    int b_stage, fixed, grp, Mv, ntn;
+    SlabRings rings;
     size_t smem;
 };
 // The form a launch takes: single blocks or block pairs (pairs_req 0 = by size, 1, 2), ring depths.
@@ -945,7 +927,11 @@ bool choose_form(int sm_count, const tnns_cuda_weights* w, const TnnsGeom& g, in
     ch->loaders = image_out && pl.taps > 1 && !ch->pairs && !fused;
     ch->b_stage = (pl.bn / (ch->pairs ? 2 : 1)) * KCH;
     ch->fixed = 1024 + SL_BAR_BYTES + (fused ? Q_STG * Q_PIX * 64 * 4 + 128 : 0);
-    if (!ring_depths(pl, ch->b_stage, ch->fixed, w->Kp / 4, ch->ntn == 1, ch->loaders, &ch->nslab, &ch->nstg, &ch->resident)) return false;
+    auto rings = [&]() {
+        const SlabFeed feed = !ch->loaders ? SLAB_COPIES : (ch->pl.bn == 64 && pl.T == 9 && g.KW == 3) ? SLAB_LOADERS_TWO : SLAB_LOADERS;
+        return slab_rings(pl.slab_bytes, ch->b_stage, 232448 - ch->fixed, w->Kp / 4, ch->ntn == 1, feed, &ch->rings);
+    };
+    if (!rings()) return false;
     if (!ch->pairs && !fused) {
         // few tiles: narrower ones (what fits with the widest tile fits with these)
         const int bn = tile_n_for(sm_count, ch->Mv, w->KN, pl.bn);
@@ -953,13 +939,14 @@ bool choose_form(int sm_count, const tnns_cuda_weights* w, const TnnsGeom& g, in
             ch->pl.bn = bn;
             ch->ntn = (w->KN + bn - 1) / bn;
             ch->b_stage = bn * KCH;
-            if (!ring_depths(pl, ch->b_stage, ch->fixed, w->Kp / 4, ch->ntn == 1, ch->loaders, &ch->nslab, &ch->nstg, &ch->resident)) return false;
+            if (!rings()) return false;
         }
     }
     // three weight stages a slot (see the kernel's GRP) where two slots fit
-    ch->grp = (pl.taps == 1 && g.KH == 3 && g.KW == 3 && !ch->resident && !ch->pairs && !fused && ch->pl.bn <= 128 && ch->nstg >= 6) ? 3 : 1;
-    ch->nstg -= ch->nstg % ch->grp;
-    ch->smem = (size_t)ch->fixed + (size_t)ch->nslab * pl.slab_bytes + (size_t)ch->nstg * ch->b_stage;
+    SlabRings& r = ch->rings;
+    ch->grp = (pl.taps == 1 && g.KH == 3 && g.KW == 3 && !r.resident && !ch->pairs && !fused && ch->pl.bn <= 128 && r.nstg >= 6) ? 3 : 1;
+    r.nstg -= r.nstg % ch->grp;
+    ch->smem = (size_t)ch->fixed + (size_t)r.nslab * pl.slab_bytes + (size_t)r.nstg * ch->b_stage;
     return true;
 }
 }  // namespace
@@ -988,7 +975,7 @@ int tnns_launch_gemm_slab(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const 
     const bool use_pairs = ch.pairs;
     const size_t smem = ch.smem;
     SlabArgs a = {};
-    a.nslab = ch.nslab; a.nstg = ch.nstg; a.b_resident = ch.resident;
+    a.nslab = ch.rings.nslab; a.nstg = ch.rings.nstg; a.b_resident = ch.rings.resident;
     a.Bimg = reinterpret_cast<const unsigned char*>(w->d_f4);
     a.y = d_y;
     a.Mv = Mv;
