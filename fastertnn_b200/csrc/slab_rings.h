@@ -20,6 +20,10 @@ struct SlabRings {
 //   two issuers   as many slabs as leave the weights resident, an even number (the issuers take them in turn), up to eight.
 //                 GEMM alone, image out, 2 / 4 / 8 slabs: 32 x 128x112x112 -> 64 (23 KB each) 22.4 / 21.6 / 18.8 us,
 //                 8 x 64x224x224 -> 64 (19 KB) 15.6 / 15.1 / 14.2, 256 x 64x56x56 -> 64 (8 KB) 27.4 / 26.3 / 26.2
+//   one issuer    loaders: two slabs, the rest for the weights.  More slabs gained nothing there and displaced weights that could stay:
+//                 2 / 4 / 8 slabs 32 x 64x80x80 -> 128 5x5 29.5 / 29.9 / 33.7 us, 64 x 128x112x112 -> 128 50.0 / 50.2 / 65.7, 256 x
+//                 128x28x28 -> 128 (weights resident with all three) 16.9 / 17.2 / 17.6.
+//   copies        four, three or two by their size
 inline bool slab_rings(int slab_bytes, int b_stage, int avail, int nchunks, bool one_kernel_tile, SlabFeed feed, SlabRings* r) {
     const bool may_stay = one_kernel_tile && nchunks <= SL_MAXSTG;
     if (feed == SLAB_LOADERS_TWO && may_stay)
@@ -28,9 +32,8 @@ inline bool slab_rings(int slab_bytes, int b_stage, int avail, int nchunks, bool
                 *r = {ns, nchunks, true};
                 return true;
             }
-    int ns = slab_bytes <= 16384 ? (feed != SLAB_COPIES ? SL_MAXSLAB : 4) : (slab_bytes <= 32768 ? 3 : 2);
-    if (feed != SLAB_COPIES) ns &= ~1;
-    for (; ns >= 2; ns -= feed != SLAB_COPIES ? 2 : 1) {
+    int ns = feed != SLAB_COPIES ? 2 : slab_bytes <= 16384 ? 4 : slab_bytes <= 32768 ? 3 : 2;
+    for (; ns >= 2; ns--) {
         const int rest = avail - ns * slab_bytes;
         if (rest < 3 * b_stage) continue;
         const int nb = std::min(SL_MAXSTG, rest / b_stage);

@@ -58,6 +58,17 @@ def test_two_issuers_use_the_memory_there_is(rings):
             assert ns == MAXSLAB or (ns + 2) * slab + nchunks * 8192 > AVAIL, slab
 
 
+def test_loaders_displace_no_weights_that_could_stay(rings):
+    """Weights that fit beside two slabs stay; four slabs of tensor copies are no reason to stream them either."""
+    for feed in (LOADERS, LOADERS_TWO):
+        for slab in SLABS:
+            for stage in (8192, 16384, 32768):
+                for nchunks in range(3, MAXSTG + 1):
+                    r = rings(slab, stage, nchunks, True, feed)
+                    if r:
+                        assert r[2] == (2 * slab + nchunks * stage <= AVAIL), (feed, slab, stage, nchunks)
+
+
 @pytest.mark.parametrize("stage", [8192, 16384, 32768])
 def test_ring_of_weights_is_sized_for_the_slabs_that_are_kept(stage, rings):
     """Streamed weights get what the slabs leave: another stage would not fit."""
