@@ -192,8 +192,8 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
     const bool ahead = LONE && warp == WARP_TMA;
     // Two warps issue the MMAs of every other tile each where a tile has few of them and the weights stay: the producer's warp has
     // nothing left to do, and a tile's two waits (110-140 clocks each even when complete) pass beside the other's MMAs.  Both take an
-    // even number of slabs and accumulators in turn, so each meets the same ones in successive phases.
-    const bool two = Cfg::TWO && p.b_resident && p.T == 9 && p.KW == 3;
+    // even number of slabs (slab_rings.h; one issuer on an odd one) and accumulators in turn, so each meets the same ones in successive phases.
+    const bool two = Cfg::TWO && p.b_resident && p.T == 9 && p.KW == 3 && (p.nslab & 1) == 0;
     uint32_t tmem_base = 0;
     if (ahead) {
         named_arrive(1, blockDim.x);
