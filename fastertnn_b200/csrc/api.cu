@@ -1052,9 +1052,13 @@ int tnns_cuda_conv_host(tnns_cuda_ctx* ctx, const tnns_cuda_weights* w, const fl
     // (Letting the one-launch kernel work on page-locked host buffers directly -- tensor copies and
     // epilogue stores over PCIe, no staging -- measured slower than the copy engines: 4.2 ms against
     // 3.2 ms on the large layer; the SMs' reads of host memory reach about 32 GB/s.)
-    // Slice the batch so that copies and kernels overlap; nb = images of a full slice.  About eight slices, but none below 4 MB of
-    // input and output: a slice costs two copies, two launches and six event calls, which a small one does not earn back
-    // (the drop-in call on 8 x 256x14x14 -> 256 s2, 2 MB of pageable memory: 508 us in eight slices, 250 in one).
+    // Slice the batch so that copies and kernels overlap; nb = images of a full slice.  About eight slices, but only as many as make
+    // a full one 4 MB of input and output (the tapered ends are parts of one, an uneven last slice is what is left): a slice costs two
+    // copies, two launches and six event calls, which a small one does not earn back (the drop-in call on 8 x 256x14x14 -> 256
+    // s2, 2 MB of pageable memory: 508 us in eight slices, 250 in one).  Page-locked buffers, one slice / two / up to eight: 5.7 MB
+    // (24 x 256x14x14 -> 256 s2) 143 / 149 / 187 us, 6.1 MB (4 x 64x56x56 -> 64) 175 / 163 / 170, 7.7 MB (8 x 64x28x28 -> 256 1x1)
+    // 173 / 178 / 182; three / eight 15.3 MB (64 x 256x14x14 -> 256 s2) 298 / 348.  A second slice below 8 MB would earn page-locked
+    // calls 7 % at most and cost pageable ones 10 to 19 (32 x 256x14x14 -> 256 s2, 7.7 MB: 467 / 539).
     const size_t in_img = (size_t)g.C * g.H * g.W * sizeof(float);
     const size_t out_img = (size_t)g.KN * g.OH * g.OW * sizeof(float);
     const int nslices = (int)std::min<size_t>(8, std::max<size_t>(1, (in_img + out_img) * (size_t)g.N / (4u << 20)));
