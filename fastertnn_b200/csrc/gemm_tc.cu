@@ -629,14 +629,18 @@ gemm_tc_kernel(GemmArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> m
                 ds[0] = row[x]; ds[1] = row[1 ^ x];
                 dz[0] = dz[1] = make_uint4(0, 0, 0, 0);
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_pempty + 8 * ps);
-            if ((ps += NG1) >= (uint32_t)NPK1) { ps = (uint32_t)grp; pph ^= 1; }
             if (!mbar_wait(bar_empty + 8 * s, ph, abort_flag, p.status, 4)) goto done;
             store_row_stage_f4(sA + s * A_STAGE, r, ds, dz);
             fence_proxy_async();  // generic-proxy smem writes -> visible to the tensor core's async proxy
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_full + 8 * s);
+            if (lane == 0) {
+                mbar_arrive(bar_full + 8 * s);
+                // The slot goes back here, where the row is stored and so has been read.  Behind the loads alone the arrival overtook them: beside
+                // the MMAs' operand reads a load of shared memory can take longer than the refill, and the last 16 bytes of a row were the
+                // next lap's (512 -> 512 @14, batch 64: 26 of 960 launches).  It costs nothing: 8 x 512x32x32 -> 512 12.8 / 12.7 us.
+                mbar_arrive(bar_pempty + 8 * ps);
+            }
+            if ((ps += NG1) >= (uint32_t)NPK1) { ps = (uint32_t)grp; pph ^= 1; }
             if ((s += NG1) >= (uint32_t)NSTG) { s -= NSTG; ph ^= 1; }
         }
     } else if (!ATMA && warp < WARP_EPI0) {

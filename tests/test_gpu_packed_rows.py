@@ -42,3 +42,42 @@ def test_packed_rows(layer, N, type_, gpu_ctx, checker):
         for p in (d_x, d_t, d_a, d_y, d_r):
             ctx.free(p)
         w.free()
+
+
+# many stages on tiles of 256 kernels: a slot of the packed-row ring is read while its refill is on the way, so every launch has to be
+# right, beside others and alone (a row read too late holds the next lap's bytes in a few launches of a hundred)
+@pytest.mark.parametrize("type_,layer,N", [(TNN, Layer(512, 14, 14, 512, 3, 3, 1, 1), 64), (TNN, Layer(512, 7, 7, 512, 3, 3, 1, 1), 256),
+                                           (BTN, Layer(1024, 7, 7, 512, 3, 3, 1, 1), 100), (BNN, Layer(512, 7, 7, 64, 3, 3, 1, 1), 100)],
+                         ids=lambda v: str(v).replace(" ", ""))
+def test_every_launch_of_many(type_, layer, N, gpu_ctx, checker):
+    import torch
+    ctx, sh, R = gpu_ctx, layer.shape(N), 6
+    case = make_case(type_, layer, 1, 9700 + layer.C, "uniform")
+    w = ctx.upload_weights(type_, checker.pack_weights(wgt_ternary(type_), case.w, case.w_thr), layer.C, layer.KH, layer.KW)
+    ternary = type_ in (TNN, TBN)
+    gen = torch.Generator(device="cuda").manual_seed(9701)
+    n_out = N * layer.KN * layer.OH * layer.OW
+    x = torch.empty(N * layer.C * layer.H * layer.W, device="cuda")
+    t = torch.full((N,), 0.25 if ternary else 0.0, device="cuda")
+    a = torch.empty((R, api.packed_bytes(type_, sh) // 8), dtype=torch.int64, device="cuda")
+    y, want = torch.empty((R, n_out), device="cuda"), torch.empty((R, n_out), device="cuda")
+    try:
+        for i in range(R):
+            x.uniform_(-1, 1, generator=gen)
+            torch.cuda.synchronize()
+            ctx.pack(ternary, x.data_ptr(), t.data_ptr(), a[i].data_ptr(), sh)
+            ctx.gemm(w, a[i].data_ptr(), want[i].data_ptr(), N, layer.OH, layer.OW, case.alpha, algo=api.GEMM_POPC_TILED)
+            ctx.sync()
+        wrong = 0
+        for rep in range(60):
+            y.fill_(float("nan"))
+            torch.cuda.synchronize()
+            for i in range(R):
+                ctx.gemm(w, a[i].data_ptr(), y[i].data_ptr(), N, layer.OH, layer.OW, case.alpha, algo=api.GEMM_F4_TC)
+                if rep % 2:
+                    ctx.sync()
+            ctx.sync()
+            wrong += int((y != want).any(1).sum())
+        assert wrong == 0, f"{wrong} of {60 * R} launches"
+    finally:
+        w.free()
