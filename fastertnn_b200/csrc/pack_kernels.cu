@@ -104,7 +104,7 @@ __device__ __forceinline__ uint32_t push_sign(uint32_t acc, float d) {
 }
 
 template <bool TERNARY, int VEC>
-__device__ __forceinline__ void quantise_batch(const float* __restrict__ q, size_t HW, float t, uint32_t (&sg)[VEC],
+__device__ __forceinline__ void quantise_batch(const float* q, size_t HW, float t, uint32_t (&sg)[VEC],
                                                uint32_t (&nzb)[VEC]) {
     // channels q[7*HW] .. q[0] (descending), eight at a time: all loads first, then the pushes
     float vals[8][VEC];
@@ -112,10 +112,10 @@ __device__ __forceinline__ void quantise_batch(const float* __restrict__ q, size
     for (int k = 0; k < 8; k++) {
         const float* pk = q + (size_t)(7 - k) * HW;
         if (VEC == 4) {
-            const float4 f = __ldg(reinterpret_cast<const float4*>(pk));
+            const float4 f = *reinterpret_cast<const float4*>(pk);
             vals[k][0] = f.x; vals[k][1 % VEC] = f.y; vals[k][2 % VEC] = f.z; vals[k][3 % VEC] = f.w;
         } else {
-            vals[k][0] = __ldg(pk);
+            vals[k][0] = *pk;
         }
     }
 #pragma unroll
@@ -133,7 +133,7 @@ __device__ __forceinline__ void quantise_batch(const float* __restrict__ q, size
 
 template <bool TERNARY, int LAYOUT, int VEC, bool PAIR>
 __global__ void __launch_bounds__(kPackThreadsMax, 2)
-pack_staged_kernel(const float* __restrict__ x, const float* __restrict__ thr, uint4* __restrict__ out, TnnsGeom g,
+pack_staged_kernel(const float* x, const float* thr, uint4* __restrict__ out, TnnsGeom g,
                    int BOH, int nbands, int Lmax, FastDiv divU, FastDiv divOW, FastDiv divL) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int PLANES = TERNARY ? 2 : 1;
@@ -165,7 +165,9 @@ pack_staged_kernel(const float* __restrict__ x, const float* __restrict__ thr, u
         joff[j] = off;
         jtap[j] = tap;
     }
-    // the input may be the output of the launch before, the matrix an operand of it
+    // The input may be the output of the launch before, the matrix an operand of it.  That launch may still write the input while this
+    // block is resident, so the input is no read-only data of this kernel: plain loads, no __ldg and no __restrict__, which would let
+    // a load be taken from the read-only path or moved ahead of the wait (times within 3 % of those of __ldg; loads past the L1 cache were up to 10 % slower).
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const float t = (LAYOUT == 2) ? 0.f : thr[n] + 0.0f, nt = -t;  // + 0.0f: a threshold of -0 behaves as +0 in every compare
 
@@ -176,8 +178,8 @@ pack_staged_kernel(const float* __restrict__ x, const float* __restrict__ thr, u
         const uint64_t* src_s = planes + (size_t)n * PLANES * HWC + (size_t)ih_lo * g.W * g.Cp;
         const int words = L * g.Cp;
         for (int i = tid; i < words; i += nthreads) {
-            sm_sign[i] = __ldg(src_s + i);
-            if (TERNARY) sm_zero[i] = __ldg(src_s + HWC + i);
+            sm_sign[i] = src_s[i];
+            if (TERNARY) sm_zero[i] = src_s[HWC + i];
         }
     } else if (LAYOUT == 0) {
         const size_t HW = (size_t)g.H * g.W;
@@ -203,7 +205,7 @@ pack_staged_kernel(const float* __restrict__ x, const float* __restrict__ thr, u
 #pragma unroll
                     for (int v = 0; v < VEC; v++) {
                         if (b < lim) {
-                            const float val = __ldg(q + v);
+                            const float val = q[v];
                             if (TERNARY) {
                                 sg[v] = push_sign(sg[v], val + t);
                                 nzb[v] = push_sign(nzb[v], t - fabsf(val));
@@ -239,7 +241,7 @@ pack_staged_kernel(const float* __restrict__ x, const float* __restrict__ thr, u
             for (int i0 = warp * UNR; i0 < items; i0 += NWARP * UNR) {
                 float v[UNR];
 #pragma unroll
-                for (int u = 0; u < UNR; u++) v[u] = (i0 + u < items) ? __ldg(base + (size_t)(i0 + u) * 32 + lane) : 0.f;
+                for (int u = 0; u < UNR; u++) v[u] = (i0 + u < items) ? base[(size_t)(i0 + u) * 32 + lane] : 0.f;
 #pragma unroll
                 for (int u = 0; u < UNR; u++) {
                     if (TERNARY) {
@@ -259,7 +261,7 @@ pack_staged_kernel(const float* __restrict__ x, const float* __restrict__ thr, u
             for (int i = warp; i < items; i += NWARP) {
                 const int p = i / halves, h = i - p * halves;
                 const int c = 32 * h + lane;
-                const float v = (c < g.C) ? __ldg(base + (size_t)p * g.C + c) : 0.f;
+                const float v = (c < g.C) ? base[(size_t)p * g.C + c] : 0.f;
                 const bool ok = c < g.C;
                 if (TERNARY) {
                     const uint32_t s = __ballot_sync(0xFFFFFFFFu, ok && v < nt);
