@@ -88,8 +88,8 @@ struct SlabCfg {
     // Epilogue warps: EPW per lane quadrant share a tile's columns, and NSETS such groups take the tiles in turn.  On tiles of
     // 64 / 128 kernels a tile's drain is a chain of latencies (barrier, row addresses, tensor-memory load, 32 columns of
     // arithmetic) several times as long as its MMAs, so three tiles are drained at once.  Eight warps on one tile / two sets /
-    // three sets, inside the 11-layer stack: 64 -> 64 @56 48.3 / 39.8 / 33.0 us, 128 -> 128 @28 25.9 / 22.1 / 19.4; four
-    // sets of the 64-kernel form gained nothing more.
+    // three sets, inside the 11-layer stack: 64 -> 64 @56 48.3 / 39.8 / 33.0 us, 128 -> 128 @28 25.9 / 22.1 / 19.4.  A fourth set gains
+    // nothing by itself; two issuers need one per accumulator (below).
     static constexpr bool LOADER = IMG && CG == 1 && TAPS > 1 && !QF;
     static constexpr bool TWO = LOADER && BN == 64;   // two MMA issuers (see the kernel)
     static constexpr int EPW = OVL ? 2 : 1, NSETS = OVL ? 1 : TWO ? 4 : (QF ? 2 : 3);
@@ -101,8 +101,8 @@ struct SlabCfg {
     // Slab loaders.  A tiled tensor copy moves one box row in about 2.6 clocks whatever its length, so slabs of 32-byte pixels came
     // at 640 clocks a tile of 64 kernels (246 rows at 56x56), whose MMAs take 432.  The slab is contiguous in the image: two warps
     // fetch it in 16-byte pieces and place them in the swizzle pattern.  Image out, one GEMM, before loaders, second issuer and the
-    // epilogue of quantise32_e2m1 / after: 256 x 64x56x56 -> 64 34.3 / 26.0 us, 256 x 128x28x28 -> 128 20.6 / 17.5, 8 x 64x112x112 ->
-    // 64 7.4 / 6.8 (the drain alone takes some 900 clocks a tile of 64 kernels, the MMAs alone 475).
+    // epilogue of quantise32_e2m1 / after: 256 x 64x56x56 -> 64 34.3 / 26.1 us, 256 x 128x28x28 -> 128 21.1 / 16.8, 8 x 64x112x112 ->
+    // 64 7.4 / 7.0 (the drain alone takes some 900 clocks a tile of 64 kernels, the MMAs alone 475).
     static constexpr int NLOAD = LOADER ? 2 : 0, WARP_LOAD0 = 2;
     static constexpr int WARP_EPI0 = 2 + NLOAD, WARP_Q0 = WARP_EPI0 + NEPI;
     static constexpr int NTHREADS = 32 * (WARP_EPI0 + NEPI + (QF ? 5 : 0));
@@ -113,7 +113,8 @@ struct SlabCfg {
 // GRP = weight stages per slot of their ring (one pair of barriers per slot).  3: a filter row of a 3x3 layer of 128-byte pixels on
 // tiles of 64 or 128 kernels whose weights stream.  There the producer's wait, announcement and copy take some 300 clocks a
 // slot and the MMA warp's wait and commit another 80, the four MMAs of a stage of 64 kernels 192.  GEMM alone, one stage a slot and a
-// division per stage / so: 8 x 512x14x14 -> 512 8.8 / 6.4 us, 8 x 1024x14x14 -> 1024 16.0 / 11.3, 8 x 256x28x28 -> 256 7.2 / 6.1.
+// division per stage / one stage / three: 8 x 512x14x14 -> 512 9.0 / 6.4 / 6.3 us, 8 x 1024x14x14 -> 1024 16.1 / 11.4 / 10.8, 8 x
+// 256x28x28 -> 256 7.3 / 6.0 / 5.9.
 template <int BN, int CG, int TAPS, bool QF, bool SINGLE, int GRP, bool IMG>
 __global__ void __launch_bounds__(SlabCfg<BN, CG, TAPS, QF, IMG>::NTHREADS, 1)
 gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)> maps) {
@@ -239,8 +240,8 @@ gemm_slab_kernel(SlabArgs p, const __grid_constant__ TensorMaps<maps_of(CG, QF)>
             for (int g = 0; g < GRP; g++) bulk_g2s(smem_u32(sB + (at + g) * B_STAGE), w + g * j_step, B_STAGE, bar_bfull + 8 * slot);
         }
     };
-    // the first stages of the block's first tile, before the wait for the launch in front (32 KB of constant weights; see gemm_tc.cu)
-    // -- whole slots of the first slab's stages
+    // the first stages of the block's first tile, before the wait for the launch in front (32 KB of constant weights, see gemm_tc.cu, in
+    // whole slots of the first slab's stages: one of 48 KB where a slot is three stages of 128 kernels)
     constexpr int EARLY = 32768 / (GRP * B_STAGE) > 0 ? 32768 / (GRP * B_STAGE) * GRP : GRP;
     const int early = min(min(EARLY, p.nstg), SPG);
     if (warp == WARP_TMA && lane == 0 && unit < ntiles) {

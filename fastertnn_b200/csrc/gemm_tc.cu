@@ -99,7 +99,7 @@ struct TcCfg {
     static constexpr int NSTG = QF ? NSTG_QF : (ATMA ? NSTG_ATMA : ((MT == 1) ? 4 : 3));
     // Stages per slot of the ring (one pair of barriers per slot).  On narrow tiles of single blocks two: a wait that finds its barrier
     // complete takes 110-140 clocks, a copy request 70, the four MMAs of a stage 192 (64 kernels) or 256 (128).  GEMM alone, one
-    // stage a slot / two: 8 x 512x14x14 -> 512 7.8 / 7.2 us, 8 x 1024x14x14 -> 1024 13.9 / 12.2, 8 x 256x28x28 -> 256 6.6 / 6.3.
+    // stage a slot / two, all else the same: 8 x 512x14x14 -> 512 7.4 / 6.7 us, 8 x 1024x14x14 -> 1024 13.4 / 11.7, 8 x 256x28x28 -> 256 6.1 / 5.8.
     static constexpr int GRP = (ATMA && !QF && CG == 1 && BN <= 128) ? 2 : 1, NSLOT = NSTG / GRP;
     static_assert(NSTG % GRP == 0, "whole slots");
     static constexpr int A_STAGE = MT * A_SUB, B_STAGE = (BN / CG) * KCH;

@@ -343,8 +343,9 @@ __device__ __forceinline__ void store_rows16_at(const float (&f)[32], float* con
 
 // Either for rows whose floats cannot be stored in pairs (an odd KN, a base of 4 bytes): the two floats one by one, two pieces of a
 // sector back to back where a row per lane would write it in eight (layer call, NHWC, row per lane / so: 64 x 64x56x56 -> 25 41.9
-// / 24.4 us, -> 63 84.8 / 43.5).  For tiles of 64 and 128 kernels, in kernels of their own (single_floats): inside the others its
-// presence cost the 11-layer stack, which never takes it, 278.7 us against 276.4.
+// / 24.4 us, -> 63 84.8 / 43.5).  In kernels of their own (single_floats), since inside the others its presence cost the 11-layer
+// stack, which never takes it, 278.7 us against 276.4: the slab-fed and the im2col-fed forms on every tile, block pairs included.
+// The GEMM over an explicit packed matrix, the gathering form and the one-launch forms have none and write a row per lane.
 inline bool single_floats(int layout, int y_vec, const void* pimg) { return !pimg && layout == TNNS_NHWC && y_vec == 1; }
 __device__ __forceinline__ void store_rows16_single(const float (&f)[32], float* const (&yrow)[4], int cols_left, int lane) {
     const int cc = 2 * (lane & 3);
