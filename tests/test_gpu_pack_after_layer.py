@@ -1,6 +1,6 @@
 """GPU suite: the pack kernel on a tensor that the launch in front has just written.  A layer, the pack of its output and the packed GEMM
 run back to back over the same intermediate buffers with other inputs each time; every launch lets its dependents in early, so nothing
-but the wait inside the pack kernel keeps it from the values of the round before."""
+but the wait inside the pack kernel keeps it from the values of the pass before."""
 import numpy as np
 import pytest
 
